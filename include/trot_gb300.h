@@ -494,6 +494,20 @@ int trot_prop_ctx_vjp(int norb, int nchol, double dt, const double* h1, const do
 int trot_tc_gemm_bf16(const uint16_t* A, const uint16_t* B, float* D, int M, int N, int K, int* status,
                       void* stream);
 
+/* Complex x real product at FP64 accuracy on the tensor cores (both operands as
+ * six FP16 digit planes per row, 26 exact digit products, FP32 accumulators in
+ * tensor memory):
+ *   C[m][n] (+)= alpha sum_k A[m][k] B(k, n)
+ * A (M x K) and C (M x N) complex row-major (lda, ldc complex elements), B real,
+ * (N x K) row-major if b_is_nk, else (K x N) (ldb elements); alpha a power of two
+ * (or its negative); K <= 2^17.  A row of A or column of B with a NaN or an
+ * infinity gives NaN outputs.  workspace: trot_zgemm_digits_workspace bytes.
+ * The building block of the FP64 contractions; no counterpart in the reference. */
+size_t trot_zgemm_digits_workspace(int M, int N, int K);
+int trot_zgemm_digits(int M, int N, int K, double alpha, const double* A, int lda, const double* B, int ldb,
+                      int b_is_nk, double* C, int ldc, int accumulate, void* workspace, size_t workspace_bytes,
+                      void* stream);
+
 /* Tuning knobs (process-wide; 0 restores the built-in default).  Chosen by
  * timing candidates on the caller's workload (trot_gb300.autotune); every
  * setting computes bit-identical results.  No counterpart in the reference.

@@ -106,6 +106,8 @@ _SIGNATURES = {
     "trot_workspace_timeouts": (_i, [_p, _i, _p]),
     "trot_local_energy_noalloc_status": (_i, [_i, _p]),
     "trot_tc_gemm_bf16": (_i, [_p, _p, _p, _i, _i, _i, _p, _p]),
+    "trot_zgemm_digits_workspace": (ctypes.c_size_t, [_i, _i, _i]),
+    "trot_zgemm_digits": (_i, [_i, _i, _i, _d, _p, _i, _p, _i, _i, _p, _i, _i, _p, ctypes.c_size_t, _p]),
     "trot_cisd_workspace_size": (ctypes.c_size_t, [ctypes.POINTER(TrotCisd), _i, _i]),
     "trot_cisd_overlap": (_i, [ctypes.POINTER(TrotCisd), _i, _p, _p, _p, ctypes.c_size_t, _p]),
     "trot_cisd_force_bias": (_i, [ctypes.POINTER(TrotCisd), _i, _p, _p, _p, ctypes.c_size_t, _p]),

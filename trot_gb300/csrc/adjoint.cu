@@ -22,6 +22,7 @@
 //             q = -sqrt(dt) st + ft + dt (E_shift + h0_prop), c = -sqrt(dt) Re(sum xs m)
 #include <algorithm>
 
+#include "digits.h"
 #include "kernels.h"
 
 namespace trot {
@@ -594,6 +595,7 @@ struct StepWs {
   double *wt_new, *wsum, *g_req, *g_c, *g_es, *opart;
   double2* kpart;  // split-K partials of the long-K products
   int* act;
+  DgScratch dg;
 };
 
 static int splitk_slices(int M, int Nn) {  // enough CTAs for two per SM
@@ -602,7 +604,20 @@ static int splitk_slices(int M, int Nn) {  // enough CTAs for two per SM
   return S < 1 ? 1 : (S > 16 ? 16 : S);
 }
 
-static void carve_step(const AdjCommon& a, Carver& c, StepWs& b) {
+// Scratch of the digit products (the largest of them), at the end of the workspace; without it the products run
+// on the FP64 pipe.
+static void take_digits(Carver& c, size_t bytes, DgScratch& dg) {
+  dg = DgScratch{};
+  if (!bytes) return;
+  dg.p = c.take<char>(bytes);
+  dg.bytes = bytes;
+  dg.status = c.status();
+}
+static void digits_for(size_t& n, size_t M, size_t Nn, size_t K) {
+  if (dg_takes((int)K)) n = std::max(n, dg_scratch_bytes(M, Nn, K));
+}
+
+static void carve_step(const AdjCommon& a, Carver& c, StepWs& b, bool digits) {
   const size_t W = a.W, G = a.G, NN = (size_t)a.N * a.N;
   b = StepWs{};
   for (int q = 0; q < a.nspin; ++q) {
@@ -647,14 +662,26 @@ static void carve_step(const AdjCommon& a, Carver& c, StepWs& b) {
   for (int q = 0; q < a.nspin; ++q) kp = std::max(kp, (size_t)splitk_slices(a.W, a.G) * W * G);
   b.kpart = c.take<double2>(kp);
   b.act = c.take<int>(W);
+  size_t nd = 0;
+  if (digits) {
+    const size_t P = a.chol_packed ? (size_t)a.N * (a.N + 1) / 2 : NN;
+    for (int q = 0; q < a.nspin; ++q) {
+      digits_for(nd, W, G, a.nN[q]);
+      digits_for(nd, W, a.nN[q], G);
+    }
+    digits_for(nd, W, P, G);
+    digits_for(nd, W, G, P);
+  }
+  take_digits(c, nd, b.dg);
 }
 
 struct EnergyWs {
   double2 *green[2], *P[2], *det, *F, *Ft, *c[2], *ctot, *D, *gG, *H;
   int* act;
+  DgScratch dg;
 };
 
-static void carve_energy(const AdjCommon& a, Carver& c, EnergyWs& b) {
+static void carve_energy(const AdjCommon& a, Carver& c, EnergyWs& b, bool digits) {
   const size_t W = a.W, G = a.G;
   b = EnergyWs{};
   size_t nmax = 0, nNmax = 0;
@@ -673,6 +700,15 @@ static void carve_energy(const AdjCommon& a, Carver& c, EnergyWs& b) {
   b.gG = c.take<double2>(W * nNmax);
   b.H = c.take<double2>(nNmax);
   b.act = c.take<int>(W);
+  size_t nd = 0;
+  if (digits)
+    for (int q = 0; q < a.nspin; ++q) {
+      const size_t n = a.n[q];
+      digits_for(nd, W * n, G * n, a.N);
+      digits_for(nd, W * n, a.N, G * n);
+      digits_for(nd, W, a.nN[q], G);
+    }
+  take_digits(c, nd, b.dg);
 }
 
 static int green_launch(const AdjCommon& a, int q, const double2* w, double2* green, double2* P, double2* det,
@@ -714,10 +750,10 @@ size_t trot_vjp_workspace_size(const trot_system* s, int op) {
   Carver c(nullptr, 0);
   if (op == TROT_OP_PROP_STEP) {
     StepWs b;
-    carve_step(a, c, b);
+    carve_step(a, c, b, true);
   } else if (op == TROT_OP_LOCAL_ENERGY) {
     EnergyWs b;
-    carve_energy(a, c, b);
+    carve_energy(a, c, b, true);
   } else if (op == TROT_OP_OVERLAP) {
     for (int q = 0; q < a.nspin; ++q) {
       c.take<double2>(a.W * a.nN[q]);
@@ -754,7 +790,11 @@ int trot_prop_step_vjp(const trot_system* s, const trot_state* in, const double*
   }
   Carver c(ws, ws_bytes);
   StepWs b;
-  carve_step(a, c, b);
+  carve_step(a, c, b, true);
+  if (!c.ok) {
+    c = Carver(ws, ws_bytes);
+    carve_step(a, c, b, false);
+  }
   if (!c.ok) { set_error("workspace too small: %zu < %zu", ws_bytes, c.used); return TROT_ERR_WORKSPACE_TOO_SMALL; }
   cudaStream_t st = (cudaStream_t)stream;
   const int W = a.W, N = a.N, G = a.G, K = a.K;
@@ -767,12 +807,11 @@ int trot_prop_step_vjp(const trot_system* s, const trot_state* in, const double*
   for (int q = 0; q < a.nspin; ++q) {
     TROT_TRY(green_launch(a, q, w[q], b.sp[q].green, b.sp[q].P, b.sp[q].det, st));
     // fb = sum_s mult_s R_s . G_s
-    TROT_TRY(launch_zgemm_cr_splitk(W, G, (int)a.nN[q], (double)a.mult[q], b.sp[q].green, (int)a.nN[q],
-                                    a.rot_chol[q], (int)a.nN[q], true, b.fb, G, q > 0, b.kpart,
-                                    splitk_slices(W, G), st));
+    TROT_TRY(launch_zgemm(W, G, (int)a.nN[q], (double)a.mult[q], b.sp[q].green, (int)a.nN[q], a.rot_chol[q],
+                          (int)a.nN[q], true, b.fb, G, q > 0, b.dg, st, b.kpart, splitk_slices(W, G)));
   }
   TROT_TRY(launch_fields(W, G, s->sqrt_dt, b.fb, s->mf_shifts_im, fields, b.xs, b.st, b.ft, st));
-  TROT_TRY(launch_vhs64(W, N, G, b.xs, s->chol_flat, a.chol_packed, b.vp, b.V, st));
+  TROT_TRY(launch_vhs64(W, N, G, b.xs, s->chol_flat, a.chol_packed, b.vp, b.V, b.dg, st));
   adj_to_complex_kernel<<<grid_of(NN), 256, 0, st>>>(NN, s->exp_h1_half, b.Bc);
   TROT_CHECK_LAUNCH("adj_to_complex_kernel");
   double2 ck[8];
@@ -875,11 +914,11 @@ int trot_prop_step_vjp(const trot_system* s, const trot_state* in, const double*
   if (a.chol_packed) {
     const int P = N * (N + 1) / 2;
     TROT_TRY(launch_pack_sym(N, W, b.gV, b.vp, st));
-    TROT_TRY(launch_zgemm_cr_splitk(W, G, P, 1.0, b.vp, P, a.chol_packed, P, true, b.gxsv, G, false, b.kpart,
-                                    splitk_slices(W, G), st));
+    TROT_TRY(launch_zgemm(W, G, P, 1.0, b.vp, P, a.chol_packed, P, true, b.gxsv, G, false, b.dg, st, b.kpart,
+                          splitk_slices(W, G)));
   } else {
-    TROT_TRY(launch_zgemm_cr_splitk(W, G, (int)NN, 1.0, b.gV, (int)NN, s->chol_flat, (int)NN, true, b.gxsv, G,
-                                    false, b.kpart, splitk_slices(W, G), st));
+    TROT_TRY(launch_zgemm(W, G, (int)NN, 1.0, b.gV, (int)NN, s->chol_flat, (int)NN, true, b.gxsv, G, false, b.dg, st,
+                          b.kpart, splitk_slices(W, G)));
   }
   adj_fields_kernel<<<grid_of((size_t)W * G), 256, 0, st>>>(W, G, s->sqrt_dt, s->mf_shifts_im, b.xs, b.gxsv, b.g_req,
                                                              b.g_c, b.gfb);
@@ -887,8 +926,8 @@ int trot_prop_step_vjp(const trot_system* s, const trot_state* in, const double*
   for (int q = 0; q < a.nspin; ++q) {
     SpinWs& x = b.sp[q];
     // fb = sum_s mult_s G_s R_s^T: g_G_s = mult_s g_fb R_s
-    TROT_TRY(launch_zgemm_cr(W, (int)a.nN[q], G, (double)a.mult[q], b.gfb, G, a.rot_chol[q], (int)a.nN[q], false,
-                             x.gG, (int)a.nN[q], false, st));
+    TROT_TRY(launch_zgemm(W, (int)a.nN[q], G, (double)a.mult[q], b.gfb, G, a.rot_chol[q], (int)a.nN[q], false, x.gG,
+                          (int)a.nN[q], false, b.dg, st));
     TROT_TRY(green_vjp_launch(a, q, x.green, x.gG, x.P, gin[q], st));
   }
   return TROT_OK;
@@ -908,7 +947,11 @@ int trot_local_energy_vjp(const trot_system* s, const double* walkers_a, const d
     if (!a.rot_chol[q] || !a.rot_h1[q]) { set_error("null measurement context"); return TROT_ERR_NULL_PTR; }
   Carver c(ws, ws_bytes);
   EnergyWs b;
-  carve_energy(a, c, b);
+  carve_energy(a, c, b, true);
+  if (!c.ok) {
+    c = Carver(ws, ws_bytes);
+    carve_energy(a, c, b, false);
+  }
   if (!c.ok) { set_error("workspace too small: %zu < %zu", ws_bytes, c.used); return TROT_ERR_WORKSPACE_TOO_SMALL; }
   cudaStream_t st = (cudaStream_t)stream;
   const int W = a.W, N = a.N, G = a.G;
@@ -922,7 +965,7 @@ int trot_local_energy_vjp(const trot_system* s, const double* walkers_a, const d
     TROT_TRY(green_launch(a, q, w[q], b.green[q], b.P[q], b.det, st));
     TROT_TRY(zero_inactive(W, a.nN[q], b.act, b.green[q], st));
     TROT_TRY(zero_inactive(W, (size_t)n * n, b.act, b.P[q], st));
-    TROT_TRY(launch_zgemm_cr(W * n, G * n, N, 1.0, b.green[q], N, a.rot_chol[q], N, true, b.F, G * n, false, st));
+    TROT_TRY(launch_zgemm(W * n, G * n, N, 1.0, b.green[q], N, a.rot_chol[q], N, true, b.F, G * n, false, b.dg, st));
     adj_trace_kernel<<<grid_of((size_t)W * G), 256, 0, st>>>(W, G, n, b.F, b.c[q]);
     TROT_CHECK_LAUNCH("adj_trace_kernel");
   }
@@ -936,12 +979,12 @@ int trot_local_energy_vjp(const trot_system* s, const double* walkers_a, const d
   for (int q = 0; q < a.nspin; ++q) {
     const int n = a.n[q];
     const double m = (double)a.mult[q];
-    TROT_TRY(launch_zgemm_cr(W * n, G * n, N, 1.0, b.green[q], N, a.rot_chol[q], N, true, b.F, G * n, false, st));
+    TROT_TRY(launch_zgemm(W * n, G * n, N, 1.0, b.green[q], N, a.rot_chol[q], N, true, b.F, G * n, false, b.dg, st));
     adj_block_transpose_kernel<<<grid_of((size_t)W * n * G * n), 256, 0, st>>>(W, G, n, b.F, b.Ft);
     TROT_CHECK_LAUNCH("adj_block_transpose_kernel");
-    TROT_TRY(launch_zgemm_cr(W * n, N, G * n, -m, b.Ft, G * n, a.rot_chol[q], N, false, b.D, N, false, st));
-    TROT_TRY(launch_zgemm_cr(W, (int)a.nN[q], G, m, b.ctot, G, a.rot_chol[q], (int)a.nN[q], false, b.D, (int)a.nN[q],
-                             true, st));
+    TROT_TRY(launch_zgemm(W * n, N, G * n, -m, b.Ft, G * n, a.rot_chol[q], N, false, b.D, N, false, b.dg, st));
+    TROT_TRY(launch_zgemm(W, (int)a.nN[q], G, m, b.ctot, G, a.rot_chol[q], (int)a.nN[q], false, b.D, (int)a.nN[q], true,
+                          b.dg, st));
     adj_energy_green_kernel<<<grid_of((size_t)W * a.nN[q]), 256, 0, st>>>(W, n, N, m, a.rot_h1[q], b.D, g_energy,
                                                                            b.gG);
     TROT_CHECK_LAUNCH("adj_energy_green_kernel");

@@ -5,6 +5,7 @@
 #include <cstdio>
 #include <cstring>
 
+#include "digits.h"
 #include "kernels.h"
 #include "mixed.h"
 #include "profile.h"
@@ -47,8 +48,21 @@ Spins make_spins(const trot_system* s) {
   return sp;
 }
 
-// Workspace layout shared by size query and the ops.
-static size_t carve_step(const trot_system* s, const Spins& sp, Carver& c, StepBuffers& b, int op) {
+// Scratch of the op's tensor-core digit products (the largest of them; they run one after another).
+static size_t digit_bytes(const trot_system* s, const Spins& sp, int op) {
+  const size_t W = s->n_walkers, N = s->norb, G = s->nchol;
+  size_t n = 0;
+  if (op == TROT_OP_FORCE_BIAS || op == TROT_OP_LOCAL_ENERGY || op == TROT_OP_PROP_STEP)
+    for (int q = 0; q < sp.nspin; ++q)
+      if (dg_takes(sp.n[q] * (int)N)) n = std::max(n, dg_scratch_bytes(W, G, sp.n[q] * N));
+  if ((op == TROT_OP_APPLY_TROTTER || op == TROT_OP_PROP_STEP) && dg_takes((int)G))
+    n = std::max(n, dg_scratch_bytes(W, N * N, G));  // full or packed
+  return n;
+}
+
+// Workspace layout shared by size query and the ops.  digits: with the scratch of the digit products at its
+// end; a workspace that is too small for it still serves the op on the FP64 pipe.
+static size_t carve_step(const trot_system* s, const Spins& sp, Carver& c, StepBuffers& b, int op, bool digits) {
   const size_t W = s->n_walkers, N = s->norb, G = s->nchol;
   b = StepBuffers{};
   if (op == TROT_OP_SR) { c.take<double>(W); return c.used; }
@@ -67,7 +81,32 @@ static size_t carve_step(const trot_system* s, const Spins& sp, Carver& c, StepB
     b.fb_term = c.take<double2>(W);
     b.node_flag = c.take<int>(W);
   }
+  const size_t nd = digits ? digit_bytes(s, sp, op) : 0;
+  if (nd) {
+    b.dg.p = c.take<char>(nd);
+    b.dg.bytes = nd;
+    b.dg.status = c.status();
+  }
   return c.used;
+}
+
+// The op's buffers in the caller's workspace, with the digit products' scratch where it fits.
+static int carve_ws(const trot_system* s, const Spins& sp, void* ws, size_t ws_bytes, StepBuffers& b, int op) {
+  Carver c(ws, ws_bytes);
+  carve_step(s, sp, c, b, op, true);
+  if (c.ok) return TROT_OK;
+  Carver d(ws, ws_bytes);
+  carve_step(s, sp, d, b, op, false);
+  if (d.ok) return TROT_OK;
+  set_error("workspace too small: %zu < %zu", ws_bytes, d.used);
+  return TROT_ERR_WORKSPACE_TOO_SMALL;
+}
+
+size_t fp64_min_workspace(const trot_system* s, int op) {
+  const Spins sp = make_spins(s);
+  Carver c(nullptr, 0);
+  StepBuffers b;
+  return carve_step(s, sp, c, b, op, false) + 256;
 }
 
 static int check_system(const trot_system* s) {
@@ -115,11 +154,11 @@ static int check_prop(const trot_system* s) {
 
 // force bias from the half Green's functions: fb = sum_s mult_s rot_chol_s G_s
 static int force_bias_from_green(const trot_system* s, const Spins& sp, const double2* green, double2* fb,
-                                 cudaStream_t st) {
+                                 const DgScratch& dg, cudaStream_t st) {
   const int W = s->n_walkers, N = s->norb, G = s->nchol, K = sp.ntot * N;
   for (int q = 0; q < sp.nspin; ++q) {
-    TROT_TRY(launch_zgemm_cr(W, G, sp.n[q] * N, (double)sp.mult[q], green + (size_t)sp.off[q] * N, K,
-                             sp.rot_chol[q], sp.n[q] * N, true, fb, G, q > 0, st));
+    TROT_TRY(launch_zgemm(W, G, sp.n[q] * N, (double)sp.mult[q], green + (size_t)sp.off[q] * N, K, sp.rot_chol[q],
+                          sp.n[q] * N, true, fb, G, q > 0, dg, st));
   }
   return TROT_OK;
 }
@@ -188,7 +227,7 @@ size_t trot_workspace_size(const trot_system* s, int op) {
     if (!s->mixed) return 0;
     return mixed_workspace_size(s, op) + 256;
   }
-  size_t n = carve_step(s, sp, c, b, op);
+  size_t n = carve_step(s, sp, c, b, op, true);
   return n + 256;
 }
 
@@ -245,13 +284,11 @@ int trot_force_bias(const trot_system* s, const double* wa, const double* wb, do
   cudaStream_t st = (cudaStream_t)stream;
   if (s->precision == TROT_MIXED)
     return mixed_force_bias(s, sp, (const double2*)wa, (const double2*)wb, (double2*)out, ws, ws_bytes, st);
-  Carver c(ws, ws_bytes);
   StepBuffers b;
-  carve_step(s, sp, c, b, TROT_OP_FORCE_BIAS);
-  if (!c.ok) { set_error("workspace too small: %zu < %zu", ws_bytes, c.used); return TROT_ERR_WORKSPACE_TOO_SMALL; }
+  TROT_TRY(carve_ws(s, sp, ws, ws_bytes, b, TROT_OP_FORCE_BIAS));
   TROT_TRY(launch_green(sp, s->n_walkers, s->norb, (const double2*)wa, (const double2*)wb, b.green, nullptr,
                         nullptr, st));
-  return force_bias_from_green(s, sp, b.green, (double2*)out, st);
+  return force_bias_from_green(s, sp, b.green, (double2*)out, b.dg, st);
 }
 
 int trot_local_energy(const trot_system* s, const double* wa, const double* wb, double* out, void* ws,
@@ -264,13 +301,11 @@ int trot_local_energy(const trot_system* s, const double* wa, const double* wb, 
   cudaStream_t st = (cudaStream_t)stream;
   if (s->precision == TROT_MIXED)
     return mixed_local_energy(s, sp, (const double2*)wa, (const double2*)wb, (double2*)out, ws, ws_bytes, st);
-  Carver c(ws, ws_bytes);
   StepBuffers b;
-  carve_step(s, sp, c, b, TROT_OP_LOCAL_ENERGY);
-  if (!c.ok) { set_error("workspace too small: %zu < %zu", ws_bytes, c.used); return TROT_ERR_WORKSPACE_TOO_SMALL; }
+  TROT_TRY(carve_ws(s, sp, ws, ws_bytes, b, TROT_OP_LOCAL_ENERGY));
   const int W = s->n_walkers, N = s->norb, G = s->nchol;
   TROT_TRY(launch_green(sp, W, N, (const double2*)wa, (const double2*)wb, b.green, nullptr, b.e1, st));
-  TROT_TRY(force_bias_from_green(s, sp, b.green, b.fb, st));
+  TROT_TRY(force_bias_from_green(s, sp, b.green, b.fb, b.dg, st));
   TROT_TRY(launch_exchange(sp, W, N, G, b.green, b.exc, st));
   return launch_energy_combine(W, G, exchange_chunks(G), s->h0, b.fb, b.e1, 1, b.exc, (double2*)out, st);
 }
@@ -289,11 +324,9 @@ int trot_apply_trotter(const trot_system* s, const double* wa, const double* wb,
   a.W = W; a.N = N; a.G = G; a.nterms = s->n_exp_terms; a.sqrt_dt = s->sqrt_dt; a.expH = s->exp_h1_half;
   a.in_a = (const double2*)wa; a.in_b = (const double2*)wb; a.out_a = (double2*)oa; a.out_b = (double2*)ob;
   if (s->precision == TROT_MIXED) return mixed_apply_trotter(s, sp, (const double2*)xs, a, ws, ws_bytes, st);
-  Carver c(ws, ws_bytes);
   StepBuffers b;
-  carve_step(s, sp, c, b, TROT_OP_APPLY_TROTTER);
-  if (!c.ok) { set_error("workspace too small: %zu < %zu", ws_bytes, c.used); return TROT_ERR_WORKSPACE_TOO_SMALL; }
-  TROT_TRY(launch_vhs64(W, N, G, (const double2*)xs, s->chol_flat, s->chol_packed, b.vp, b.vhs, st));
+  TROT_TRY(carve_ws(s, sp, ws, ws_bytes, b, TROT_OP_APPLY_TROTTER));
+  TROT_TRY(launch_vhs64(W, N, G, (const double2*)xs, s->chol_flat, s->chol_packed, b.vp, b.vhs, b.dg, st));
   a.vhs = b.vhs;
   return launch_trotter(sp, a, st);
 }
@@ -313,17 +346,15 @@ int trot_prop_step(const trot_system* s, const trot_state* state, const double* 
   cudaStream_t st = (cudaStream_t)stream;
   if (s->precision == TROT_MIXED)
     return mixed_prop_step(s, sp, state, fields, (double2*)energy_out, ws, ws_bytes, st);
-  Carver c(ws, ws_bytes);
   StepBuffers b;
-  carve_step(s, sp, c, b, TROT_OP_PROP_STEP);
-  if (!c.ok) { set_error("workspace too small: %zu < %zu", ws_bytes, c.used); return TROT_ERR_WORKSPACE_TOO_SMALL; }
+  TROT_TRY(carve_ws(s, sp, ws, ws_bytes, b, TROT_OP_PROP_STEP));
   const int W = s->n_walkers, N = s->norb, G = s->nchol;
   double2* wa = (double2*)state->walkers_a;
   double2* wb = (double2*)state->walkers_b;
   // 1. Green's functions (+ one-body energy) of the current walkers
   TROT_TIMED("green", st, launch_green(sp, W, N, wa, wb, b.green, nullptr, energy_out ? b.e1 : nullptr, st));
   // 2. force bias
-  TROT_TIMED("force_bias_fp64", st, force_bias_from_green(s, sp, b.green, b.fb, st));
+  TROT_TIMED("force_bias_fp64", st, force_bias_from_green(s, sp, b.green, b.fb, b.dg, st));
   // 3. optional local energy of the current walkers (reuses G and fb)
   if (energy_out) {
     TROT_TIMED("exchange_fp64", st, launch_exchange(sp, W, N, G, b.green, b.exc, st));
@@ -333,7 +364,7 @@ int trot_prop_step(const trot_system* s, const trot_state* state, const double* 
   // 4. shifted fields
   TROT_TIMED("fields", st, launch_fields(W, G, s->sqrt_dt, b.fb, s->mf_shifts_im, fields, b.xs, b.shift_term, b.fb_term, st));
   // 5. VHS
-  TROT_TIMED("vhs_fp64", st, launch_vhs64(W, N, G, b.xs, s->chol_flat, s->chol_packed, b.vp, b.vhs, st));
+  TROT_TIMED("vhs_fp64", st, launch_vhs64(W, N, G, b.xs, s->chol_flat, s->chol_packed, b.vp, b.vhs, b.dg, st));
   // 6. propagation + overlaps + weights
   TrotterArgs a{};
   a.W = W; a.N = N; a.G = G; a.nterms = s->n_exp_terms; a.sqrt_dt = s->sqrt_dt; a.expH = s->exp_h1_half;

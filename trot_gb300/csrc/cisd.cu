@@ -18,6 +18,7 @@
 
 #include <algorithm>
 
+#include "digits.h"
 #include "ff.cuh"
 #include "kernels.h"
 #include "mixed.h"
@@ -53,6 +54,7 @@ struct CisdBuffers {
   // propagation step
   double2 *fb, *xs, *shift_term, *fb_term, *vhs, *ov_new;
   int* node_flag;
+  DgScratch dg;  // scratch of the digit products; p == null: none
 };
 
 static constexpr int kCisdGChunk = 8;
@@ -71,7 +73,25 @@ static int cisd_splitk(int M, int Nn, int K) {
   return std::max(1, std::min(S, 16));
 }
 
-static size_t carve_cisd(const trot_cisd* c, int W, int op, Carver& cv, CisdBuffers& b) {
+// Scratch of the tensor-core digit products of an op (the largest of them; they run one after another)
+static size_t cisd_digit_bytes(const trot_cisd* c, size_t W, int op) {
+  const size_t N = c->norb, n = c->nocc, G = c->nchol, nv = n * c->nvir;
+  size_t d = 0;
+  auto add = [&](size_t M, size_t Nn, size_t K) {
+    if (dg_takes((int)K)) d = std::max(d, dg_scratch_bytes(M, Nn, K));
+  };
+  add(W, nv, nv);  // ci2g
+  if (op == TROT_OP_OVERLAP) return d;
+  add(W, G, n * N);                                          // lg
+  add(W, G, N * N);                                          // lcs (packed or full)
+  add(W, G, N * (N + 1) / 2);
+  if (op == TROT_OP_FORCE_BIAS) return d;
+  if (c->l2ci2_precision != TROT_MIXED) add(W * G, nv, nv);  // l2ci2
+  if (op == TROT_OP_PROP_STEP) add(W, N * N, G);             // VHS (FP64 propagation)
+  return d;
+}
+
+static size_t carve_cisd_buffers(const trot_cisd* c, int W, int op, Carver& cv, CisdBuffers& b) {
   const size_t N = c->norb, n = c->nocc, v = c->nvir, G = c->nchol, nv = n * v;
   b = CisdBuffers{};
   b.status = cv.status();
@@ -127,6 +147,18 @@ static size_t carve_cisd(const trot_cisd* c, int W, int op, Carver& cv, CisdBuff
   b.vhs = cv.take<double2>((size_t)W * N * N);
   b.ov_new = cv.take<double2>(W);
   b.node_flag = cv.take<int>(W);
+  return cv.used;
+}
+
+// digits: with the scratch of the digit products at the end (without it they run on the FP64 pipe)
+static size_t carve_cisd(const trot_cisd* c, int W, int op, Carver& cv, CisdBuffers& b, bool digits) {
+  carve_cisd_buffers(c, W, op, cv, b);
+  const size_t nd = digits ? cisd_digit_bytes(c, W, op) : 0;
+  if (nd) {
+    b.dg.p = cv.take<char>(nd);
+    b.dg.bytes = nd;
+    b.dg.status = cv.status();
+  }
   return cv.used;
 }
 
@@ -781,8 +813,8 @@ static int cisd_run(const trot_cisd* c, int W, const double2* w, CisdBuffers& b,
   CISD_LAUNCH("cisd_x", cisd_x_kernel, W, 256, 0, st, N, n, v, b.green, c->ci1, b.x,
               stage >= 1 ? b.ci1g1 : nullptr, b.wsc);
   TROT_TIMED("cisd_ci2g", st,
-             launch_zgemm_cr_splitk(W, nv, nv, 1.0, b.x, nv, c->ci2m, nv, false, b.cg, nv, false, b.kpart,
-                                    cisd_splitk(W, nv, nv), st));
+             launch_zgemm(W, nv, nv, 1.0, b.x, nv, c->ci2m, nv, false, b.cg, nv, false, b.dg, st, b.kpart,
+                          cisd_splitk(W, nv, nv)));
   if (stage == 0) return TROT_OK;
   const size_t smem = cisd_mats_smem(N, n, v);
   if (smem > 40 * 1024) cudaFuncSetAttribute(cisd_mats_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -790,8 +822,8 @@ static int cisd_run(const trot_cisd* c, int W, const double2* w, CisdBuffers& b,
               b.m2, b.p2, b.wsc);
   // lg = rot_chol . G  (rot_chol rows g: chol[g][:n][:] = first n N entries of chol_flat row g)
   TROT_TIMED("cisd_chol_gemm", st,
-             launch_zgemm_cr_splitk(W, G, n * N, 1.0, b.green, n * N, c->chol, N * N, true, b.lg, G, false, b.kpart,
-                                    cisd_splitk(W, G, n * N), st));
+             launch_zgemm(W, G, n * N, 1.0, b.green, n * N, c->chol, N * N, true, b.lg, G, false, b.dg, st, b.kpart,
+                          cisd_splitk(W, G, n * N)));
   // lcs = (ci1_green + ci2_green) . chol^T: one (W, N^2) x (N^2, G) FP64 product, over the packed
   // upper triangle when every chol[g] is symmetric.
   // (FP32-class products here, as the reference's mixed_real_dtype contraction, move
@@ -804,12 +836,12 @@ static int cisd_run(const trot_cisd* c, int W, const double2* w, CisdBuffers& b,
     CISD_LAUNCH("cisd_lci_gemm", cisd_pack_ms_kernel, (unsigned)std::min<size_t>((wnn + 255) / 256, 152 * 16), 256, 0,
                 st, N, W, b.ms, b.msp);
     TROT_TIMED("cisd_lci_gemm", st,
-               launch_zgemm_cr_splitk(W, G, P, 1.0, b.msp, P, b.lp, P, true, b.lcs, G, false, b.kpart,
-                                      cisd_splitk(W, G, P), st));
+               launch_zgemm(W, G, P, 1.0, b.msp, P, b.lp, P, true, b.lcs, G, false, b.dg, st, b.kpart,
+                            cisd_splitk(W, G, P)));
   } else {
     TROT_TIMED("cisd_lci_gemm", st,
-               launch_zgemm_cr_splitk(W, G, N * N, 1.0, b.ms, N * N, c->chol, N * N, true, b.lcs, G, false,
-                                      b.kpart, cisd_splitk(W, G, N * N), st));
+               launch_zgemm(W, G, N * N, 1.0, b.ms, N * N, c->chol, N * N, true, b.lcs, G, false, b.dg, st, b.kpart,
+                            cisd_splitk(W, G, N * N)));
   }
   if (stage == 1) return TROT_OK;
   const int nch = cisd_chunks(G);
@@ -843,9 +875,22 @@ static int cisd_run(const trot_cisd* c, int W, const double2* w, CisdBuffers& b,
   }
   if ((size_t)W * G > 65535u * 64u) { set_error("CISD: W*G too large"); return TROT_ERR_UNSUPPORTED; }
   TROT_TIMED("cisd_l2ci2", st,
-             launch_zgemm_cr(W * G, nv, nv, 1.0, b.xg, nv, c->ci2m, nv, false, b.y, nv, false, st));
+             launch_zgemm(W * G, nv, nv, 1.0, b.xg, nv, c->ci2m, nv, false, b.y, nv, false, b.dg, st));
   CISD_LAUNCH("cisd_l2_reduce", cisd_l2_reduce_kernel, dim3(kL2Parts, W), 256, 0, st, G, nv, b.xg, b.y, b.l2part);
   return TROT_OK;
+}
+
+// The op's buffers in the caller's workspace, `after` more bytes kept free behind them; with the digit products'
+// scratch where it fits.
+static int carve_cisd_ws(const trot_cisd* c, int W, int op, void* ws, size_t ws_bytes, size_t after, Carver& cv,
+                         CisdBuffers& b) {
+  for (int digits = 1; digits >= 0; --digits) {
+    cv = Carver(ws, ws_bytes);
+    carve_cisd(c, W, op, cv, b, digits != 0);
+    if (cv.ok && (!digits || ((cv.used + 255) & ~(size_t)255) + after <= ws_bytes)) return TROT_OK;
+  }
+  set_error("workspace too small: %zu < %zu", ws_bytes, cv.used);
+  return TROT_ERR_WORKSPACE_TOO_SMALL;
 }
 
 }  // namespace trot
@@ -862,7 +907,7 @@ size_t trot_cisd_workspace_size(const trot_cisd* c, int n_walkers, int op) {
   }
   Carver cv(nullptr, 0);
   CisdBuffers b;
-  return carve_cisd(c, n_walkers, op, cv, b) + 256;
+  return carve_cisd(c, n_walkers, op, cv, b, true) + 256;
 }
 
 int trot_cisd_overlap(const trot_cisd* c, int W, const double* walkers, double* out, void* ws, size_t ws_bytes,
@@ -871,8 +916,7 @@ int trot_cisd_overlap(const trot_cisd* c, int W, const double* walkers, double* 
   if (!walkers || !out) { set_error("null walkers or output"); return TROT_ERR_NULL_PTR; }
   Carver cv(ws, ws_bytes);
   CisdBuffers b;
-  carve_cisd(c, W, TROT_OP_OVERLAP, cv, b);
-  if (!cv.ok) { set_error("workspace too small: %zu < %zu", ws_bytes, cv.used); return TROT_ERR_WORKSPACE_TOO_SMALL; }
+  TROT_TRY(carve_cisd_ws(c, W, TROT_OP_OVERLAP, ws, ws_bytes, 0, cv, b));
   cudaStream_t st = (cudaStream_t)stream;
   TROT_TRY(cisd_run(c, W, (const double2*)walkers, b, 0, st));
   cisd_overlap_kernel<<<W, 256, 0, st>>>(c->nocc * c->nvir, b.x, b.cg, b.wsc, b.det2, (double2*)out);
@@ -886,8 +930,7 @@ int trot_cisd_force_bias(const trot_cisd* c, int W, const double* walkers, doubl
   if (!walkers || !out) { set_error("null walkers or output"); return TROT_ERR_NULL_PTR; }
   Carver cv(ws, ws_bytes);
   CisdBuffers b;
-  carve_cisd(c, W, TROT_OP_FORCE_BIAS, cv, b);
-  if (!cv.ok) { set_error("workspace too small: %zu < %zu", ws_bytes, cv.used); return TROT_ERR_WORKSPACE_TOO_SMALL; }
+  TROT_TRY(carve_cisd_ws(c, W, TROT_OP_FORCE_BIAS, ws, ws_bytes, 0, cv, b));
   cudaStream_t st = (cudaStream_t)stream;
   TROT_TRY(cisd_run(c, W, (const double2*)walkers, b, 1, st));
   const size_t n = (size_t)W * c->nchol;
@@ -902,8 +945,7 @@ int trot_cisd_local_energy(const trot_cisd* c, int W, const double* walkers, dou
   if (!walkers || !out) { set_error("null walkers or output"); return TROT_ERR_NULL_PTR; }
   Carver cv(ws, ws_bytes);
   CisdBuffers b;
-  carve_cisd(c, W, TROT_OP_LOCAL_ENERGY, cv, b);
-  if (!cv.ok) { set_error("workspace too small: %zu < %zu", ws_bytes, cv.used); return TROT_ERR_WORKSPACE_TOO_SMALL; }
+  TROT_TRY(carve_cisd_ws(c, W, TROT_OP_LOCAL_ENERGY, ws, ws_bytes, 0, cv, b));
   cudaStream_t st = (cudaStream_t)stream;
   TROT_TRY(cisd_run(c, W, (const double2*)walkers, b, 2, st));
   cisd_energy_kernel<<<W, 256, 0, st>>>(c->nchol, cisd_chunks(c->nchol), c->h0, b.wsc, b.hg2, b.lg, b.lcs,
@@ -918,8 +960,7 @@ int trot_cisd_rdm1(const trot_cisd* c, int W, const double* walkers, double* out
   if (!walkers || !out) { set_error("null walkers or output"); return TROT_ERR_NULL_PTR; }
   Carver cv(ws, ws_bytes);
   CisdBuffers b;
-  carve_cisd(c, W, TROT_OP_FORCE_BIAS, cv, b);
-  if (!cv.ok) { set_error("workspace too small: %zu < %zu", ws_bytes, cv.used); return TROT_ERR_WORKSPACE_TOO_SMALL; }
+  TROT_TRY(carve_cisd_ws(c, W, TROT_OP_FORCE_BIAS, ws, ws_bytes, 0, cv, b));
   cudaStream_t st = (cudaStream_t)stream;
   TROT_TRY(cisd_run(c, W, (const double2*)walkers, b, 1, st));
   const int N = c->norb;
@@ -957,16 +998,17 @@ int trot_cisd_prop_step(const trot_cisd* c, const trot_system* prop, const trot_
     set_error("null state buffer");
     return TROT_ERR_NULL_PTR;
   }
-  Carver cv(ws, ws_bytes);
-  CisdBuffers b;
-  carve_cisd(c, W, TROT_OP_PROP_STEP, cv, b);
-  if (!cv.ok) { set_error("workspace too small: %zu < %zu", ws_bytes, cv.used); return TROT_ERR_WORKSPACE_TOO_SMALL; }
   // mixed propagation: the tensor-core Trotter path gets its own workspace after the CISD buffers
-  const size_t cisd_bytes = (cv.used + 255) & ~(size_t)255;
   size_t prop_bytes = 0;
   if (prop->precision == TROT_MIXED) {
     prop_bytes = trot_workspace_size(prop, TROT_OP_APPLY_TROTTER);
     if (prop_bytes == 0) return TROT_ERR_BAD_SHAPE;
+  }
+  Carver cv(ws, ws_bytes);
+  CisdBuffers b;
+  TROT_TRY(carve_cisd_ws(c, W, TROT_OP_PROP_STEP, ws, ws_bytes, prop_bytes, cv, b));
+  const size_t cisd_bytes = (cv.used + 255) & ~(size_t)255;
+  if (prop->precision == TROT_MIXED) {
     if (cisd_bytes + prop_bytes > ws_bytes) {
       set_error("workspace too small: %zu < %zu", ws_bytes, cisd_bytes + prop_bytes);
       return TROT_ERR_WORKSPACE_TOO_SMALL;
@@ -997,7 +1039,7 @@ int trot_cisd_prop_step(const trot_cisd* c, const trot_system* prop, const trot_
     TROT_TRY(launch_status_merge(reinterpret_cast<const int*>(static_cast<char*>(ws) + cisd_bytes), b.status, st));
   } else {
     TROT_TIMED("vhs_fp64", st,
-               launch_zgemm_cr(W, N * N, G, 1.0, b.xs, G, prop->chol_flat, N * N, false, b.vhs, N * N, false, st));
+               launch_zgemm(W, N * N, G, 1.0, b.xs, G, prop->chol_flat, N * N, false, b.vhs, N * N, false, b.dg, st));
     a.vhs = b.vhs;
     TROT_TIMED("trotter_fp64", st, launch_trotter(sp, a, st));
   }

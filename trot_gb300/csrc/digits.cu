@@ -1,0 +1,642 @@
+// Complex x real FP64 products on the tensor cores (tcgen05), exact digit slices.
+//
+// This GPU's FP64 pipe retires two FMAs per clock and SM (about 1.2 TFLOP/s), so a contraction on
+// it is bound by that pipe whatever its tiling.  Here both operands are written as integer digits
+// and multiplied on the FP16 tensor cores, about forty times the rate, at FP64 accuracy:
+//
+//  * a row x[0..K) (a row of A: real or imaginary part; a column of B) is x ~= 2^e sum_{t<6} q_t 2^-(9 + 9 t)
+//    with integers |q_0| <= 512, |q_t| <= 256 (exact in FP16), one exponent e per row: 54 bits below the row's
+//    largest element;
+//  * products q_t q_u of equal order d = t + u <= 6 (26 of the 36) share one FP32 accumulator in TMEM.  Over a slab
+//    of 64 k every partial sum of the orders d <= 3 stays below 2^24, so it is an exact integer (a row whose |q_0|
+//    would sum past 8192 over 32 k gets e + 1: then |q_0| <= 256); the orders above carry 2^-54 of the row maxima
+//    and less, where the last bit does not matter;
+//  * after each slab the seven sums are added into one 64-bit integer per output, which is converted to FP64 once.
+//
+// Error against a long-double product, on the force bias, exchange, VHS and CISD operands of systems of 24 to 135
+// orbitals (K = 24 ... 2160): 1.0e-16 ... 6.1e-16 of the result, against 1.7e-16 ... 1.5e-15 for an FP64 sum over k
+// (0.2 to 0.86 of it; five digits, or orders d <= 5 only, are worse than FP64 where one element dominates its
+// row).  The result does not depend on the tiling or on the other rows.
+//
+// Rate (1024 x 7260, K = 600, the VHS of 120 orbitals): 0.455 ms + 0.040 ms for the digits = 36 TFLOP/s, against
+// 14.5 ms on the FP64 pipe; bound by the MMAs' operand reads from shared memory (about 50 cycles per MMA and 0.75 per
+// column and K16 step).  (1024 x 7200, K = 120): 0.123 ms, where the epilogue's conversions take half of the time.
+//
+// One persistent CTA per SM: MMA rows are the columns of B (128 per tile), MMA columns the rows of A in
+// tiles of 32 (16 complex rows: re, im).  A CTA takes NT such tiles against one 128-row tile at a time, so each 24 KB
+// K16 step of the latter serves NT x 26 products from shared memory; per K16 step six (seven in a slab's first)
+// MMAs: digit plane t of B against planes 0..min(5, 6 - t) of A stacked along the MMA's N.  Two TMEM accumulators (7 x 32
+// columns) let the tensor core run the next tile's slab while 16 epilogue warps empty this one.
+#include <cooperative_groups.h>
+#include <cuda_fp16.h>
+
+#include <algorithm>
+#include <cmath>
+
+#include "digits.h"
+#include "tc.cuh"
+
+namespace trot {
+
+static constexpr int kDgS = 6;           // digit planes
+static constexpr int kDgGroups = 7;      // orders d = 0..6
+static constexpr int kDgTop = 9, kDgLow = 9;
+static constexpr int kDgBits = kDgTop + kDgLow * (kDgS - 1);  // 54
+static constexpr int kDgP = 32;          // real rows of A per tile
+static constexpr int kDgSlab = 4;        // K16 steps per slab
+static constexpr uint32_t kDgAStep = kDgS * 128 * 32;    // 24576 B: one K16 step of a 128-row tile
+static constexpr uint32_t kDgBStep = kDgS * kDgP * 32;   // 6144 B: one K16 step of a 32-row tile
+static constexpr int kDgASlots = 6, kDgBSlots = 3;
+static constexpr int kDgEpi = 512;
+static constexpr int kDgThreads = kDgEpi + 3 * 32;       // 16 epilogue warps, MMA warp, two loader warps
+static constexpr size_t kDgOffB = (size_t)kDgASlots * kDgAStep;
+static constexpr size_t kDgOffBar = kDgOffB + (size_t)kDgBSlots * kDgSlab * kDgBStep;
+static constexpr size_t kDgSmem = kDgOffBar + 256 + 128;  // + base alignment
+static_assert(kDgSmem <= 232448, "digit product: shared memory");
+static constexpr int kDgNonFinite = 0x4000;               // exponent code of a row with inf or NaN
+
+// 16-bit index of element (r, k) of a [rows x 16] block (8 x 8 core matrices, K-adjacent ones
+// 128 B apart, 8-row groups 256 B apart)
+TROT_HD uint32_t dg_idx(int r, int k) { return (uint32_t)((r >> 3) * 128 + (k >> 3) * 64 + (r & 7) * 8 + (k & 7)); }
+
+// ------------------------------------------------------------------ digits
+// Digit planes of eight consecutive k of one row, w[t] = 16 B of FP16: q = rint(|x| 2^(54 - e)) <= 2^54 (half away
+// from zero; subnormal x gives 0) split by 32-bit operations into five balanced 9-bit digits (mod 512, in
+// [-256, 256)) and the leading one (<= 512), the sign of x flipped in afterwards.  A digit d becomes FP16 as the bits
+// 0x6600 + d of 1536 + d less 1536, two at a time: the conversion instructions run at a quarter of the rate.
+TROT_D void dg_split8(const double* x, int e, uint4* w) {
+  const __half2 off = __half2half2(__ushort_as_half((unsigned short)0x6600));
+  uint32_t h[kDgS][4];
+#pragma unroll
+  for (int i = 0; i < 8; i += 2) {
+    int d[2][kDgS];
+    uint32_t sign[2];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const unsigned long long u = (unsigned long long)__double_as_longlong(x[i + c]);
+      const unsigned uh = (unsigned)(u >> 32);
+      const int ex = (int)((uh >> 20) & 0x7FFu);
+      sign[c] = uh & 0x80000000u;
+      const unsigned long long M = (u & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
+      const int sh = 1075 - kDgBits + e - ex;  // |x| 2^(54 - e) = M 2^-sh; |x| < 2^e: sh >= -1
+      unsigned long long q = (2 * M + (1ull << (sh + 1 < 63 ? sh + 1 : 63)) / 2) >> (sh + 1 < 63 ? sh + 1 : 63);
+      if (ex == 0) q = 0;
+      int lo = (int)((unsigned)q & 0x7FFFFFFu), hi = (int)(unsigned)(q >> 27);
+#pragma unroll
+      for (int t = kDgS - 1; t >= 3; --t) {
+        d[c][t] = (lo << 23) >> 23;
+        lo = (lo - d[c][t]) >> kDgLow;
+      }
+      hi += lo;  // the carry out of the low three digits
+      d[c][2] = (hi << 23) >> 23;
+      hi = (hi - d[c][2]) >> kDgLow;
+      d[c][1] = (hi << 23) >> 23;
+      d[c][0] = (hi - d[c][1]) >> kDgLow;
+    }
+    const uint32_t sg = (sign[0] >> 16) | sign[1];
+#pragma unroll
+    for (int t = 0; t < kDgS; ++t) {
+      const uint32_t b = (uint32_t)((0x6600 + d[0][t]) & 0xFFFF) | ((uint32_t)(0x6600 + d[1][t]) << 16);
+      const __half2 v = __hsub2(*reinterpret_cast<const __half2*>(&b), off);
+      h[t][i >> 1] = *reinterpret_cast<const uint32_t*>(&v) ^ sg;
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < kDgS; ++t) w[t] = make_uint4(h[t][0], h[t][1], h[t][2], h[t][3]);
+}
+
+// exponent e (max |x| < 2^e) of a row from the high words of its largest |x| and its largest sum of |x| over 32 k
+TROT_D int dg_exponent(unsigned mx, float l1) {
+  const int E = (int)(mx >> 20);
+  if (E == 0x7FF) return kDgNonFinite;
+  if (E == 0) return 0;  // zero (or subnormal: dropped)
+  int e = E - 1022;
+  // sum |q_0| <= l1 2^(9 - e) + 16 over 32 k: keep it at 8192 or below
+  // (rows outside FP32's range, whose sum is not known: always)
+  if (e <= -110 || e >= 110 || l1 > ldexpf(8160.f, e - kDgTop)) ++e;
+  return e;
+}
+
+// Real rows (complex A: row 2 m + c = real / imaginary part of row m; real B: a row or, with kst = ldb, a column) as
+// digit images [tile][K16][plane][R][16].  A CTA takes one group of eight rows, lane = (row, k group), so a warp
+// writes 128 B runs.  A cluster of KS CTAs (grid.x) shares one row group along K and exchanges the row maxima through
+// distributed shared memory, so that long rows fill the chip; with K <= 256 KS every element is read once.
+// The integer work (about 100 instructions per element) bounds it: 4.4M elements (7260 x 600) take 74 us with one CTA
+// per 32 columns, 20 us like this.
+struct DgSrc {
+  const double* p;
+  int rows, K, nk16, R;  // R = 32 or 128 rows per tile
+  int rpb;               // complex rows per block of bstride doubles (complex A only)
+  long long bstride, rst, kst;  // strides in doubles
+  int cplx;
+  uint16_t* img;
+  int16_t* ex;
+};
+
+__global__ void __launch_bounds__(256) dg_rows_kernel(DgSrc a) {
+  __shared__ unsigned smx[8][8], cmx[8];
+  __shared__ float sl1[8][8], cl1[8];
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  const int KS = (int)gridDim.x, rank = (int)blockIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int rl = lane & 7, kg = lane >> 3;
+  const int row = blockIdx.y * 8 + rl;
+  const bool valid = row < a.rows;
+  const double* p = a.p;
+  if (valid) {
+    if (a.cplx) {
+      const int cr = row >> 1;
+      p += (long long)(cr / a.rpb) * a.bstride + (long long)(cr % a.rpb) * a.rst + (row & 1);
+    } else {
+      p += (long long)row * a.rst;
+    }
+  }
+  const int kpad = a.nk16 * 16, kstep = 256 * KS;
+  unsigned mx = 0;
+  float l1 = 0.f;
+  double x[8];
+  for (int k0 = (rank * 8 + warp) * 32; k0 < kpad; k0 += kstep) {
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int k = k0 + kg * 8 + i;
+      x[i] = (valid && k < a.K) ? p[(long long)k * a.kst] : 0.0;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const unsigned b = (unsigned)__double2hiint(x[i]) & 0x7FFFFFFFu;
+      mx = b > mx ? b : mx;
+      // |x| as a float from its high word (the range only matters near the row maximum)
+      const unsigned f = b - (896u << 20);
+      s += f < (254u << 20) ? __uint_as_float(f << 3) : 0.f;
+    }
+    s += __shfl_xor_sync(0xffffffffu, s, 8);
+    s += __shfl_xor_sync(0xffffffffu, s, 16);
+    l1 = fmaxf(l1, s);
+  }
+#pragma unroll
+  for (int o = 8; o < 32; o <<= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if (lane < 8) {
+    smx[warp][lane] = mx;
+    sl1[warp][lane] = l1;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < 8; ++w) {
+    mx = max(mx, smx[w][rl]);
+    l1 = fmaxf(l1, sl1[w][rl]);
+  }
+  if (KS > 1) {
+    if (threadIdx.x < 8) {
+      cmx[rl] = mx;
+      cl1[rl] = l1;
+    }
+    cl.sync();
+    for (int c = 0; c < KS; ++c) {
+      mx = max(mx, cl.map_shared_rank(cmx, c)[rl]);
+      l1 = fmaxf(l1, cl.map_shared_rank(cl1, c)[rl]);
+    }
+  }
+  const int e = dg_exponent(mx, l1);
+  if (rank == 0 && warp == 0 && lane < 8) a.ex[row] = (int16_t)e;
+  const bool live = valid && e != kDgNonFinite;
+  const int r = row % a.R;
+  uint16_t* out = a.img + (size_t)(row / a.R) * a.nk16 * kDgS * a.R * 16;
+  const bool once = kpad <= kstep;
+  for (int k0 = (rank * 8 + warp) * 32; k0 < kpad; k0 += kstep) {
+    const int kb = k0 + kg * 8;
+    if (kb >= kpad) continue;
+    if (!once) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] = (live && kb + i < a.K) ? p[(long long)(kb + i) * a.kst] : 0.0;
+    }
+    if (!live) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] = 0.0;
+    }
+    uint4 w[kDgS];
+    dg_split8(x, live ? e : 0, w);
+    uint16_t* o = out + (size_t)(kb >> 4) * kDgS * a.R * 16 + dg_idx(r, kb & 15);
+#pragma unroll
+    for (int t = 0; t < kDgS; ++t) *reinterpret_cast<uint4*>(o + (size_t)t * a.R * 16) = w[t];
+  }
+  if (KS > 1) cl.sync();  // the maxima stay readable until every CTA of the cluster has them
+}
+
+static int dg_rows_launch(const DgSrc& a, int groups, cudaStream_t st) {
+  int ks = 1;
+  while (ks < 8 && a.nk16 * 16 > 256 * ks && groups * ks < 304) ks *= 2;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(ks, groups);
+  cfg.blockDim = dim3(256);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = ks;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = ks > 1 ? 1 : 0;
+  const cudaError_t rc = cudaLaunchKernelEx(&cfg, dg_rows_kernel, a);
+  if (rc != cudaSuccess) return cuda_status(rc, "dg_rows_kernel");
+  TROT_CHECK_LAUNCH("dg_rows_kernel");
+  return TROT_OK;
+}
+
+// ------------------------------------------------------------------ product
+struct DgArgs {
+  const uint16_t* imgB;  // MMA rows: columns n of B, [rt][nk16][6][128][16]
+  const int16_t* exB;
+  const uint16_t* imgA;  // MMA columns: rows of A, [tile][nk16][6][32][16]
+  const int16_t* exA;
+  int Nn, M;             // outputs: n < Nn, complex rows m < M
+  int nrt, ntile, nct;   // 128-row tiles, 32-row tiles, groups of NT 32-row tiles
+  int nk16, shift;       // K16 steps; the outputs' integers are in units 2^(eA + eB - 54 + shift)
+  double2* C;
+  long long ldc;
+  int salpha, ealpha, accumulate;  // alpha = salpha 2^ealpha, salpha = +-1
+  int* status;
+};
+
+// v 2^E rounded to a double, by integer operations (conversions and FP64 additions run on the
+// narrow FP64 pipe: two of them per output took longer than the output's 26 products)
+TROT_D double dg_double(long long v, int E) {
+  if (v == 0) return 0.0;
+  const unsigned long long a = v < 0 ? 0ull - (unsigned long long)v : (unsigned long long)v;
+  const int lz = __clzll((long long)a);
+  const unsigned long long m = a << lz;  // 2^63 <= m < 2^64
+  unsigned long long q = m >> 11;
+  const unsigned r = (unsigned)m & 0x7FFu;
+  q += (r > 0x400u || (r == 0x400u && (q & 1ull))) ? 1ull : 0ull;  // half to even; 2^53 carries into the exponent
+  const int ex = 1023 + 63 - lz + E;  // of the unrounded value
+  const unsigned long long sign = (unsigned long long)v & 0x8000000000000000ull;
+  if (ex > 0 && ex < 0x7FE) return __longlong_as_double((long long)(((unsigned long long)(ex - 1) << 52) + q + sign));
+  const double d = __longlong_as_double((long long)(((unsigned long long)(1023 + 51) << 52) + q + sign));  // q 1.f form
+  return ldexp(d, ex - 1023 - 52);
+}
+
+// out of line, so that its FP64 instructions are not issued (predicated off) for plain stores
+__device__ __noinline__ void dg_add(double2* o, double2 v) { *o = cadd(*o, v); }
+
+template <int NT>
+__global__ void __launch_bounds__(kDgThreads, 1) dg_gemm_kernel(DgArgs a) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  unsigned char* base = smem_raw + ((128 - (tc::smem_u32(smem_raw) & 127)) & 127);
+  unsigned char* sA = base;             // B's 128-row tile, K16 steps (kDgASlots)
+  unsigned char* sB = base + kDgOffB;   // A's 32-row tiles, slabs (kDgBSlots)
+  uint64_t* bars = reinterpret_cast<uint64_t*>(base + kDgOffBar);
+  uint64_t* a_full = bars;
+  uint64_t* a_free = a_full + kDgASlots;
+  uint64_t* b_full = a_free + kDgASlots;
+  uint64_t* b_free = b_full + kDgBSlots;
+  uint64_t* acc_full = b_free + kDgBSlots;   // [2]
+  uint64_t* acc_empty = acc_full + 2;        // [2]
+  uint64_t* drain = acc_empty + 2;
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(drain + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(drain + 2);
+  static_assert((2 * kDgASlots + 2 * kDgBSlots + 4 + 3) * 8 <= 256, "barrier table");
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int n_items = a.nrt * a.nct, nk = a.nk16;
+  const int nslab = (nk + kDgSlab - 1) / kDgSlab;
+  if (warp == 16) tc::tmem_alloc(tslot, 512);
+  if (tid == kDgEpi) {
+    for (int k = 0; k < kDgASlots; ++k) {
+      tc::mbar_init(&a_full[k], 1);
+      tc::mbar_init(&a_free[k], 1);
+    }
+    for (int k = 0; k < kDgBSlots; ++k) {
+      tc::mbar_init(&b_full[k], 1);
+      tc::mbar_init(&b_free[k], 1);
+    }
+    for (int k = 0; k < 2; ++k) {
+      tc::mbar_init(&acc_full[k], 1);
+      tc::mbar_init(&acc_empty[k], 16);
+    }
+    tc::mbar_init(drain, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t taddr = *tslot;
+  // item -> (128-row tile, group of NT 32-row tiles)
+  if (warp == 16) {
+    if (lane == 0) {
+      bool ok = true;
+      const uint64_t ad0 = tc::smem_desc(tc::smem_u32(sA), 128, 256);
+      const uint64_t bd0 = tc::smem_desc(tc::smem_u32(sB), 128, 256);
+      const uint32_t adlo = (uint32_t)ad0, bdlo = (uint32_t)bd0, dhi = (uint32_t)(ad0 >> 32);
+      int ca = 0, cb = 0, cacc = 0;  // chunk, slab-tile and accumulator counters of this CTA
+      for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+        const int ntv = min(NT, a.ntile - (item / a.nrt) * NT);
+        for (int s = 0; s < nslab && ok; ++s) {
+          const int ks = min(kDgSlab, nk - s * kDgSlab);
+          for (int j = 0; j < ntv && ok; ++j, ++cb, ++cacc) {
+            const int buf = cacc & 1;
+            if (cacc >= 2) ok = tc::mbar_wait(&acc_empty[buf], (uint32_t)(((cacc >> 1) - 1) & 1));
+            if (ok) ok = tc::mbar_wait(&b_full[cb % kDgBSlots], (uint32_t)((cb / kDgBSlots) & 1));
+            if (!ok) break;
+            const uint32_t dcol = taddr + (uint32_t)(buf * 256);
+            for (int k = 0; k < ks; ++k) {
+              const int slot = (ca + k) % kDgASlots;
+              if (j == 0) {
+                ok = tc::mbar_wait(&a_full[slot], (uint32_t)(((ca + k) / kDgASlots) & 1));
+                if (!ok) break;
+              }
+              tc::fence_after_sync();
+              const uint32_t alo = adlo + (uint32_t)((slot * kDgAStep) >> 4);
+              const uint32_t blo = bdlo + (uint32_t)(((cb % kDgBSlots) * kDgSlab * kDgBStep + k * kDgBStep) >> 4);
+#pragma unroll
+              for (int t = 0; t < kDgS; ++t) {
+                const int np = t < 1 ? kDgS : kDgGroups - t;  // planes 0 .. np - 1
+                if (t == 1 && k == 0) {  // order 6 starts here: its columns are overwritten
+                  tc::mma_bf16_lo(dcol + 32, alo + 256, blo, dhi, tc::idesc_f16_f32(128, 160), 1u);
+                  tc::mma_bf16_lo(dcol + 192, alo + 256, blo + (5 * kDgP * 32) / 16, dhi, tc::idesc_f16_f32(128, 32), 0u);
+                } else {
+                  tc::mma_bf16_lo(dcol + (uint32_t)(t * kDgP), alo + (uint32_t)(t * 256), blo, dhi,
+                                  tc::idesc_f16_f32(128, np * kDgP), (k > 0 || t > 0) ? 1u : 0u);
+                }
+              }
+              if (j == ntv - 1) tc::mma_commit(&a_free[slot]);
+            }
+            if (ok) {
+              tc::mma_commit(&b_free[cb % kDgBSlots]);
+              tc::mma_commit(&acc_full[buf]);
+            }
+          }
+          ca += ks;
+        }
+      }
+      if (!ok) {
+        if (a.status) report_timeout(a.status);
+        *abort_flag = 1;
+        tc::mma_commit(drain);  // the MMAs already issued complete before the epilogue is released
+        tc::mbar_wait(drain, 0u, 1000000u);
+        tc::mbar_arrive(&acc_full[0]);
+        tc::mbar_arrive(&acc_full[1]);
+      }
+    }
+    __syncwarp();
+  } else if (warp > 16) {
+    if (lane == 0) {
+      const bool la = warp == 17;  // loader of the 128-row tile; the other one loads the 32-row tiles
+      const int slots = la ? kDgASlots : kDgBSlots;
+      uint64_t* full = la ? a_full : b_full;
+      uint64_t* free_ = la ? a_free : b_free;
+      bool ok = true;
+      int c = 0;
+      for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+        const int rt = item % a.nrt, ct = item / a.nrt;
+        const int ntv = min(NT, a.ntile - ct * NT);
+        for (int s = 0; s < nslab && ok; ++s) {
+          const int ks = min(kDgSlab, nk - s * kDgSlab);
+          const int nc = la ? ks : ntv;
+          for (int j = 0; j < nc; ++j, ++c) {
+            const int slot = c % slots;
+            if (c >= slots) {  // the MMAs that read the slot's previous contents are done
+              const uint32_t par = (uint32_t)(((c / slots) - 1) & 1);
+              uint32_t polls = 0;
+              while (!tc::mbar_try_wait(&free_[slot], par))
+                if (*abort_flag || ++polls > 20000000u) {
+                  ok = false;
+                  break;
+                }
+              if (!ok) break;
+            }
+            if (la) {
+              tc::mbar_expect_tx(&full[slot], kDgAStep);
+              tc::bulk_g2s(sA + (size_t)slot * kDgAStep,
+                           a.imgB + ((size_t)rt * nk + s * kDgSlab + j) * (kDgAStep / 2), kDgAStep, &full[slot]);
+            } else {
+              tc::mbar_expect_tx(&full[slot], ks * kDgBStep);
+              tc::bulk_g2s(sB + (size_t)slot * kDgSlab * kDgBStep,
+                           a.imgA + ((size_t)(ct * NT + j) * nk + s * kDgSlab) * (kDgBStep / 2), ks * kDgBStep,
+                           &full[slot]);
+            }
+          }
+        }
+      }
+      if (!ok) {
+        if (!*abort_flag && a.status) report_timeout(a.status);
+        for (int u = c - 1; u >= 0 && u >= c - slots; --u)  // bounded drain of the copies in flight
+          tc::mbar_wait(&full[u % slots], (uint32_t)((u / slots) & 1), 1000000u);
+      }
+    }
+    __syncwarp();
+  } else {
+    const int q = warp & 3, h = warp >> 2;
+    const uint32_t tl = taddr + ((uint32_t)(q * 32) << 16) + (uint32_t)(h * 8);
+    const int sh = a.shift;
+    // digit weights in the accumulator's units (sh >= 1, so that the largest stays an int32)
+    const int m0 = 1 << (31 - sh), m1 = 1 << (27 - sh), m2 = 1 << (18 - sh), m3 = 1 << (9 - sh);
+    const float lscale = __int_as_float((127 - sh) << 23);
+    int cacc = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
+      const int rt = item % a.nrt, ct = item / a.nrt;
+      const int ntv = min(NT, a.ntile - ct * NT);
+      const int n = rt * 128 + q * 32 + lane;
+      long long acc[NT][8];
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int x = 0; x < 8; ++x) acc[j][x] = 0;
+      for (int s = 0; s < nslab; ++s) {
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+          if (j >= ntv) break;
+          const int buf = cacc & 1;
+          if (ok && (!tc::mbar_wait(&acc_full[buf], (uint32_t)((cacc >> 1) & 1)) || *abort_flag)) {
+            if (!*abort_flag && a.status && lane == 0) report_timeout(a.status);
+            ok = false;
+          }
+          ++cacc;
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) continue;
+          tc::fence_after_sync();
+#pragma unroll
+          for (int c4 = 0; c4 < 8; c4 += 2) {
+            uint32_t raw[kDgGroups][2];
+#pragma unroll
+            for (int d = 0; d < kDgGroups; ++d) tc::tmem_ld2(tl + (uint32_t)(buf * 256 + d * kDgP + c4), raw[d][0], raw[d][1]);
+            tc::tmem_wait_ld();
+            if (c4 == 6) {
+              tc::fence_before_sync();
+              __syncwarp();
+              if (lane == 0) tc::mbar_arrive(&acc_empty[buf]);
+            }
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+              float f[kDgGroups];
+#pragma unroll
+              for (int d = 0; d < kDgGroups; ++d) {
+                uint32_t v = raw[d][x];
+                asm volatile("" : "+r"(v));  // consume after tcgen05.wait::ld
+                f[d] = __uint_as_float(v);
+              }
+              // sum_d S_d 2^(-9 d) in units 2^(sh - 36): orders 0-3 exactly, the rest rounded once
+              const float f4 = fmaf(fmaf(f[6], 1.953125e-03f, f[5]), 1.953125e-03f, f[4]) * lscale;
+              long long v = acc[j][c4 + x];
+              v += (long long)(__float2int_rn(f[0]) << 5) * m0;
+              v += (long long)__float2int_rn(f[1]) * m1;
+              v += (long long)__float2int_rn(f[2]) * m2;
+              v += (long long)__float2int_rn(f[3]) * m3;
+              v += (long long)__float2int_rn(f4);
+              acc[j][c4 + x] = v;
+            }
+          }
+        }
+      }
+      // outputs: lane = column n of C, register pairs = (re, im) of four complex rows
+      int eb = n < a.Nn ? a.exB[n] : 0;
+      if (!ok) eb = kDgNonFinite;
+      const bool bad = eb == kDgNonFinite;
+      eb += sh - kDgBits + a.ealpha;
+      uint4 ea[NT];  // the rows' exponents, eight int16
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+        ea[j] = j < ntv ? __ldg(reinterpret_cast<const uint4*>(a.exA + (ct * NT + j) * kDgP + h * 8)) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int j = 0; j < NT; ++j) {
+        if (j >= ntv) break;
+        const int m0r = (ct * NT + j) * (kDgP / 2) + h * 4;
+        double2* o = a.C + (long long)m0r * a.ldc + n;
+        const uint32_t ew[4] = {ea[j].x, ea[j].y, ea[j].z, ea[j].w};
+#pragma unroll
+        for (int y = 0; y < 4; ++y, o += a.ldc) {
+          const int e0 = (int)(int16_t)(ew[y] & 0xFFFFu), e1 = (int)(int16_t)(ew[y] >> 16);
+          const double nan = __longlong_as_double(0x7FF8000000000000ll);
+          double2 v = cmk(dg_double(acc[j][2 * y] * a.salpha, e0 + eb), dg_double(acc[j][2 * y + 1] * a.salpha, e1 + eb));
+          if (bad || e0 == kDgNonFinite) v.x = nan;
+          if (bad || e1 == kDgNonFinite) v.y = nan;
+          if (m0r + y < a.M && n < a.Nn) {
+            if (a.accumulate) dg_add(o, v);
+            else *o = v;
+          }
+        }
+      }
+    }
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  if (warp == 16) tc::tmem_dealloc(taddr, 512);
+}
+
+// ------------------------------------------------------------------ host
+static constexpr size_t kDgRowBytes(size_t nk16) { return nk16 * 16 * kDgS * 2; }
+// rows of A per pass are limited so that their image stays in L2
+static constexpr size_t kDgImageCap = size_t(64) << 20;
+
+static size_t dg_chunk_rows(size_t M, size_t K) {
+  const size_t nk16 = (K + 15) / 16, per = 2 * kDgRowBytes(nk16);
+  size_t mc = kDgImageCap / per / 64 * 64;
+  if (mc < 64) mc = 64;
+  return mc < M ? mc : (M + 15) / 16 * 16;
+}
+
+size_t dg_scratch_bytes(size_t M, size_t Nn, size_t K) {
+  const size_t nk16 = (K + 15) / 16, mc = dg_chunk_rows(M, K), nb = (Nn + 127) / 128 * 128;
+  return nb * kDgRowBytes(nk16) + 2 * mc * kDgRowBytes(nk16) + nb * 2 + 2 * mc * 2 + 5 * 256;
+}
+
+template <int NT>
+static void dg_launch(DgArgs a, cudaStream_t st) {
+  a.nct = (a.ntile + NT - 1) / NT;
+  cudaFuncSetAttribute(dg_gemm_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgSmem);
+  const int items = a.nrt * a.nct;
+  dg_gemm_kernel<NT><<<items < 152 ? items : 152, kDgThreads, kDgSmem, st>>>(a);
+}
+
+// Tiles per CTA pass: the fewest rounds of the 152 CTAs, counted in 32-row tiles; NT = 4 reads the 128-row tile
+// least often, so it wins ties.
+static int dg_pick_nt(int nrt, int ntile) {
+  int best = 4;
+  long long cost = -1;
+  for (int nt = 4; nt >= 1; nt >>= 1) {
+    const long long items = (long long)nrt * ((ntile + nt - 1) / nt);
+    const long long c = (items + 151) / 152 * nt;
+    if (cost < 0 || c < cost) {
+      cost = c;
+      best = nt;
+    }
+  }
+  return best;
+}
+
+int launch_zgemm_dg(int M, int Nn, int K, double alpha, DgRows A, const double* B, int ldb, bool b_is_nk, double2* C,
+                    long long ldc, bool accumulate, const DgScratch& s, cudaStream_t st) {
+  if (M <= 0 || Nn <= 0) return TROT_OK;
+  if (K <= 0 || K > (1 << 17) || s.bytes < dg_scratch_bytes(M, Nn, K)) {
+    set_error("digit product: K=%d, scratch %zu < %zu", K, s.bytes, dg_scratch_bytes(M, Nn, K));
+    return TROT_ERR_WORKSPACE_TOO_SMALL;
+  }
+  const int nk16 = (K + 15) / 16, nrt = (Nn + 127) / 128;
+  const size_t mc = dg_chunk_rows(M, K);
+  char* p = reinterpret_cast<char*>(((uintptr_t)s.p + 255) & ~(uintptr_t)255);
+  auto take = [&](size_t n) {
+    char* r = p;
+    p += (n + 255) & ~(size_t)255;
+    return r;
+  };
+  DgArgs a{};
+  uint16_t* imgB = reinterpret_cast<uint16_t*>(take((size_t)nrt * 128 * kDgRowBytes(nk16)));
+  uint16_t* imgA = reinterpret_cast<uint16_t*>(take(2 * mc * kDgRowBytes(nk16)));
+  int16_t* exB = reinterpret_cast<int16_t*>(take((size_t)nrt * 128 * 2));
+  int16_t* exA = reinterpret_cast<int16_t*>(take(2 * mc * 2));
+  DgSrc sb{B, Nn, K, nk16, 128, 1, 0, b_is_nk ? ldb : 1, b_is_nk ? 1 : ldb, 0, imgB, exB};
+  TROT_TRY(dg_rows_launch(sb, nrt * 16, st));
+  int lk = 0;
+  while ((1 << lk) < K) ++lk;
+  a.imgB = imgB; a.exB = exB; a.imgA = imgA; a.exA = exA;
+  a.Nn = Nn; a.nrt = nrt; a.nk16 = nk16;
+  // |sum| <= K 2^17 2^36 2^-shift <= 2^62 (the leading digits of a row average 256 at most); at most 8 (K <= 2^17)
+  a.shift = lk > 10 ? lk - 9 : 1;
+  int ea = 0;
+  const double fa = frexp(alpha, &ea);  // alpha = fa 2^ea
+  if (fa != 0.5 && fa != -0.5) { set_error("digit product: alpha %g is not a power of two", alpha); return TROT_ERR_UNSUPPORTED; }
+  a.salpha = fa < 0 ? -1 : 1;
+  a.ealpha = ea - 1;
+  a.ldc = ldc; a.accumulate = accumulate ? 1 : 0; a.status = s.status;
+  for (size_t m0 = 0; m0 < (size_t)M; m0 += mc) {
+    const int mm = (int)std::min(mc, (size_t)M - m0);
+    a.ntile = (2 * mm + kDgP - 1) / kDgP;
+    DgSrc sa{reinterpret_cast<const double*>(A.p + (long long)(m0 / A.rpb) * A.bstride), 2 * mm, K, nk16, kDgP, A.rpb,
+             2 * A.bstride, 2ll * A.lda, 2, 1, imgA, exA};  // chunks start on whole row blocks
+    TROT_TRY(dg_rows_launch(sa, a.ntile * 4, st));
+    a.M = mm;
+    a.C = C + (long long)m0 * ldc;
+    const int nt = dg_pick_nt(nrt, a.ntile);
+    if (nt == 4) dg_launch<4>(a, st);
+    else if (nt == 2) dg_launch<2>(a, st);
+    else dg_launch<1>(a, st);
+    TROT_CHECK_LAUNCH("dg_gemm_kernel");
+  }
+  return TROT_OK;
+}
+
+}  // namespace trot
+
+extern "C" size_t trot_zgemm_digits_workspace(int M, int N, int K) {
+  return M > 0 && N > 0 && K > 0 ? trot::dg_scratch_bytes(M, N, K) + 512 : 0;
+}
+
+extern "C" int trot_zgemm_digits(int M, int N, int K, double alpha, const double* A, int lda, const double* B, int ldb,
+                                 int b_is_nk, double* C, int ldc, int accumulate, void* ws, size_t ws_bytes,
+                                 void* stream) {
+  using namespace trot;
+  if (!A || !B || !C || !ws) { set_error("null digit product buffer"); return TROT_ERR_NULL_PTR; }
+  if (M <= 0 || N <= 0 || K <= 0 || lda < K || ldc < N || ldb < (b_is_nk ? K : N)) {
+    set_error("zgemm_digits: bad sizes M=%d N=%d K=%d lda=%d ldb=%d ldc=%d", M, N, K, lda, ldb, ldc);
+    return TROT_ERR_BAD_SHAPE;
+  }
+  Carver c(ws, ws_bytes);
+  DgScratch s;
+  s.bytes = dg_scratch_bytes(M, N, K);
+  s.p = c.take<char>(s.bytes);
+  s.status = c.status();
+  if (!c.ok) { set_error("workspace too small: %zu < %zu", ws_bytes, c.used); return TROT_ERR_WORKSPACE_TOO_SMALL; }
+  return launch_zgemm_dg(M, N, K, alpha, dg_rows((const double2*)A, lda), B, ldb, b_is_nk != 0, (double2*)C, ldc,
+                         accumulate != 0, s, (cudaStream_t)stream);
+}

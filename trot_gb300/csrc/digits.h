@@ -1,0 +1,31 @@
+// FP64-accurate products on the tensor cores by exact digit slices (digits.cu).
+// Shorter rows than 20 stay on the FP64 pipe: the digits' error does not fall with K (1.05e-16 of the result at K = 3,
+// 1.1e-16 at 16, 1.2e-16 at 135), that of an FP64 sum does (0.8e-16, 1.5e-16, 3.9e-16).  Past 2^17 the 64-bit sums
+// would overflow.  There is no limit on the other sizes: one 64 x 64 x 16 step of the FP64 kernel takes 34 us on its
+// SM, a whole small product here 20 us.
+#pragma once
+#include "kernels.h"
+
+namespace trot {
+
+static constexpr int kDgMinK = 20, kDgMaxK = 1 << 17;
+inline bool dg_takes(int K) { return K >= kDgMinK && K <= kDgMaxK; }
+
+// Bytes that launch_zgemm_dg wants for C (M x Nn) = alpha A (M x K complex) B (K x Nn real).
+size_t dg_scratch_bytes(size_t M, size_t Nn, size_t K);
+
+// A complex rows: row r at A + (r / rpb) bstride + (r % rpb) lda (rpb = 1, bstride = lda: plain row-major).
+struct DgRows {
+  const double2* p;
+  int rpb;
+  long long bstride;
+  int lda;
+};
+inline DgRows dg_rows(const double2* p, int lda) { return DgRows{p, 1, lda, lda}; }
+
+// C[m][n] (+)= alpha sum_k A[m][k] B(k, n) as launch_zgemm_cr, with both operands as six
+// FP16 digit planes per row and 26 exact tensor-core products.
+int launch_zgemm_dg(int M, int Nn, int K, double alpha, DgRows A, const double* B, int ldb, bool b_is_nk, double2* C,
+                    long long ldc, bool accumulate, const DgScratch& s, cudaStream_t st);
+
+}  // namespace trot

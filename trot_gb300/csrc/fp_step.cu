@@ -98,8 +98,10 @@ int trot_fp_step(const trot_system* s, const trot_state* state, const double* fi
     return TROT_ERR_NULL_PTR;
   }
   if (!s->mf_shifts_im) { set_error("null propagation context"); return TROT_ERR_NULL_PTR; }
-  const size_t tb = trotter_bytes(s);
+  size_t tb = trotter_bytes(s);
   if (tb == 0) return TROT_ERR_BAD_SHAPE;  // trot_workspace_size recorded the reason
+  if (s->precision == TROT_FP64 && ws_bytes < trot_fp_workspace_size(s))  // too small for the digit products' scratch
+    tb = (fp64_min_workspace(s, TROT_OP_APPLY_TROTTER) + 255) & ~(size_t)255;
   if (ws_bytes < tb) { set_error("workspace too small: %zu < %zu", ws_bytes, tb); return TROT_ERR_WORKSPACE_TOO_SMALL; }
   Spins sp = make_spins(s);
   Carver c(ws ? static_cast<char*>(ws) + tb : nullptr, ws_bytes - tb);

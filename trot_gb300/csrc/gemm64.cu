@@ -9,7 +9,7 @@
 // (trot/prop/chol_afqmc_ops.py:83-87: Re(x) @ chol_flat + i Im(x) @ chol_flat).
 // GB300's FP64 rate is ~2 FMA/clk/SM, so this kernel is FP64-pipe bound with
 // any reasonable register tiling: 64x64 tiles, 4x4 complex outputs per thread.
-#include "kernels.h"
+#include "digits.h"
 
 namespace trot {
 
@@ -134,6 +134,12 @@ int launch_zgemm_cr_splitk(int M, int Nn, int K, double alpha, const double2* A,
   return TROT_OK;
 }
 
+int launch_zgemm(int M, int Nn, int K, double alpha, const double2* A, int lda, const double* B, int ldb, bool b_is_nk,
+                 double2* C, int ldc, bool accumulate, const DgScratch& dg, cudaStream_t st, double2* part, int S) {
+  if (M > 0 && Nn > 0 && dg.p && dg_takes(K) && dg.bytes >= dg_scratch_bytes(M, Nn, K))
+    return launch_zgemm_dg(M, Nn, K, alpha, dg_rows(A, lda), B, ldb, b_is_nk, C, ldc, accumulate, dg, st);
+  return launch_zgemm_cr_splitk(M, Nn, K, alpha, A, lda, B, ldb, b_is_nk, C, ldc, accumulate, part, S, st);
+}
 
 // ------------------------------------------------------------------ packed symmetric VHS
 // With every L_g symmetric, V_b = sum_g xs[b][g] L_g is symmetric: its upper triangle
@@ -171,11 +177,11 @@ static int grid_1d(size_t total) {
 }
 
 int launch_vhs64(int W, int N, int G, const double2* xs, const double* chol_flat, const double* chol_packed,
-                 double2* vp, double2* vhs, cudaStream_t st) {
+                 double2* vp, double2* vhs, const DgScratch& dg, cudaStream_t st) {
   if (!chol_packed || !vp)
-    return launch_zgemm_cr(W, N * N, G, 1.0, xs, G, chol_flat, N * N, false, vhs, N * N, false, st);
+    return launch_zgemm(W, N * N, G, 1.0, xs, G, chol_flat, N * N, false, vhs, N * N, false, dg, st);
   const int P = N * (N + 1) / 2;
-  TROT_TRY(launch_zgemm_cr(W, P, G, 1.0, xs, G, chol_packed, P, false, vp, P, false, st));
+  TROT_TRY(launch_zgemm(W, P, G, 1.0, xs, G, chol_packed, P, false, vp, P, false, dg, st));
   vhs_unpack_kernel<<<grid_1d((size_t)W * N * N), 256, 0, st>>>(W, N, vp, vhs);
   TROT_CHECK_LAUNCH("vhs_unpack_kernel");
   return TROT_OK;

@@ -29,14 +29,25 @@ struct Carver {
   }
 };
 
+// Scratch of the tensor-core digit products (digits.h), carved out of the caller's workspace; status: the
+// workspace's status words (see report_timeout), may be null.  p == null: none.
+struct DgScratch {
+  void* p = nullptr;
+  size_t bytes = 0;
+  int* status = nullptr;
+};
+
 struct StepBuffers {
   double2 *green, *e1, *fb, *xs, *shift_term, *fb_term, *vhs, *exc;
   double2* vp;  // packed upper triangle of the VHS (W, N(N+1)/2) when chol_packed is set
   int* node_flag;
+  DgScratch dg;  // scratch of the digit products; p == null: none
 };
 
 Spins make_spins(const trot_system* s);
 int tune_get(int knob);  // tune.cu: 0 = default
+// bytes with which an FP64 op runs at all: its workspace without the digit products' scratch
+size_t fp64_min_workspace(const trot_system* s, int op);
 
 // Green's function / overlap per walker (green.cu).
 // green: complex (W, ntot*N) half Green's functions, spin blocks concatenated
@@ -55,10 +66,15 @@ int launch_zgemm_cr(int M, int Nn, int K, double alpha, const double2* A, int ld
 int launch_zgemm_cr_splitk(int M, int Nn, int K, double alpha, const double2* A, int lda, const double* B, int ldb,
                            bool b_is_nk, double2* C, int ldc, bool accumulate, double2* part, int S,
                            cudaStream_t st);
+// The product on the tensor cores (digits.cu) where `dg` holds its scratch and K is in its range, else on the
+// FP64 pipe (split over K when part is given).
+int launch_zgemm(int M, int Nn, int K, double alpha, const double2* A, int lda, const double* B, int ldb, bool b_is_nk,
+                 double2* C, int ldc, bool accumulate, const DgScratch& dg, cudaStream_t st,
+                 double2* part = nullptr, int S = 1);
 // FP64 VHS = xs . chol (W x N^2): over the packed upper triangle (then mirrored) when
 // chol_packed and vp (W x N(N+1)/2 complex scratch) are given, else the full product.
 int launch_vhs64(int W, int N, int G, const double2* xs, const double* chol_flat, const double* chol_packed,
-                 double2* vp, double2* vhs, cudaStream_t st);
+                 double2* vp, double2* vhs, const DgScratch& dg, cudaStream_t st);
 // Mp = the packed upper triangle of M + M^T (diagonal once), W matrices of N x N.
 int launch_pack_sym(int N, int W, const double2* m, double2* mp, cudaStream_t st);
 

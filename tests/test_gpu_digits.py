@@ -117,3 +117,45 @@ def test_small_workspace_runs_without_the_digit_products(kind):
     assert len(out) >= 2
     for e in out[1:]:
         assert np.max(np.abs(e - out[0])) <= 1e-12 * np.max(np.abs(out[0]))
+
+
+@pytest.mark.parametrize("kind,N,na,nb,G,W", [
+    ("rhf_r", 20, 1, 1, 65, 3), ("rhf_r", 33, 2, 2, 64, 17), ("rhf_u", 40, 7, 7, 63, 5), ("uhf_u", 48, 16, 3, 130, 18),
+    ("uhf_u", 37, 9, 17, 129, 33), ("rhf_r", 70, 33, 33, 71, 2), ("rhf_r", 129, 5, 5, 200, 20)])
+def test_energy_from_digit_products(kind, N, na, nb, G, W):
+    """Local energy (exchange sums and traces of f_g) and the step's force bias against the oracle: electrons per spin
+    from 1 past 32, vectors and walkers off the kernel's chunks of 64 and 16.  FP64 sums over K <= 129 terms and G n^2
+    products of a well-conditioned Green's function: 1e-11 of the largest energy."""
+    from oracle import afqmc_oracle as orc
+
+    rng = np.random.default_rng(N)
+    h0, h1, chol = synthetic.hamiltonian(N, G, 30.0, seed=N, h0=0.3)
+    mo = np.linalg.qr(rng.standard_normal((N, N)))[0]
+    ma, mb = np.ascontiguousarray(mo[:, :na]), np.ascontiguousarray(mo[:, -nb:] if kind == "uhf_u" else mo[:, :nb])
+    S = Setup(kind, h0, h1, chol, ma, mb, 0.005, W)
+    w = synthetic.perturbed_walkers(ma, W, 0.05, 3)
+    if kind != "rhf_r":
+        w = (w, synthetic.perturbed_walkers(mb, W, 0.05, 4))
+    if kind == "uhf_u":
+        ctx, mo_o = orc.build_uhf_meas_ctx(h1, chol, ma, mb), (ma, mb)
+    else:
+        ctx, mo_o = orc.build_rhf_meas_ctx(h1, chol, ma), ma
+    m = orc.Model(kind, h0, mo_o, ctx, orc.build_prop_ctx(h0, h1, chol, np.stack([ma @ ma.T, mb @ mb.T]), 0.005))
+    e_ref, fb_ref = m.energy(w), m.force_bias(w)
+    wd = S.walkers(w)
+    e, fb = cpu(S.energy(wd)), cpu(S.force_bias(wd))
+    assert np.max(np.abs(e - e_ref)) <= 1e-11 * np.max(np.abs(e_ref))
+    assert np.max(np.abs(fb - fb_ref)) <= 1e-11 * np.max(np.abs(fb_ref))
+    # the step takes its force bias from the traces of f_g when it also returns the energies, else from a product
+    fields, outs = dev(rng.standard_normal((W, G))), []
+    for with_energy in (True, False):
+        wk = S.walkers(w)
+        st = S.state(wk, np.ones(W), cpu(S.overlap(wk)), -1.0, -1.0)
+        en = torch.zeros(W, dtype=torch.complex128, device="cuda") if with_energy else None
+        S.step(st, fields, energy_out=en)
+        if with_energy:
+            assert np.array_equal(cpu(en), e)
+        ws = st.walkers if isinstance(st.walkers, tuple) else (st.walkers,)
+        outs.append([cpu(x) for x in ws])
+    for x, y in zip(*outs):
+        assert np.max(np.abs(x - y)) <= 1e-11 * np.max(np.abs(y))

@@ -55,6 +55,8 @@ static size_t digit_bytes(const trot_system* s, const Spins& sp, int op) {
   if (op == TROT_OP_FORCE_BIAS || op == TROT_OP_LOCAL_ENERGY || op == TROT_OP_PROP_STEP)
     for (int q = 0; q < sp.nspin; ++q)
       if (dg_takes(sp.n[q] * (int)N)) n = std::max(n, dg_scratch_bytes(W, G, sp.n[q] * N));
+  if ((op == TROT_OP_LOCAL_ENERGY || op == TROT_OP_PROP_STEP) && dg_takes((int)N) && N <= 1024)
+    n = std::max(n, exchange_dg_bytes(sp, W, N, G));
   if ((op == TROT_OP_APPLY_TROTTER || op == TROT_OP_PROP_STEP) && dg_takes((int)G))
     n = std::max(n, dg_scratch_bytes(W, N * N, G));  // full or packed
   return n;
@@ -160,6 +162,23 @@ static int force_bias_from_green(const trot_system* s, const Spins& sp, const do
     TROT_TRY(launch_zgemm(W, G, sp.n[q] * N, (double)sp.mult[q], green + (size_t)sp.off[q] * N, K, sp.rot_chol[q],
                           sp.n[q] * N, true, fb, G, q > 0, dg, st));
   }
+  return TROT_OK;
+}
+
+// force bias and exchange sums (nchunks of them per walker) of the local energy, on the tensor cores where
+// the digit products apply
+static int force_bias_and_exchange(const trot_system* s, const Spins& sp, const StepBuffers& b, int& nchunks,
+                                   cudaStream_t st) {
+  const int W = s->n_walkers, N = s->norb, G = s->nchol;
+  TROT_TRY(check_exchange_tile(sp, N));
+  if (b.dg.p && dg_takes(N) && N <= 1024) {
+    nchunks = exchange_dg_chunks(G);
+    TROT_TIMED("exchange_digits", st, launch_exchange_dg(sp, W, N, G, b.green, b.exc, b.fb, b.dg, st));
+    return TROT_OK;
+  }
+  nchunks = exchange_chunks(G);
+  TROT_TIMED("force_bias_fp64", st, force_bias_from_green(s, sp, b.green, b.fb, b.dg, st));
+  TROT_TIMED("exchange_fp64", st, launch_exchange(sp, W, N, G, b.green, b.exc, st));
   return TROT_OK;
 }
 
@@ -305,9 +324,9 @@ int trot_local_energy(const trot_system* s, const double* wa, const double* wb, 
   TROT_TRY(carve_ws(s, sp, ws, ws_bytes, b, TROT_OP_LOCAL_ENERGY));
   const int W = s->n_walkers, N = s->norb, G = s->nchol;
   TROT_TRY(launch_green(sp, W, N, (const double2*)wa, (const double2*)wb, b.green, nullptr, b.e1, st));
-  TROT_TRY(force_bias_from_green(s, sp, b.green, b.fb, b.dg, st));
-  TROT_TRY(launch_exchange(sp, W, N, G, b.green, b.exc, st));
-  return launch_energy_combine(W, G, exchange_chunks(G), s->h0, b.fb, b.e1, 1, b.exc, (double2*)out, st);
+  int nchunks = 0;
+  TROT_TRY(force_bias_and_exchange(s, sp, b, nchunks, st));
+  return launch_energy_combine(W, G, nchunks, s->h0, b.fb, b.e1, 1, b.exc, (double2*)out, st);
 }
 
 int trot_apply_trotter(const trot_system* s, const double* wa, const double* wb, const double* xs,
@@ -353,13 +372,14 @@ int trot_prop_step(const trot_system* s, const trot_state* state, const double* 
   double2* wb = (double2*)state->walkers_b;
   // 1. Green's functions (+ one-body energy) of the current walkers
   TROT_TIMED("green", st, launch_green(sp, W, N, wa, wb, b.green, nullptr, energy_out ? b.e1 : nullptr, st));
-  // 2. force bias
-  TROT_TIMED("force_bias_fp64", st, force_bias_from_green(s, sp, b.green, b.fb, b.dg, st));
-  // 3. optional local energy of the current walkers (reuses G and fb)
-  if (energy_out) {
-    TROT_TIMED("exchange_fp64", st, launch_exchange(sp, W, N, G, b.green, b.exc, st));
+  // 2. force bias, 3. optional local energy of the current walkers (reuses G; f_g gives both)
+  if (!energy_out) {
+    TROT_TIMED("force_bias_fp64", st, force_bias_from_green(s, sp, b.green, b.fb, b.dg, st));
+  } else {
+    int nchunks = 0;
+    TROT_TRY(force_bias_and_exchange(s, sp, b, nchunks, st));
     TROT_TIMED("energy_combine", st,
-               launch_energy_combine(W, G, exchange_chunks(G), s->h0, b.fb, b.e1, 1, b.exc, (double2*)energy_out, st));
+               launch_energy_combine(W, G, nchunks, s->h0, b.fb, b.e1, 1, b.exc, (double2*)energy_out, st));
   }
   // 4. shifted fields
   TROT_TIMED("fields", st, launch_fields(W, G, s->sqrt_dt, b.fb, s->mf_shifts_im, fields, b.xs, b.shift_term, b.fb_term, st));

@@ -125,13 +125,25 @@ TROT_D int dg_exponent(unsigned mx, float l1) {
 // per 32 columns, 20 us like this.
 struct DgSrc {
   const double* p;
-  int rows, K, nk16, R;  // R = 32 or 128 rows per tile
-  int rpb;               // complex rows per block of bstride doubles (complex A only)
-  long long bstride, rst, kst;  // strides in doubles
+  int K, nk16, R;        // R = 32 or 128 rows per tile
   int cplx;
+  // image row -> block (of bstride doubles) row / rpad, row r = row % rpad of it; rows r >= rpb and blocks
+  // >= nblk are padding
+  int rpb, rpad, nblk;
+  long long bstride, rst, kst;  // strides in doubles (rst: of a complex row)
+  // complex rows r >= split come from a second array (the other spin's walkers)
+  int split;
+  const double* p2;
+  long long bstride2, kst2;
   uint16_t* img;
   int16_t* ex;
 };
+static constexpr int kDgOneBlock = 1 << 30;
+// `rows` rows of stride rst (complex ones count twice), one block
+static DgSrc dg_src(const double* p, int cplx, int rows, int K, int R, long long rst, long long kst, uint16_t* img,
+                    int16_t* ex) {
+  return DgSrc{p, K, (K + 15) / 16, R, cplx, rows, kDgOneBlock, 1, 0, rst, kst, kDgOneBlock, nullptr, 0, 0, img, ex};
+}
 
 __global__ void __launch_bounds__(256) dg_rows_kernel(DgSrc a) {
   __shared__ unsigned smx[8][8], cmx[8];
@@ -142,14 +154,18 @@ __global__ void __launch_bounds__(256) dg_rows_kernel(DgSrc a) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int rl = lane & 7, kg = lane >> 3;
   const int row = blockIdx.y * 8 + rl;
-  const bool valid = row < a.rows;
+  const int blk = row / a.rpad, rr = row - blk * a.rpad;
+  const bool valid = blk < a.nblk && rr < a.rpb;
   const double* p = a.p;
+  long long kst = a.kst;
   if (valid) {
-    if (a.cplx) {
-      const int cr = row >> 1;
-      p += (long long)(cr / a.rpb) * a.bstride + (long long)(cr % a.rpb) * a.rst + (row & 1);
+    if (rr >= a.split) {
+      p = a.p2 + blk * a.bstride2 + ((rr - a.split) >> 1) * a.rst + (rr & 1);
+      kst = a.kst2;
+    } else if (a.cplx) {
+      p += blk * a.bstride + (rr >> 1) * a.rst + (rr & 1);
     } else {
-      p += (long long)row * a.rst;
+      p += blk * a.bstride + rr * a.rst;
     }
   }
   const int kpad = a.nk16 * 16, kstep = 256 * KS;
@@ -161,7 +177,7 @@ __global__ void __launch_bounds__(256) dg_rows_kernel(DgSrc a) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int k = k0 + kg * 8 + i;
-      x[i] = (valid && k < a.K) ? p[(long long)k * a.kst] : 0.0;
+      x[i] = (valid && k < a.K) ? p[k * kst] : 0.0;
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -209,7 +225,7 @@ __global__ void __launch_bounds__(256) dg_rows_kernel(DgSrc a) {
     if (kb >= kpad) continue;
     if (!once) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) x[i] = (live && kb + i < a.K) ? p[(long long)(kb + i) * a.kst] : 0.0;
+      for (int i = 0; i < 8; ++i) x[i] = (live && kb + i < a.K) ? p[(kb + i) * kst] : 0.0;
     }
     if (!live) {
 #pragma unroll
@@ -251,7 +267,9 @@ struct DgArgs {
   const uint16_t* imgA;  // MMA columns: rows of A, [tile][nk16][6][32][16]
   const int16_t* exA;
   int Nn, M;             // outputs: n < Nn, complex rows m < M
-  int nrt, ntile, nct;   // 128-row tiles, 32-row tiles, groups of NT 32-row tiles
+  int nrt, ntile, nct;   // 128-row tiles, 32-row tiles, groups of NT 32-row tiles (per batch)
+  int nbatch, bB;        // batches: ntile 32-row tiles each, bB 128-row tiles (0: all share them)
+  long long cstride;     // and cstride complex outputs
   int nk16, shift;       // K16 steps; the outputs' integers are in units 2^(eA + eB - 54 + shift)
   double2* C;
   long long ldc;
@@ -279,7 +297,9 @@ TROT_D double dg_double(long long v, int E) {
 // out of line, so that its FP64 instructions are not issued (predicated off) for plain stores
 __device__ __noinline__ void dg_add(double2* o, double2 v) { *o = cadd(*o, v); }
 
-template <int NT>
+// PAIR: the 128-row tiles hold complex rows (row 2 p = real, 2 p + 1 = imaginary part of V[p]) and the product is the
+// complex V T: C[m][p] = V_p . A_m.  Lanes 2 p and 2 p + 1 exchange the cross terms; each stores its part.
+template <int NT, bool PAIR>
 __global__ void __launch_bounds__(kDgThreads, 1) dg_gemm_kernel(DgArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   unsigned char* base = smem_raw + ((128 - (tc::smem_u32(smem_raw) & 127)) & 127);
@@ -297,7 +317,7 @@ __global__ void __launch_bounds__(kDgThreads, 1) dg_gemm_kernel(DgArgs a) {
   volatile int* abort_flag = reinterpret_cast<volatile int*>(drain + 2);
   static_assert((2 * kDgASlots + 2 * kDgBSlots + 4 + 3) * 8 <= 256, "barrier table");
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n_items = a.nrt * a.nct, nk = a.nk16;
+  const int n_items = a.nrt * a.nct * a.nbatch, nk = a.nk16;
   const int nslab = (nk + kDgSlab - 1) / kDgSlab;
   if (warp == 16) tc::tmem_alloc(tslot, 512);
   if (tid == kDgEpi) {
@@ -330,7 +350,7 @@ __global__ void __launch_bounds__(kDgThreads, 1) dg_gemm_kernel(DgArgs a) {
       const uint32_t adlo = (uint32_t)ad0, bdlo = (uint32_t)bd0, dhi = (uint32_t)(ad0 >> 32);
       int ca = 0, cb = 0, cacc = 0;  // chunk, slab-tile and accumulator counters of this CTA
       for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-        const int ntv = min(NT, a.ntile - (item / a.nrt) * NT);
+        const int ntv = min(NT, a.ntile - ((item / a.nrt) % a.nct) * NT);
         for (int s = 0; s < nslab && ok; ++s) {
           const int ks = min(kDgSlab, nk - s * kDgSlab);
           for (int j = 0; j < ntv && ok; ++j, ++cb, ++cacc) {
@@ -388,7 +408,8 @@ __global__ void __launch_bounds__(kDgThreads, 1) dg_gemm_kernel(DgArgs a) {
       bool ok = true;
       int c = 0;
       for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-        const int rt = item % a.nrt, ct = item / a.nrt;
+        const int bt = item / (a.nrt * a.nct);
+        const int rt = item % a.nrt + bt * a.bB, ct = (item / a.nrt) % a.nct;
         const int ntv = min(NT, a.ntile - ct * NT);
         for (int s = 0; s < nslab && ok; ++s) {
           const int ks = min(kDgSlab, nk - s * kDgSlab);
@@ -412,7 +433,7 @@ __global__ void __launch_bounds__(kDgThreads, 1) dg_gemm_kernel(DgArgs a) {
             } else {
               tc::mbar_expect_tx(&full[slot], ks * kDgBStep);
               tc::bulk_g2s(sB + (size_t)slot * kDgSlab * kDgBStep,
-                           a.imgA + ((size_t)(ct * NT + j) * nk + s * kDgSlab) * (kDgBStep / 2), ks * kDgBStep,
+                           a.imgA + ((size_t)(bt * a.ntile + ct * NT + j) * nk + s * kDgSlab) * (kDgBStep / 2), ks * kDgBStep,
                            &full[slot]);
             }
           }
@@ -435,7 +456,7 @@ __global__ void __launch_bounds__(kDgThreads, 1) dg_gemm_kernel(DgArgs a) {
     int cacc = 0;
     bool ok = true;
     for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-      const int rt = item % a.nrt, ct = item / a.nrt;
+      const int rt = item % a.nrt, ct = (item / a.nrt) % a.nct, bt = item / (a.nrt * a.nct);
       const int ntv = min(NT, a.ntile - ct * NT);
       const int n = rt * 128 + q * 32 + lane;
       long long acc[NT][8];
@@ -490,19 +511,19 @@ __global__ void __launch_bounds__(kDgThreads, 1) dg_gemm_kernel(DgArgs a) {
         }
       }
       // outputs: lane = column n of C, register pairs = (re, im) of four complex rows
-      int eb = n < a.Nn ? a.exB[n] : 0;
+      int eb = n < a.Nn ? a.exB[bt * a.bB * 128 + n] : 0;
       if (!ok) eb = kDgNonFinite;
       const bool bad = eb == kDgNonFinite;
       eb += sh - kDgBits + a.ealpha;
       uint4 ea[NT];  // the rows' exponents, eight int16
 #pragma unroll
       for (int j = 0; j < NT; ++j)
-        ea[j] = j < ntv ? __ldg(reinterpret_cast<const uint4*>(a.exA + (ct * NT + j) * kDgP + h * 8)) : make_uint4(0, 0, 0, 0);
+        ea[j] = j < ntv ? __ldg(reinterpret_cast<const uint4*>(a.exA + (size_t)(bt * a.ntile + ct * NT + j) * kDgP + h * 8)) : make_uint4(0, 0, 0, 0);
 #pragma unroll
       for (int j = 0; j < NT; ++j) {
         if (j >= ntv) break;
         const int m0r = (ct * NT + j) * (kDgP / 2) + h * 4;
-        double2* o = a.C + (long long)m0r * a.ldc + n;
+        double2* o = a.C + bt * a.cstride + (long long)m0r * a.ldc + (PAIR ? n >> 1 : n);
         const uint32_t ew[4] = {ea[j].x, ea[j].y, ea[j].z, ea[j].w};
 #pragma unroll
         for (int y = 0; y < 4; ++y, o += a.ldc) {
@@ -511,7 +532,14 @@ __global__ void __launch_bounds__(kDgThreads, 1) dg_gemm_kernel(DgArgs a) {
           double2 v = cmk(dg_double(acc[j][2 * y] * a.salpha, e0 + eb), dg_double(acc[j][2 * y + 1] * a.salpha, e1 + eb));
           if (bad || e0 == kDgNonFinite) v.x = nan;
           if (bad || e1 == kDgNonFinite) v.y = nan;
-          if (m0r + y < a.M && n < a.Nn) {
+          if (PAIR) {
+            const double w = __shfl_xor_sync(0xffffffffu, v.y, 1);
+            if (m0r + y < a.M && n < a.Nn) {
+              double* od = reinterpret_cast<double*>(o);
+              if (n & 1) od[1] = v.x + w;
+              else od[0] = v.x - w;
+            }
+          } else if (m0r + y < a.M && n < a.Nn) {
             if (a.accumulate) dg_add(o, v);
             else *o = v;
           }
@@ -541,21 +569,21 @@ size_t dg_scratch_bytes(size_t M, size_t Nn, size_t K) {
   return nb * kDgRowBytes(nk16) + 2 * mc * kDgRowBytes(nk16) + nb * 2 + 2 * mc * 2 + 5 * 256;
 }
 
-template <int NT>
+template <int NT, bool PAIR>
 static void dg_launch(DgArgs a, cudaStream_t st) {
   a.nct = (a.ntile + NT - 1) / NT;
-  cudaFuncSetAttribute(dg_gemm_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgSmem);
-  const int items = a.nrt * a.nct;
-  dg_gemm_kernel<NT><<<items < 152 ? items : 152, kDgThreads, kDgSmem, st>>>(a);
+  cudaFuncSetAttribute(dg_gemm_kernel<NT, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgSmem);
+  const int items = a.nrt * a.nct * a.nbatch;
+  dg_gemm_kernel<NT, PAIR><<<items < 152 ? items : 152, kDgThreads, kDgSmem, st>>>(a);
 }
 
 // Tiles per CTA pass: the fewest rounds of the 152 CTAs, counted in 32-row tiles; NT = 4 reads the 128-row tile
 // least often, so it wins ties.
-static int dg_pick_nt(int nrt, int ntile) {
+static int dg_pick_nt(int nrt, int ntile, int nbatch) {
   int best = 4;
   long long cost = -1;
   for (int nt = 4; nt >= 1; nt >>= 1) {
-    const long long items = (long long)nrt * ((ntile + nt - 1) / nt);
+    const long long items = (long long)nrt * ((ntile + nt - 1) / nt) * nbatch;
     const long long c = (items + 151) / 152 * nt;
     if (cost < 0 || c < cost) {
       cost = c;
@@ -565,8 +593,15 @@ static int dg_pick_nt(int nrt, int ntile) {
   return best;
 }
 
-int launch_zgemm_dg(int M, int Nn, int K, double alpha, DgRows A, const double* B, int ldb, bool b_is_nk, double2* C,
-                    long long ldc, bool accumulate, const DgScratch& s, cudaStream_t st) {
+static void dg_gemm(const DgArgs& a, cudaStream_t st) {
+  const int nt = dg_pick_nt(a.nrt, a.ntile, a.nbatch);
+  if (nt == 4) dg_launch<4, false>(a, st);
+  else if (nt == 2) dg_launch<2, false>(a, st);
+  else dg_launch<1, false>(a, st);
+}
+
+int launch_zgemm_dg(int M, int Nn, int K, double alpha, const double2* A, int lda, const double* B, int ldb,
+                    bool b_is_nk, double2* C, long long ldc, bool accumulate, const DgScratch& s, cudaStream_t st) {
   if (M <= 0 || Nn <= 0) return TROT_OK;
   if (K <= 0 || K > (1 << 17) || s.bytes < dg_scratch_bytes(M, Nn, K)) {
     set_error("digit product: K=%d, scratch %zu < %zu", K, s.bytes, dg_scratch_bytes(M, Nn, K));
@@ -585,12 +620,11 @@ int launch_zgemm_dg(int M, int Nn, int K, double alpha, DgRows A, const double* 
   uint16_t* imgA = reinterpret_cast<uint16_t*>(take(2 * mc * kDgRowBytes(nk16)));
   int16_t* exB = reinterpret_cast<int16_t*>(take((size_t)nrt * 128 * 2));
   int16_t* exA = reinterpret_cast<int16_t*>(take(2 * mc * 2));
-  DgSrc sb{B, Nn, K, nk16, 128, 1, 0, b_is_nk ? ldb : 1, b_is_nk ? 1 : ldb, 0, imgB, exB};
-  TROT_TRY(dg_rows_launch(sb, nrt * 16, st));
+  TROT_TRY(dg_rows_launch(dg_src(B, 0, Nn, K, 128, b_is_nk ? ldb : 1, b_is_nk ? 1 : ldb, imgB, exB), nrt * 16, st));
   int lk = 0;
   while ((1 << lk) < K) ++lk;
   a.imgB = imgB; a.exB = exB; a.imgA = imgA; a.exA = exA;
-  a.Nn = Nn; a.nrt = nrt; a.nk16 = nk16;
+  a.Nn = Nn; a.nrt = nrt; a.nk16 = nk16; a.nbatch = 1;
   // |sum| <= K 2^17 2^36 2^-shift <= 2^62 (the leading digits of a row average 256 at most); at most 8 (K <= 2^17)
   a.shift = lk > 10 ? lk - 9 : 1;
   int ea = 0;
@@ -602,16 +636,151 @@ int launch_zgemm_dg(int M, int Nn, int K, double alpha, DgRows A, const double* 
   for (size_t m0 = 0; m0 < (size_t)M; m0 += mc) {
     const int mm = (int)std::min(mc, (size_t)M - m0);
     a.ntile = (2 * mm + kDgP - 1) / kDgP;
-    DgSrc sa{reinterpret_cast<const double*>(A.p + (long long)(m0 / A.rpb) * A.bstride), 2 * mm, K, nk16, kDgP, A.rpb,
-             2 * A.bstride, 2ll * A.lda, 2, 1, imgA, exA};  // chunks start on whole row blocks
-    TROT_TRY(dg_rows_launch(sa, a.ntile * 4, st));
+    TROT_TRY(dg_rows_launch(dg_src(reinterpret_cast<const double*>(A + (long long)m0 * lda), 1, 2 * mm, K, kDgP, 2ll * lda,
+                                   2, imgA, exA), a.ntile * 4, st));
     a.M = mm;
     a.C = C + (long long)m0 * ldc;
-    const int nt = dg_pick_nt(nrt, a.ntile);
-    if (nt == 4) dg_launch<4>(a, st);
-    else if (nt == 2) dg_launch<2>(a, st);
-    else dg_launch<1>(a, st);
+    dg_gemm(a, st);
     TROT_CHECK_LAUNCH("dg_gemm_kernel");
+  }
+  return TROT_OK;
+}
+
+// ------------------------------------------------------------------ exchange
+// f_g[i][j] = sum_p rot_chol_g[i][p] G[j][p] of a chunk of walkers as one product F (rows (b, j), columns (g, i)), then
+// per walker sum_g sum_ij f_gij f_gji and the traces tr f_g (trot/meas/rhf.py:33-60,119-125).  F of a chunk stays in
+// L2 (96 MB cap), so only the products cost: padding every walker's 2 n columns to the 32 of a tile, for sums
+// in the product's own epilogue, would cost more than writing and reading F (n = 10: 38 % idle columns).
+//
+// exchange_pairs_kernel, one CTA per (64 Cholesky vectors, walker): the vectors' n x n blocks in shared memory, row i
+// takes the pairs (i, i + k mod n), k <= n / 2, each product once (weight 2 off the diagonal), four FP64 FMAs each:
+// 0.6 ms of the FP64 pipe at 120 orbitals, 12 + 10 electrons, 600 vectors, 1024 walkers, which bounds it.  The CTA's
+// own reduction (20 FP64 additions per warp) costs as much as 16 vectors' products, hence 64 vectors per CTA.
+static constexpr int kExgChunk = 64;     // vectors per partial sum
+static constexpr int kExgThreads = 128;  // a thread per (vector, i) of the vectors in shared memory
+
+int exchange_dg_chunks(int G) { return (G + kExgChunk - 1) / kExgChunk; }
+
+__global__ void __launch_bounds__(kExgThreads)
+exchange_pairs_kernel(int n, int G, int gsub, int nchunks, int mult, int add, const double2* __restrict__ F,
+                      double2* __restrict__ partial, double2* __restrict__ fb) {
+  extern __shared__ double2 sm[];
+  __shared__ double2 red[32];
+  const int b = blockIdx.y, chunk = blockIdx.x, tid = threadIdx.x;
+  const int g0 = chunk * kExgChunk, g1 = min(G, g0 + kExgChunk);
+  const size_t ld = (size_t)G * n;
+  const double2* Fb = F + (size_t)b * n * ld;
+  const int lds = gsub * n, g = tid / n, i = tid - g * n;
+  double2 once = cmk(0.0, 0.0), twice = cmk(0.0, 0.0);
+  for (int gs = g0; gs < g1; gs += gsub) {
+    const int ng = min(gsub, g1 - gs), cols = ng * n;
+    __syncthreads();
+    if (tid < cols) {
+      const double2* src = Fb + (size_t)gs * n + tid;
+#pragma unroll 4
+      for (int j = 0; j < n; ++j) sm[j * lds + tid] = src[(size_t)j * ld];
+    }
+    __syncthreads();
+    if (tid < cols) {
+      const double2* row = sm + (size_t)i * lds + g * n;  // f_{., i} of this thread's vector: element j is f[j][i]
+      double2 x = sm[i * lds + tid];
+      cfma(once, x, x);
+      int j = i;
+      for (int k = 1; 2 * k < n; ++k) {
+        j = j + 1 == n ? 0 : j + 1;
+        cfma(twice, sm[j * lds + tid], row[j]);
+      }
+      if ((n & 1) == 0) {  // both rows of an antipodal pair visit it
+        j = j + 1 == n ? 0 : j + 1;
+        cfma(once, sm[j * lds + tid], row[j]);
+      }
+    }
+    if (tid < ng) {
+      double2 t = cmk(0.0, 0.0);
+      for (int r = 0; r < n; ++r) t = cadd(t, sm[r * lds + tid * n + r]);
+      if (mult == 2) t = cadd(t, t);
+      double2* o = fb + (size_t)b * G + gs + tid;
+      *o = add ? cadd(*o, t) : t;
+    }
+  }
+  once = cadd(once, cadd(twice, twice));
+  once = block_sum2(once, red);
+  if (tid == 0) {
+    if (mult == 2) once = cadd(once, once);
+    double2* o = partial + (size_t)b * nchunks + chunk;
+    *o = add ? cadd(*o, once) : once;
+  }
+}
+
+static size_t exg_chunk(size_t W, size_t n, size_t G) {  // walkers per pass, a multiple of 16 (whole 32-row tiles)
+  size_t wc = (size_t(96) << 20) / (n * n * G * sizeof(double2)) / 16 * 16;
+  if (wc < 16) wc = 16;
+  return std::min(wc, (W + 15) / 16 * 16);
+}
+
+size_t exchange_dg_bytes(const Spins& sp, size_t W, size_t N, size_t G) {
+  const size_t rb = kDgRowBytes((N + 15) / 16);
+  size_t rows = 0, brows = 0, f = 0;
+  for (int q = 0; q < sp.nspin; ++q) {
+    const size_t n = sp.n[q];
+    rows = std::max(rows, (2 * W * n + 31) / 32 * 32);
+    brows = std::max(brows, (G * n + 127) / 128 * 128);
+    f = std::max(f, exg_chunk(W, n, G) * n * n * G * sizeof(double2));
+  }
+  return (rows + brows) * (rb + 2) + f + 6 * 256;
+}
+
+int launch_exchange_dg(const Spins& sp, int W, int N, int G, const double2* green, double2* partial, double2* fb,
+                       const DgScratch& s, cudaStream_t st) {
+  const int nk16 = (N + 15) / 16, nchunks = exchange_dg_chunks(G);
+  const size_t rb = kDgRowBytes(nk16);
+  if (s.bytes < exchange_dg_bytes(sp, W, N, G)) { set_error("exchange: scratch %zu", s.bytes); return TROT_ERR_WORKSPACE_TOO_SMALL; }
+  const int nmax = std::max(sp.n[0], sp.nspin == 2 ? sp.n[1] : 0);
+  const size_t rows = ((size_t)2 * W * nmax + 31) / 32 * 32, brows = ((size_t)G * nmax + 127) / 128 * 128;
+  char* p = reinterpret_cast<char*>(((uintptr_t)s.p + 255) & ~(uintptr_t)255);
+  auto take = [&](size_t n) {
+    char* r = p;
+    p += (n + 255) & ~(size_t)255;
+    return r;
+  };
+  DgArgs a{};
+  uint16_t* imgB = reinterpret_cast<uint16_t*>(take(brows * rb));
+  uint16_t* imgA = reinterpret_cast<uint16_t*>(take(rows * rb));
+  int16_t* exB = reinterpret_cast<int16_t*>(take(brows * 2));
+  int16_t* exA = reinterpret_cast<int16_t*>(take(rows * 2));
+  double2* F = reinterpret_cast<double2*>(p);
+  for (int q = 0; q < sp.nspin; ++q) {
+    const int n = sp.n[q], Gn = G * n;
+    a.nrt = (Gn + 127) / 128;
+    if (q == 0 || sp.rot_chol[q] != sp.rot_chol[0] || n != sp.n[0]) {
+      TROT_TRY(dg_rows_launch(dg_src(sp.rot_chol[q], 0, Gn, N, 128, N, 1, imgB, exB), a.nrt * 16, st));
+    }
+    const int tiles = (2 * W * n + kDgP - 1) / kDgP;
+    DgSrc sa = dg_src(reinterpret_cast<const double*>(green + (size_t)sp.off[q] * N), 1, 2 * n, N, kDgP, 2ll * N, 2, imgA, exA);
+    sa.rpad = 2 * n;
+    sa.nblk = W;
+    sa.bstride = 2ll * sp.ntot * N;
+    TROT_TRY(dg_rows_launch(sa, tiles * 4, st));
+    a.imgB = imgB; a.exB = exB;
+    a.Nn = Gn; a.nk16 = nk16; a.nbatch = 1; a.shift = 1;  // N <= 1024
+    a.C = F; a.ldc = Gn; a.salpha = 1; a.ealpha = 0; a.accumulate = 0; a.status = s.status;
+    const int wc = (int)exg_chunk(W, n, G);
+    const int gsub = kExgThreads / n;  // n <= 64
+    const size_t smem = (size_t)n * n * gsub * sizeof(double2);
+    if (smem > 40 * 1024) cudaFuncSetAttribute(exchange_pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    for (int w0 = 0; w0 < W; w0 += wc) {
+      const int wn = std::min(wc, W - w0);
+      const size_t t0 = (size_t)w0 * 2 * n / kDgP;
+      a.imgA = imgA + t0 * kDgP * (rb / 2);
+      a.exA = exA + t0 * kDgP;
+      a.M = wn * n;
+      a.ntile = (2 * wn * n + kDgP - 1) / kDgP;
+      dg_gemm(a, st);
+      TROT_CHECK_LAUNCH("dg_gemm_kernel");
+      exchange_pairs_kernel<<<dim3(nchunks, wn), kExgThreads, smem, st>>>(n, G, gsub, nchunks, sp.mult[q], q > 0, F,
+                                                                  partial + (size_t)w0 * nchunks, fb + (size_t)w0 * G);
+      TROT_CHECK_LAUNCH("exchange_pairs_kernel");
+    }
   }
   return TROT_OK;
 }
@@ -637,6 +806,6 @@ extern "C" int trot_zgemm_digits(int M, int N, int K, double alpha, const double
   s.p = c.take<char>(s.bytes);
   s.status = c.status();
   if (!c.ok) { set_error("workspace too small: %zu < %zu", ws_bytes, c.used); return TROT_ERR_WORKSPACE_TOO_SMALL; }
-  return launch_zgemm_dg(M, N, K, alpha, dg_rows((const double2*)A, lda), B, ldb, b_is_nk != 0, (double2*)C, ldc,
+  return launch_zgemm_dg(M, N, K, alpha, (const double2*)A, lda, B, ldb, b_is_nk != 0, (double2*)C, ldc,
                          accumulate != 0, s, (cudaStream_t)stream);
 }

@@ -14,18 +14,17 @@ inline bool dg_takes(int K) { return K >= kDgMinK && K <= kDgMaxK; }
 // Bytes that launch_zgemm_dg wants for C (M x Nn) = alpha A (M x K complex) B (K x Nn real).
 size_t dg_scratch_bytes(size_t M, size_t Nn, size_t K);
 
-// A complex rows: row r at A + (r / rpb) bstride + (r % rpb) lda (rpb = 1, bstride = lda: plain row-major).
-struct DgRows {
-  const double2* p;
-  int rpb;
-  long long bstride;
-  int lda;
-};
-inline DgRows dg_rows(const double2* p, int lda) { return DgRows{p, 1, lda, lda}; }
-
 // C[m][n] (+)= alpha sum_k A[m][k] B(k, n) as launch_zgemm_cr, with both operands as six
 // FP16 digit planes per row and 26 exact tensor-core products.
-int launch_zgemm_dg(int M, int Nn, int K, double alpha, DgRows A, const double* B, int ldb, bool b_is_nk, double2* C,
-                    long long ldc, bool accumulate, const DgScratch& s, cudaStream_t st);
+int launch_zgemm_dg(int M, int Nn, int K, double alpha, const double2* A, int lda, const double* B, int ldb,
+                    bool b_is_nk, double2* C, long long ldc, bool accumulate, const DgScratch& s, cudaStream_t st);
+
+
+// Exchange sums and force bias of all walkers from one set of digit products f_g = rot_chol_g G^T (N >= kDgMinK
+// orbitals): partial[b][chunk] as launch_exchange but exchange_dg_chunks(G) of them (fewer), fb[b][g] = sum_s mult_s tr f_sg.
+int exchange_dg_chunks(int G);
+size_t exchange_dg_bytes(const Spins& sp, size_t W, size_t N, size_t G);
+int launch_exchange_dg(const Spins& sp, int W, int N, int G, const double2* green, double2* partial, double2* fb,
+                       const DgScratch& s, cudaStream_t st);
 
 }  // namespace trot

@@ -137,7 +137,7 @@ int launch_zgemm_cr_splitk(int M, int Nn, int K, double alpha, const double2* A,
 int launch_zgemm(int M, int Nn, int K, double alpha, const double2* A, int lda, const double* B, int ldb, bool b_is_nk,
                  double2* C, int ldc, bool accumulate, const DgScratch& dg, cudaStream_t st, double2* part, int S) {
   if (M > 0 && Nn > 0 && dg.p && dg_takes(K) && dg.bytes >= dg_scratch_bytes(M, Nn, K))
-    return launch_zgemm_dg(M, Nn, K, alpha, dg_rows(A, lda), B, ldb, b_is_nk, C, ldc, accumulate, dg, st);
+    return launch_zgemm_dg(M, Nn, K, alpha, A, lda, B, ldb, b_is_nk, C, ldc, accumulate, dg, st);
   return launch_zgemm_cr_splitk(M, Nn, K, alpha, A, lda, B, ldb, b_is_nk, C, ldc, accumulate, part, S, st);
 }
 

@@ -106,6 +106,7 @@ int launch_step_finalize(int W, double* weights, double* scalars, long long* nod
                          const int* status = nullptr);
 
 int exchange_chunks(int G);
+int check_exchange_tile(const Spins& sp, int N);  // TROT_ERR_UNSUPPORTED past the FP64 kernel's shared memory
 int launch_exchange(const Spins& sp, int W, int N, int G, const double2* green, double2* partial,
                     cudaStream_t st);
 // Fixed-point partial sum of the tensor-core exchange kernel: value v[c] 2^-s[c] (c = re, im);

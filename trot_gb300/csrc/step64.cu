@@ -204,14 +204,21 @@ exchange_kernel(Spins sp, int N, int G, const double2* __restrict__ green, doubl
   if (tid == 0) partial[(size_t)b * gridDim.x + chunk] = acc_all;
 }
 
+static size_t exchange_smem(const Spins& sp, int N) {
+  const int nmax = sp.n[0] > sp.n[1] ? sp.n[0] : sp.n[1];
+  return (size_t)(nmax * N + nmax * nmax) * sizeof(double2) + (size_t)nmax * N * sizeof(double);
+}
+
+int check_exchange_tile(const Spins& sp, int N) {
+  if (exchange_smem(sp, N) <= 200 * 1024) return TROT_OK;
+  set_error("exchange: tile of %zu bytes exceeds shared memory", exchange_smem(sp, N));
+  return TROT_ERR_UNSUPPORTED;
+}
+
 int launch_exchange(const Spins& sp, int W, int N, int G, const double2* green, double2* partial,
                     cudaStream_t st) {
-  int nmax = sp.n[0] > sp.n[1] ? sp.n[0] : sp.n[1];
-  size_t smem = (size_t)(nmax * N + nmax * nmax) * sizeof(double2) + (size_t)nmax * N * sizeof(double);
-  if (smem > 200 * 1024) {
-    set_error("exchange: tile of %zu bytes exceeds shared memory", smem);
-    return TROT_ERR_UNSUPPORTED;
-  }
+  const size_t smem = exchange_smem(sp, N);
+  TROT_TRY(check_exchange_tile(sp, N));
   if (smem > 40 * 1024)
     cudaFuncSetAttribute(exchange_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   dim3 grid(exchange_chunks(G), W);

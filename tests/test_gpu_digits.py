@@ -159,3 +159,41 @@ def test_energy_from_digit_products(kind, N, na, nb, G, W):
         outs.append([cpu(x) for x in ws])
     for x, y in zip(*outs):
         assert np.max(np.abs(x - y)) <= 1e-11 * np.max(np.abs(y))
+
+
+@pytest.mark.parametrize("kind,N,na,nb,terms,W", [
+    ("rhf_r", 50, 6, 6, 6, 3), ("rhf_r", 63, 16, 16, 1, 5), ("uhf_u", 64, 5, 12, 6, 2), ("uhf_u", 65, 17, 16, 10, 2),
+    ("rhf_u", 96, 3, 3, 0, 4), ("rhf_r", 128, 1, 1, 6, 7), ("rhf_r", 129, 15, 15, 6, 2), ("rhf_r", 260, 3, 3, 3, 2)])
+def test_trotter_from_digit_products(kind, N, na, nb, terms, W):
+    """Trotter action and one step against the oracle: orbitals at the edges of the 128-row tiles of (re, im) rows and
+    of K runs of 256, columns at the edges of the 32-row tiles, no and many Taylor terms.  FP64 sums over K <= 260
+    terms: 1e-12 of the largest walker element."""
+    from oracle import afqmc_oracle as orc
+
+    G = 30
+    rng = np.random.default_rng(N + na)
+    h0, h1, chol = synthetic.hamiltonian(N, G, 30.0, seed=N)
+    chol = 0.3 * chol
+    mo = np.linalg.qr(rng.standard_normal((N, N)))[0]
+    ma, mb = np.ascontiguousarray(mo[:, :na]), np.ascontiguousarray(mo[:, -nb:] if kind == "uhf_u" else mo[:, :nb])
+    S = Setup(kind, h0, h1, chol, ma, mb, 0.01, W, n_exp_terms=terms)
+    w = synthetic.perturbed_walkers(ma, W, 0.1, 3)
+    if kind != "rhf_r":
+        w = (w, synthetic.perturbed_walkers(mb, W, 0.1, 4))
+    rho = np.stack([ma @ ma.T, mb @ mb.T])
+    ctx = orc.build_prop_ctx(h0, h1, chol, rho, 0.01)
+    xs = rng.standard_normal((W, G)) + 0.3j * rng.standard_normal((W, G))
+    from trot_gb300.prop import make_trotter_ops
+
+    got = make_trotter_ops("restricted", S.walker_kind).apply_trotter(S.walkers(w), dev(xs), S.prop_ctx, terms)
+    ref = orc.apply_trotter_r(w, xs, ctx, terms) if kind == "rhf_r" else orc.apply_trotter_u(*w, xs, ctx, terms)
+    for a, b in zip(*[(x if isinstance(x, tuple) else (x,)) for x in (got, ref)]):
+        assert np.max(np.abs(cpu(a) - b)) <= 1e-12 * np.max(np.abs(b))
+    mctx = orc.build_uhf_meas_ctx(h1, chol, ma, mb) if kind == "uhf_u" else orc.build_rhf_meas_ctx(h1, chol, ma)
+    m = orc.Model(kind, h0, (ma, mb) if kind == "uhf_u" else ma, mctx, ctx)
+    ov = m.overlap(w)
+    x = rng.standard_normal((W, G))
+    o = orc.afqmc_step(orc.State(w, np.ones(W), ov, -1.0, -1.0, 0), m, orc.Params(dt=0.01, n_exp_terms=terms), x)
+    st = S.step(S.state(S.walkers(w), np.ones(W), ov, -1.0, -1.0), dev(x))
+    assert np.max(np.abs(cpu(st.overlaps) - o.overlaps)) <= 1e-10 * np.max(np.abs(o.overlaps))
+    assert np.allclose(cpu(st.weights), o.weights, rtol=1e-9, atol=1e-12)

@@ -59,6 +59,8 @@ static size_t digit_bytes(const trot_system* s, const Spins& sp, int op) {
     n = std::max(n, exchange_dg_bytes(sp, W, N, G));
   if ((op == TROT_OP_APPLY_TROTTER || op == TROT_OP_PROP_STEP) && dg_takes((int)G))
     n = std::max(n, dg_scratch_bytes(W, N * N, G));  // full or packed
+  if ((op == TROT_OP_APPLY_TROTTER || op == TROT_OP_PROP_STEP) && trotter_takes_digits(sp, (int)N))
+    n = std::max(n, trotter_dg_bytes(sp, W, N));
   return n;
 }
 
@@ -347,7 +349,7 @@ int trot_apply_trotter(const trot_system* s, const double* wa, const double* wb,
   TROT_TRY(carve_ws(s, sp, ws, ws_bytes, b, TROT_OP_APPLY_TROTTER));
   TROT_TRY(launch_vhs64(W, N, G, (const double2*)xs, s->chol_flat, s->chol_packed, b.vp, b.vhs, b.dg, st));
   a.vhs = b.vhs;
-  return launch_trotter(sp, a, st);
+  return launch_trotter(sp, a, b.dg, st);
 }
 
 int trot_prop_step(const trot_system* s, const trot_state* state, const double* fields, double* energy_out,
@@ -392,7 +394,7 @@ int trot_prop_step(const trot_system* s, const trot_state* state, const double* 
   a.overlaps = (double2*)state->overlaps; a.weights = state->weights; a.scalars = state->scalars;
   a.shift_term = b.shift_term; a.fb_term = b.fb_term; a.node_flag = b.node_flag;
   a.dt = s->dt; a.h0_prop = s->h0_prop; a.w_floor = s->weight_floor; a.w_cap = s->weight_cap;
-  TROT_TIMED("trotter_fp64", st, launch_trotter(sp, a, st));
+  TROT_TIMED("trotter_fp64", st, launch_trotter(sp, a, b.dg, st));
   // 7. population-control shift, node count
   TROT_TIMED("step_finalize", st, launch_step_finalize(W, state->weights, state->scalars, (long long*)state->node_encounters,
                                                        b.node_flag, s->pop_control_damping, s->dt, st));

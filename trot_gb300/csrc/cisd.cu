@@ -87,7 +87,13 @@ static size_t cisd_digit_bytes(const trot_cisd* c, size_t W, int op) {
   add(W, G, N * (N + 1) / 2);
   if (op == TROT_OP_FORCE_BIAS) return d;
   if (c->l2ci2_precision != TROT_MIXED) add(W * G, nv, nv);  // l2ci2
-  if (op == TROT_OP_PROP_STEP) add(W, N * N, G);             // VHS (FP64 propagation)
+  if (op == TROT_OP_PROP_STEP) {                             // FP64 propagation
+    add(W, N * N, G);
+    Spins sp{};
+    sp.nspin = 1;
+    sp.n[0] = sp.ntot = c->nocc;
+    if (trotter_takes_digits(sp, (int)N)) d = std::max(d, trotter_dg_bytes(sp, W, N));
+  }
   return d;
 }
 
@@ -1041,7 +1047,7 @@ int trot_cisd_prop_step(const trot_cisd* c, const trot_system* prop, const trot_
     TROT_TIMED("vhs_fp64", st,
                launch_zgemm(W, N * N, G, 1.0, b.xs, G, prop->chol_flat, N * N, false, b.vhs, N * N, false, b.dg, st));
     a.vhs = b.vhs;
-    TROT_TIMED("trotter_fp64", st, launch_trotter(sp, a, st));
+    TROT_TIMED("trotter_fp64", st, launch_trotter(sp, a, b.dg, st));
   }
   // 5. CISD overlaps of the new walkers, weights, population shift
   TROT_TRY(cisd_run(c, W, w, b, 0, st));

@@ -22,11 +22,12 @@
 // 14.5 ms on the FP64 pipe; bound by the MMAs' operand reads from shared memory (about 50 cycles per MMA and 0.75 per
 // column and K16 step).  (1024 x 7200, K = 120): 0.123 ms, where the epilogue's conversions take half of the time.
 //
-// One persistent CTA per SM: MMA rows are the columns of B (128 per tile), MMA columns the rows of A in
-// tiles of 32 (16 complex rows: re, im).  A CTA takes NT such tiles against one 128-row tile at a time, so each 24 KB
-// K16 step of the latter serves NT x 26 products from shared memory; per K16 step six (seven in a slab's first)
-// MMAs: digit plane t of B against planes 0..min(5, 6 - t) of A stacked along the MMA's N.  Two TMEM accumulators (7 x 32
-// columns) let the tensor core run the next tile's slab while 16 epilogue warps empty this one.
+// One persistent CTA per SM: MMA rows are the columns of B (128 per tile), MMA columns the rows of A in tiles of 32
+// (16 complex rows: re, im).  Per K16 step six (seven in a slab's first) MMAs: digit plane t of B against planes
+// 0..min(5, 6 - t) of A stacked along the MMA's N.  Two TMEM accumulators (7 x 32 columns) let the tensor core run
+// the next slab while 16 epilogue warps empty this one.  Keeping a 128-row tile in shared memory for two or four 32-row
+// tiles saves loads but not time (VHS 0.460 ms, K = 120 0.117 / 0.125 against 0.442 and 0.112 ms: the outputs of
+// several tiles come in a burst that the two accumulators cannot hide, and small products leave CTAs without work).
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>
 
@@ -34,6 +35,7 @@
 #include <cmath>
 
 #include "digits.h"
+#include "step_tail.cuh"
 #include "tc.cuh"
 
 namespace trot {
@@ -105,6 +107,23 @@ TROT_D void dg_split8(const double* x, int e, uint4* w) {
   for (int t = 0; t < kDgS; ++t) w[t] = make_uint4(h[t][0], h[t][1], h[t][2], h[t][3]);
 }
 
+// the same as stores of the six planes, `plane` entries apart
+TROT_D void dg_store8(const double* x, int e, uint16_t* o, size_t plane) {
+  uint4 w[kDgS];
+  dg_split8(x, e, w);
+#pragma unroll
+  for (int t = 0; t < kDgS; ++t) *reinterpret_cast<uint4*>(o + t * plane) = w[t];
+}
+
+// high word of the largest |x| so far, and sum of |x| as a float from its high word (the range only matters near
+// the row maximum)
+TROT_D void dg_row_max(double x, unsigned& mx, float& s) {
+  const unsigned b = (unsigned)__double2hiint(x) & 0x7FFFFFFFu;
+  mx = b > mx ? b : mx;
+  const unsigned f = b - (896u << 20);
+  s += f < (254u << 20) ? __uint_as_float(f << 3) : 0.f;
+}
+
 // exponent e (max |x| < 2^e) of a row from the high words of its largest |x| and its largest sum of |x| over 32 k
 TROT_D int dg_exponent(unsigned mx, float l1) {
   const int E = (int)(mx >> 20);
@@ -168,11 +187,11 @@ __global__ void __launch_bounds__(256) dg_rows_kernel(DgSrc a) {
       p += blk * a.bstride + rr * a.rst;
     }
   }
-  const int kpad = a.nk16 * 16, kstep = 256 * KS;
+  const int nwarp = (int)blockDim.x >> 5, kpad = a.nk16 * 16, kstep = nwarp * 32 * KS;
   unsigned mx = 0;
   float l1 = 0.f;
   double x[8];
-  for (int k0 = (rank * 8 + warp) * 32; k0 < kpad; k0 += kstep) {
+  for (int k0 = (rank * nwarp + warp) * 32; k0 < kpad; k0 += kstep) {
     float s = 0.f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -180,13 +199,7 @@ __global__ void __launch_bounds__(256) dg_rows_kernel(DgSrc a) {
       x[i] = (valid && k < a.K) ? p[k * kst] : 0.0;
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const unsigned b = (unsigned)__double2hiint(x[i]) & 0x7FFFFFFFu;
-      mx = b > mx ? b : mx;
-      // |x| as a float from its high word (the range only matters near the row maximum)
-      const unsigned f = b - (896u << 20);
-      s += f < (254u << 20) ? __uint_as_float(f << 3) : 0.f;
-    }
+    for (int i = 0; i < 8; ++i) dg_row_max(x[i], mx, s);
     s += __shfl_xor_sync(0xffffffffu, s, 8);
     s += __shfl_xor_sync(0xffffffffu, s, 16);
     l1 = fmaxf(l1, s);
@@ -198,8 +211,7 @@ __global__ void __launch_bounds__(256) dg_rows_kernel(DgSrc a) {
     sl1[warp][lane] = l1;
   }
   __syncthreads();
-#pragma unroll
-  for (int w = 0; w < 8; ++w) {
+  for (int w = 0; w < nwarp; ++w) {
     mx = max(mx, smx[w][rl]);
     l1 = fmaxf(l1, sl1[w][rl]);
   }
@@ -220,7 +232,7 @@ __global__ void __launch_bounds__(256) dg_rows_kernel(DgSrc a) {
   const int r = row % a.R;
   uint16_t* out = a.img + (size_t)(row / a.R) * a.nk16 * kDgS * a.R * 16;
   const bool once = kpad <= kstep;
-  for (int k0 = (rank * 8 + warp) * 32; k0 < kpad; k0 += kstep) {
+  for (int k0 = (rank * nwarp + warp) * 32; k0 < kpad; k0 += kstep) {
     const int kb = k0 + kg * 8;
     if (kb >= kpad) continue;
     if (!once) {
@@ -231,21 +243,20 @@ __global__ void __launch_bounds__(256) dg_rows_kernel(DgSrc a) {
 #pragma unroll
       for (int i = 0; i < 8; ++i) x[i] = 0.0;
     }
-    uint4 w[kDgS];
-    dg_split8(x, live ? e : 0, w);
-    uint16_t* o = out + (size_t)(kb >> 4) * kDgS * a.R * 16 + dg_idx(r, kb & 15);
-#pragma unroll
-    for (int t = 0; t < kDgS; ++t) *reinterpret_cast<uint4*>(o + (size_t)t * a.R * 16) = w[t];
+    dg_store8(x, live ? e : 0, out + (size_t)(kb >> 4) * kDgS * a.R * 16 + dg_idx(r, kb & 15), a.R * 16);
   }
   if (KS > 1) cl.sync();  // the maxima stay readable until every CTA of the cluster has them
 }
+
+// a warp per 32 k, eight at most
+static int dg_row_threads(int nk16) { return 32 * std::min(8, (nk16 + 1) / 2); }
 
 static int dg_rows_launch(const DgSrc& a, int groups, cudaStream_t st) {
   int ks = 1;
   while (ks < 8 && a.nk16 * 16 > 256 * ks && groups * ks < 304) ks *= 2;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(ks, groups);
-  cfg.blockDim = dim3(256);
+  cfg.blockDim = dim3(dg_row_threads(a.nk16));
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -267,7 +278,7 @@ struct DgArgs {
   const uint16_t* imgA;  // MMA columns: rows of A, [tile][nk16][6][32][16]
   const int16_t* exA;
   int Nn, M;             // outputs: n < Nn, complex rows m < M
-  int nrt, ntile, nct;   // 128-row tiles, 32-row tiles, groups of NT 32-row tiles (per batch)
+  int nrt, ntile;        // 128-row tiles and 32-row tiles (per batch)
   int nbatch, bB;        // batches: ntile 32-row tiles each, bB 128-row tiles (0: all share them)
   long long cstride;     // and cstride complex outputs
   int nk16, shift;       // K16 steps; the outputs' integers are in units 2^(eA + eB - 54 + shift)
@@ -277,21 +288,25 @@ struct DgArgs {
   int* status;
 };
 
-// v 2^E rounded to a double, by integer operations (conversions and FP64 additions run on the
+// q 2^(ex - 1075) for results next to or outside the normal range
+__device__ __noinline__ double dg_ldexp(unsigned long long q, unsigned sign, int ex) {
+  const double d = ldexp((double)q, ex - 1075);
+  return sign ? -d : d;
+}
+
+// v 2^E rounded to a double (ties away from zero), by integer operations (conversions and FP64 additions run on the
 // narrow FP64 pipe: two of them per output took longer than the output's 26 products)
 TROT_D double dg_double(long long v, int E) {
-  if (v == 0) return 0.0;
   const unsigned long long a = v < 0 ? 0ull - (unsigned long long)v : (unsigned long long)v;
-  const int lz = __clzll((long long)a);
-  const unsigned long long m = a << lz;  // 2^63 <= m < 2^64
-  unsigned long long q = m >> 11;
-  const unsigned r = (unsigned)m & 0x7FFu;
-  q += (r > 0x400u || (r == 0x400u && (q & 1ull))) ? 1ull : 0ull;  // half to even; 2^53 carries into the exponent
-  const int ex = 1023 + 63 - lz + E;  // of the unrounded value
-  const unsigned long long sign = (unsigned long long)v & 0x8000000000000000ull;
-  if (ex > 0 && ex < 0x7FE) return __longlong_as_double((long long)(((unsigned long long)(ex - 1) << 52) + q + sign));
-  const double d = __longlong_as_double((long long)(((unsigned long long)(1023 + 51) << 52) + q + sign));  // q 1.f form
-  return ldexp(d, ex - 1023 - 52);
+  const unsigned hi = (unsigned)(a >> 32);
+  const int lz = __clz((int)(hi ? hi : (unsigned)a)) + (hi ? 0 : 32);  // 64 for v = 0
+  const unsigned long long m = a << (lz & 63);              // 2^63 <= m < 2^64
+  const unsigned long long q = ((m >> 10) + 1) >> 1;        // 53 bits; 2^53 carries into the exponent
+  const int ex = 1023 + 63 - lz + E;                        // of the unrounded value
+  const unsigned sign = (unsigned)((unsigned long long)v >> 32) & 0x80000000u;
+  double d = __hiloint2double((int)(((unsigned)(ex - 1) << 20) + (unsigned)(q >> 32) + sign), (int)(unsigned)q);
+  if (ex <= 0 || ex >= 0x7FE) d = dg_ldexp(q, sign, ex);
+  return v == 0 ? 0.0 : d;
 }
 
 // out of line, so that its FP64 instructions are not issued (predicated off) for plain stores
@@ -299,7 +314,7 @@ __device__ __noinline__ void dg_add(double2* o, double2 v) { *o = cadd(*o, v); }
 
 // PAIR: the 128-row tiles hold complex rows (row 2 p = real, 2 p + 1 = imaginary part of V[p]) and the product is the
 // complex V T: C[m][p] = V_p . A_m.  Lanes 2 p and 2 p + 1 exchange the cross terms; each stores its part.
-template <int NT, bool PAIR>
+template <bool PAIR>
 __global__ void __launch_bounds__(kDgThreads, 1) dg_gemm_kernel(DgArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   unsigned char* base = smem_raw + ((128 - (tc::smem_u32(smem_raw) & 127)) & 127);
@@ -317,7 +332,7 @@ __global__ void __launch_bounds__(kDgThreads, 1) dg_gemm_kernel(DgArgs a) {
   volatile int* abort_flag = reinterpret_cast<volatile int*>(drain + 2);
   static_assert((2 * kDgASlots + 2 * kDgBSlots + 4 + 3) * 8 <= 256, "barrier table");
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n_items = a.nrt * a.nct * a.nbatch, nk = a.nk16;
+  const int n_items = a.nrt * a.ntile * a.nbatch, nk = a.nk16;
   const int nslab = (nk + kDgSlab - 1) / kDgSlab;
   if (warp == 16) tc::tmem_alloc(tslot, 512);
   if (tid == kDgEpi) {
@@ -341,52 +356,45 @@ __global__ void __launch_bounds__(kDgThreads, 1) dg_gemm_kernel(DgArgs a) {
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t taddr = *tslot;
-  // item -> (128-row tile, group of NT 32-row tiles)
+  // item -> (batch, 32-row tile, 128-row tile), the last fastest
   if (warp == 16) {
     if (lane == 0) {
       bool ok = true;
       const uint64_t ad0 = tc::smem_desc(tc::smem_u32(sA), 128, 256);
       const uint64_t bd0 = tc::smem_desc(tc::smem_u32(sB), 128, 256);
       const uint32_t adlo = (uint32_t)ad0, bdlo = (uint32_t)bd0, dhi = (uint32_t)(ad0 >> 32);
-      int ca = 0, cb = 0, cacc = 0;  // chunk, slab-tile and accumulator counters of this CTA
+      int ca = 0, cs = 0;  // K16 step and slab counters of this CTA
       for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-        const int ntv = min(NT, a.ntile - ((item / a.nrt) % a.nct) * NT);
-        for (int s = 0; s < nslab && ok; ++s) {
-          const int ks = min(kDgSlab, nk - s * kDgSlab);
-          for (int j = 0; j < ntv && ok; ++j, ++cb, ++cacc) {
-            const int buf = cacc & 1;
-            if (cacc >= 2) ok = tc::mbar_wait(&acc_empty[buf], (uint32_t)(((cacc >> 1) - 1) & 1));
-            if (ok) ok = tc::mbar_wait(&b_full[cb % kDgBSlots], (uint32_t)((cb / kDgBSlots) & 1));
+        for (int s = 0; s < nslab && ok; ++s, ++cs) {
+          const int ks = min(kDgSlab, nk - s * kDgSlab), buf = cs & 1, bs = cs % kDgBSlots;
+          if (cs >= 2) ok = tc::mbar_wait(&acc_empty[buf], (uint32_t)(((cs >> 1) - 1) & 1));
+          if (ok) ok = tc::mbar_wait(&b_full[bs], (uint32_t)((cs / kDgBSlots) & 1));
+          if (!ok) break;
+          const uint32_t dcol = taddr + (uint32_t)(buf * 256);
+          for (int k = 0; k < ks; ++k, ++ca) {
+            const int slot = ca % kDgASlots;
+            ok = tc::mbar_wait(&a_full[slot], (uint32_t)((ca / kDgASlots) & 1));
             if (!ok) break;
-            const uint32_t dcol = taddr + (uint32_t)(buf * 256);
-            for (int k = 0; k < ks; ++k) {
-              const int slot = (ca + k) % kDgASlots;
-              if (j == 0) {
-                ok = tc::mbar_wait(&a_full[slot], (uint32_t)(((ca + k) / kDgASlots) & 1));
-                if (!ok) break;
-              }
-              tc::fence_after_sync();
-              const uint32_t alo = adlo + (uint32_t)((slot * kDgAStep) >> 4);
-              const uint32_t blo = bdlo + (uint32_t)(((cb % kDgBSlots) * kDgSlab * kDgBStep + k * kDgBStep) >> 4);
+            tc::fence_after_sync();
+            const uint32_t alo = adlo + (uint32_t)((slot * kDgAStep) >> 4);
+            const uint32_t blo = bdlo + (uint32_t)((bs * kDgSlab * kDgBStep + k * kDgBStep) >> 4);
 #pragma unroll
-              for (int t = 0; t < kDgS; ++t) {
-                const int np = t < 1 ? kDgS : kDgGroups - t;  // planes 0 .. np - 1
-                if (t == 1 && k == 0) {  // order 6 starts here: its columns are overwritten
-                  tc::mma_bf16_lo(dcol + 32, alo + 256, blo, dhi, tc::idesc_f16_f32(128, 160), 1u);
-                  tc::mma_bf16_lo(dcol + 192, alo + 256, blo + (5 * kDgP * 32) / 16, dhi, tc::idesc_f16_f32(128, 32), 0u);
-                } else {
-                  tc::mma_bf16_lo(dcol + (uint32_t)(t * kDgP), alo + (uint32_t)(t * 256), blo, dhi,
-                                  tc::idesc_f16_f32(128, np * kDgP), (k > 0 || t > 0) ? 1u : 0u);
-                }
+            for (int t = 0; t < kDgS; ++t) {
+              const int np = t < 1 ? kDgS : kDgGroups - t;  // planes 0 .. np - 1
+              if (t == 1 && k == 0) {  // order 6 starts here: its columns are overwritten
+                tc::mma_bf16_lo(dcol + 32, alo + 256, blo, dhi, tc::idesc_f16_f32(128, 160), 1u);
+                tc::mma_bf16_lo(dcol + 192, alo + 256, blo + (5 * kDgP * 32) / 16, dhi, tc::idesc_f16_f32(128, 32), 0u);
+              } else {
+                tc::mma_bf16_lo(dcol + (uint32_t)(t * kDgP), alo + (uint32_t)(t * 256), blo, dhi,
+                                tc::idesc_f16_f32(128, np * kDgP), (k > 0 || t > 0) ? 1u : 0u);
               }
-              if (j == ntv - 1) tc::mma_commit(&a_free[slot]);
             }
-            if (ok) {
-              tc::mma_commit(&b_free[cb % kDgBSlots]);
-              tc::mma_commit(&acc_full[buf]);
-            }
+            tc::mma_commit(&a_free[slot]);
           }
-          ca += ks;
+          if (ok) {
+            tc::mma_commit(&b_free[bs]);
+            tc::mma_commit(&acc_full[buf]);
+          }
         }
       }
       if (!ok) {
@@ -408,12 +416,11 @@ __global__ void __launch_bounds__(kDgThreads, 1) dg_gemm_kernel(DgArgs a) {
       bool ok = true;
       int c = 0;
       for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-        const int bt = item / (a.nrt * a.nct);
-        const int rt = item % a.nrt + bt * a.bB, ct = (item / a.nrt) % a.nct;
-        const int ntv = min(NT, a.ntile - ct * NT);
+        const int bt = item / (a.nrt * a.ntile);
+        const int rt = item % a.nrt + bt * a.bB, tile = (item / a.nrt) % a.ntile + bt * a.ntile;
         for (int s = 0; s < nslab && ok; ++s) {
           const int ks = min(kDgSlab, nk - s * kDgSlab);
-          const int nc = la ? ks : ntv;
+          const int nc = la ? ks : 1;
           for (int j = 0; j < nc; ++j, ++c) {
             const int slot = c % slots;
             if (c >= slots) {  // the MMAs that read the slot's previous contents are done
@@ -433,7 +440,7 @@ __global__ void __launch_bounds__(kDgThreads, 1) dg_gemm_kernel(DgArgs a) {
             } else {
               tc::mbar_expect_tx(&full[slot], ks * kDgBStep);
               tc::bulk_g2s(sB + (size_t)slot * kDgSlab * kDgBStep,
-                           a.imgA + ((size_t)(bt * a.ntile + ct * NT + j) * nk + s * kDgSlab) * (kDgBStep / 2), ks * kDgBStep,
+                           a.imgA + ((size_t)tile * nk + s * kDgSlab) * (kDgBStep / 2), ks * kDgBStep,
                            &full[slot]);
             }
           }
@@ -453,96 +460,78 @@ __global__ void __launch_bounds__(kDgThreads, 1) dg_gemm_kernel(DgArgs a) {
     // digit weights in the accumulator's units (sh >= 1, so that the largest stays an int32)
     const int m0 = 1 << (31 - sh), m1 = 1 << (27 - sh), m2 = 1 << (18 - sh), m3 = 1 << (9 - sh);
     const float lscale = __int_as_float((127 - sh) << 23);
-    int cacc = 0;
+    int cs = 0;
     bool ok = true;
     for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-      const int rt = item % a.nrt, ct = (item / a.nrt) % a.nct, bt = item / (a.nrt * a.nct);
-      const int ntv = min(NT, a.ntile - ct * NT);
+      const int rt = item % a.nrt, ct = (item / a.nrt) % a.ntile, bt = item / (a.nrt * a.ntile);
       const int n = rt * 128 + q * 32 + lane;
-      long long acc[NT][8];
+      // exponents of this column and of the warp's eight rows (int16), loaded before the first wait
+      int eb = n < a.Nn ? a.exB[(size_t)bt * a.bB * 128 + n] : 0;
+      const uint4 ea = __ldg(reinterpret_cast<const uint4*>(a.exA + (size_t)(bt * a.ntile + ct) * kDgP + h * 8));
+      long long acc[8];
 #pragma unroll
-      for (int j = 0; j < NT; ++j)
+      for (int x = 0; x < 8; ++x) acc[x] = 0;
+      for (int s = 0; s < nslab; ++s, ++cs) {
+        const int buf = cs & 1;
+        if (ok && (!tc::mbar_wait(&acc_full[buf], (uint32_t)((cs >> 1) & 1)) || *abort_flag)) {
+          if (!*abort_flag && a.status && lane == 0) report_timeout(a.status);
+          ok = false;
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) continue;
+        tc::fence_after_sync();
+        uint32_t raw[kDgGroups][8];
 #pragma unroll
-        for (int x = 0; x < 8; ++x) acc[j][x] = 0;
-      for (int s = 0; s < nslab; ++s) {
+        for (int d = 0; d < kDgGroups; ++d) tc::tmem_ld8_raw(tl + (uint32_t)(buf * 256 + d * kDgP), raw[d]);
+        tc::tmem_wait_ld();
+        tc::fence_before_sync();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&acc_empty[buf]);
 #pragma unroll
-        for (int j = 0; j < NT; ++j) {
-          if (j >= ntv) break;
-          const int buf = cacc & 1;
-          if (ok && (!tc::mbar_wait(&acc_full[buf], (uint32_t)((cacc >> 1) & 1)) || *abort_flag)) {
-            if (!*abort_flag && a.status && lane == 0) report_timeout(a.status);
-            ok = false;
+        for (int x = 0; x < 8; ++x) {
+          float f[kDgGroups];
+#pragma unroll
+          for (int d = 0; d < kDgGroups; ++d) {
+            uint32_t v = raw[d][x];
+            asm volatile("" : "+r"(v));  // consume after tcgen05.wait::ld
+            f[d] = __uint_as_float(v);
           }
-          ++cacc;
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) continue;
-          tc::fence_after_sync();
-#pragma unroll
-          for (int c4 = 0; c4 < 8; c4 += 2) {
-            uint32_t raw[kDgGroups][2];
-#pragma unroll
-            for (int d = 0; d < kDgGroups; ++d) tc::tmem_ld2(tl + (uint32_t)(buf * 256 + d * kDgP + c4), raw[d][0], raw[d][1]);
-            tc::tmem_wait_ld();
-            if (c4 == 6) {
-              tc::fence_before_sync();
-              __syncwarp();
-              if (lane == 0) tc::mbar_arrive(&acc_empty[buf]);
-            }
-#pragma unroll
-            for (int x = 0; x < 2; ++x) {
-              float f[kDgGroups];
-#pragma unroll
-              for (int d = 0; d < kDgGroups; ++d) {
-                uint32_t v = raw[d][x];
-                asm volatile("" : "+r"(v));  // consume after tcgen05.wait::ld
-                f[d] = __uint_as_float(v);
-              }
-              // sum_d S_d 2^(-9 d) in units 2^(sh - 36): orders 0-3 exactly, the rest rounded once
-              const float f4 = fmaf(fmaf(f[6], 1.953125e-03f, f[5]), 1.953125e-03f, f[4]) * lscale;
-              long long v = acc[j][c4 + x];
-              v += (long long)(__float2int_rn(f[0]) << 5) * m0;
-              v += (long long)__float2int_rn(f[1]) * m1;
-              v += (long long)__float2int_rn(f[2]) * m2;
-              v += (long long)__float2int_rn(f[3]) * m3;
-              v += (long long)__float2int_rn(f4);
-              acc[j][c4 + x] = v;
-            }
-          }
+          // sum_d S_d 2^(-9 d) in units 2^(sh - 36): orders 0-3 exactly, the rest rounded once
+          const float f4 = fmaf(fmaf(f[6], 1.953125e-03f, f[5]), 1.953125e-03f, f[4]) * lscale;
+          long long v = acc[x];
+          v += (long long)(__float2int_rn(f[0]) << 5) * m0;
+          v += (long long)__float2int_rn(f[1]) * m1;
+          v += (long long)__float2int_rn(f[2]) * m2;
+          v += (long long)__float2int_rn(f[3]) * m3;
+          v += (long long)__float2int_rn(f4);
+          acc[x] = v;
         }
       }
       // outputs: lane = column n of C, register pairs = (re, im) of four complex rows
-      int eb = n < a.Nn ? a.exB[bt * a.bB * 128 + n] : 0;
       if (!ok) eb = kDgNonFinite;
       const bool bad = eb == kDgNonFinite;
       eb += sh - kDgBits + a.ealpha;
-      uint4 ea[NT];  // the rows' exponents, eight int16
+      const int m0r = ct * (kDgP / 2) + h * 4;
+      double2* o = a.C + bt * a.cstride + (long long)m0r * a.ldc + (PAIR ? n >> 1 : n);
+      const uint32_t ew[4] = {ea.x, ea.y, ea.z, ea.w};
 #pragma unroll
-      for (int j = 0; j < NT; ++j)
-        ea[j] = j < ntv ? __ldg(reinterpret_cast<const uint4*>(a.exA + (size_t)(bt * a.ntile + ct * NT + j) * kDgP + h * 8)) : make_uint4(0, 0, 0, 0);
-#pragma unroll
-      for (int j = 0; j < NT; ++j) {
-        if (j >= ntv) break;
-        const int m0r = (ct * NT + j) * (kDgP / 2) + h * 4;
-        double2* o = a.C + bt * a.cstride + (long long)m0r * a.ldc + (PAIR ? n >> 1 : n);
-        const uint32_t ew[4] = {ea[j].x, ea[j].y, ea[j].z, ea[j].w};
-#pragma unroll
-        for (int y = 0; y < 4; ++y, o += a.ldc) {
-          const int e0 = (int)(int16_t)(ew[y] & 0xFFFFu), e1 = (int)(int16_t)(ew[y] >> 16);
-          const double nan = __longlong_as_double(0x7FF8000000000000ll);
-          double2 v = cmk(dg_double(acc[j][2 * y] * a.salpha, e0 + eb), dg_double(acc[j][2 * y + 1] * a.salpha, e1 + eb));
-          if (bad || e0 == kDgNonFinite) v.x = nan;
-          if (bad || e1 == kDgNonFinite) v.y = nan;
-          if (PAIR) {
-            const double w = __shfl_xor_sync(0xffffffffu, v.y, 1);
-            if (m0r + y < a.M && n < a.Nn) {
-              double* od = reinterpret_cast<double*>(o);
-              if (n & 1) od[1] = v.x + w;
-              else od[0] = v.x - w;
-            }
-          } else if (m0r + y < a.M && n < a.Nn) {
-            if (a.accumulate) dg_add(o, v);
-            else *o = v;
+      for (int y = 0; y < 4; ++y, o += a.ldc) {
+        const int e0 = (int)(int16_t)(ew[y] & 0xFFFFu), e1 = (int)(int16_t)(ew[y] >> 16);
+        const double nan = __longlong_as_double(0x7FF8000000000000ll);
+        double2 v = cmk(dg_double(a.salpha < 0 ? -acc[2 * y] : acc[2 * y], e0 + eb),
+                        dg_double(a.salpha < 0 ? -acc[2 * y + 1] : acc[2 * y + 1], e1 + eb));
+        if (bad || e0 == kDgNonFinite) v.x = nan;
+        if (bad || e1 == kDgNonFinite) v.y = nan;
+        if (PAIR) {
+          const double w = __shfl_xor_sync(0xffffffffu, v.y, 1);
+          if (m0r + y < a.M && n < a.Nn) {
+            double* od = reinterpret_cast<double*>(o);
+            if (n & 1) od[1] = v.x + w;
+            else od[0] = v.x - w;
           }
+        } else if (m0r + y < a.M && n < a.Nn) {
+          if (a.accumulate) dg_add(o, v);
+          else *o = v;
         }
       }
     }
@@ -569,35 +558,13 @@ size_t dg_scratch_bytes(size_t M, size_t Nn, size_t K) {
   return nb * kDgRowBytes(nk16) + 2 * mc * kDgRowBytes(nk16) + nb * 2 + 2 * mc * 2 + 5 * 256;
 }
 
-template <int NT, bool PAIR>
-static void dg_launch(DgArgs a, cudaStream_t st) {
-  a.nct = (a.ntile + NT - 1) / NT;
-  cudaFuncSetAttribute(dg_gemm_kernel<NT, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgSmem);
-  const int items = a.nrt * a.nct * a.nbatch;
-  dg_gemm_kernel<NT, PAIR><<<items < 152 ? items : 152, kDgThreads, kDgSmem, st>>>(a);
-}
-
-// Tiles per CTA pass: the fewest rounds of the 152 CTAs, counted in 32-row tiles; NT = 4 reads the 128-row tile
-// least often, so it wins ties.
-static int dg_pick_nt(int nrt, int ntile, int nbatch) {
-  int best = 4;
-  long long cost = -1;
-  for (int nt = 4; nt >= 1; nt >>= 1) {
-    const long long items = (long long)nrt * ((ntile + nt - 1) / nt) * nbatch;
-    const long long c = (items + 151) / 152 * nt;
-    if (cost < 0 || c < cost) {
-      cost = c;
-      best = nt;
-    }
-  }
-  return best;
-}
-
-static void dg_gemm(const DgArgs& a, cudaStream_t st) {
-  const int nt = dg_pick_nt(a.nrt, a.ntile, a.nbatch);
-  if (nt == 4) dg_launch<4, false>(a, st);
-  else if (nt == 2) dg_launch<2, false>(a, st);
-  else dg_launch<1, false>(a, st);
+template <bool PAIR>
+static int dg_gemm(const DgArgs& a, cudaStream_t st) {
+  cudaFuncSetAttribute(dg_gemm_kernel<PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgSmem);
+  const int items = a.nrt * a.ntile * a.nbatch;
+  dg_gemm_kernel<PAIR><<<items < 152 ? items : 152, kDgThreads, kDgSmem, st>>>(a);
+  TROT_CHECK_LAUNCH("dg_gemm_kernel");
+  return TROT_OK;
 }
 
 int launch_zgemm_dg(int M, int Nn, int K, double alpha, const double2* A, int lda, const double* B, int ldb,
@@ -640,8 +607,7 @@ int launch_zgemm_dg(int M, int Nn, int K, double alpha, const double2* A, int ld
                                    2, imgA, exA), a.ntile * 4, st));
     a.M = mm;
     a.C = C + (long long)m0 * ldc;
-    dg_gemm(a, st);
-    TROT_CHECK_LAUNCH("dg_gemm_kernel");
+    TROT_TRY(dg_gemm<false>(a, st));
   }
   return TROT_OK;
 }
@@ -775,13 +741,203 @@ int launch_exchange_dg(const Spins& sp, int W, int N, int G, const double2* gree
       a.exA = exA + t0 * kDgP;
       a.M = wn * n;
       a.ntile = (2 * wn * n + kDgP - 1) / kDgP;
-      dg_gemm(a, st);
-      TROT_CHECK_LAUNCH("dg_gemm_kernel");
+      TROT_TRY(dg_gemm<false>(a, st));
       exchange_pairs_kernel<<<dim3(nchunks, wn), kExgThreads, smem, st>>>(n, G, gsub, nchunks, sp.mult[q], q > 0, F,
                                                                   partial + (size_t)w0 * nchunks, fb + (size_t)w0 * G);
       TROT_CHECK_LAUNCH("exchange_pairs_kernel");
     }
   }
+  return TROT_OK;
+}
+
+// ------------------------------------------------------------------ Trotter propagation
+// w' = E sum_k ((i sqrt(dt))^k / k!) V^k E w of every walker (trot/prop/chol_afqmc_ops.py:198-222,
+// trot/prop/utils.py:20-30) as a chain of batched digit products: per walker V (2 N rows, re / im interleaved) against
+// the 2 nc columns (j, re / im) of U_k = V^k E w, U_{k+1}[j][p] = sum_q V[p][q] U_k[j][q] (PAIR).  Between two products
+// dg_taylor_kernel adds the term to the sum O and rewrites U_k as digits.  U and O are kept transposed (walker, j, p), so
+// that the products' rows are contiguous.  Bound by the products (0.11 ms per term at 120 orbitals, 22 columns, 1024
+// walkers, with the digit image of V, 0.4 GB, streaming from HBM at half its rate).
+struct DgTaylor {
+  int W, N, nc, rpad;       // rpad: 32-row-tile rows per walker
+  int k, last;              // term k of the sum; last: the digits are those of O (the operand of the final E)
+  double coef;              // sqrt(dt)^k / k!
+  const double* U;          // (W, nc, N) complex
+  double* O;                // (W, nc, N) complex
+  uint16_t* img;
+  int16_t* ex;
+};
+
+// rows r = 2 j + c of a walker as in dg_rows_kernel; each thread also updates component c of O[j][k]
+__global__ void __launch_bounds__(256) dg_taylor_kernel(DgTaylor a) {
+  __shared__ unsigned smx[8][8];
+  __shared__ float sl1[8][8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int rl = lane & 7, kg = lane >> 3;
+  const int row = blockIdx.x * 8 + rl;
+  const int b = row / a.rpad, r = row - b * a.rpad, c = r & 1;
+  const bool valid = (r >> 1) < a.nc;
+  const size_t base = valid ? 2 * ((size_t)(b * a.nc + (r >> 1)) * a.N) + c : 0;
+  const int nk16 = (a.N + 15) / 16, kpad = nk16 * 16, nwarp = (int)blockDim.x >> 5, kstep = nwarp * 32;
+  // i^k = 1, i, -1, -i: component c of i^k U is +- component c ^ (k & 1) of U
+  const int flip = (a.k & 1) ? 1 - 2 * c : 0;  // offset of the other component
+  const int q = a.k & 3;
+  const double cf = (q == 2 || (q == 1 && c == 0) || (q == 3 && c == 1)) ? -a.coef : a.coef;
+  unsigned mx = 0;
+  float l1 = 0.f;
+  double x[8];
+  for (int k0 = warp * 32; k0 < kpad; k0 += kstep) {
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int k = k0 + kg * 8 + i;
+      x[i] = 0.0;
+      if (valid && k < a.N) {
+        const size_t e = base + 2 * (size_t)k;
+        const double u = a.U[e];
+        double o = a.U[e + flip];
+        o = a.k == 0 ? o : fma(cf, o, a.O[e]);
+        a.O[e] = o;
+        x[i] = a.last ? o : u;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) dg_row_max(x[i], mx, s);
+    s += __shfl_xor_sync(0xffffffffu, s, 8);
+    s += __shfl_xor_sync(0xffffffffu, s, 16);
+    l1 = fmaxf(l1, s);
+  }
+#pragma unroll
+  for (int o = 8; o < 32; o <<= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if (lane < 8) {
+    smx[warp][lane] = mx;
+    sl1[warp][lane] = l1;
+  }
+  __syncthreads();
+  for (int w = 0; w < nwarp; ++w) {
+    mx = max(mx, smx[w][rl]);
+    l1 = fmaxf(l1, sl1[w][rl]);
+  }
+  const int e = dg_exponent(mx, l1);
+  if (warp == 0 && lane < 8) a.ex[row] = (int16_t)e;
+  const bool live = valid && e != kDgNonFinite;
+  uint16_t* out = a.img + (size_t)(row / kDgP) * nk16 * kDgS * kDgP * 16;
+  const double* src = a.last ? a.O : a.U;
+  for (int k0 = warp * 32; k0 < kpad; k0 += kstep) {
+    const int kb = k0 + kg * 8;
+    if (kb >= kpad) continue;
+    if (kpad > kstep) {  // more than one run per thread: read again
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] = (live && kb + i < a.N) ? src[base + 2 * (size_t)(kb + i)] : 0.0;
+    }
+    if (!live) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] = 0.0;
+    }
+    dg_store8(x, live ? e : 0, out + (size_t)(kb >> 4) * kDgS * kDgP * 16 + dg_idx(row % kDgP, kb & 15), kDgP * 16);
+  }
+}
+
+// propagated walkers from the transposed w'[j][p]; in step mode their overlap and weight
+__global__ void __launch_bounds__(256) dg_trotter_tail_kernel(Spins sp, TrotterArgs a, const double2* __restrict__ wt) {
+  extern __shared__ double2 smem[];
+  __shared__ double2 red[32];
+  __shared__ int piv;
+  const int b = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
+  const int N = a.N, nc = sp.ntot;
+  double2* W2 = smem;           // N x nc
+  double2* Ms = W2 + N * nc;    // n x n
+  const double2* src = wt + (size_t)b * nc * N;
+  for (int e = tid; e < N * nc; e += nt) W2[(e % N) * nc + e / N] = src[e];
+  __syncthreads();
+  for (int s = 0; s < sp.nspin; ++s) {
+    const int n = sp.n[s];
+    double2* w = (s == 0 ? a.out_a : a.out_b) + (size_t)b * N * n;
+    for (int e = tid; e < N * n; e += nt) w[e] = W2[(e / n) * nc + sp.off[s] + e % n];
+  }
+  if (a.overlaps == nullptr) return;
+  overlap_and_weight(sp, a, N, nc, W2, Ms, &piv, red);
+}
+
+struct DgTrotterPlan {
+  int nk16, vtiles, tiles, rpad;  // K16 steps; 128-row tiles of V, 32-row tiles and rows of U per walker
+  size_t rb, bytes;
+};
+static DgTrotterPlan dg_trotter_plan(const Spins& sp, size_t W, size_t N) {
+  DgTrotterPlan p{};
+  p.nk16 = (int)((N + 15) / 16);
+  p.vtiles = (int)((2 * N + 127) / 128);
+  p.tiles = (2 * sp.ntot + kDgP - 1) / kDgP;
+  p.rpad = p.tiles * kDgP;
+  p.rb = kDgRowBytes(p.nk16);
+  const size_t erows = (N + 127) / 128 * 128;
+  p.bytes = (W * p.vtiles * 128 + W * p.rpad + erows) * (p.rb + 2) + 2 * W * sp.ntot * N * sizeof(double2) + 10 * 256;
+  return p;
+}
+
+size_t trotter_dg_bytes(const Spins& sp, size_t W, size_t N) { return dg_trotter_plan(sp, W, N).bytes; }
+
+int launch_trotter_dg(const Spins& sp, const TrotterArgs& t, const DgScratch& s, cudaStream_t st) {
+  const int W = t.W, N = t.N, nc = sp.ntot;
+  const DgTrotterPlan pl = dg_trotter_plan(sp, W, N);
+  if (s.bytes < pl.bytes) { set_error("trotter: scratch %zu < %zu", s.bytes, pl.bytes); return TROT_ERR_WORKSPACE_TOO_SMALL; }
+  char* p = reinterpret_cast<char*>(((uintptr_t)s.p + 255) & ~(uintptr_t)255);
+  auto take = [&](size_t n) {
+    char* r = p;
+    p += (n + 255) & ~(size_t)255;
+    return r;
+  };
+  const size_t vrows = (size_t)W * pl.vtiles * 128, urows = (size_t)W * pl.rpad, erows = (size_t)(N + 127) / 128 * 128;
+  uint16_t* vimg = reinterpret_cast<uint16_t*>(take(vrows * pl.rb));
+  uint16_t* uimg = reinterpret_cast<uint16_t*>(take(urows * pl.rb));
+  uint16_t* eimg = reinterpret_cast<uint16_t*>(take(erows * pl.rb));
+  int16_t* vex = reinterpret_cast<int16_t*>(take(vrows * 2));
+  int16_t* uex = reinterpret_cast<int16_t*>(take(urows * 2));
+  int16_t* eex = reinterpret_cast<int16_t*>(take(erows * 2));
+  double2* U = reinterpret_cast<double2*>(take((size_t)W * nc * N * sizeof(double2)));
+  double2* O = reinterpret_cast<double2*>(take((size_t)W * nc * N * sizeof(double2)));
+  // digits of V (walker, 2 p + c), of E and of the walkers (walker, 2 j + c; K along the orbitals)
+  DgSrc sv = dg_src(reinterpret_cast<const double*>(t.vhs), 1, 2 * N, N, 128, 2ll * N, 2, vimg, vex);
+  sv.rpad = pl.vtiles * 128;
+  sv.nblk = W;
+  sv.bstride = 2ll * N * N;
+  if (t.nterms > 0) TROT_TRY(dg_rows_launch(sv, W * pl.vtiles * 16, st));
+  TROT_TRY(dg_rows_launch(dg_src(t.expH, 0, N, N, 128, N, 1, eimg, eex), (int)erows / 8, st));
+  DgSrc sw = dg_src(reinterpret_cast<const double*>(t.in_a), 1, 2 * nc, N, kDgP, 2, 2ll * sp.n[0], uimg, uex);
+  sw.rpad = pl.rpad;
+  sw.nblk = W;
+  sw.bstride = 2ll * N * sp.n[0];
+  if (sp.nspin == 2) {
+    sw.split = 2 * sp.n[0];
+    sw.p2 = reinterpret_cast<const double*>(t.in_b);
+    sw.bstride2 = 2ll * N * sp.n[1];
+    sw.kst2 = 2ll * sp.n[1];
+  }
+  TROT_TRY(dg_rows_launch(sw, W * pl.tiles * 4, st));
+  DgArgs e{};  // E x
+  e.imgB = eimg; e.exB = eex; e.imgA = uimg; e.exA = uex;
+  e.Nn = N; e.M = nc; e.nrt = (N + 127) / 128; e.ntile = pl.tiles; e.nk16 = pl.nk16; e.shift = 1;
+  e.nbatch = W; e.bB = 0; e.cstride = (long long)nc * N;
+  e.C = U; e.ldc = N; e.salpha = 1; e.status = s.status;
+  DgArgs v = e;  // V x
+  v.imgB = vimg; v.exB = vex; v.Nn = 2 * N; v.nrt = v.bB = pl.vtiles;
+  TROT_TRY(dg_gemm<false>(e, st));
+  DgTaylor ty{W, N, nc, pl.rpad, 0, t.nterms == 0, 1.0, (const double*)U, (double*)O, uimg, uex};
+  for (int k = 0;; ++k) {
+    ty.k = k;
+    ty.last = k == t.nterms;
+    dg_taylor_kernel<<<W * pl.tiles * 4, dg_row_threads(pl.nk16), 0, st>>>(ty);
+    TROT_CHECK_LAUNCH("dg_taylor_kernel");
+    if (k == t.nterms) break;
+    TROT_TRY(dg_gemm<true>(v, st));
+    ty.coef *= t.sqrt_dt / (double)(k + 1);
+  }
+  TROT_TRY(dg_gemm<false>(e, st));
+  const int nmax = std::max(sp.n[0], sp.nspin == 2 ? sp.n[1] : 0);
+  const size_t smem = (size_t)(N * nc + nmax * nmax) * sizeof(double2);
+  if (smem > 40 * 1024)
+    cudaFuncSetAttribute(dg_trotter_tail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  dg_trotter_tail_kernel<<<W, 256, smem, st>>>(sp, t, U);
+  TROT_CHECK_LAUNCH("dg_trotter_tail_kernel");
   return TROT_OK;
 }
 

@@ -27,4 +27,8 @@ size_t exchange_dg_bytes(const Spins& sp, size_t W, size_t N, size_t G);
 int launch_exchange_dg(const Spins& sp, int W, int N, int G, const double2* green, double2* partial, double2* fb,
                        const DgScratch& s, cudaStream_t st);
 
+// Trotter propagation (with overlaps and weights in step mode) by digit products; same results as launch_trotter.
+size_t trotter_dg_bytes(const Spins& sp, size_t W, size_t N);
+int launch_trotter_dg(const Spins& sp, const TrotterArgs& a, const DgScratch& s, cudaStream_t st);
+
 }  // namespace trot

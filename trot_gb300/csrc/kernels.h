@@ -97,7 +97,9 @@ struct TrotterArgs {
   int* node_flag;
   double dt, h0_prop, w_floor, w_cap;
 };
-int launch_trotter(const Spins& sp, const TrotterArgs& a, cudaStream_t st);
+// by digit products where `dg` holds their scratch and trotter_takes_digits, else on the FP64 pipe
+bool trotter_takes_digits(const Spins& sp, int N);
+int launch_trotter(const Spins& sp, const TrotterArgs& a, const DgScratch& dg, cudaStream_t st);
 // status (optional): the mixed-precision status words of the step (int[4], see
 // report_timeout); when status[0] is set the step's weights and population shift
 // become NaN instead of numbers computed from skipped tensor-core results

@@ -1,4 +1,5 @@
 // FP64 kernels of the phaseless step and the local energy.
+#include "digits.h"
 #include "kernels.h"
 #include "step_tail.cuh"
 
@@ -110,12 +111,22 @@ trotter_kernel(Spins sp, TrotterArgs a) {
   overlap_and_weight(sp, a, N, nc, T2, O, &piv, red);
 }
 
-int launch_trotter(const Spins& sp, const TrotterArgs& a, cudaStream_t st) {
-  size_t smem = (size_t)3 * a.N * sp.ntot * sizeof(double2);
+// The chain of digit products takes 19 launches, 150 us at least; this kernel's time is the FP64 pipe's, one walker's
+// N^2 nc products on one SM at a time.  Measured (6 terms; FP64 kernel / digit products, us): N = 24, 5 columns: 60 / 150
+// (64 walkers), 216 / 355 (1024); N = 40, 7: 150 / 152, 654 / 427; N = 50, 8: 190 / 168, 1110 / 479; N = 64, 10: 345 /
+// 164, 2107 / 550; N = 96, 12: 843 / 193, 5505 / 1003.
+bool trotter_takes_digits(const Spins& sp, int N) {
+  return dg_takes(N) && N <= 1024 && (long long)N * N * sp.ntot >= 14000;
+}
+
+int launch_trotter(const Spins& sp, const TrotterArgs& a, const DgScratch& dg, cudaStream_t st) {
+  const size_t smem = (size_t)3 * a.N * sp.ntot * sizeof(double2);
   if (smem > 220 * 1024) {
     set_error("trotter: 3 walker tiles of %zu bytes exceed shared memory", smem);
     return TROT_ERR_UNSUPPORTED;
   }
+  if (dg.p && trotter_takes_digits(sp, a.N) && dg.bytes >= trotter_dg_bytes(sp, a.W, a.N))
+    return launch_trotter_dg(sp, a, dg, st);
   if (smem > 40 * 1024)
     cudaFuncSetAttribute(trotter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   trotter_kernel<<<a.W, kTrotThreads, smem, st>>>(sp, a);

@@ -38,3 +38,40 @@ def test_half_green_matches_oracle(kind, N, nelec, W):
     assert rel(cpu(green), ref) <= 1e-12
     assert rel(cpu(ov), cpu(S.trial_ops.overlap(walkers, S.trial))) <= 1e-14
     assert rel(cpu(half_green_batched(walkers, S.trial, S.walker_kind)), ref) <= 1e-12
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(not torch.cuda.is_available(), reason="needs a CUDA device")
+@pytest.mark.parametrize("kind,N,na,nb,W", [("rhf_r", 3, 1, 1, 2), ("rhf_r", 90, 33, 33, 3), ("uhf_u", 64, 31, 64, 2),
+                                            ("uhf_u", 130, 2, 17, 5), ("rhf_u", 41, 16, 16, 3), ("rhf_r", 1500, 4, 4, 2)])
+def test_green_and_overlap_sizes(kind, N, na, nb, W):
+    """Half Green's functions and overlaps at the edges of the kernel: one electron, more than a warp's lanes of
+    electrons, tiles that only fit without row padding, walkers of extreme magnitude.  Condition numbers of order ten,
+    so 1e-12 of the largest element."""
+    import trot_gb300 as tg
+    from oracle import afqmc_oracle as orc
+    from tests.gpu_helpers import cpu, dev
+    from trot_gb300 import synthetic
+    from trot_gb300.trial import half_green_batched
+
+    rng = np.random.default_rng(N + na)
+    q = np.linalg.qr(rng.standard_normal((N, max(na, nb))))[0]
+    ma, mb = np.ascontiguousarray(q[:, :na]), np.ascontiguousarray(q[:, :nb])
+    wk = "restricted" if kind == "rhf_r" else "unrestricted"
+    trial = tg.UhfTrial(ma, mb) if kind == "uhf_u" else tg.RhfTrial(ma)
+    noise = 0.3 / np.sqrt(N)
+    w = [synthetic.perturbed_walkers(ma, W, noise, 3), synthetic.perturbed_walkers(mb, W, noise, 4)]
+    if na <= 2:
+        w[0] = w[0] * np.array([1e150, 1e-150, 1, 1, 1])[:W, None, None]  # G does not depend on the scale
+    wd = dev(w[0]) if wk == "restricted" else (dev(w[0]), dev(w[1]))
+    g, ov = half_green_batched(wd, trial, wk, with_overlaps=True)
+    ref = [orc.half_green(w[0], ma)] + ([] if wk == "restricted" else [orc.half_green(w[1], mb)])
+    scale = [np.max(np.abs(r), axis=(1, 2), keepdims=True) for r in ref]
+    ref = np.concatenate([r / s for r, s in zip(ref, scale)], axis=1)
+    got = cpu(g)
+    got = np.concatenate([got[:, :na] / scale[0]] + ([] if wk == "restricted" else [got[:, na:] / scale[1]]), axis=1)
+    assert np.max(np.abs(got - ref)) <= 1e-12
+    d = [np.linalg.det(orc._ovlp_mat(m, x)) for m, x in zip((ma, mb), w)]
+    want = d[0] * d[0] if wk == "restricted" else d[0] * d[1]
+    fin = np.isfinite(want) & (np.abs(want) > 1e-290)
+    assert np.all(np.abs(cpu(ov) - want)[fin] <= (1e-11 * np.abs(want))[fin])

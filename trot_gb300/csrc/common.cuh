@@ -55,6 +55,18 @@ TROT_HD double2 cexp(double2 a) {
   return cmk(e * c, e * s);
 }
 
+// 1 / b by one division: b scaled by the power of two of its larger part (exact, against overflow), conj(b) / |b|^2, and
+// one correction by the residual 1 - b r
+TROT_D double2 crcp(double2 b) {
+  const int ex = max((__double2hiint(b.x) >> 20) & 0x7FF, (__double2hiint(b.y) >> 20) & 0x7FF);
+  if (ex < 64 || ex > 1982) return cdiv(cmk(1.0, 0.0), b);
+  const double s = __hiloint2double((2046 - ex) << 20, 0);  // 2^(1023 - ex)
+  const double x = b.x * s, y = b.y * s, r = 1.0 / fma(x, x, y * y);
+  const double u = x * r, v = -y * r;
+  const double er = fma(y, v, fma(-x, u, 1.0)), ei = -fma(y, u, x * v);
+  return cmk(fma(u, er, fma(-v, ei, u)) * s, fma(u, ei, fma(v, er, v)) * s);
+}
+
 // ---------------------------------------------------------------- reductions
 TROT_D double warp_sum(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -100,27 +112,28 @@ struct Spins {
 // Returns det(A) to all threads; A is overwritten by its LU factors.
 // If `inv` is non-null it receives A^{-1} (Gauss-Jordan on [A | I]).
 // One warp, an n x n matrix A (row stride n) in shared memory, partial pivoting (the first
-// largest |A[i][k]| wins, as in block_gauss_jordan).  Returns det(A).  With `inverse`, A is
+// largest |A[i][k]| wins, as in block_gauss_jordan, by integer reductions of the squares' words: five
+// shuffles of FP64 comparisons took longer than the elimination).  Returns det(A).  With `inverse`, A is
 // overwritten by its inverse (in-place Gauss-Jordan: each pivot step updates the n x n working
 // array once, half the work of eliminating [A | I]; the row interchanges are undone as column
 // interchanges in reverse order at the end, `perm` holds n ints of scratch); without it, A
 // holds its LU factors.  Phases are separated by __syncwarp, so no CTA barrier is involved.
-// The determinant is returned in lane 0.
-TROT_D double2 warp_gauss_jordan(double2* A, int n, bool inverse, int* perm) {
+// The determinant is returned in lane 0.  `smith`: the pivots' reciprocals by cdiv (three divisions) instead of crcp
+// (one), for results that are rounded to FP32 afterwards and must not move.
+TROT_D double2 warp_gauss_jordan(double2* A, int n, bool inverse, int* perm, bool smith = false) {
   const int lane = threadIdx.x & 31;
   double2 det = cmk(1.0, 0.0);
   for (int k = 0; k < n; ++k) {
-    double best = -1.0;
+    unsigned long long best = 0;  // bits of the square, with one added to the high word (0: no row)
     int bi = k;
     for (int i = k + lane; i < n; i += 32) {
-      const double a = cabs2(A[i * n + k]);
+      const unsigned long long a = (unsigned long long)__double_as_longlong(cabs2(A[i * n + k])) + (1ull << 32);
       if (a > best) { best = a; bi = i; }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-    }
+    const unsigned th = __reduce_max_sync(0xffffffffu, (unsigned)(best >> 32));
+    const bool cand = (unsigned)(best >> 32) == th;
+    const unsigned tl = __reduce_max_sync(0xffffffffu, cand ? (unsigned)best : 0u);
+    bi = (int)__reduce_min_sync(0xffffffffu, cand && (unsigned)best == tl ? (unsigned)bi : 0x7fffffffu);
     if (bi != k) {
       for (int j = lane; j < n; j += 32) {
         const double2 t = A[k * n + j];
@@ -137,7 +150,7 @@ TROT_D double2 warp_gauss_jordan(double2* A, int n, bool inverse, int* perm) {
     if (lane == 0) {
       const double2 piv = A[k * n + k];
       det = cmul(det, piv);
-      rp = cdiv(cmk(1.0, 0.0), piv);
+      rp = smith ? cdiv(cmk(1.0, 0.0), piv) : crcp(piv);
     }
     rp.x = __shfl_sync(0xffffffffu, rp.x, 0);
     rp.y = __shfl_sync(0xffffffffu, rp.y, 0);

@@ -84,7 +84,7 @@ green_ff_kernel(Spins sp, int N, const double2* __restrict__ wa, const double2* 
     }
     __syncthreads();
     // M^{-1} in place, FP64, by one warp (warp-synchronous phases; the other warps wait here)
-    if (tid < 32) warp_gauss_jordan(Md, n, true, perm);
+    if (tid < 32) warp_gauss_jordan(Md, n, true, perm, true);
     __syncthreads();
     for (int e = tid; e < n * n; e += nt) Mif[e] = ffc{ff_from_d(Md[e].x), ff_from_d(Md[e].y)};
     __syncthreads();

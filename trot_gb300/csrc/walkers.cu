@@ -306,30 +306,54 @@ int launch_qr(const Spins& sp, int W, int N, double2* wa, double2* wb, double2* 
 // ------------------------------------------------------------------ SR
 // Comb resampling (trot/walkers.py:249-293): cw = cumsum|w| (sequential, same
 // order as numpy), z_k = cw[-1] (k + zeta) / W, idx_k = first i with cw[i] >= z_k.
+// The sums are one chain of W dependent FP64 additions, which bounds the kernel; the weights come to it, and the sums
+// go to the searches, through shared memory (4096 at a time), so that nothing else waits between two additions.
+static constexpr int kSrTile = 4096;
+
 __global__ void __launch_bounds__(1024)
 sr_index_kernel(int W, const double* __restrict__ weights, const double* __restrict__ zeta_dev, double zeta,
                 double* __restrict__ cw, long long* __restrict__ idx, double* __restrict__ weights_out) {
-  __shared__ double tot_s;
+  __shared__ double c_s[kSrTile];
   if (zeta_dev) zeta = zeta_dev[0];
-  if (threadIdx.x == 0) {
-    double c = 0.0;
-    for (int i = 0; i < W; ++i) {
-      c += fabs(weights[i]);
-      cw[i] = c;
+  double c = 0.0;  // thread 0's running sum
+  for (int t0 = 0; t0 < W; t0 += kSrTile) {
+    const int m = min(kSrTile, W - t0);
+    __syncthreads();
+    for (int i = threadIdx.x; i < m; i += blockDim.x) c_s[i] = fabs(weights[t0 + i]);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int i = 0;
+      for (; i + 16 <= m; i += 16) {
+        double v[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) v[u] = c_s[i + u];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) {
+          c += v[u];
+          c_s[i + u] = c;
+        }
+      }
+      for (; i < m; ++i) {
+        c += c_s[i];
+        c_s[i] = c;
+      }
     }
-    tot_s = c;
+    __syncthreads();
+    if (W > kSrTile)
+      for (int i = threadIdx.x; i < m; i += blockDim.x) cw[t0 + i] = c_s[i];
   }
   __syncthreads();
-  const double tot = tot_s;
+  const double* cum = W > kSrTile ? cw : c_s;
+  const double tot = cum[W - 1], per = tot / (double)W;
   for (int k = threadIdx.x; k < W; k += blockDim.x) {
     const double z = tot * ((double)k + zeta) / (double)W;
     int lo = 0, hi = W;  // first i in [0, W) with cw[i] >= z; W if none
     while (lo < hi) {
       int mid = (lo + hi) >> 1;
-      if (cw[mid] < z) lo = mid + 1; else hi = mid;
+      if (cum[mid] < z) lo = mid + 1; else hi = mid;
     }
     idx[k] = lo < W ? lo : W - 1;
-    weights_out[k] = tot / (double)W;
+    weights_out[k] = per;
   }
 }
 

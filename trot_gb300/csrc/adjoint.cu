@@ -325,6 +325,71 @@ static int combine(size_t len, const Comb& cb, double2* out, bool accumulate, cu
   return TROT_OK;
 }
 
+// ---------------------------------------------------------------- Taylor chain on (walker, l, j, p) arrays
+// With the digit products the columns of both spins run through the chain together, transposed and, in the backward
+// direction, conjugated: V^H v = conj(V^T conj(v)) and g_V = conj(sum_l conj(s_l) u_l^T), so that only V (or V^T) is
+// ever an operand.  c_k = (i sqrt(dt))^k / k! has one non-zero part: times c_k is a real factor and a rotation by i^k.
+struct AdjCoef {
+  int K;
+  double r[8];  // sqrt(dt)^k / k!
+};
+TROT_D void adj_fma_ck(double2& acc, double r, int k, double2 x) {  // acc += r i^k x
+  const double2 y = (k & 1) ? cmk(-x.y, x.x) : x;
+  const double f = (k & 2) ? -r : r;
+  acc.x = fma(f, y.x, acc.x);
+  acc.y = fma(f, y.y, acc.y);
+}
+// O[b][e] = sum_k c_k U[b][k][e], e < per
+__global__ void adj_chain_sum_kernel(int W, size_t per, AdjCoef c, const double2* __restrict__ U, double2* __restrict__ O) {
+  const size_t total = (size_t)W * per;
+  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
+    const size_t b = t / per, e = t - b * per;
+    const double2* u = U + b * (c.K + 1) * per + e;
+    double2 acc = u[0];
+    for (int k = 1; k <= c.K; ++k) adj_fma_ck(acc, c.r[k], k, u[k * per]);
+    O[t] = acc;
+  }
+}
+// g[b][e] = sum_k c_k v[b][k][e];  S[b][l][e] = sum_{j <= K-1-l} c_{j+l+1} v[b][j][e], l < K
+__global__ void adj_chain_back_kernel(int W, size_t per, AdjCoef c, const double2* __restrict__ v,
+                                      double2* __restrict__ g, double2* __restrict__ S) {
+  const size_t total = (size_t)W * per;
+  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
+    const size_t b = t / per, e = t - b * per;
+    const double2* u = v + b * (c.K + 1) * per + e;
+    double2* s = S + b * c.K * per + e;
+    double2 x[8], acc = u[0];
+    x[0] = acc;
+#pragma unroll
+    for (int k = 1; k < 8; ++k)
+      if (k <= c.K) {
+        x[k] = u[k * per];
+        adj_fma_ck(acc, c.r[k], k, x[k]);
+      }
+    g[t] = acc;
+#pragma unroll
+    for (int l = 0; l < 7; ++l) {
+      if (l >= c.K) break;
+      double2 y = cmk(0.0, 0.0);
+#pragma unroll
+      for (int j = 0; j < 7; ++j)
+        if (j + l + 1 <= c.K) adj_fma_ck(y, c.r[j + l + 1], j + l + 1, x[j]);
+      s[l * per] = y;
+    }
+  }
+}
+// w[b][p][j] = x[b][off + j][p] (walkers of x nc N apart), conjugated if conj
+__global__ void adj_from_rows_kernel(int N, int n, int nc, int off, int conj, const double2* __restrict__ x,
+                                     double2* __restrict__ w) {
+  const int b = blockIdx.x;
+  const double2* src = x + ((size_t)b * nc + off) * N;
+  for (int e = threadIdx.x; e < N * n; e += blockDim.x) {
+    const int p = e / n, j = e - p * n;
+    const double2 v = src[(size_t)j * N + p];
+    w[(size_t)b * N * n + e] = conj ? cmk(v.x, -v.y) : v;
+  }
+}
+
 // Walkers that cannot influence the objective (zero weight before the step, or
 // a weight the step's guards set to zero; zero energy / overlap cotangent) get
 // exactly zero cotangents: their recomputed data, which may be non-finite, is
@@ -452,7 +517,7 @@ __global__ void adj_step_bwd_kernel(int W, const double2* __restrict__ ov_old, c
 // st = i sum xs m, ft = sum (x fs - fs^2 / 2), c = -sqrt(dt) Re(sum xs m).
 __global__ void adj_fields_kernel(int W, int G, double sqrt_dt, const double* __restrict__ mf_im,
                                   const double2* __restrict__ xs, const double2* __restrict__ gxsv,
-                                  const double* __restrict__ g_req, const double* __restrict__ g_c,
+                                  int conj_gxsv, const double* __restrict__ g_req, const double* __restrict__ g_c,
                                   double2* __restrict__ gfb) {
   const size_t total = (size_t)W * G;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
@@ -460,7 +525,7 @@ __global__ void adj_fields_kernel(int W, int G, double sqrt_dt, const double* __
     const double m = mf_im[g];
     const double greq = g_req[b];
     const double gst = -sqrt_dt * greq;  // g_st (real): Re q = -sqrt(dt) Re st + ...
-    const double2 gv = gxsv[e];
+    const double2 gv = conj_gxsv ? cmk(gxsv[e].x, -gxsv[e].y) : gxsv[e];
     const double2 gxs = cmk(gv.x - sqrt_dt * m * g_c[b], gv.y - m * gst);
     const double2 x = xs[e];
     const double2 gfs = csub(cscale(cmk(x.x, -x.y), greq), gxs);
@@ -596,7 +661,14 @@ struct StepWs {
   double2* kpart;  // split-K partials of the long-K products
   int* act;
   DgScratch dg;
+  // digit products: (W, K + 1, nc, N) forward and backward chains, (W, K, nc, N) s_l, (W, nc, N) sums
+  double2 *Ut, *Vt, *St, *Ot, *Tt;
+  DgAdjoint ad;
+  bool chain;
 };
+
+// the Taylor chains on the tensor cores (both spins' columns together)
+static bool adj_chain_digits(const AdjCommon& a) { return dg_takes(a.N) && a.N <= 1024; }
 
 static int splitk_slices(int M, int Nn) {  // enough CTAs for two per SM
   const int base = ((Nn + 63) / 64) * ((M + 63) / 64);
@@ -620,13 +692,14 @@ static void digits_for(size_t& n, size_t M, size_t Nn, size_t K) {
 static void carve_step(const AdjCommon& a, Carver& c, StepWs& b, bool digits) {
   const size_t W = a.W, G = a.G, NN = (size_t)a.N * a.N;
   b = StepWs{};
+  b.chain = digits && adj_chain_digits(a);
   for (int q = 0; q < a.nspin; ++q) {
     SpinWs& x = b.sp[q];
     const size_t wn = a.wn[q], n = a.n[q];
     x.green = c.take<double2>(W * a.nN[q]);
     x.P = c.take<double2>(W * n * n);
     x.det = c.take<double2>(W);
-    x.U = c.take<double2>((size_t)(a.K + 1) * wn);
+    if (!b.chain) x.U = c.take<double2>((size_t)(a.K + 1) * wn);
     x.w2 = c.take<double2>(wn);
     x.wnew = c.take<double2>(wn);
     x.greenn = c.take<double2>(W * a.nN[q]);
@@ -634,8 +707,10 @@ static void carve_step(const AdjCommon& a, Carver& c, StepWs& b, bool digits) {
     x.detn = c.take<double2>(W);
     x.gwn = c.take<double2>(wn);
     x.gw2 = c.take<double2>(wn);
-    x.Vv = c.take<double2>((size_t)(a.K + 1) * wn);
-    x.S = c.take<double2>((size_t)a.K * wn);
+    if (!b.chain) {
+      x.Vv = c.take<double2>((size_t)(a.K + 1) * wn);
+      x.S = c.take<double2>((size_t)a.K * wn);
+    }
     x.gG = c.take<double2>(W * a.nN[q]);
     x.gw1 = c.take<double2>(wn);
     x.wz = c.take<double2>(wn);
@@ -671,6 +746,17 @@ static void carve_step(const AdjCommon& a, Carver& c, StepWs& b, bool digits) {
     }
     digits_for(nd, W, P, G);
     digits_for(nd, W, G, P);
+  }
+  if (b.chain) {
+    const size_t nc = a.n[0] + (a.nspin == 2 ? a.n[1] : 0), one = W * nc * a.N;
+    b.Ut = c.take<double2>((a.K + 1) * one);
+    b.Vt = c.take<double2>((a.K + 1) * one);
+    b.St = c.take<double2>(a.K * one);
+    b.Ot = c.take<double2>(one);
+    b.Tt = c.take<double2>(one);
+    DgScratch s{};
+    take_digits(c, adjoint_dg_bytes(W, a.N, nc, a.K * nc), s);
+    adjoint_dg_carve(b.ad, (int)W, a.N, (int)nc, (int)(a.K * nc), s);
   }
   take_digits(c, nd, b.dg);
 }
@@ -730,6 +816,12 @@ static int ov_launch(const AdjCommon& a, const double2* d0, const double2* d1, d
   adj_ov_kernel<<<(a.W + 127) / 128, 128, 0, st>>>(a.W, d0, a.mult[0], a.nspin == 2 ? d1 : nullptr,
                                                     a.nspin == 2 ? a.mult[1] : 0, ov);
   TROT_CHECK_LAUNCH("adj_ov_kernel");
+  return TROT_OK;
+}
+
+static int from_rows(int W, int N, int n, int nc, int off, bool conj, const double2* x, double2* w, cudaStream_t st) {
+  adj_from_rows_kernel<<<W, 256, 0, st>>>(N, n, nc, off, conj ? 1 : 0, x, w);
+  TROT_CHECK_LAUNCH("adj_from_rows_kernel");
   return TROT_OK;
 }
 
@@ -812,8 +904,10 @@ int trot_prop_step_vjp(const trot_system* s, const trot_state* in, const double*
   }
   TROT_TRY(launch_fields(W, G, s->sqrt_dt, b.fb, s->mf_shifts_im, fields, b.xs, b.st, b.ft, st));
   TROT_TRY(launch_vhs64(W, N, G, b.xs, s->chol_flat, a.chol_packed, b.vp, b.V, b.dg, st));
-  adj_to_complex_kernel<<<grid_of(NN), 256, 0, st>>>(NN, s->exp_h1_half, b.Bc);
-  TROT_CHECK_LAUNCH("adj_to_complex_kernel");
+  if (!b.chain) {
+    adj_to_complex_kernel<<<grid_of(NN), 256, 0, st>>>(NN, s->exp_h1_half, b.Bc);
+    TROT_CHECK_LAUNCH("adj_to_complex_kernel");
+  }
   double2 ck[8];
   {  // c_k = (i sqrt(dt))^k / k!
     double2 t = one;
@@ -823,7 +917,32 @@ int trot_prop_step_vjp(const trot_system* s, const trot_state* in, const double*
       ck[k] = t;
     }
   }
-  for (int q = 0; q < a.nspin; ++q) {
+  const int nc = a.n[0] + (two ? a.n[1] : 0);
+  const size_t per1 = (size_t)nc * N;
+  const long long sU = (long long)(K + 1) * per1;
+  AdjCoef co{};
+  co.K = K;
+  co.r[0] = 1.0;
+  for (int k = 1; k <= K; ++k) co.r[k] = co.r[k - 1] * s->sqrt_dt / k;
+  if (b.chain) {
+    // u_0 = E w, u_{l+1} = V u_l, w2 = sum_k c_k u_k, w' = E w2 (both spins' columns)
+    TROT_TRY(adjoint_dg_e(b.ad, s->exp_h1_half, st));
+    TROT_TRY(adjoint_dg_v(b.ad, b.V, false, st));
+    TROT_TRY(adjoint_dg_from_walkers(b.ad, kDgE, w[0], a.n[0], two ? w[1] : nullptr, a.n[1], false, b.Ut, sU, st));
+    for (int l = 0; l < K; ++l)
+      TROT_TRY(adjoint_dg_from_rows(b.ad, kDgV, b.Ut + l * per1, sU, b.Ut + (l + 1) * per1, sU, st));
+    adj_chain_sum_kernel<<<grid_of(W * per1), 256, 0, st>>>(W, per1, co, b.Ut, b.Ot);
+    TROT_CHECK_LAUNCH("adj_chain_sum_kernel");
+    TROT_TRY(adjoint_dg_from_rows(b.ad, kDgE, b.Ot, (long long)per1, b.Tt, (long long)per1, st));
+    for (int q = 0; q < a.nspin; ++q) {
+      SpinWs& x = b.sp[q];
+      const int off = q ? a.n[0] : 0;
+      TROT_TRY(from_rows(W, N, a.n[q], nc, off, false, b.Ot, x.w2, st));
+      TROT_TRY(from_rows(W, N, a.n[q], nc, off, false, b.Tt, x.wnew, st));
+      TROT_TRY(green_launch(a, q, x.wnew, x.greenn, x.Pn, x.detn, st));
+    }
+  }
+  for (int q = 0; q < a.nspin && !b.chain; ++q) {
     SpinWs& x = b.sp[q];
     const int n = a.n[q];
     const long long sw = (long long)N * n;
@@ -853,13 +972,14 @@ int trot_prop_step_vjp(const trot_system* s, const trot_state* in, const double*
     const size_t per = (size_t)N * a.n[q], nn = (size_t)a.n[q] * a.n[q];
     TROT_TRY(dcopy(x.wz, w[q], a.wn[q] * sizeof(double2), st));
     TROT_TRY(zero_inactive(W, per, b.act, x.wz, st));
-    for (int l = 0; l <= K; ++l) TROT_TRY(zero_inactive(W, per, b.act, x.U + (size_t)l * a.wn[q], st));
+    for (int l = 0; l <= K && !b.chain; ++l) TROT_TRY(zero_inactive(W, per, b.act, x.U + (size_t)l * a.wn[q], st));
     TROT_TRY(zero_inactive(W, per, b.act, x.w2, st));
     TROT_TRY(zero_inactive(W, a.nN[q], b.act, x.green, st));
     TROT_TRY(zero_inactive(W, nn, b.act, x.P, st));
     TROT_TRY(zero_inactive(W, nn, b.act, x.Pn, st));
   }
-  TROT_TRY(zero_inactive(W, NN, b.act, b.V, st));
+  if (b.chain) TROT_TRY(zero_inactive(W, (K + 1) * per1, b.act, b.Ut, st));
+  if (!b.chain || !a.chol_packed) TROT_TRY(zero_inactive(W, NN, b.act, b.V, st));
   TROT_TRY(zero_inactive(W, G, b.act, b.xs, st));
   // ---------------- backward
   adj_step_bwd_kernel<<<wb, 128, 0, st>>>(W, (const double2*)in->overlaps, b.ov_new, b.st, b.ft, in->weights,
@@ -885,6 +1005,7 @@ int trot_prop_step_vjp(const trot_system* s, const trot_state* in, const double*
     TROT_CHECK_LAUNCH("adj_overlap_kernel");
     // w' = B w2: g_B += Re sum g_w' w2^H; g_w2 = B^T g_w'
     TROT_TRY(outer_sum(W, N, n, x.gwn, x.w2, b.opart, g_exp_h1_half, st));
+    if (b.chain) continue;
     TROT_TRY(zgemm_batched(W, N, n, N, one, b.Bc, 0, N, 1, x.gwn, sw, n, 0, zero, x.gw2, sw, n, st));
     // v_0 = g_w2, v_{j+1} = V^H v_j
     TROT_TRY(dcopy(x.Vv, x.gw2, a.wn[q] * sizeof(double2), st));
@@ -909,6 +1030,28 @@ int trot_prop_step_vjp(const trot_system* s, const trot_state* in, const double*
     TROT_TRY(outer_sum(W, N, n, x.gw1, x.wz, b.opart, g_exp_h1_half, st));
     TROT_TRY(zgemm_batched(W, N, n, N, one, b.Bc, 0, N, 1, x.gw1, sw, n, 0, zero, gin[q], sw, n, st));
   }
+  if (b.chain) {
+    // conj(v_0) = E^T conj(g_w'), conj(v_{j+1}) = V^T conj(v_j); V is symmetric with symmetric L_g
+    if (a.chol_packed) TROT_TRY(adjoint_dg_v_active(b.ad, b.act, st));
+    else TROT_TRY(adjoint_dg_v(b.ad, b.V, true, st));
+    TROT_TRY(adjoint_dg_from_walkers(b.ad, kDgET, b.sp[0].gwn, a.n[0], two ? b.sp[1].gwn : nullptr, a.n[1], true, b.Vt, sU,
+                                     st));
+    for (int j = 0; j < K; ++j)
+      TROT_TRY(adjoint_dg_from_rows(b.ad, kDgV, b.Vt + j * per1, sU, b.Vt + (j + 1) * per1, sU, st));
+    adj_chain_back_kernel<<<grid_of(W * per1), 256, 0, st>>>(W, per1, co, b.Vt, b.Ot, b.St);
+    TROT_CHECK_LAUNCH("adj_chain_back_kernel");
+    // conj(g_V)[p][q] = sum_{l,j} conj(s_l)[j][p] u_l[j][q]
+    TROT_TRY(adjoint_dg_gv(b.ad, b.St, (long long)K * per1, b.Ut, sU, b.gV, st));
+    TROT_TRY(adjoint_dg_from_rows(b.ad, kDgET, b.Ot, (long long)per1, b.Tt, (long long)per1, st));
+    for (int q = 0; q < a.nspin; ++q) {
+      SpinWs& x = b.sp[q];
+      const int n = a.n[q], off = q ? a.n[0] : 0;
+      // w1 = B w: g_B += Re sum g_w1 w^H; g_w = B^T g_w1 (the Green's-function term is added below)
+      TROT_TRY(from_rows(W, N, n, nc, off, true, b.Ot, x.gw1, st));
+      TROT_TRY(outer_sum(W, N, n, x.gw1, x.wz, b.opart, g_exp_h1_half, st));
+      TROT_TRY(from_rows(W, N, n, nc, off, true, b.Tt, gin[q], st));
+    }
+  }
   // V = sum_g xs_g L_g: g_xs^V[b][g] = sum_pq L_g[pq] g_V[b][pq] (with symmetric L_g: over the packed
   // upper triangle of g_V + g_V^T, half the FP64 products)
   if (a.chol_packed) {
@@ -920,7 +1063,7 @@ int trot_prop_step_vjp(const trot_system* s, const trot_state* in, const double*
     TROT_TRY(launch_zgemm(W, G, (int)NN, 1.0, b.gV, (int)NN, s->chol_flat, (int)NN, true, b.gxsv, G, false, b.dg, st,
                           b.kpart, splitk_slices(W, G)));
   }
-  adj_fields_kernel<<<grid_of((size_t)W * G), 256, 0, st>>>(W, G, s->sqrt_dt, s->mf_shifts_im, b.xs, b.gxsv, b.g_req,
+  adj_fields_kernel<<<grid_of((size_t)W * G), 256, 0, st>>>(W, G, s->sqrt_dt, s->mf_shifts_im, b.xs, b.gxsv, b.chain ? 1 : 0, b.g_req,
                                                              b.g_c, b.gfb);
   TROT_CHECK_LAUNCH("adj_fields_kernel");
   for (int q = 0; q < a.nspin; ++q) {
@@ -976,10 +1119,11 @@ int trot_local_energy_vjp(const trot_system* s, const double* walkers_a, const d
     TROT_TRY(combine((size_t)W * G, cb, b.ctot, false, st));
   }
   // dE/dG_s = mult_s (rot_h1_s + sum_g c_tot,g R_{s,g} - sum_g f_{s,g} R_{s,g})
-  for (int q = 0; q < a.nspin; ++q) {
+  for (int q = a.nspin - 1; q >= 0; --q) {
     const int n = a.n[q];
     const double m = (double)a.mult[q];
-    TROT_TRY(launch_zgemm(W * n, G * n, N, 1.0, b.green[q], N, a.rot_chol[q], N, true, b.F, G * n, false, b.dg, st));
+    if (q != a.nspin - 1)  // F holds the last spin's f from the traces above
+      TROT_TRY(launch_zgemm(W * n, G * n, N, 1.0, b.green[q], N, a.rot_chol[q], N, true, b.F, G * n, false, b.dg, st));
     adj_block_transpose_kernel<<<grid_of((size_t)W * n * G * n), 256, 0, st>>>(W, G, n, b.F, b.Ft);
     TROT_CHECK_LAUNCH("adj_block_transpose_kernel");
     TROT_TRY(launch_zgemm(W * n, N, G * n, -m, b.Ft, G * n, a.rot_chol[q], N, false, b.D, N, false, b.dg, st));

@@ -115,6 +115,8 @@ TROT_D void dg_store8(const double* x, int e, uint16_t* o, size_t plane) {
   for (int t = 0; t < kDgS; ++t) *reinterpret_cast<uint4*>(o + t * plane) = w[t];
 }
 
+TROT_D double dg_neg(double x) { return __hiloint2double(__double2hiint(x) ^ (int)0x80000000u, __double2loint(x)); }
+
 // high word of the largest |x| so far, and sum of |x| as a float from its high word (the range only matters near
 // the row maximum)
 TROT_D void dg_row_max(double x, unsigned& mx, float& s) {
@@ -145,7 +147,7 @@ TROT_D int dg_exponent(unsigned mx, float l1) {
 struct DgSrc {
   const double* p;
   int K, nk16, R;        // R = 32 or 128 rows per tile
-  int cplx;
+  int cplx, conj;        // conj: imaginary rows change sign
   // image row -> block (of bstride doubles) row / rpad, row r = row % rpad of it; rows r >= rpb and blocks
   // >= nblk are padding
   int rpb, rpad, nblk;
@@ -161,7 +163,7 @@ static constexpr int kDgOneBlock = 1 << 30;
 // `rows` rows of stride rst (complex ones count twice), one block
 static DgSrc dg_src(const double* p, int cplx, int rows, int K, int R, long long rst, long long kst, uint16_t* img,
                     int16_t* ex) {
-  return DgSrc{p, K, (K + 15) / 16, R, cplx, rows, kDgOneBlock, 1, 0, rst, kst, kDgOneBlock, nullptr, 0, 0, img, ex};
+  return DgSrc{p, K, (K + 15) / 16, R, cplx, 0, rows, kDgOneBlock, 1, 0, rst, kst, kDgOneBlock, nullptr, 0, 0, img, ex};
 }
 
 __global__ void __launch_bounds__(256) dg_rows_kernel(DgSrc a) {
@@ -174,7 +176,7 @@ __global__ void __launch_bounds__(256) dg_rows_kernel(DgSrc a) {
   const int rl = lane & 7, kg = lane >> 3;
   const int row = blockIdx.y * 8 + rl;
   const int blk = row / a.rpad, rr = row - blk * a.rpad;
-  const bool valid = blk < a.nblk && rr < a.rpb;
+  const bool valid = blk < a.nblk && rr < a.rpb, flip = a.conj && (rr & 1);
   const double* p = a.p;
   long long kst = a.kst;
   if (valid) {
@@ -197,6 +199,7 @@ __global__ void __launch_bounds__(256) dg_rows_kernel(DgSrc a) {
     for (int i = 0; i < 8; ++i) {
       const int k = k0 + kg * 8 + i;
       x[i] = (valid && k < a.K) ? p[k * kst] : 0.0;
+      if (flip) x[i] = dg_neg(x[i]);
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i) dg_row_max(x[i], mx, s);
@@ -237,7 +240,10 @@ __global__ void __launch_bounds__(256) dg_rows_kernel(DgSrc a) {
     if (kb >= kpad) continue;
     if (!once) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) x[i] = (live && kb + i < a.K) ? p[(kb + i) * kst] : 0.0;
+      for (int i = 0; i < 8; ++i) {
+        x[i] = (live && kb + i < a.K) ? p[(kb + i) * kst] : 0.0;
+        if (flip) x[i] = dg_neg(x[i]);
+      }
     }
     if (!live) {
 #pragma unroll
@@ -939,6 +945,127 @@ int launch_trotter_dg(const Spins& sp, const TrotterArgs& t, const DgScratch& s,
   dg_trotter_tail_kernel<<<W, 256, smem, st>>>(sp, t, U);
   TROT_CHECK_LAUNCH("dg_trotter_tail_kernel");
   return TROT_OK;
+}
+
+// ------------------------------------------------------------------ step adjoint
+static size_t adj_rows(size_t rows, size_t tile) { return (rows + tile - 1) / tile * tile; }
+
+size_t adjoint_dg_bytes(size_t W, size_t N, size_t nc, size_t K2) {
+  DgAdjoint d{};
+  DgScratch s{};
+  adjoint_dg_carve(d, (int)W, (int)N, (int)nc, (int)K2, s);
+  return (size_t)((char*)d.etex - (char*)nullptr) + adj_rows(N, 128) * 2 + 512;
+}
+
+// (with s.p null the pointers are offsets from the start, for the size)
+void adjoint_dg_carve(DgAdjoint& d, int W, int N, int nc, int K2, const DgScratch& s) {
+  d.W = W; d.N = N; d.nc = nc; d.K2 = K2; d.status = s.status;
+  char* p = reinterpret_cast<char*>(((uintptr_t)s.p + 255) & ~(uintptr_t)255);
+  auto take = [&](size_t n) {
+    char* r = p;
+    p += (n + 255) & ~(size_t)255;
+    return r;
+  };
+  const size_t rb = kDgRowBytes((N + 15) / 16), rb2 = kDgRowBytes((K2 + 15) / 16);
+  const size_t vr = (size_t)W * adj_rows(2 * N, 128), ur = (size_t)W * adj_rows(2 * nc, kDgP);
+  const size_t gr = (size_t)W * adj_rows(2 * N, kDgP), er = adj_rows(N, 128);
+  d.vimg = reinterpret_cast<uint16_t*>(take(vr * std::max(rb, rb2)));
+  d.uimg = reinterpret_cast<uint16_t*>(take(std::max(ur * rb, gr * rb2)));
+  d.eimg = reinterpret_cast<uint16_t*>(take(er * rb));
+  d.etimg = reinterpret_cast<uint16_t*>(take(er * rb));
+  d.vex = reinterpret_cast<int16_t*>(take(vr * 2));
+  d.uex = reinterpret_cast<int16_t*>(take(std::max(ur, gr) * 2));
+  d.eex = reinterpret_cast<int16_t*>(take(er * 2));
+  d.etex = reinterpret_cast<int16_t*>(take(er * 2));
+}
+
+int adjoint_dg_e(const DgAdjoint& d, const double* E, cudaStream_t st) {
+  const int groups = (int)adj_rows(d.N, 128) / 8;
+  TROT_TRY(dg_rows_launch(dg_src(E, 0, d.N, d.N, 128, d.N, 1, d.eimg, d.eex), groups, st));
+  return dg_rows_launch(dg_src(E, 0, d.N, d.N, 128, 1, d.N, d.etimg, d.etex), groups, st);
+}
+
+int adjoint_dg_v(const DgAdjoint& d, const double2* V, bool transposed, cudaStream_t st) {
+  const int N = d.N, rpad = (int)adj_rows(2 * N, 128);
+  DgSrc s = dg_src(reinterpret_cast<const double*>(V), 1, 2 * N, N, 128, transposed ? 2 : 2ll * N,
+                   transposed ? 2ll * N : 2, d.vimg, d.vex);
+  s.rpad = rpad;
+  s.nblk = d.W;
+  s.bstride = 2ll * N * N;
+  return dg_rows_launch(s, d.W * (rpad / 8), st);
+}
+
+__global__ void dg_clear_flags_kernel(int W, int rpad, const int* __restrict__ act, int16_t* __restrict__ ex) {
+  const size_t total = (size_t)W * rpad;
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x)
+    if (!act[e / rpad] && ex[e] == kDgNonFinite) ex[e] = 0;  // such a row's digits are zeros
+}
+
+int adjoint_dg_v_active(const DgAdjoint& d, const int* act, cudaStream_t st) {
+  const int rpad = (int)adj_rows(2 * d.N, 128);
+  const size_t total = (size_t)d.W * rpad;
+  dg_clear_flags_kernel<<<(int)std::min<size_t>((total + 255) / 256, 1024), 256, 0, st>>>(d.W, rpad, act, d.vex);
+  TROT_CHECK_LAUNCH("dg_clear_flags_kernel");
+  return TROT_OK;
+}
+
+static int adj_apply(const DgAdjoint& d, DgOperand op, DgSrc s, double2* out, long long ostride, cudaStream_t st) {
+  const int rpad = (int)adj_rows(2 * d.nc, kDgP);
+  s.rpad = rpad;
+  s.nblk = d.W;
+  TROT_TRY(dg_rows_launch(s, d.W * (rpad / 8), st));
+  DgArgs a{};
+  a.imgA = d.uimg; a.exA = d.uex;
+  a.imgB = op == kDgV ? d.vimg : op == kDgE ? d.eimg : d.etimg;
+  a.exB = op == kDgV ? d.vex : op == kDgE ? d.eex : d.etex;
+  a.Nn = op == kDgV ? 2 * d.N : d.N; a.M = d.nc;
+  a.nrt = (a.Nn + 127) / 128; a.bB = op == kDgV ? a.nrt : 0;
+  a.ntile = rpad / kDgP; a.nbatch = d.W; a.cstride = ostride;
+  a.nk16 = (d.N + 15) / 16; a.shift = 1;
+  a.C = out; a.ldc = d.N; a.salpha = 1; a.status = d.status;
+  return op == kDgV ? dg_gemm<true>(a, st) : dg_gemm<false>(a, st);
+}
+
+int adjoint_dg_from_walkers(const DgAdjoint& d, DgOperand op, const double2* wa, int na, const double2* wb, int nb,
+                            bool conj, double2* out, long long ostride, cudaStream_t st) {
+  DgSrc s = dg_src(reinterpret_cast<const double*>(wa), 1, 2 * d.nc, d.N, kDgP, 2, 2ll * na, d.uimg, d.uex);
+  s.conj = conj;
+  s.bstride = 2ll * d.N * na;
+  if (wb) {
+    s.split = 2 * na;
+    s.p2 = reinterpret_cast<const double*>(wb);
+    s.bstride2 = 2ll * d.N * nb;
+    s.kst2 = 2ll * nb;
+  }
+  return adj_apply(d, op, s, out, ostride, st);
+}
+
+int adjoint_dg_from_rows(const DgAdjoint& d, DgOperand op, const double2* src, long long sstride, double2* out,
+                         long long ostride, cudaStream_t st) {
+  DgSrc s = dg_src(reinterpret_cast<const double*>(src), 1, 2 * d.nc, d.N, kDgP, 2ll * d.N, 2, d.uimg, d.uex);
+  s.bstride = 2 * sstride;
+  return adj_apply(d, op, s, out, ostride, st);
+}
+
+int adjoint_dg_gv(const DgAdjoint& d, const double2* S, long long sstride, const double2* U, long long ustride,
+                  double2* gv, cudaStream_t st) {
+  const int N = d.N, rpad = (int)adj_rows(2 * N, kDgP), vpad = (int)adj_rows(2 * N, 128);
+  DgSrc s = dg_src(reinterpret_cast<const double*>(S), 1, 2 * N, d.K2, kDgP, 2, 2ll * N, d.uimg, d.uex);
+  s.rpad = rpad;
+  s.nblk = d.W;
+  s.bstride = 2 * sstride;
+  TROT_TRY(dg_rows_launch(s, d.W * (rpad / 8), st));
+  DgSrc u = dg_src(reinterpret_cast<const double*>(U), 1, 2 * N, d.K2, 128, 2, 2ll * N, d.vimg, d.vex);
+  u.rpad = vpad;
+  u.nblk = d.W;
+  u.bstride = 2 * ustride;
+  TROT_TRY(dg_rows_launch(u, d.W * (vpad / 8), st));
+  DgArgs a{};
+  a.imgA = d.uimg; a.exA = d.uex; a.imgB = d.vimg; a.exB = d.vex;
+  a.Nn = 2 * N; a.M = N; a.nrt = a.bB = vpad / 128; a.ntile = rpad / kDgP; a.nbatch = d.W;
+  a.cstride = (long long)N * N; a.nk16 = (d.K2 + 15) / 16; a.shift = 1;  // K2 <= 7 x 64
+  a.C = gv; a.ldc = N; a.salpha = 1; a.status = d.status;
+  return dg_gemm<true>(a, st);
 }
 
 }  // namespace trot

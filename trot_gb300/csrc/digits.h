@@ -31,4 +31,30 @@ int launch_exchange_dg(const Spins& sp, int W, int N, int G, const double2* gree
 size_t trotter_dg_bytes(const Spins& sp, size_t W, size_t N);
 int launch_trotter_dg(const Spins& sp, const TrotterArgs& a, const DgScratch& s, cudaStream_t st);
 
+// Batched products of the step adjoint on arrays (walker, column j, orbital p) of nc columns: V (complex N x N per
+// walker), E (real N x N) or E^T against every column.
+struct DgAdjoint {
+  int W, N, nc, K2;                    // K2: terms (l, j) of the cotangent of V
+  uint16_t *vimg, *uimg, *eimg, *etimg;
+  int16_t *vex, *uex, *eex, *etex;
+  int* status;
+};
+enum DgOperand { kDgE, kDgET, kDgV };
+size_t adjoint_dg_bytes(size_t W, size_t N, size_t nc, size_t K2);
+void adjoint_dg_carve(DgAdjoint& d, int W, int N, int nc, int K2, const DgScratch& s);
+// digits of E and E^T; of V, or of V^T (transposed)
+int adjoint_dg_e(const DgAdjoint& d, const double* E, cudaStream_t st);
+int adjoint_dg_v(const DgAdjoint& d, const double2* V, bool transposed, cudaStream_t st);
+// walkers with act[b] == 0: a row of V that is not finite counts as zero
+int adjoint_dg_v_active(const DgAdjoint& d, const int* act, cudaStream_t st);
+// out[b][j][p] (walkers ostride apart) = op . columns of wa (W, N, na) and wb (W, N, nb), conjugated if conj
+int adjoint_dg_from_walkers(const DgAdjoint& d, DgOperand op, const double2* wa, int na, const double2* wb, int nb,
+                            bool conj, double2* out, long long ostride, cudaStream_t st);
+// the same from an array (walker, j, p), walkers sstride apart
+int adjoint_dg_from_rows(const DgAdjoint& d, DgOperand op, const double2* src, long long sstride, double2* out,
+                         long long ostride, cudaStream_t st);
+// gv[b][p][q] = sum_{k < K2} S[b][k][p] U[b][k][q] (the digits of V are overwritten)
+int adjoint_dg_gv(const DgAdjoint& d, const double2* S, long long sstride, const double2* U, long long ustride,
+                  double2* gv, cudaStream_t st);
+
 }  // namespace trot

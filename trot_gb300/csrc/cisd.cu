@@ -49,7 +49,8 @@ struct CisdBuffers {
   double2* y;                   // xg ci2m (W G, n v)    (FP64 l2ci2)
   uint16_t* xq;                 // split3 image of xg    (mixed l2ci2)
   float* yd;                    // xg ci2m, FP32         (mixed l2ci2)
-  double2* gpart;               // per (walker, gamma chunk) partial sums (W, nchunk, 4)
+  double2* gpart;               // per (walker, gamma chunk) partial sums (W, nchunk, 4), nchunk <= cisd_chunks
+  int nchunk;
   double2* l2part;              // l2ci2 partial sums (W, kL2Parts)
   // propagation step
   double2 *fb, *xs, *shift_term, *fb_term, *vhs, *ov_new;
@@ -73,6 +74,11 @@ static int cisd_splitk(int M, int Nn, int K) {
   return std::max(1, std::min(S, 16));
 }
 
+// the per-vector terms in FP64 by digit products
+static bool cisd_gamma_digits(const trot_cisd* c) {
+  return c->gl_precision != TROT_MIXED && dg_takes(c->norb) && c->norb <= 1024;
+}
+
 // Scratch of the tensor-core digit products of an op (the largest of them; they run one after another)
 static size_t cisd_digit_bytes(const trot_cisd* c, size_t W, int op) {
   const size_t N = c->norb, n = c->nocc, G = c->nchol, nv = n * c->nvir;
@@ -87,6 +93,7 @@ static size_t cisd_digit_bytes(const trot_cisd* c, size_t W, int op) {
   add(W, G, N * (N + 1) / 2);
   if (op == TROT_OP_FORCE_BIAS) return d;
   if (c->l2ci2_precision != TROT_MIXED) add(W * G, nv, nv);  // l2ci2
+  if (cisd_gamma_digits(c)) d = std::max(d, cisd_gamma_dg_bytes(W, N, n, G));
   if (op == TROT_OP_PROP_STEP) {                             // FP64 propagation
     add(W, N * N, G);
     Spins sp{};
@@ -850,7 +857,8 @@ static int cisd_run(const trot_cisd* c, int W, const double2* w, CisdBuffers& b,
                             cisd_splitk(W, G, N * N)));
   }
   if (stage == 1) return TROT_OK;
-  const int nch = cisd_chunks(G);
+  b.nchunk = cisd_chunks(G);
+  const int nch = b.nchunk;
   if (c->gl_precision == TROT_MIXED) {
     const size_t smem2 = cisd_gamma_f32_smem(N, n);
     cudaFuncSetAttribute(cisd_gamma_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
@@ -866,6 +874,10 @@ static int cisd_run(const trot_cisd* c, int W, const double2* w, CisdBuffers& b,
     TROT_TIMED("cisd_gl_tc", st, launch_split3_gemm(W * n, N, kp, np, b.green, b.glimg, b.glq, b.gld, b.status, st));
     CISD_LAUNCH("cisd_gamma_f32", cisd_gamma_f32_kernel, dim3(nch, W), 256, smem2, st, N, n, v, G, b.green, b.gld, np,
                 b.rd, b.lc, b.p2, b.ci1g1, b.xg, b.gpart);
+  } else if (b.dg.p && cisd_gamma_digits(c)) {
+    b.nchunk = cisd_gamma_dg_chunks(G);
+    CisdGammaArgs ga{W, N, n, v, G, b.green, c->chol, c->lci1, b.p2, b.ci1g1, b.xg, b.gpart};
+    TROT_TIMED("cisd_gamma", st, launch_cisd_gamma_dg(ga, b.dg, st));
   } else {
     const size_t smem2 = cisd_gamma_smem(N, n);
     cudaFuncSetAttribute(cisd_gamma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
@@ -954,7 +966,7 @@ int trot_cisd_local_energy(const trot_cisd* c, int W, const double* walkers, dou
   TROT_TRY(carve_cisd_ws(c, W, TROT_OP_LOCAL_ENERGY, ws, ws_bytes, 0, cv, b));
   cudaStream_t st = (cudaStream_t)stream;
   TROT_TRY(cisd_run(c, W, (const double2*)walkers, b, 2, st));
-  cisd_energy_kernel<<<W, 256, 0, st>>>(c->nchol, cisd_chunks(c->nchol), c->h0, b.wsc, b.hg2, b.lg, b.lcs,
+  cisd_energy_kernel<<<W, 256, 0, st>>>(c->nchol, b.nchunk, c->h0, b.wsc, b.hg2, b.lg, b.lcs,
                                         b.gpart, b.l2part, (double2*)out, b.status);
   TROT_CHECK_LAUNCH("cisd_energy_kernel");
   return TROT_OK;
@@ -1029,7 +1041,7 @@ int trot_cisd_prop_step(const trot_cisd* c, const trot_system* prop, const trot_
   CISD_LAUNCH("cisd_fb", cisd_fb_kernel, (unsigned)((wg + 255) / 256), 256, 0, st, W, G, b.wsc, b.lg, b.lcs,
               b.fb);
   if (energy_out)
-    CISD_LAUNCH("cisd_energy", cisd_energy_kernel, W, 256, 0, st, G, cisd_chunks(G), c->h0, b.wsc, b.hg2, b.lg,
+    CISD_LAUNCH("cisd_energy", cisd_energy_kernel, W, 256, 0, st, G, b.nchunk, c->h0, b.wsc, b.hg2, b.lg,
                 b.lcs, b.gpart, b.l2part, (double2*)energy_out, b.status);
   // 2. shifted fields, 3. VHS, 4. propagation in place
   TROT_TIMED("fields", st,

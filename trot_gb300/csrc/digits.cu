@@ -287,6 +287,11 @@ struct DgArgs {
   int nrt, ntile;        // 128-row tiles and 32-row tiles (per batch)
   int nbatch, bB;        // batches: ntile 32-row tiles each, bB 128-row tiles (0: all share them)
   long long cstride;     // and cstride complex outputs
+  // PAIR: outputs p >= psplit (0: none) go to C2 (row stride ldc2, batches cstride2 apart), column p - psplit; rows m
+  // are stored at (m % perm) permn + m / perm (perm = 0: at m)
+  int psplit, perm, permn;
+  double2* C2;
+  long long ldc2, cstride2;
   int nk16, shift;       // K16 steps; the outputs' integers are in units 2^(eA + eB - 54 + shift)
   double2* C;
   long long ldc;
@@ -532,6 +537,13 @@ __global__ void __launch_bounds__(kDgThreads, 1) dg_gemm_kernel(DgArgs a) {
           const double w = __shfl_xor_sync(0xffffffffu, v.y, 1);
           if (m0r + y < a.M && n < a.Nn) {
             double* od = reinterpret_cast<double*>(o);
+            if (a.perm | a.psplit) {
+              const int m = m0r + y, pp = n >> 1;
+              const long long mm = a.perm ? (long long)(m % a.perm) * a.permn + m / a.perm : m;
+              od = reinterpret_cast<double*>(a.psplit && pp >= a.psplit
+                                                 ? a.C2 + bt * a.cstride2 + mm * a.ldc2 + (pp - a.psplit)
+                                                 : a.C + bt * a.cstride + mm * a.ldc + pp);
+            }
             if (n & 1) od[1] = v.x + w;
             else od[0] = v.x - w;
           }
@@ -1066,6 +1078,174 @@ int adjoint_dg_gv(const DgAdjoint& d, const double2* S, long long sstride, const
   a.cstride = (long long)N * N; a.nk16 = (d.K2 + 15) / 16; a.shift = 1;  // K2 <= 7 x 64
   a.C = gv; a.ldc = N; a.salpha = 1; a.status = d.status;
   return dg_gemm<true>(a, st);
+}
+
+// ------------------------------------------------------------------ CISD per-vector terms
+// Per walker and Cholesky vector (L = chol_g, R = L[:n, :]): lg1 = R G^T, B = G lci1_g, gl = G L, glgp = gl gp and
+// sum gl o lci2_green = <lg1, gl P2> (lci2_green = lg1 P2^T).  For a chunk of walkers: three products of the rows of G
+// (all vectors), then gl's rows against [gp | P2] (N columns per walker), so that no contraction over orbitals is left on
+// the FP64 pipe; cisd_pairs_kernel sums what is left, 4 n^2 (n + 3) FMAs per vector.  Chunks keep gl (64 MB) in L2.
+// 41 orbitals, 6 + 6 electrons, 164 vectors, 96 walkers: 1.74 ms with every contraction on the FP64 pipe (per vector, in
+// shared memory), 0.38 ms like this.
+static constexpr int kPairsChunk = 64;
+
+int cisd_gamma_dg_chunks(int G) { return (G + kPairsChunk - 1) / kPairsChunk; }
+
+// Q[b][i][c]: gp (c < v: rows i < n hold x[i][c] = G[i][n + c], row n + c holds -1) and P2 (c >= v)
+__global__ void cisd_q_kernel(int N, int n, int v, const double2* __restrict__ green, const double2* __restrict__ p2,
+                              double2* __restrict__ Q) {
+  const int b = blockIdx.y;
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < N * N; e += gridDim.x * blockDim.x) {
+    const int i = e / N, c = e - i * N;
+    double2 x = cmk(0.0, 0.0);
+    if (c >= v) x = p2[((size_t)b * N + i) * n + c - v];
+    else if (i < n) x = green[((size_t)b * n + i) * N + n + c];
+    else if (i - n == c) x = cmk(-1.0, 0.0);
+    Q[(size_t)b * N * N + e] = x;
+  }
+}
+
+// F1[(b, q)][(g, p)] = lg1[p][q], F2[(b, p)][(g, q)] = B[p][q], F3[b][g][p][k] = (gl P2)[p][k]:
+// [0] sum lg1 o lg1^T, [1] tr(lg1 lg1 ci1g1), [2] sum B o lg1, [3] sum F3 o lg1
+__global__ void __launch_bounds__(128)
+cisd_pairs_kernel(int n, int G, int gsub, int nchunk, const double2* __restrict__ F1, const double2* __restrict__ F2,
+                  const double2* __restrict__ F3, const double2* __restrict__ ci1g1, double2* __restrict__ gpart) {
+  extern __shared__ double2 sm[];
+  __shared__ double2 red[32];
+  const int chunk = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, nt = blockDim.x, nn = n * n;
+  double2* C1 = sm;       // n x n
+  double2* A = C1 + nn;   // gsub x n x n
+  for (int e = tid; e < nn; e += nt) C1[e] = ci1g1[(size_t)b * nn + e];
+  const size_t ld = (size_t)G * n;
+  const double2* f1 = F1 + (size_t)b * n * ld;
+  const double2* f2 = F2 + (size_t)b * n * ld;
+  const double2* f3 = F3 + (size_t)b * G * nn;
+  double2 s0 = cmk(0.0, 0.0), s1 = cmk(0.0, 0.0), s2 = cmk(0.0, 0.0), s3 = cmk(0.0, 0.0);
+  const int g0 = chunk * kPairsChunk, g1 = min(G, g0 + kPairsChunk);
+  for (int gs = g0; gs < g1; gs += gsub) {
+    const int cols = min(gsub, g1 - gs) * n, items = cols * n;
+    __syncthreads();
+    for (int e = tid; e < items; e += nt) {  // (q, g, p), p fastest
+      const int q = e / cols, r = e - q * cols, g = r / n, p = r - g * n;
+      A[g * nn + p * n + q] = f1[(size_t)q * ld + (size_t)gs * n + r];
+    }
+    __syncthreads();
+    for (int e = tid; e < items; e += nt) {
+      const int g = e / nn, pq = e - g * nn, p = pq / n, q = pq - p * n;
+      const double2* Ag = A + g * nn;
+      const double2 apq = Ag[pq];
+      double2 t = cmk(0.0, 0.0);
+      for (int a = 0; a < n; ++a) cfma(t, Ag[q * n + a], C1[a * n + p]);
+      cfma(s0, apq, Ag[q * n + p]);
+      cfma(s1, apq, t);
+      cfma(s2, apq, f2[(size_t)p * ld + (size_t)(gs + g) * n + q]);
+      cfma(s3, apq, f3[(size_t)(gs + g) * nn + pq]);
+    }
+  }
+  s0 = block_sum2(s0, red);
+  s1 = block_sum2(s1, red);
+  s2 = block_sum2(s2, red);
+  s3 = block_sum2(s3, red);
+  if (tid == 0) {
+    double2* o = gpart + ((size_t)b * nchunk + chunk) * 4;
+    o[0] = s0; o[1] = s1; o[2] = s2; o[3] = s3;
+  }
+}
+
+static size_t cgd_chunk(size_t W, size_t N, size_t n, size_t G) {
+  const size_t wc = std::max<size_t>(1, (size_t(64) << 20) / (n * G * N * sizeof(double2)));
+  return std::min(wc, W);
+}
+
+struct CgdBuffers {
+  uint16_t *icol, *irow, *ilc, *ig, *igl, *iq;
+  int16_t *ecol, *erow, *elc, *eg, *egl, *eq;
+  double2 *gl, *F1, *F2, *F3, *Q;
+};
+static size_t cgd_carve(CgdBuffers& b, size_t wc, size_t N, size_t n, size_t G, void* base) {
+  char* p0 = reinterpret_cast<char*>(((uintptr_t)base + 255) & ~(uintptr_t)255);
+  char* p = p0;
+  auto take = [&](size_t k) {
+    char* r = p;
+    p += (k + 255) & ~(size_t)255;
+    return r;
+  };
+  const size_t rb = kDgRowBytes((N + 15) / 16);
+  const size_t col = adj_rows(G * N, 128), row = adj_rows(G * n, 128), g = adj_rows(2 * wc * n, kDgP);
+  const size_t gl = wc * adj_rows(2 * G * n, kDgP), q = wc * adj_rows(2 * N, 128);
+  b.icol = (uint16_t*)take(col * rb); b.irow = (uint16_t*)take(row * rb); b.ilc = (uint16_t*)take(row * rb);
+  b.ig = (uint16_t*)take(g * rb); b.igl = (uint16_t*)take(gl * rb); b.iq = (uint16_t*)take(q * rb);
+  b.ecol = (int16_t*)take(col * 2); b.erow = (int16_t*)take(row * 2); b.elc = (int16_t*)take(row * 2);
+  b.eg = (int16_t*)take(g * 2); b.egl = (int16_t*)take(gl * 2); b.eq = (int16_t*)take(q * 2);
+  b.gl = (double2*)take(wc * n * G * N * sizeof(double2));
+  b.F1 = (double2*)take(wc * n * n * G * sizeof(double2));
+  b.F2 = (double2*)take(wc * n * n * G * sizeof(double2));
+  b.F3 = (double2*)take(wc * n * n * G * sizeof(double2));
+  b.Q = (double2*)take(wc * N * N * sizeof(double2));
+  return (size_t)(p - p0) + 256;
+}
+
+size_t cisd_gamma_dg_bytes(size_t W, size_t N, size_t n, size_t G) {
+  CgdBuffers b;
+  return cgd_carve(b, cgd_chunk(W, N, n, G), N, n, G, nullptr);
+}
+
+int launch_cisd_gamma_dg(const CisdGammaArgs& c, const DgScratch& s, cudaStream_t st) {
+  const int W = c.W, N = c.N, n = c.n, v = c.v, G = c.G, nn = n * n;
+  const int wc = (int)cgd_chunk(W, N, n, G);
+  CgdBuffers b;
+  if (s.bytes < cgd_carve(b, wc, N, n, G, s.p)) { set_error("CISD terms: scratch %zu", s.bytes); return TROT_ERR_WORKSPACE_TOO_SMALL; }
+  // rows (g, i) = columns of L_g; (g, p) = rows p < n of L_g; (g, a) = columns of lci1_g
+  DgSrc sc = dg_src(c.chol, 0, N, N, 128, 1, N, b.icol, b.ecol);
+  sc.rpad = N; sc.nblk = G; sc.bstride = (long long)N * N;
+  TROT_TRY(dg_rows_launch(sc, (int)(adj_rows((size_t)G * N, 128) / 8), st));
+  DgSrc sr = dg_src(c.chol, 0, n, N, 128, N, 1, b.irow, b.erow);
+  sr.rpad = n; sr.nblk = G; sr.bstride = (long long)N * N;
+  TROT_TRY(dg_rows_launch(sr, (int)(adj_rows((size_t)G * n, 128) / 8), st));
+  DgSrc sl = dg_src(c.lci1, 0, n, N, 128, 1, n, b.ilc, b.elc);
+  sl.rpad = n; sl.nblk = G; sl.bstride = (long long)N * n;
+  TROT_TRY(dg_rows_launch(sl, (int)(adj_rows((size_t)G * n, 128) / 8), st));
+  const int gsub = std::max(1, std::min(kPairsChunk, 256 / nn)), nchunk = cisd_gamma_dg_chunks(G);
+  const size_t smem = (size_t)(gsub + 1) * nn * sizeof(double2);
+  if (smem > 40 * 1024) cudaFuncSetAttribute(cisd_pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const int qpad = (int)adj_rows(2 * N, 128), glpad = (int)adj_rows((size_t)2 * G * n, kDgP);
+  for (int w0 = 0; w0 < W; w0 += wc) {
+    const int wn = std::min(wc, W - w0);
+    const double2* gr = c.green + (size_t)w0 * n * N;
+    const int tiles = (2 * wn * n + kDgP - 1) / kDgP;
+    TROT_TRY(dg_rows_launch(dg_src(reinterpret_cast<const double*>(gr), 1, 2 * wn * n, N, kDgP, 2ll * N, 2, b.ig, b.eg),
+                            tiles * 4, st));
+    DgArgs a{};
+    a.imgA = b.ig; a.exA = b.eg; a.M = wn * n; a.ntile = tiles; a.nbatch = 1;
+    a.nk16 = (N + 15) / 16; a.shift = 1; a.salpha = 1; a.status = s.status;
+    a.imgB = b.irow; a.exB = b.erow; a.Nn = G * n; a.nrt = (G * n + 127) / 128; a.C = b.F1; a.ldc = (long long)G * n;
+    TROT_TRY(dg_gemm<false>(a, st));
+    a.imgB = b.ilc; a.exB = b.elc; a.C = b.F2;
+    TROT_TRY(dg_gemm<false>(a, st));
+    a.imgB = b.icol; a.exB = b.ecol; a.Nn = G * N; a.nrt = (G * N + 127) / 128; a.C = b.gl; a.ldc = (long long)G * N;
+    TROT_TRY(dg_gemm<false>(a, st));
+    // gl rows (p, g) of each walker against the columns of [gp | P2]
+    cisd_q_kernel<<<dim3((N * N + 255) / 256, wn), 256, 0, st>>>(N, n, v, gr, c.p2 + (size_t)w0 * N * n, b.Q);
+    TROT_CHECK_LAUNCH("cisd_q_kernel");
+    DgSrc sq = dg_src(reinterpret_cast<const double*>(b.Q), 1, 2 * N, N, 128, 2, 2ll * N, b.iq, b.eq);
+    sq.rpad = qpad; sq.nblk = wn; sq.bstride = 2ll * N * N;
+    TROT_TRY(dg_rows_launch(sq, wn * (qpad / 8), st));
+    DgSrc s2 = dg_src(reinterpret_cast<const double*>(b.gl), 1, 2 * G * n, N, kDgP, 2ll * N, 2, b.igl, b.egl);
+    s2.rpad = glpad; s2.nblk = wn; s2.bstride = 2ll * n * G * N;
+    TROT_TRY(dg_rows_launch(s2, wn * (glpad / 8), st));
+    DgArgs q{};
+    q.imgA = b.igl; q.exA = b.egl; q.imgB = b.iq; q.exB = b.eq;
+    q.M = G * n; q.ntile = glpad / kDgP; q.Nn = 2 * N; q.nrt = q.bB = qpad / 128; q.nbatch = wn;
+    q.nk16 = (N + 15) / 16; q.shift = 1; q.salpha = 1; q.status = s.status;
+    q.C = c.xg + (size_t)w0 * G * n * v; q.ldc = v; q.cstride = (long long)G * n * v;
+    q.C2 = b.F3; q.ldc2 = n; q.cstride2 = (long long)G * nn; q.psplit = v;
+    q.perm = G; q.permn = n;
+    TROT_TRY(dg_gemm<true>(q, st));
+    cisd_pairs_kernel<<<dim3(nchunk, wn), 128, smem, st>>>(n, G, gsub, nchunk, b.F1, b.F2, b.F3,
+                                                           c.ci1g1 + (size_t)w0 * nn, c.gpart + (size_t)w0 * nchunk * 4);
+    TROT_CHECK_LAUNCH("cisd_pairs_kernel");
+  }
+  return TROT_OK;
 }
 
 }  // namespace trot

@@ -57,4 +57,20 @@ int adjoint_dg_from_rows(const DgAdjoint& d, DgOperand op, const double2* src, l
 int adjoint_dg_gv(const DgAdjoint& d, const double2* S, long long sstride, const double2* U, long long ustride,
                   double2* gv, cudaStream_t st);
 
+// The CISD energy's per-vector terms (cisd_gamma_kernel's) with every contraction over orbitals as a digit product:
+// xg[b][g][p][t] = glgp, gpart[b][chunk][4] the four sums (cisd_gamma_dg_chunks(G) chunks per walker).
+struct CisdGammaArgs {
+  int W, N, n, v, G;
+  const double2* green;   // (W, n, N)
+  const double* chol;     // (G, N, N)
+  const double* lci1;     // (G, N, n)
+  const double2* p2;      // (W, N, n)
+  const double2* ci1g1;   // (W, n, n)
+  double2* xg;
+  double2* gpart;
+};
+int cisd_gamma_dg_chunks(int G);
+size_t cisd_gamma_dg_bytes(size_t W, size_t N, size_t n, size_t G);
+int launch_cisd_gamma_dg(const CisdGammaArgs& c, const DgScratch& s, cudaStream_t st);
+
 }  // namespace trot

@@ -45,7 +45,7 @@ struct CisdBuffers {
   ff *rd, *lc;                  // chol rows < n transposed, lci1: float-float (G, N, n)   (FP32 gl)
   uint16_t *glimg, *glq;        // split3 images of chol (rows (g, j), K = i) and of G     (FP32 gl)
   float* gld;                   // gl = G L_g for all (walker, p) x (g, j), FP32           (FP32 gl)
-  double2* xg;                  // glgp rows (W G, n v)
+  double2* xg;                  // glgp rows (W G, n v); FP32 complex when both gl and l2ci2 are mixed
   double2* y;                   // xg ci2m (W G, n v)    (FP64 l2ci2)
   uint16_t* xq;                 // split3 image of xg    (mixed l2ci2)
   float* yd;                    // xg ci2m, FP32         (mixed l2ci2)
@@ -451,7 +451,8 @@ TROT_D ffc ffc_quad_sum(ffc a) {
 __global__ void __launch_bounds__(256, 4)
 cisd_gamma_f32_kernel(int N, int n, int v, int G, const double2* __restrict__ green, const float* __restrict__ gld,
                       int ldd, const ff* __restrict__ rd, const ff* __restrict__ lc, const double2* __restrict__ p2,
-                      const double2* __restrict__ ci1g1, double2* __restrict__ xg, double2* __restrict__ gpart) {
+                      const double2* __restrict__ ci1g1, double2* __restrict__ xg, float2* __restrict__ xf,
+                      double2* __restrict__ gpart) {
   extern __shared__ double2 sm[];
   __shared__ double2 red[32];
   const int chunk = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, nt = blockDim.x;
@@ -562,7 +563,7 @@ cisd_gamma_f32_kernel(int N, int n, int v, int G, const double2* __restrict__ gr
     s1 = ffc_norm(s1);
     s2 = ffc_norm(s2);
     s3 = ffc_norm(s3);
-    double2* xo = xg + ((size_t)b * G + gg) * n * v;
+    const size_t xo = ((size_t)b * G + gg) * n * v;
     for (int e = tid; e < n * v; e += nt) {
       const int p = e / v, t = e % v;
       const float2 gl = GLf[p * N + n + t];
@@ -572,7 +573,8 @@ cisd_gamma_f32_kernel(int N, int n, int v, int G, const double2* __restrict__ gr
         ar = fmaf(a.x, x.x, fmaf(-a.y, x.y, ar));
         ai = fmaf(a.x, x.y, fmaf(a.y, x.x, ai));
       }
-      xo[e] = make_double2(f2d_bits(ar), f2d_bits(ai));
+      if (xf) xf[xo + e] = make_float2(ar, ai);
+      else xg[xo + e] = make_double2(f2d_bits(ar), f2d_bits(ai));
     }
   }
   double2 d0 = block_sum2(ffc_d(s0), red);
@@ -594,8 +596,12 @@ cisd_gamma_f32_kernel(int N, int n, int v, int G, const double2* __restrict__ gr
 // Y is FP32 and X is rounded to FP32 (by integer operations): FP32 complex products,
 // summed per thread in float-float and across the block in FP64 (no FP64-pipe work
 // per element)
+TROT_D float2 cisd_x32(double2 x) { return make_float2(d2f_bits(x.x), d2f_bits(x.y)); }
+TROT_D float2 cisd_x32(float2 x) { return x; }
+
+template <class C2>
 __global__ void __launch_bounds__(256)
-cisd_l2_reduce_tc_kernel(int G, int nv, int ldy, const double2* __restrict__ xg, const float* __restrict__ yd,
+cisd_l2_reduce_tc_kernel(int G, int nv, int ldy, const C2* __restrict__ xg, const float* __restrict__ yd,
                          double2* __restrict__ part) {
   __shared__ double2 red[32];
   const int c = blockIdx.x, b = blockIdx.y, nparts = gridDim.x;
@@ -604,12 +610,12 @@ cisd_l2_reduce_tc_kernel(int G, int nv, int ldy, const double2* __restrict__ xg,
   ff ar{0.f, 0.f}, ai{0.f, 0.f};
   for (int g = g0 + warp; g < g1; g += nw) {
     const size_t r = (size_t)b * G + g;
-    const double2* xr = xg + r * nv;
+    const C2* xr = xg + r * nv;
     const float* y0 = yd + 2 * r * (size_t)ldy;
     const float* y1 = y0 + ldy;
     for (int k = lane; k < nv; k += 32) {
-      const double2 xv = xr[k];
-      const float xre = d2f_bits(xv.x), xim = d2f_bits(xv.y);
+      const float2 xv = cisd_x32(xr[k]);
+      const float xre = xv.x, xim = xv.y;
       const float yr = y0[k], yi = y1[k];
       const float pr = fmaf(xre, yr, __fmul_rn(-xim, yi)), pi = fmaf(xre, yi, __fmul_rn(xim, yr));
       const ff tr = ff_two_sum(ar.hi, pr), ti = ff_two_sum(ai.hi, pi);
@@ -871,9 +877,10 @@ static int cisd_run(const trot_cisd* c, int W, const double2* w, CisdBuffers& b,
     const size_t nimg = (size_t)np * kp;
     CISD_LAUNCH("cisd_gl_tc", cisd_gl_image_kernel, (unsigned)std::min<size_t>((nimg + 255) / 256, 152 * 16), 256, 0,
                 st, N, G, kp, np, c->chol, b.glimg);
-    TROT_TIMED("cisd_gl_tc", st, launch_split3_gemm(W * n, N, kp, np, b.green, b.glimg, b.glq, b.gld, b.status, st));
+    TROT_TIMED("cisd_gl_tc", st, launch_split3_gemm(W * n, N, kp, G * N, np, b.green, b.glimg, b.glq, b.gld, b.status, st));
     CISD_LAUNCH("cisd_gamma_f32", cisd_gamma_f32_kernel, dim3(nch, W), 256, smem2, st, N, n, v, G, b.green, b.gld, np,
-                b.rd, b.lc, b.p2, b.ci1g1, b.xg, b.gpart);
+                b.rd, b.lc, b.p2, b.ci1g1, b.xg,
+                c->l2ci2_precision == TROT_MIXED ? reinterpret_cast<float2*>(b.xg) : nullptr, b.gpart);
   } else if (b.dg.p && cisd_gamma_digits(c)) {
     b.nchunk = cisd_gamma_dg_chunks(G);
     CisdGammaArgs ga{W, N, n, v, G, b.green, c->chol, c->lci1, b.p2, b.ci1g1, b.xg, b.gpart};
@@ -885,9 +892,17 @@ static int cisd_run(const trot_cisd* c, int W, const double2* w, CisdBuffers& b,
                 b.m2, b.ci1g1, b.xg, b.gpart);
   }
   if (c->l2ci2_precision == TROT_MIXED) {
+    if (c->gl_precision == TROT_MIXED) {  // xg holds FP32 values
+      const float2* xf = reinterpret_cast<const float2*>(b.xg);
+      TROT_TIMED("cisd_l2ci2_tc", st,
+                 launch_split3_gemm(W * G, nv, c->nvpad, nv, c->ncpad, xf, c->ci2_image, b.xq, b.yd, b.status, st));
+      CISD_LAUNCH("cisd_l2_reduce", cisd_l2_reduce_tc_kernel<float2>, dim3(kL2Parts, W), 256, 0, st, G, nv, c->ncpad,
+                  xf, b.yd, b.l2part);
+      return TROT_OK;
+    }
     TROT_TIMED("cisd_l2ci2_tc", st,
-               launch_split3_gemm(W * G, nv, c->nvpad, c->ncpad, b.xg, c->ci2_image, b.xq, b.yd, b.status, st));
-    CISD_LAUNCH("cisd_l2_reduce", cisd_l2_reduce_tc_kernel, dim3(kL2Parts, W), 256, 0, st, G, nv, c->ncpad, b.xg,
+               launch_split3_gemm(W * G, nv, c->nvpad, nv, c->ncpad, b.xg, c->ci2_image, b.xq, b.yd, b.status, st));
+    CISD_LAUNCH("cisd_l2_reduce", cisd_l2_reduce_tc_kernel<double2>, dim3(kL2Parts, W), 256, 0, st, G, nv, c->ncpad, b.xg,
                 b.yd, b.l2part);
     return TROT_OK;
   }

@@ -817,33 +817,74 @@ static constexpr uint32_t kVStage = 6 * kVSlice;          // 3 X + 3 L slices: 9
 static constexpr int kVThreads = 160;                     // 4 epilogue warps + 1 producer warp
 static constexpr size_t kVhsSmem = 2 * (size_t)kVStage + 16 * 8 + 1024;
 
-// Shifted fields -> 3-term bf16 split in the X image layout.
-__global__ void x_slices_kernel(int W, int G, int gpad, int mpad, const double2* __restrict__ xs,
-                                uint16_t* __restrict__ xq) {
-  const int nkc = gpad / kVK;
-  const size_t total = (size_t)mpad * gpad;
+__device__ __forceinline__ void split3_bf16(float x, uint16_t& h, uint16_t& m, uint16_t& l) {
+  const __nv_bfloat16 bh = __float2bfloat16_rn(x);
+  const float r1 = x - __bfloat162float(bh);
+  const __nv_bfloat16 bm = __float2bfloat16_rn(r1);
+  const __nv_bfloat16 bl = __float2bfloat16_rn(r1 - __bfloat162float(bm));
+  h = *reinterpret_cast<const uint16_t*>(&bh);
+  m = *reinterpret_cast<const uint16_t*>(&bm);
+  l = *reinterpret_cast<const uint16_t*>(&bl);
+}
+
+// Complex rows (FP64, or FP32 as the CISD kernels keep them) -> 3-term bf16 split of their FP32 values in the X image
+// layout, row 2b + c = component c of row b.  A thread takes eight k of one complex row: a warp reads four rows x 64
+// values and writes 1 KB runs of each slice (one 2-byte store per element and slice took three times as long).
+__device__ __forceinline__ float x_val(double v) { return (float)v; }
+__device__ __forceinline__ float x_val(float v) { return v; }
+
+template <class C2>
+__global__ void __launch_bounds__(256)
+x_slices_kernel(int W, int G, int gpad, int mpad, const C2* __restrict__ xs, uint16_t* __restrict__ xq) {
+  const int nkc = gpad / kVK, nkg = gpad / 8;
+  const size_t total = (size_t)(mpad / 8) * nkg * 4;  // (group of four rows, k group, row), the row fastest
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-    const int row = (int)(e / gpad), g = (int)(e % gpad);
-    const int b = row >> 1, c = row & 1;
-    float x = 0.f;
-    if (b < W && g < G) {
-      const double2 v = xs[(size_t)b * G + g];
-      x = (float)(c ? v.y : v.x);
+    const size_t t = e >> 2;
+    const int grp = (int)(t / nkg), kg = (int)(t - (size_t)grp * nkg), b = grp * 4 + (int)(e & 3), g0 = kg * 8;
+    uint32_t w[2][3][4];  // [component][slice]
+#pragma unroll
+    for (int i = 0; i < 8; i += 2) {
+      float re[2], im[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int g = g0 + i + u;
+        re[u] = im[u] = 0.f;
+        if (b < W && g < G) {
+          const C2 v = xs[(size_t)b * G + g];
+          re[u] = x_val(v.x);
+          im[u] = x_val(v.y);
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint16_t h[2], m[2], l[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) split3_bf16(c ? im[u] : re[u], h[u], m[u], l[u]);
+        w[c][0][i / 2] = (uint32_t)h[0] | ((uint32_t)h[1] << 16);
+        w[c][1][i / 2] = (uint32_t)m[0] | ((uint32_t)m[1] << 16);
+        w[c][2][i / 2] = (uint32_t)l[0] | ((uint32_t)l[1] << 16);
+      }
     }
-    const __nv_bfloat16 h = __float2bfloat16_rn(x);
-    const float r1 = x - __bfloat162float(h);
-    const __nv_bfloat16 m = __float2bfloat16_rn(r1);
-    const __nv_bfloat16 l = __float2bfloat16_rn(r1 - __bfloat162float(m));
-    const int mt = row >> 7, rr = row & 127, kc = g / kVK, kk = g % kVK;
-    const size_t base = (((size_t)mt * nkc + kc) * 3) * (kVSlice / 2) + tc::tile_off(rr, kk) / 2;
-    xq[base] = *reinterpret_cast<const uint16_t*>(&h);
-    xq[base + kVSlice / 2] = *reinterpret_cast<const uint16_t*>(&m);
-    xq[base + kVSlice] = *reinterpret_cast<const uint16_t*>(&l);
+    const int row = 2 * b, mt = row >> 7, rr = row & 127, kc = g0 / kVK, kk = g0 % kVK;
+    unsigned char* o = reinterpret_cast<unsigned char*>(xq) + (((size_t)mt * nkc + kc) * 3) * kVSlice + tc::tile_off(rr, kk);
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+      for (int sl = 0; sl < 3; ++sl)
+        *reinterpret_cast<uint4*>(o + (size_t)sl * kVSlice + c * 16) = make_uint4(w[c][sl][0], w[c][sl][1], w[c][sl][2], w[c][sl][3]);
   }
 }
 
+template <class C2>
+static int launch_x_slices(int W, int G, int gpad, int mpad, const C2* xs, uint16_t* xq, cudaStream_t st) {
+  const size_t blocks = ((size_t)(mpad / 8) * (gpad / 8) * 4 + 255) / 256;
+  x_slices_kernel<<<(unsigned)std::min<size_t>(blocks, 152 * 32), 256, 0, st>>>(W, G, gpad, mpad, xs, xq);
+  TROT_CHECK_LAUNCH("x_slices_kernel");
+  return TROT_OK;
+}
+
 __global__ void __launch_bounds__(kVThreads, 1)
-vhs_gemm_kernel(int mtiles, int ntiles, int gpad, int n2pad, const uint16_t* __restrict__ xq,
+vhs_gemm_kernel(int mtiles, int ntiles, int gpad, int n2pad, int ncols, int kvalid, const uint16_t* __restrict__ xq,
                 const uint16_t* __restrict__ lq, float* __restrict__ D, int* status) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = smem_raw + ((1024 - (tc::smem_u32(smem_raw) & 1023)) & 1023);
@@ -875,15 +916,17 @@ vhs_gemm_kernel(int mtiles, int ntiles, int gpad, int n2pad, const uint16_t* __r
   if (warp == 4) {
     if (lane == 0) {
       bool ok = true;
-      const uint32_t idesc = tc::idesc_bf16_f32(128, 128);
       const uint32_t su = tc::smem_u32(base);
       int chunk = 0;  // global K-chunk counter of this CTA (stage = chunk & 1)
       int nt = 0;     // tiles of this CTA
       for (int tl = blockIdx.x; tl < ntot && ok; tl += gridDim.x, ++nt) {
         const int mt = tl / ntiles, ntl = tl % ntiles;
         const int abuf = nt & 1;
+        // a last tile of few valid columns takes narrow MMAs, the last chunk only its valid K16 steps
+        const int nv = min(128, (ncols - ntl * 128 + 15) / 16 * 16);
+        const uint32_t idesc = tc::idesc_bf16_f32(128, nv);
         if (nt >= 2) ok = tc::mbar_wait(&acc_empty[abuf], (uint32_t)(((nt - 2) / 2) & 1));
-        for (int kc = 0; kc < nkc && ok; ++kc, ++chunk) {
+        for (int kc = 0; kc * kVK < kvalid && ok; ++kc, ++chunk) {  // the padding past K is not multiplied
           const int st = chunk & 1;
           if (chunk >= 2) ok = tc::mbar_wait(&empty[st], (uint32_t)(((chunk - 2) / 2) & 1));
           if (!ok) break;
@@ -899,13 +942,14 @@ vhs_gemm_kernel(int mtiles, int ntiles, int gpad, int n2pad, const uint16_t* __r
           const uint64_t s0d = tc::smem_desc(su + (uint32_t)st * kVStage, 128, 1024);
           const uint32_t slo = (uint32_t)s0d, dhi = (uint32_t)(s0d >> 32);  // A and B share the high word
           const uint32_t dcol = taddr + (uint32_t)(abuf * 128);
+          const int nks = min(kVK / 16, (kvalid - kc * kVK + 15) / 16);
 #pragma unroll
           for (int t = 0; t < 3; ++t)
 #pragma unroll
             for (int u = 0; t + u <= 2; ++u)
 #pragma unroll
               for (int ks = 0; ks < kVK / 16; ++ks)
-                tc::mma_bf16_lo(dcol, slo + (uint32_t)((t * kVSlice + ks * 256) >> 4),
+                if (ks < nks) tc::mma_bf16_lo(dcol, slo + (uint32_t)((t * kVSlice + ks * 256) >> 4),
                                 slo + (uint32_t)(((3 + u) * kVSlice + ks * 256) >> 4), dhi, idesc,
                                 (kc | t | u | ks) ? 1u : 0u);
           tc::mma_commit(&empty[st]);
@@ -933,7 +977,8 @@ vhs_gemm_kernel(int mtiles, int ntiles, int gpad, int n2pad, const uint16_t* __r
       tc::fence_after_sync();
       const uint32_t trow = taddr + ((uint32_t)(warp * 32) << 16) + (uint32_t)(abuf * 128);
       float* drow = D + (size_t)(mt * 128 + warp * 32 + lane) * n2pad + (size_t)ntl * 128;
-      for (int c = 0; c < 8; ++c) {
+      const int nc16 = min(8, (ncols - ntl * 128 + 15) / 16);  // column groups with valid outputs
+      for (int c = 0; c < nc16; ++c) {
         float v[16];
         tc::tmem_ld16(trow + c * 16, v);
         float4* d4 = reinterpret_cast<float4*>(drow + c * 16);
@@ -1172,16 +1217,6 @@ struct TrotTcArgs {
   const uint16_t* eimg;  // (4 chunks, 3, 128, 32) bf16 image of E
   int* status;
 };
-
-__device__ __forceinline__ void split3_bf16(float x, uint16_t& h, uint16_t& m, uint16_t& l) {
-  const __nv_bfloat16 bh = __float2bfloat16_rn(x);
-  const float r1 = x - __bfloat162float(bh);
-  const __nv_bfloat16 bm = __float2bfloat16_rn(r1);
-  const __nv_bfloat16 bl = __float2bfloat16_rn(r1 - __bfloat162float(bm));
-  h = *reinterpret_cast<const uint16_t*>(&bh);
-  m = *reinterpret_cast<const uint16_t*>(&bm);
-  l = *reinterpret_cast<const uint16_t*>(&bl);
-}
 
 // B element (row j, k < 128) = x as 3 slices; B image = [kchunk][slice][NB rows][32]
 template <int NB>
@@ -1655,21 +1690,31 @@ static void vhs_gemm_attr() {
   }
 }
 
-int launch_split3_gemm(int rows, int K, int kpad, int npad, const double2* x, const uint16_t* b_image,
+template <class C2>
+static int split3_gemm(int rows, int K, int kpad, int ncols, int npad, const C2* x, const uint16_t* b_image,
                        uint16_t* xq, float* D, int* status, cudaStream_t st) {
-  if (kpad % kVK || npad % 128 || K > kpad || rows <= 0) {
-    set_error("split3 GEMM: bad layout rows=%d K=%d kpad=%d npad=%d", rows, K, kpad, npad);
+  if (kpad % kVK || npad % 128 || K > kpad || K <= 0 || ncols <= 0 || ncols > npad || rows <= 0) {
+    set_error("split3 GEMM: bad layout rows=%d K=%d kpad=%d ncols=%d npad=%d", rows, K, kpad, ncols, npad);
     return TROT_ERR_BAD_SHAPE;
   }
   const int mpad = split3_mpad(rows);
-  x_slices_kernel<<<152 * 8, 256, 0, st>>>(rows, K, kpad, mpad, x, xq);
-  TROT_CHECK_LAUNCH("x_slices_kernel");
+  TROT_TRY(launch_x_slices(rows, K, kpad, mpad, x, xq, st));
   vhs_gemm_attr();
-  const int mtiles = mpad / 128, ntiles = npad / 128;
+  const int mtiles = mpad / 128, ntiles = (ncols + 127) / 128;
   const int grid = mtiles * ntiles > 152 ? 152 : mtiles * ntiles;
-  vhs_gemm_kernel<<<grid, kVThreads, kVhsSmem, st>>>(mtiles, ntiles, kpad, npad, xq, b_image, D, status);
+  vhs_gemm_kernel<<<grid, kVThreads, kVhsSmem, st>>>(mtiles, ntiles, kpad, npad, ncols, K, xq, b_image,
+                                                     D, status);
   TROT_CHECK_LAUNCH("vhs_gemm_kernel");
   return TROT_OK;
+}
+
+int launch_split3_gemm(int rows, int K, int kpad, int ncols, int npad, const double2* x, const uint16_t* b_image,
+                       uint16_t* xq, float* D, int* status, cudaStream_t st) {
+  return split3_gemm(rows, K, kpad, ncols, npad, x, b_image, xq, D, status, st);
+}
+int launch_split3_gemm(int rows, int K, int kpad, int ncols, int npad, const float2* x, const uint16_t* b_image,
+                       uint16_t* xq, float* D, int* status, cudaStream_t st) {
+  return split3_gemm(rows, K, kpad, ncols, npad, x, b_image, xq, D, status, st);
 }
 
 static int run_vhs(const trot_system* s, MixedBuffers& m, const double2* xs, cudaStream_t st) {
@@ -1679,17 +1724,15 @@ static int run_vhs(const trot_system* s, MixedBuffers& m, const double2* xs, cud
     set_error("mixed context: VHS operand layout mismatch");
     return TROT_ERR_BAD_SHAPE;
   }
-  TROT_TIMED("x_slices", st, ([&]() -> int {
-    x_slices_kernel<<<152 * 8, 256, 0, st>>>(W, G, mx->gpad, m.mpad, xs, m.xq);
-    TROT_CHECK_LAUNCH("x_slices_kernel");
-    return TROT_OK;
-  })());
+  TROT_TIMED("x_slices", st, launch_x_slices(W, G, mx->gpad, m.mpad, xs, m.xq, st));
   vhs_gemm_attr();
-  const int mtiles = m.mpad / 128, ntiles = mx->n2pad / 128;
+  const int mtiles = m.mpad / 128, N = s->norb;
+  const int ncols = std::min(mx->n2pad, mx->vhs_packed ? N * (N + 1) / 2 : N * N);
+  const int ntiles = (ncols + 127) / 128;
   int grid = mtiles * ntiles;
   if (grid > 152) grid = 152;
   TROT_TIMED("vhs_tc", st, ([&]() -> int {
-    vhs_gemm_kernel<<<grid, kVThreads, kVhsSmem, st>>>(mtiles, ntiles, mx->gpad, mx->n2pad, m.xq,
+    vhs_gemm_kernel<<<grid, kVThreads, kVhsSmem, st>>>(mtiles, ntiles, mx->gpad, mx->n2pad, ncols, std::min(G, mx->gpad), m.xq,
                                                        mx->chol_t_slices, m.vhs, m.status);
     TROT_CHECK_LAUNCH("vhs_gemm_kernel");
     return TROT_OK;

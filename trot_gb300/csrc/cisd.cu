@@ -79,6 +79,11 @@ static bool cisd_gamma_digits(const trot_cisd* c) {
   return c->gl_precision != TROT_MIXED && dg_takes(c->norb) && c->norb <= 1024;
 }
 
+// mixed gl: lg1 and G lci1_g by digit products
+static bool cisd_lg_digits(const trot_cisd* c) {
+  return c->gl_precision == TROT_MIXED && dg_takes(c->norb) && c->norb <= 1024;
+}
+
 // Scratch of the tensor-core digit products of an op (the largest of them; they run one after another)
 static size_t cisd_digit_bytes(const trot_cisd* c, size_t W, int op) {
   const size_t N = c->norb, n = c->nocc, G = c->nchol, nv = n * c->nvir;
@@ -94,6 +99,7 @@ static size_t cisd_digit_bytes(const trot_cisd* c, size_t W, int op) {
   if (op == TROT_OP_FORCE_BIAS) return d;
   if (c->l2ci2_precision != TROT_MIXED) add(W * G, nv, nv);  // l2ci2
   if (cisd_gamma_digits(c)) d = std::max(d, cisd_gamma_dg_bytes(W, N, n, G));
+  if (cisd_lg_digits(c)) d = std::max(d, cisd_lg_dg_bytes(W, N, n, G));
   if (op == TROT_OP_PROP_STEP) {                             // FP64 propagation
     add(W, N * N, G);
     Spins sp{};
@@ -231,8 +237,8 @@ __global__ void cisd_x_kernel(int N, int n, int v, const double2* __restrict__ g
 // ------------------------------------------------------------------ per-walker N x N matrices
 // gci2g = sum ci2g o x; P_Y = gp Y^T (N x n); M = P_Y G (N x N) for Y = ci1, ci2g;
 // e1_1_2 = -2 sum h1 o M1, e1_2_2 = -2 sum h1 o M2.  Stores M1 + M2 (the force bias,
-// the energy and the 1-RDM use chol . ci1_green and chol . ci2_green only in that sum)
-// and M2 (lci2_green).
+// the energy and the 1-RDM use chol . ci1_green and chol . ci2_green only in that sum, as they do e1_1_2 and
+// e1_2_2) and, for the FP64 per-vector kernel (lci2_green), M2.
 __global__ void __launch_bounds__(256)
 cisd_mats_kernel(int N, int n, int v, const double2* __restrict__ green, const double* __restrict__ ci1,
                  const double2* __restrict__ cg, const double2* __restrict__ x,
@@ -275,7 +281,18 @@ cisd_mats_kernel(int N, int n, int v, const double2* __restrict__ green, const d
   }
   __syncthreads();
   double2 h1s = cmk(0.0, 0.0), h2s = cmk(0.0, 0.0);
-  for (int e = tid; e < N * N; e += nt) {
+  if (!m2) {  // only the sum is wanted: one product of P1 + P2 (in P1), its h1 sum in the first slot
+    for (int e = tid; e < N * n; e += nt) P1[e] = cadd(P1[e], P2[e]);
+    __syncthreads();
+    for (int e = tid; e < N * N; e += nt) {
+      const int i = e / N, j = e % N;
+      double2 s = cmk(0.0, 0.0);
+      for (int p = 0; p < n; ++p) cfma(s, P1[i * n + p], Gs[p * N + j]);
+      ms[(size_t)b * N * N + e] = s;
+      crfma(h1s, h1[e], s);
+    }
+  }
+  for (int e = m2 ? tid : N * N; e < N * N; e += nt) {
     const int i = e / N, j = e % N;
     double2 s1 = cmk(0.0, 0.0), s2 = cmk(0.0, 0.0);
     for (int p = 0; p < n; ++p) {
@@ -587,6 +604,132 @@ cisd_gamma_f32_kernel(int N, int n, int v, int G, const double2* __restrict__ gr
   }
 }
 
+// The same sums with lg1 and B = G lci1_g given (F1, F2: digit products, FP64), a warp per Cholesky vector: gl_g of the
+// walker, lg1 and the n x n sums stay in the warp's shared memory, no CTA barrier between vectors.  What is left per
+// vector is gl P2 and glgp in FP32 (7 n N + 4 n^2 v operations) and n^3 float-float products; the two float-float
+// products over N that cisd_gamma_f32_kernel forms per vector were 3/4 of its work.
+static constexpr int kGammaChunk = 32;  // vectors per CTA
+static constexpr int kGammaTile = 8;    // rows p of glgp at a time
+
+static size_t cisd_gamma_w_shared(int N, int n) { return (size_t)2 * n * N * sizeof(float2) + (size_t)n * (n | 1) * 16; }
+static size_t cisd_gamma_w_warp(int N, int n) { return ((size_t)n * N * sizeof(float2) + 15) / 16 * 16 + (size_t)n * (n | 1) * 16; }
+static int cisd_gamma_w_warps(int N, int n) {
+  const size_t sh = cisd_gamma_w_shared(N, n), pw = cisd_gamma_w_warp(N, n);
+  return (int)std::max<size_t>(1, std::min<size_t>(8, sh + pw > 56 * 1024 ? (100 * 1024 > sh ? (100 * 1024 - sh) / pw : 1)
+                                                                           : (56 * 1024 - sh) / pw));
+}
+
+__global__ void __launch_bounds__(256)
+cisd_gamma_w_kernel(int N, int n, int v, int G, const double2* __restrict__ green, const float* __restrict__ gld, int ldd,
+                    const double2* __restrict__ F1, const double2* __restrict__ F2, const double2* __restrict__ p2,
+                    const double2* __restrict__ ci1g1, double2* __restrict__ xg, float2* __restrict__ xf,
+                    double2* __restrict__ gpart) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ double2 red[32];
+  const int chunk = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, nt = blockDim.x;
+  const int lane = tid & 31, warp = tid >> 5, nw = nt >> 5, ns = n | 1, nn = n * n;
+  ffc* C1 = reinterpret_cast<ffc*>(smraw);                // n x ns: ci1g1
+  float2* Gf = reinterpret_cast<float2*>(C1 + n * ns);    // n x N
+  float2* P2f = Gf + n * N;                               // N x n
+  unsigned char* mine = smraw + (size_t)n * ns * 16 + (size_t)2 * n * N * sizeof(float2);
+  mine += (size_t)warp * (((size_t)n * N * sizeof(float2) + 15) / 16 * 16 + (size_t)n * ns * 16);
+  ffc* A = reinterpret_cast<ffc*>(mine);                  // n x ns: lg1
+  float2* GL = reinterpret_cast<float2*>(A + n * ns);     // n x N: gl_g
+  for (int e = tid; e < n * N; e += nt) {
+    const double2 g = green[(size_t)b * n * N + e];
+    Gf[e] = make_float2(d2f_bits(g.x), d2f_bits(g.y));
+    const double2 m = p2[(size_t)b * N * n + e];
+    P2f[e] = make_float2(d2f_bits(m.x), d2f_bits(m.y));
+  }
+  for (int e = tid; e < nn; e += nt) {
+    const double2 c = ci1g1[(size_t)b * nn + e];
+    C1[(e / n) * ns + e % n] = ffc{ff_from_d(c.x), ff_from_d(c.y)};
+  }
+  __syncthreads();
+  const ffc z{{0.f, 0.f}, {0.f, 0.f}};
+  ffc s0 = z, s1 = z, s2 = z, s3 = z;
+  const int g1 = min(G, (chunk + 1) * kGammaChunk);
+  for (int gg = chunk * kGammaChunk + warp; gg < g1; gg += nw) {
+    __syncwarp();
+    for (int p = 0; p < n; ++p) {  // rows 2 (b n + p) (Re) and + 1 (Im), columns gg N + j
+      const float* r0 = gld + 2 * ((size_t)b * n + p) * ldd + (size_t)gg * N;
+      for (int j = lane; j < N; j += 32) GL[p * N + j] = make_float2(r0[j], r0[ldd + j]);
+    }
+    for (int e = lane; e < nn; e += 32) {
+      const int q = e / n, p = e - q * n;
+      const double2 x = F1[(((size_t)b * n + q) * G + gg) * n + p];
+      A[p * ns + q] = ffc{ff_from_d(x.x), ff_from_d(x.y)};
+    }
+    __syncwarp();
+    for (int e = lane; e < nn; e += 32) {
+      const int p = e / n, q = e - p * n;
+      const double2 x = F2[(((size_t)b * n + p) * G + gg) * n + q];
+      // (gl P2)[p][q]: four partial sums over j mod 4
+      float zr[4] = {0.f, 0.f, 0.f, 0.f}, zi[4] = {0.f, 0.f, 0.f, 0.f};
+      int j = 0;
+      for (; j + 4 <= N; j += 4)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const float2 a = GL[p * N + j + u], m = P2f[(j + u) * n + q];
+          zr[u] = fmaf(a.x, m.x, fmaf(-a.y, m.y, zr[u]));
+          zi[u] = fmaf(a.x, m.y, fmaf(a.y, m.x, zi[u]));
+        }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (j + u < N) {
+          const float2 a = GL[p * N + j + u], m = P2f[(j + u) * n + q];
+          zr[u] = fmaf(a.x, m.x, fmaf(-a.y, m.y, zr[u]));
+          zi[u] = fmaf(a.x, m.y, fmaf(a.y, m.x, zi[u]));
+        }
+      ffc t = z;  // (lg1 ci1g1)[q][p]
+      for (int a = 0; a < n; ++a) ffc_mad(t, A[q * ns + a], C1[a * ns + p]);
+      const ffc apq = A[p * ns + q];
+      ffc_mad(s0, apq, A[q * ns + p]);
+      ffc_mad(s1, apq, ffc_norm(t));
+      ffc_mad(s2, ffc{ff_from_d(x.x), ff_from_d(x.y)}, apq);
+      ffc_mad(s3, apq, ffc{ff{(zr[0] + zr[1]) + (zr[2] + zr[3]), 0.f}, ff{(zi[0] + zi[1]) + (zi[2] + zi[3]), 0.f}});
+    }
+    s0 = ffc_norm(s0);
+    s1 = ffc_norm(s1);
+    s2 = ffc_norm(s2);
+    s3 = ffc_norm(s3);
+    // glgp[p][t] = sum_{i < n} gl[p][i] x[i][t] - gl[p][n + t]
+    const size_t xo = ((size_t)b * G + gg) * n * v;
+    for (int p0 = 0; p0 < n; p0 += kGammaTile)
+      for (int t = lane; t < v; t += 32) {
+        float ar[kGammaTile], ai[kGammaTile];
+#pragma unroll
+        for (int r = 0; r < kGammaTile; ++r) {
+          const float2 g = p0 + r < n ? GL[(p0 + r) * N + n + t] : make_float2(0.f, 0.f);
+          ar[r] = -g.x;
+          ai[r] = -g.y;
+        }
+        for (int i = 0; i < n; ++i) {
+          const float2 x = Gf[i * N + n + t];
+#pragma unroll
+          for (int r = 0; r < kGammaTile; ++r) {
+            const float2 a = GL[min(p0 + r, n - 1) * N + i];
+            ar[r] = fmaf(a.x, x.x, fmaf(-a.y, x.y, ar[r]));
+            ai[r] = fmaf(a.x, x.y, fmaf(a.y, x.x, ai[r]));
+          }
+        }
+#pragma unroll
+        for (int r = 0; r < kGammaTile; ++r)
+          if (p0 + r < n) {
+            const size_t o = xo + (size_t)(p0 + r) * v + t;
+            if (xf) xf[o] = make_float2(ar[r], ai[r]);
+            else xg[o] = make_double2(f2d_bits(ar[r]), f2d_bits(ai[r]));
+          }
+      }
+  }
+  const double2 d0 = block_sum2(ffc_d(s0), red), d1 = block_sum2(ffc_d(s1), red);
+  const double2 d2 = block_sum2(ffc_d(s2), red), d3 = block_sum2(ffc_d(s3), red);
+  if (tid == 0) {
+    double2* o = gpart + ((size_t)b * gridDim.x + chunk) * 4;
+    o[0] = d0; o[1] = d1; o[2] = d2; o[3] = d3;
+  }
+}
+
 // l2ci2 from the tensor-core product: Y = xg ci2m in FP32, rows 2r (Re) / 2r+1 (Im) of yd
 // (row stride ldy); per walker sum over g of X_g . Y_g, FP64 accumulation.
 // l2ci2 partial sums: CTA (c, b) takes Cholesky rows [c G/P, (c+1) G/P) of walker b
@@ -823,6 +966,11 @@ static Spins cisd_spins(const trot_cisd* c) {
     return TROT_OK;                                             \
   })())
 
+// ci2_green by itself is read by cisd_gamma_kernel only
+static bool cisd_wants_m2(const trot_cisd* c, const CisdBuffers& b, int stage) {
+  return stage == 2 && c->gl_precision != TROT_MIXED && !(b.dg.p && cisd_gamma_digits(c));
+}
+
 // green, x, C_c / C_e, scalars; stage 0 = overlap only, 1 = + N x N matrices and chol contractions, 2 = + energy terms
 static int cisd_run(const trot_cisd* c, int W, const double2* w, CisdBuffers& b, int stage, cudaStream_t st) {
   const int N = c->norb, n = c->nocc, v = c->nvir, G = c->nchol, nv = n * v;
@@ -838,7 +986,7 @@ static int cisd_run(const trot_cisd* c, int W, const double2* w, CisdBuffers& b,
   const size_t smem = cisd_mats_smem(N, n, v);
   if (smem > 40 * 1024) cudaFuncSetAttribute(cisd_mats_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   CISD_LAUNCH("cisd_mats", cisd_mats_kernel, W, 256, smem, st, N, n, v, b.green, c->ci1, b.cg, b.x, c->h1, b.ms,
-              b.m2, b.p2, b.wsc);
+              cisd_wants_m2(c, b, stage) ? b.m2 : nullptr, b.p2, b.wsc);
   // lg = rot_chol . G  (rot_chol rows g: chol[g][:n][:] = first n N entries of chol_flat row g)
   TROT_TIMED("cisd_chol_gemm", st,
              launch_zgemm(W, G, n * N, 1.0, b.green, n * N, c->chol, N * N, true, b.lg, G, false, b.dg, st, b.kpart,
@@ -866,21 +1014,32 @@ static int cisd_run(const trot_cisd* c, int W, const double2* w, CisdBuffers& b,
   b.nchunk = cisd_chunks(G);
   const int nch = b.nchunk;
   if (c->gl_precision == TROT_MIXED) {
-    const size_t smem2 = cisd_gamma_f32_smem(N, n);
-    cudaFuncSetAttribute(cisd_gamma_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
-    const size_t gnn = (size_t)G * N * n;
-    CISD_LAUNCH("cisd_chol_forms", cisd_chol_forms_kernel, (unsigned)std::min<size_t>((gnn + 255) / 256, 152 * 16),
-                256, 0, st, N, n, G, c->chol, c->lci1, b.rd, b.lc);
     // gl = G L_g for all walkers and Cholesky vectors: one split-BF16 tensor-core product
     // (FP32-class, the reference's float32 gl), rows (walker, p), columns (g, j)
     const int kp = (int)cisd_gl_kpad(N), np = (int)cisd_gl_npad(N, G);
-    const size_t nimg = (size_t)np * kp;
+    const size_t nimg = (size_t)np * kp, gnn = (size_t)G * N * n;
     CISD_LAUNCH("cisd_gl_tc", cisd_gl_image_kernel, (unsigned)std::min<size_t>((nimg + 255) / 256, 152 * 16), 256, 0,
                 st, N, G, kp, np, c->chol, b.glimg);
     TROT_TIMED("cisd_gl_tc", st, launch_split3_gemm(W * n, N, kp, G * N, np, b.green, b.glimg, b.glq, b.gld, b.status, st));
-    CISD_LAUNCH("cisd_gamma_f32", cisd_gamma_f32_kernel, dim3(nch, W), 256, smem2, st, N, n, v, G, b.green, b.gld, np,
-                b.rd, b.lc, b.p2, b.ci1g1, b.xg,
-                c->l2ci2_precision == TROT_MIXED ? reinterpret_cast<float2*>(b.xg) : nullptr, b.gpart);
+    float2* xf = c->l2ci2_precision == TROT_MIXED ? reinterpret_cast<float2*>(b.xg) : nullptr;
+    if (b.dg.p && cisd_lg_digits(c)) {
+      double2 *F1 = nullptr, *F2 = nullptr;
+      CisdGammaArgs ga{W, N, n, v, G, b.green, c->chol, c->lci1, b.p2, b.ci1g1, b.xg, b.gpart};
+      TROT_TIMED("cisd_lg", st, launch_cisd_lg_dg(ga, b.dg, &F1, &F2, st));
+      const int nw = cisd_gamma_w_warps(N, n);
+      const size_t smem2 = cisd_gamma_w_shared(N, n) + nw * cisd_gamma_w_warp(N, n);
+      cudaFuncSetAttribute(cisd_gamma_w_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
+      b.nchunk = (G + kGammaChunk - 1) / kGammaChunk;
+      CISD_LAUNCH("cisd_gamma_f32", cisd_gamma_w_kernel, dim3(b.nchunk, W), 32 * nw, smem2, st, N, n, v, G, b.green, b.gld,
+                  np, F1, F2, b.p2, b.ci1g1, b.xg, xf, b.gpart);
+    } else {
+      const size_t smem2 = cisd_gamma_f32_smem(N, n);
+      cudaFuncSetAttribute(cisd_gamma_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
+      CISD_LAUNCH("cisd_chol_forms", cisd_chol_forms_kernel, (unsigned)std::min<size_t>((gnn + 255) / 256, 152 * 16),
+                  256, 0, st, N, n, G, c->chol, c->lci1, b.rd, b.lc);
+      CISD_LAUNCH("cisd_gamma_f32", cisd_gamma_f32_kernel, dim3(nch, W), 256, smem2, st, N, n, v, G, b.green, b.gld, np,
+                  b.rd, b.lc, b.p2, b.ci1g1, b.xg, xf, b.gpart);
+    }
   } else if (b.dg.p && cisd_gamma_digits(c)) {
     b.nchunk = cisd_gamma_dg_chunks(G);
     CisdGammaArgs ga{W, N, n, v, G, b.green, c->chol, c->lci1, b.p2, b.ci1g1, b.xg, b.gpart};

@@ -1152,6 +1152,9 @@ cisd_pairs_kernel(int n, int G, int gsub, int nchunk, const double2* __restrict_
   }
 }
 
+static int cisd_lg_rows(const CisdGammaArgs& c, uint16_t* irow, int16_t* erow, uint16_t* ilc, int16_t* elc,
+                        cudaStream_t st);
+
 static size_t cgd_chunk(size_t W, size_t N, size_t n, size_t G) {
   const size_t wc = std::max<size_t>(1, (size_t(64) << 20) / (n * G * N * sizeof(double2)));
   return std::min(wc, W);
@@ -1199,12 +1202,7 @@ int launch_cisd_gamma_dg(const CisdGammaArgs& c, const DgScratch& s, cudaStream_
   DgSrc sc = dg_src(c.chol, 0, N, N, 128, 1, N, b.icol, b.ecol);
   sc.rpad = N; sc.nblk = G; sc.bstride = (long long)N * N;
   TROT_TRY(dg_rows_launch(sc, (int)(adj_rows((size_t)G * N, 128) / 8), st));
-  DgSrc sr = dg_src(c.chol, 0, n, N, 128, N, 1, b.irow, b.erow);
-  sr.rpad = n; sr.nblk = G; sr.bstride = (long long)N * N;
-  TROT_TRY(dg_rows_launch(sr, (int)(adj_rows((size_t)G * n, 128) / 8), st));
-  DgSrc sl = dg_src(c.lci1, 0, n, N, 128, 1, n, b.ilc, b.elc);
-  sl.rpad = n; sl.nblk = G; sl.bstride = (long long)N * n;
-  TROT_TRY(dg_rows_launch(sl, (int)(adj_rows((size_t)G * n, 128) / 8), st));
+  TROT_TRY(cisd_lg_rows(c, b.irow, b.erow, b.ilc, b.elc, st));
   const int gsub = std::max(1, std::min(kPairsChunk, 256 / nn)), nchunk = cisd_gamma_dg_chunks(G);
   const size_t smem = (size_t)(gsub + 1) * nn * sizeof(double2);
   if (smem > 40 * 1024) cudaFuncSetAttribute(cisd_pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1245,6 +1243,64 @@ int launch_cisd_gamma_dg(const CisdGammaArgs& c, const DgScratch& s, cudaStream_
                                                            c.ci1g1 + (size_t)w0 * nn, c.gpart + (size_t)w0 * nchunk * 4);
     TROT_CHECK_LAUNCH("cisd_pairs_kernel");
   }
+  return TROT_OK;
+}
+
+struct ClgBuffers {
+  uint16_t *irow, *ilc, *ig;
+  int16_t *erow, *elc, *eg;
+  double2 *F1, *F2;
+};
+static size_t clg_carve(ClgBuffers& b, size_t W, size_t N, size_t n, size_t G, void* base) {
+  char* p0 = reinterpret_cast<char*>(((uintptr_t)base + 255) & ~(uintptr_t)255);
+  char* p = p0;
+  auto take = [&](size_t k) {
+    char* r = p;
+    p += (k + 255) & ~(size_t)255;
+    return r;
+  };
+  const size_t rb = kDgRowBytes((N + 15) / 16), row = adj_rows(G * n, 128), g = adj_rows(2 * W * n, kDgP);
+  b.irow = (uint16_t*)take(row * rb); b.ilc = (uint16_t*)take(row * rb); b.ig = (uint16_t*)take(g * rb);
+  b.erow = (int16_t*)take(row * 2); b.elc = (int16_t*)take(row * 2); b.eg = (int16_t*)take(g * 2);
+  b.F1 = (double2*)take(W * n * n * G * sizeof(double2));
+  b.F2 = (double2*)take(W * n * n * G * sizeof(double2));
+  return (size_t)(p - p0) + 256;
+}
+
+size_t cisd_lg_dg_bytes(size_t W, size_t N, size_t n, size_t G) {
+  ClgBuffers b;
+  return clg_carve(b, W, N, n, G, nullptr);
+}
+
+// digits of the rows p < n of every L_g and of the columns of every lci1_g
+static int cisd_lg_rows(const CisdGammaArgs& c, uint16_t* irow, int16_t* erow, uint16_t* ilc, int16_t* elc,
+                        cudaStream_t st) {
+  const int N = c.N, n = c.n, G = c.G, groups = (int)(adj_rows((size_t)G * n, 128) / 8);
+  DgSrc sr = dg_src(c.chol, 0, n, N, 128, N, 1, irow, erow);
+  sr.rpad = n; sr.nblk = G; sr.bstride = (long long)N * N;
+  TROT_TRY(dg_rows_launch(sr, groups, st));
+  DgSrc sl = dg_src(c.lci1, 0, n, N, 128, 1, n, ilc, elc);
+  sl.rpad = n; sl.nblk = G; sl.bstride = (long long)N * n;
+  return dg_rows_launch(sl, groups, st);
+}
+
+int launch_cisd_lg_dg(const CisdGammaArgs& c, const DgScratch& s, double2** F1, double2** F2, cudaStream_t st) {
+  const int W = c.W, N = c.N, n = c.n, G = c.G;
+  ClgBuffers b;
+  if (s.bytes < clg_carve(b, W, N, n, G, s.p)) { set_error("CISD terms: scratch %zu", s.bytes); return TROT_ERR_WORKSPACE_TOO_SMALL; }
+  TROT_TRY(cisd_lg_rows(c, b.irow, b.erow, b.ilc, b.elc, st));
+  const int tiles = (2 * W * n + kDgP - 1) / kDgP;
+  TROT_TRY(dg_rows_launch(dg_src(reinterpret_cast<const double*>(c.green), 1, 2 * W * n, N, kDgP, 2ll * N, 2, b.ig, b.eg),
+                          tiles * 4, st));
+  DgArgs a{};
+  a.imgA = b.ig; a.exA = b.eg; a.M = W * n; a.ntile = tiles; a.nbatch = 1;
+  a.nk16 = (N + 15) / 16; a.shift = 1; a.salpha = 1; a.status = s.status;
+  a.imgB = b.irow; a.exB = b.erow; a.Nn = G * n; a.nrt = (G * n + 127) / 128; a.C = b.F1; a.ldc = (long long)G * n;
+  TROT_TRY(dg_gemm<false>(a, st));
+  a.imgB = b.ilc; a.exB = b.elc; a.C = b.F2;
+  TROT_TRY(dg_gemm<false>(a, st));
+  *F1 = b.F1;
+  *F2 = b.F2;
   return TROT_OK;
 }
 

@@ -69,6 +69,11 @@ struct CisdGammaArgs {
   double2* xg;
   double2* gpart;
 };
+// lg1 and B alone, for all walkers: F1[(b, q)][(g, p)] = lg1[p][q], F2[(b, p)][(g, q)] = (G lci1_g)[p][q] (complex,
+// W n x G n), both inside the scratch
+size_t cisd_lg_dg_bytes(size_t W, size_t N, size_t n, size_t G);
+int launch_cisd_lg_dg(const CisdGammaArgs& c, const DgScratch& s, double2** F1, double2** F2, cudaStream_t st);
+
 int cisd_gamma_dg_chunks(int G);
 size_t cisd_gamma_dg_bytes(size_t W, size_t N, size_t n, size_t G);
 int launch_cisd_gamma_dg(const CisdGammaArgs& c, const DgScratch& s, cudaStream_t st);

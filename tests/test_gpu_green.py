@@ -75,3 +75,30 @@ def test_green_and_overlap_sizes(kind, N, na, nb, W):
     want = d[0] * d[0] if wk == "restricted" else d[0] * d[1]
     fin = np.isfinite(want) & (np.abs(want) > 1e-290)
     assert np.all(np.abs(cpu(ov) - want)[fin] <= (1e-11 * np.abs(want))[fin])
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 5, 12, 13, 14, 15, 32, 33, 64])
+def test_eliminations(n):
+    """Inverses and determinants on both sides of the line between one and four warps, with walkers whose pivots are
+    real, imaginary, or outside the range of the fast reciprocal (2^-300 to 2^300).  Same bounds as above."""
+    N = min(2 * n + 1, 66)
+    q = np.linalg.qr(np.random.default_rng(n).standard_normal((N, n)))[0]
+    _check_scaled(N, n, q, np.array([1.0, 1j, -1j, 2.0 ** 310, 2.0 ** -310, 2.0 ** 299, 0.6 - 0.8j]))
+
+
+def _check_scaled(N, n, q, scales):
+    import trot_gb300 as tg
+    from oracle import afqmc_oracle as orc
+    from tests.gpu_helpers import cpu, dev
+    from trot_gb300 import synthetic
+    from trot_gb300.trial import half_green_batched
+
+    base = synthetic.perturbed_walkers(q, len(scales), 0.3 / np.sqrt(N), 3)
+    g, ov = half_green_batched(dev(base * scales[:, None, None]), tg.RhfTrial(np.ascontiguousarray(q)), "restricted",
+                               with_overlaps=True)
+    ref = orc.half_green(base, q)  # G does not depend on the scale
+    assert np.max(np.abs(cpu(g) - ref)) <= 1e-12 * np.max(np.abs(ref))
+    with np.errstate(all="ignore"):
+        want = np.linalg.det(orc._ovlp_mat(q, base)) ** 2 * (scales ** n) ** 2
+    fin = np.isfinite(want) & (np.abs(want) > 1e-290)
+    assert np.all(np.abs(cpu(ov) - want)[fin] <= (1e-11 * np.abs(want))[fin])

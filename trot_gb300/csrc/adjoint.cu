@@ -106,19 +106,19 @@ static int grid_of_(size_t len) { return (int)((len + 255) / 256 < 4096 ? (len +
 // O = C^T w, P = O^-1, G = (w P)^T (n x N), det(O); one block per walker (n <= 32).
 __global__ void adj_green_kernel(int N, int n, const double* __restrict__ C, const double2* __restrict__ w,
                                  double2* __restrict__ green, double2* __restrict__ Pout, double2* __restrict__ det) {
-  __shared__ double2 O[32 * 32], P[32 * 32];
-  __shared__ int piv;
-  __shared__ double2 red[32];
+  __shared__ double2 P[32 * 32];
+  __shared__ GjScratch gj;
   const int b = blockIdx.x, tid = threadIdx.x;
   const double2* wb = w + (size_t)b * N * n;
   for (int e = tid; e < n * n; e += blockDim.x) {
     const int i = e / n, j = e % n;
     double2 acc = cmk(0.0, 0.0);
     for (int p = 0; p < N; ++p) crfma(acc, C[(size_t)p * n + i], wb[(size_t)p * n + j]);
-    O[i * n + j] = acc;
+    P[i * n + j] = acc;
   }
   __syncthreads();
-  const double2 d = block_gauss_jordan(O, n, n, P, &piv, red);
+  double2 d = cmk(0.0, 0.0);
+  if (tid < 128) d = gauss_jordan(P, n, true, gj, b);
   __syncthreads();
   for (int e = tid; e < n * N; e += blockDim.x) {
     const int j = e / N, p = e % N;  // G[j][p] = sum_k w[p][k] P[k][j]
@@ -209,9 +209,8 @@ __global__ void adj_green_vjp_kernel(int N, int n, const double* __restrict__ C,
 // QR: g_w = g_Q (w^H Q)^-1 per walker (n <= 32)
 __global__ void adj_qr_kernel(int N, int n, const double2* __restrict__ w, const double2* __restrict__ q,
                               const double2* __restrict__ gq, double2* __restrict__ gw) {
-  __shared__ double2 M[32 * 32], Mi[32 * 32];
-  __shared__ int piv;
-  __shared__ double2 red[32];
+  __shared__ double2 M[32 * 32];  // w^H Q, then its inverse
+  __shared__ GjScratch gj;
   const int b = blockIdx.x, tid = threadIdx.x;
   const double2* wb = w + (size_t)b * N * n;
   const double2* qb = q + (size_t)b * N * n;
@@ -225,7 +224,7 @@ __global__ void adj_qr_kernel(int N, int n, const double2* __restrict__ w, const
     M[e] = acc;
   }
   __syncthreads();
-  block_gauss_jordan(M, n, n, Mi, &piv, red);
+  if (tid < 128) gauss_jordan(M, n, true, gj, b);
   __syncthreads();
   const double2* g = gq + (size_t)b * N * n;
   // a walker with a zero cotangent (no influence on the objective) gets exactly zero
@@ -238,7 +237,7 @@ __global__ void adj_qr_kernel(int N, int n, const double2* __restrict__ w, const
   for (int e = tid; e < N * n; e += blockDim.x) {
     const int p = e / n, k = e % n;
     double2 acc = cmk(0.0, 0.0);
-    for (int j = 0; j < n; ++j) cfma(acc, g[(size_t)p * n + j], Mi[j * n + k]);
+    for (int j = 0; j < n; ++j) cfma(acc, g[(size_t)p * n + j], M[j * n + k]);
     gw[(size_t)b * N * n + e] = acc;
   }
 }

@@ -55,18 +55,6 @@ TROT_HD double2 cexp(double2 a) {
   return cmk(e * c, e * s);
 }
 
-// 1 / b by one division: b scaled by the power of two of its larger part (exact, against overflow), conj(b) / |b|^2, and
-// one correction by the residual 1 - b r
-TROT_D double2 crcp(double2 b) {
-  const int ex = max((__double2hiint(b.x) >> 20) & 0x7FF, (__double2hiint(b.y) >> 20) & 0x7FF);
-  if (ex < 64 || ex > 1982) return cdiv(cmk(1.0, 0.0), b);
-  const double s = __hiloint2double((2046 - ex) << 20, 0);  // 2^(1023 - ex)
-  const double x = b.x * s, y = b.y * s, r = 1.0 / fma(x, x, y * y);
-  const double u = x * r, v = -y * r;
-  const double er = fma(y, v, fma(-x, u, 1.0)), ei = -fma(y, u, x * v);
-  return cmk(fma(u, er, fma(-v, ei, u)) * s, fma(u, ei, fma(v, er, v)) * s);
-}
-
 // ---------------------------------------------------------------- reductions
 TROT_D double warp_sum(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -107,25 +95,70 @@ struct Spins {
   const double* rot_chol[2];
 };
 
-// Small-matrix LU with partial pivoting on an n x n complex matrix in shared
-// memory (row-major, leading dimension ld), executed by the whole block.
-// Returns det(A) to all threads; A is overwritten by its LU factors.
-// If `inv` is non-null it receives A^{-1} (Gauss-Jordan on [A | I]).
-// One warp, an n x n matrix A (row stride n) in shared memory, partial pivoting (the first
-// largest |A[i][k]| wins, as in block_gauss_jordan, by integer reductions of the squares' words: five
-// shuffles of FP64 comparisons took longer than the elimination).  Returns det(A).  With `inverse`, A is
-// overwritten by its inverse (in-place Gauss-Jordan: each pivot step updates the n x n working
-// array once, half the work of eliminating [A | I]; the row interchanges are undone as column
-// interchanges in reverse order at the end, `perm` holds n ints of scratch); without it, A
-// holds its LU factors.  Phases are separated by __syncwarp, so no CTA barrier is involved.
-// The determinant is returned in lane 0.  `smith`: the pivots' reciprocals by cdiv (three divisions) instead of crcp
-// (one), for results that are rounded to FP32 afterwards and must not move.
-TROT_D double2 warp_gauss_jordan(double2* A, int n, bool inverse, int* perm, bool smith = false) {
+// Small complex matrices A (n x n <= kGjMax, row stride n) in shared memory, partial pivoting (the first largest
+// |A[i][k]| wins, by integer reductions of the squares' words: five shuffles of FP64 comparisons took longer than the
+// elimination).  Threads 0..127 of the block call gauss_jordan, which returns det(A) to thread 0.  With `inverse`, A is
+// overwritten by its inverse (in-place Gauss-Jordan: each pivot step updates the n x n array once, half the work of
+// eliminating [A | I]; the row interchanges are undone as column interchanges at the end); without it, A holds its LU
+// factors.  Each quarter of an SM has an FP64 pipe of its own that takes an instruction of a warp every 64 cycles (72
+// for a dependent one, 405 for a division), so a pivot costs one warp about 2 divisions + 6 n^2 / 32 instructions in a
+// row.  The inverse (and the factors from kGjQuadLu on) updates on four warps and the serial part of a pivot (search,
+// interchange, reciprocal) moves from warp to warp (quad_gauss_jordan); smaller factors stay in one warp without
+// barriers (warp_lu).  FP64 instructions that are predicated off take the pipe as well: the loops are not unrolled.
+// Cycles per pivot, one block: inverse, n = 5 / 12 / 16: 4850 / 7940 / 10070 (one warp, divisions) -> 2870 / 3320 /
+// 3420; factors, n = 5 / 12 / 16: 3190 / 3900 / 4570 -> 2360 / 2980 / 3580 (one warp), 2470 / 2650 / 2820 (four); with
+// the SMs full of blocks one warp stays ahead up to n = 13 (N = 120, n = 12, W = 1024: 95 against 97 us).
+// float-float Green's functions, N = 97, n = 12, W = 128: 65 -> 39 us.
+static constexpr int kGjMax = 64, kGjQuadLu = 14;
+struct GjScratch {
+  double2 rp, piv, det, col[kGjMax];
+  int perm[kGjMax];
+};
+// e / m for e < m^2 <= kGjMax^2 by a product (an integer division takes as long as two FP64 instructions)
+TROT_D unsigned gj_magic(int m) { return m > 0 ? ((1u << 20) + m - 1) / m : 0u; }
+TROT_D int gj_div(int e, unsigned magic) { return (int)(((unsigned)e * magic) >> 20); }
+// 1/u for 2^-300 <= |u| <= 2^300 to about 2^-46: an FP32 reciprocal of the leading 24 bits of the mantissa, one
+// second-order Newton step in FP32 over all its 53 bits, joined as a fixed-point number
+TROT_D double gj_seed(double u) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(u), m = b & 0xFFFFFFFFFFFFFull;
+  const float h = __int_as_float(0x3F800000 | (int)(m >> 29));
+  const float l = __fmul_rn(__uint2float_rn((unsigned)m & 0x1FFFFFFFu), 0x1p-52f);
+  const float r = __fdividef(1.0f, h);
+  const float e = fmaf(-r, l, fmaf(-r, h, 1.0f));
+  const int lo = __float2int_rn(__fmul_rn(__fmul_rn(r, fmaf(e, e, e)), 0x1p53f));
+  const long long f = ((long long)__float2int_rn(__fmul_rn(r, 0x1p24f)) << 29) + lo;  // 2^53 / mantissa
+  const long long ex = (long long)((b >> 52) & 0x7FF) - 1023;
+  return __longlong_as_double((long long)(b & 0x8000000000000000ull) | (f + ((1021ll - ex) << 52)));
+}
+// a / u from that: Markstein's correction by the residual, the rounded quotient but for about one case in 2^39
+TROT_D double gj_div_by(double a, double u, double ru) {
+  const double q = a * ru;
+  return fma(fma(-q, u, a), ru, q);
+}
+static __device__ __noinline__ double2 gj_rcp_general(double2 p) { return cdiv(cmk(1.0, 0.0), p); }
+// Re (part = 0) or Im (part = 1) of 1/p by Smith's two steps, every lane alike but for the last numerator.  (The
+// division routine takes 600 to 750 cycles; three in a row were half of a pivot.)
+TROT_D double gj_reciprocal(double2 p, int part) {
+  const unsigned long long mx = (unsigned long long)__double_as_longlong(p.x) << 1,
+                           my = (unsigned long long)__double_as_longlong(p.y) << 1;
+  const bool c = mx >= my;  // |Re p| >= |Im p|
+  const double u = c ? p.x : p.y, o = c ? p.y : p.x;
+  const int eu = (int)((c ? mx : my) >> 53) - 1023, eo = (int)((c ? my : mx) >> 53) - 1023;
+  if (eu > 300 || eu < -300 || (eo < -300 && (c ? my : mx) != 0)) {
+    const double2 r = gj_rcp_general(p);
+    return part ? r.y : r.x;
+  }
+  const double r = gj_div_by(o, u, gj_seed(u)), d = u + o * r;
+  return gj_div_by(part ? (c ? -r : -1.0) : (c ? 1.0 : r), d, gj_seed(d));
+}
+TROT_D void gj_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+TROT_D double2 warp_lu(double2* A, int n) {
   const int lane = threadIdx.x & 31;
   double2 det = cmk(1.0, 0.0);
   for (int k = 0; k < n; ++k) {
     unsigned long long best = 0;  // bits of the square, with one added to the high word (0: no row)
     int bi = k;
+#pragma unroll 1
     for (int i = k + lane; i < n; i += 32) {
       const unsigned long long a = (unsigned long long)__double_as_longlong(cabs2(A[i * n + k])) + (1ull << 32);
       if (a > best) { best = a; bi = i; }
@@ -135,6 +168,7 @@ TROT_D double2 warp_gauss_jordan(double2* A, int n, bool inverse, int* perm, boo
     const unsigned tl = __reduce_max_sync(0xffffffffu, cand ? (unsigned)best : 0u);
     bi = (int)__reduce_min_sync(0xffffffffu, cand && (unsigned)best == tl ? (unsigned)bi : 0x7fffffffu);
     if (bi != k) {
+#pragma unroll 1
       for (int j = lane; j < n; j += 32) {
         const double2 t = A[k * n + j];
         A[k * n + j] = A[bi * n + j];
@@ -142,60 +176,126 @@ TROT_D double2 warp_gauss_jordan(double2* A, int n, bool inverse, int* perm, boo
       }
       det = cmk(-det.x, -det.y);
     }
-    if (inverse && lane == 0) perm[k] = bi;
     __syncwarp();
-    // the pivot's reciprocal and the running determinant by lane 0 only (the FP64 pipe is
-    // narrow: an FP64 division issued by the whole warp costs as much as an elimination step)
-    double2 rp = cmk(0.0, 0.0);
-    if (lane == 0) {
-      const double2 piv = A[k * n + k];
-      det = cmul(det, piv);
-      rp = smith ? cdiv(cmk(1.0, 0.0), piv) : crcp(piv);
-    }
-    rp.x = __shfl_sync(0xffffffffu, rp.x, 0);
-    rp.y = __shfl_sync(0xffffffffu, rp.y, 0);
-    if (inverse) {
-      __syncwarp();
-      for (int j = lane; j < n; j += 32) A[k * n + j] = j == k ? rp : cmul(A[k * n + j], rp);
-      __syncwarp();
-      // A[i][j] -= A[i][k] A[k][j] for i != k, j != k (the (n-1)^2 elements, row / column k
-      // skipped by the index map); then column k: A[i][k] = -A[i][k] rp
-      const int m = n - 1;
-      for (int e = lane; e < m * m; e += 32) {
-        int i = e / m, j = e - (e / m) * m;
-        i += i >= k;
-        j += j >= k;
-        A[i * n + j] = csub(A[i * n + j], cmul(A[i * n + k], A[k * n + j]));
-      }
-      __syncwarp();
-      for (int i = lane; i < n; i += 32)
-        if (i != k) A[i * n + k] = cmul(cmk(-A[i * n + k].x, -A[i * n + k].y), rp);
-    } else {
-      for (int i = k + 1 + lane; i < n; i += 32) A[i * n + k] = cmul(A[i * n + k], rp);
-      __syncwarp();
-      const int m = n - k - 1;
-      for (int e = lane; e < m * m; e += 32) {
-        const int i = k + 1 + e / m, j = k + 1 + (e - (e / m) * m);
-        A[i * n + j] = csub(A[i * n + j], cmul(A[i * n + k], A[k * n + j]));
-      }
+    const double2 piv = A[k * n + k];
+    const double v = k + 1 < n ? gj_reciprocal(piv, lane & 1) : 0.0;
+    if (lane == 0) det = cmul(det, piv);
+    const double2 rp = cmk(__shfl_sync(0xffffffffu, v, 0), __shfl_sync(0xffffffffu, v, 1));
+#pragma unroll 1
+    for (int i = k + 1 + lane; i < n; i += 32) A[i * n + k] = cmul(A[i * n + k], rp);
+    __syncwarp();
+    const int m = n - k - 1;
+    const unsigned im = gj_magic(m);
+#pragma unroll 1
+    for (int e = lane; e < m * m; e += 32) {
+      const int r = gj_div(e, im), i = k + 1 + r, j = k + 1 + e - r * m;
+      A[i * n + j] = csub(A[i * n + j], cmul(A[i * n + k], A[k * n + j]));
     }
     __syncwarp();
-  }
-  if (inverse) {
-    for (int k = n - 1; k >= 0; --k) {
-      const int p = perm[k];
-      if (p != k)
-        for (int i = lane; i < n; i += 32) {
-          const double2 t = A[i * n + k];
-          A[i * n + k] = A[i * n + p];
-          A[i * n + p] = t;
-        }
-      __syncwarp();
-    }
   }
   return det;
 }
 
+TROT_D double2 quad_gauss_jordan(double2* A, int n, bool inverse, GjScratch& S, int turn) {
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const unsigned in = gj_magic(n);
+  if (t == 0) S.det = cmk(1.0, 0.0);
+  for (int k = 0; k < n; ++k) {
+    const int role = (warp - k - turn) & 3;
+    if (role == 0) {
+      unsigned long long best = 0;  // bits of the square, with one added to the high word (0: no row)
+      int bi = k;
+#pragma unroll 1
+      for (int i = k + lane; i < n; i += 32) {
+        const unsigned long long a = (unsigned long long)__double_as_longlong(cabs2(A[i * n + k])) + (1ull << 32);
+        if (a > best) { best = a; bi = i; }
+      }
+      const unsigned th = __reduce_max_sync(0xffffffffu, (unsigned)(best >> 32));
+      const bool cand = (unsigned)(best >> 32) == th;
+      const unsigned tl = __reduce_max_sync(0xffffffffu, cand ? (unsigned)best : 0u);
+      bi = (int)__reduce_min_sync(0xffffffffu, cand && (unsigned)best == tl ? (unsigned)bi : 0x7fffffffu);
+      const double2 p = A[bi * n + k];
+      __syncwarp();
+      if (bi != k) {
+#pragma unroll 1
+        for (int j = lane; j < n; j += 32) {
+          const double2 x = A[k * n + j];
+          A[k * n + j] = A[bi * n + j];
+          A[bi * n + j] = x;
+        }
+      }
+      if (lane == 0) {
+        S.perm[k] = bi;
+        S.piv = p;
+      }
+      if (inverse || k + 1 < n) {
+        const double v = gj_reciprocal(p, lane & 1);
+        if (lane < 2) (lane == 0 ? S.rp.x : S.rp.y) = v;
+      }
+    }
+    gj_sync();
+    if (role == 1) {
+      const double2 rp = S.rp;
+      if (inverse) {
+#pragma unroll 1
+        for (int j = lane; j < n; j += 32) A[k * n + j] = j == k ? rp : cmul(A[k * n + j], rp);
+      } else {
+#pragma unroll 1
+        for (int i = k + 1 + lane; i < n; i += 32) A[i * n + k] = cmul(A[i * n + k], rp);
+      }
+    } else if (role == 2) {
+      if (inverse)
+#pragma unroll 1
+        for (int i = lane; i < n; i += 32)
+          if (i != k) S.col[i] = A[i * n + k];
+    } else if (role == 3 && lane == 0) {
+      const double2 d = S.det;
+      S.det = cmul(S.perm[k] != k ? cmk(-d.x, -d.y) : d, S.piv);
+    }
+    gj_sync();
+    if (inverse) {  // A[i][j] -= A[i][k] A[k][j] for i != k; in column k the old value counts as 0
+#pragma unroll 1
+      for (int e = t; e < (n - 1) * n; e += 128) {
+        int i = gj_div(e, in);
+        const int j = e - i * n;
+        i += i >= k;
+        A[i * n + j] = csub(j == k ? cmk(0.0, 0.0) : A[i * n + j], cmul(S.col[i], A[k * n + j]));
+      }
+    } else {
+      const int m = n - k - 1;
+      const unsigned im = gj_magic(m);
+#pragma unroll 1
+      for (int e = t; e < m * m; e += 128) {
+        const int r = gj_div(e, im), i = k + 1 + r, j = k + 1 + e - r * m;
+        A[i * n + j] = csub(A[i * n + j], cmul(A[i * n + k], A[k * n + j]));
+      }
+    }
+    gj_sync();
+  }
+  if (inverse) {
+    if (t < n)
+      for (int k = n - 1; k >= 0; --k) {
+        const int p = S.perm[k];
+        if (p != k) {
+          const double2 x = A[t * n + k];
+          A[t * n + k] = A[t * n + p];
+          A[t * n + p] = x;
+        }
+      }
+    gj_sync();
+  }
+  return S.det;
+}
+
+TROT_D double2 gauss_jordan(double2* A, int n, bool inverse, GjScratch& S, int turn) {
+  if (inverse || n >= kGjQuadLu) return quad_gauss_jordan(A, n, inverse, S, turn);
+  return threadIdx.x < 32 ? warp_lu(A, n) : cmk(0.0, 0.0);
+}
+
+// Small-matrix LU with partial pivoting on an n x n complex matrix in shared
+// memory (row-major, leading dimension ld), executed by the whole block.
+// Returns det(A) to all threads; A is overwritten by its LU factors.
+// If `inv` is non-null it receives A^{-1} (Gauss-Jordan on [A | I]).
 TROT_D double2 block_gauss_jordan(double2* A, int n, int ld, double2* inv, int* piv_s, double2* red) {
   const int tid = threadIdx.x, nt = blockDim.x;
   if (inv) {

@@ -28,15 +28,22 @@ TROT_D ff ff_mul(ff x, ff y) {
   e = fmaf(x.lo, y.hi, e);
   return ff_fast(p, e);
 }
-// float -> double by moving the bits (exact for normal floats; zero, subnormal, inf and
-// NaN take the conversion instruction)
+// float -> double by moving the bits (exact).  Integer operations also in the rare cases: a conversion instruction
+// would be issued to the FP64 pipe as a predicated one for every value (64 cycles of a quarter SM).
 TROT_D double f2d_bits(float f) {
   const unsigned v = (unsigned)__float_as_int(f);
   const unsigned e = (v >> 23) & 0xFFu;
-  if (e == 0u || e == 0xFFu) return (double)f;
-  const unsigned long long d = ((unsigned long long)(v & 0x80000000u) << 32) |
-                               ((unsigned long long)(e - 127u + 1023u) << 52) |
-                               ((unsigned long long)(v & 0x7FFFFFu) << 29);
+  unsigned ed = e - 127u + 1023u, m = v & 0x7FFFFFu;
+  if (e == 0u) {  // subnormal: normalise; zero
+    const unsigned lz = (unsigned)__clz((int)m) - 8u;
+    ed = m ? 897u - lz : 0u;
+    m = m ? (m << lz) & 0x7FFFFFu : 0u;
+  } else if (e == 0xFFu) {
+    ed = 0x7FFu;
+    m |= m ? 0x400000u : 0u;
+  }
+  const unsigned long long d = ((unsigned long long)(v & 0x80000000u) << 32) | ((unsigned long long)ed << 52) |
+                               ((unsigned long long)m << 29);
   return __longlong_as_double((long long)d);
 }
 TROT_D double ff_d(ff x) { return f2d_bits(x.hi) + f2d_bits(x.lo); }
@@ -68,7 +75,7 @@ TROT_D ff ff_from_d(double x) {
   const unsigned long long u = (unsigned long long)__double_as_longlong(x);
   const unsigned sign = (unsigned)(u >> 32) & 0x80000000u;
   const int ex = (int)((u >> 52) & 0x7FF);
-  if (ex == 0x7FF) return ff{__double2float_rn(x), 0.f};
+  if (ex == 0x7FF) return ff{__int_as_float((int)((u << 12) ? 0x7FFFFFFFu : sign | 0x7F800000u)), 0.f};
   const int ef = ex - 1023 + 127;
   if (ex == 0 || ef <= 0) return ff{__int_as_float((int)sign), 0.f};
   if (ef >= 255) return ff{__int_as_float((int)(sign | 0x7F800000u)), 0.f};
@@ -87,7 +94,7 @@ TROT_D float d2f_bits(double x) {
   const unsigned long long u = (unsigned long long)__double_as_longlong(x);
   const unsigned sign = (unsigned)(u >> 32) & 0x80000000u;
   const int ex = (int)((u >> 52) & 0x7FF);
-  if (ex == 0x7FF) return __double2float_rn(x);
+  if (ex == 0x7FF) return __int_as_float((int)((u << 12) ? 0x7FFFFFFFu : sign | 0x7F800000u));
   const int ef = ex - 1023 + 127;
   if (ex == 0 || ef <= 0) return __int_as_float((int)sign);
   if (ef >= 255) return __int_as_float((int)(sign | 0x7F800000u));

@@ -26,7 +26,7 @@ green_kernel(Spins sp, int N, int padded, const double2* __restrict__ wa, const 
   extern __shared__ double2 smem[];
   __shared__ double2 red[32];
   __shared__ double2 sums[2];  // det^mult, mult e1 of this spin
-  __shared__ int perm[kMaxOcc];
+  __shared__ GjScratch gj;
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   const int s = sp.nspin == 2 ? blockIdx.x & 1 : 0, b = sp.nspin == 2 ? blockIdx.x >> 1 : blockIdx.x;
@@ -54,10 +54,8 @@ green_kernel(Spins sp, int N, int padded, const double2* __restrict__ wa, const 
   }
   __syncthreads();
   const int mult = s ? sp.mult[1] : sp.mult[0];
-  if (tid < 32) {
-    const double2 det = warp_gauss_jordan(Ms, n, want_green, perm);
-    if (tid == 0) sums[0] = mult == 2 ? cmul(det, det) : det;
-  }
+  const double2 det = gauss_jordan(Ms, n, want_green, gj, b);
+  if (tid == 0) sums[0] = mult == 2 ? cmul(det, det) : det;
   __syncthreads();
   if (want_green) {
     // G[i][p] = sum_j w[p][j] Minv[j][i]
@@ -78,13 +76,13 @@ green_kernel(Spins sp, int N, int padded, const double2* __restrict__ wa, const 
   }
   if (sp.nspin == 2) cl.sync();
   if (s == 0 && tid == 0) {
-    double2 det = cmul(cmk(1.0, 0.0), sums[0]), e1 = cadd(cmk(0.0, 0.0), sums[1]);
+    double2 d = cmul(cmk(1.0, 0.0), sums[0]), e1 = cadd(cmk(0.0, 0.0), sums[1]);
     if (sp.nspin == 2) {
       const double2* other = cl.map_shared_rank(sums, 1);
-      det = cmul(det, other[0]);
+      d = cmul(d, other[0]);
       if (e1_out) e1 = cadd(e1, other[1]);
     }
-    if (ovlp_out) ovlp_out[b] = det;
+    if (ovlp_out) ovlp_out[b] = d;
     if (e1_out) e1_out[b] = e1;
   }
   if (sp.nspin == 2) cl.sync();  // the other CTA's sums stay readable until here

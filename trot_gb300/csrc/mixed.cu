@@ -19,7 +19,7 @@
 
 namespace trot {
 
-static constexpr int kMaxOccGJ = 16;  // largest n of the warp Gauss-Jordan kernels (perm scratch)
+static constexpr int kMaxOccGJ = 16;  // largest n of the float-float kernels
 
 // ------------------------------------------------------------------ Green's functions in float-float
 // Same quantities as green_kernel (green.cu): M_s = C_s^T w_s, M_s^{-1} by FP64
@@ -32,7 +32,7 @@ green_ff_kernel(Spins sp, int N, const double2* __restrict__ wa, const double2* 
                 double2* __restrict__ green, double2* __restrict__ e1_out) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ double2 red[32];
-  __shared__ int perm[kMaxOccGJ];
+  __shared__ GjScratch gj;
   const int b = blockIdx.x, s = blockIdx.y, tid = threadIdx.x, nt = blockDim.x;
   const int nmax = sp.n[0] > sp.n[1] ? sp.n[0] : sp.n[1];
   ffc* Wf = reinterpret_cast<ffc*>(smem_raw);                    // N x n
@@ -83,8 +83,8 @@ green_ff_kernel(Spins sp, int N, const double2* __restrict__ wa, const double2* 
       Md[e] = make_double2(ff_d(sr), ff_d(si));
     }
     __syncthreads();
-    // M^{-1} in place, FP64, by one warp (warp-synchronous phases; the other warps wait here)
-    if (tid < 32) warp_gauss_jordan(Md, n, true, perm, true);
+    // M^{-1} in place, FP64, by four warps (the others wait here)
+    if (tid < 128) gauss_jordan(Md, n, true, gj, b);
     __syncthreads();
     for (int e = tid; e < n * n; e += nt) Mif[e] = ffc{ff_from_d(Md[e].x), ff_from_d(Md[e].y)};
     __syncthreads();
@@ -1541,6 +1541,7 @@ __global__ void tc_weight_kernel(TrotterArgs a, const double2* __restrict__ ov_n
 // overlap_weight_finish_kernel multiplies the spins and applies phaseless_update.
 __global__ void __launch_bounds__(256) overlap_weight_ff_kernel(Spins sp, TrotterArgs a, double2* __restrict__ ovp) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
+  __shared__ GjScratch gj;
   const int b = blockIdx.x, s = blockIdx.y, tid = threadIdx.x, nt = blockDim.x;
   const int N = a.N;
   const int nmax = sp.n[0] > sp.n[1] ? sp.n[0] : sp.n[1];
@@ -1586,8 +1587,8 @@ __global__ void __launch_bounds__(256) overlap_weight_ff_kernel(Spins sp, Trotte
     Md[e] = make_double2(ff_d(sr), ff_d(si));
   }
   __syncthreads();
-  if (tid < 32) {  // LU determinant in FP64 by one warp
-    const double2 det = warp_gauss_jordan(Md, n, false, nullptr);
+  if (tid < 128) {  // LU determinant in FP64
+    const double2 det = gauss_jordan(Md, n, false, gj, b);
     if (tid == 0) ovp[(size_t)s * a.W + b] = (s ? sp.mult[1] : sp.mult[0]) == 2 ? cmul(det, det) : det;
   }
 }

@@ -81,6 +81,30 @@ TROT_D double2 block_sum2(double2 v, double2* red) {
   return t;
 }
 
+// Sums of eight doubles over a block of 256 threads, into out[0..7] (shared, visible to all on return; red: 64 doubles).
+// Each step of the exchange halves the values a lane carries: 9 additions a warp instead of 40.
+TROT_D void block_sum8(double (&v)[8], double* red, double* out) {
+  const int t = threadIdx.x, l = t & 31;
+#pragma unroll
+  for (int o = 16, n = 4; n >= 1; o >>= 1, n >>= 1)
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const double keep = (l & o) ? v[i + n] : v[i], give = (l & o) ? v[i] : v[i + n];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+  if ((l & 3) == 0) red[(t >> 5) * 8 + (l >> 2)] = v[0];  // lane l holds value l >> 2
+  __syncthreads();
+  if (t < 32) {
+    double s = red[t] + red[t + 32];
+    s += __shfl_xor_sync(0xffffffffu, s, 8);
+    s += __shfl_xor_sync(0xffffffffu, s, 16);
+    if (t < 8) out[t] = s;
+  }
+  __syncthreads();
+}
+
 // ---------------------------------------------------------------- spin layout
 // Per-system spin description used by every kernel: up to two spins; a
 // restricted walker has one spin with multiplicity 2.
@@ -238,7 +262,10 @@ TROT_D double2 quad_gauss_jordan(double2* A, int n, bool inverse, GjScratch& S, 
       const double2 rp = S.rp;
       if (inverse) {
 #pragma unroll 1
-        for (int j = lane; j < n; j += 32) A[k * n + j] = j == k ? rp : cmul(A[k * n + j], rp);
+        for (int j = lane; j < n; j += 32) {
+          const double2 x = A[k * n + j];
+          A[k * n + j] = j == k ? rp : cmk(fma(x.x, rp.x, -__dmul_rn(x.y, rp.y)), fma(x.x, rp.y, __dmul_rn(x.y, rp.x)));
+        }
       } else {
 #pragma unroll 1
         for (int i = k + 1 + lane; i < n; i += 32) A[i * n + k] = cmul(A[i * n + k], rp);
@@ -253,13 +280,19 @@ TROT_D double2 quad_gauss_jordan(double2* A, int n, bool inverse, GjScratch& S, 
       S.det = cmul(S.perm[k] != k ? cmk(-d.x, -d.y) : d, S.piv);
     }
     gj_sync();
-    if (inverse) {  // A[i][j] -= A[i][k] A[k][j] for i != k; in column k the old value counts as 0
+    // A[i][j] -= A[i][k] A[k][j] for i != k; in column k the old value counts as 0.  Which of two products is rounded
+    // first is spelled out (and differs in column k): results that are rounded to FP32 later must not move.
+    if (inverse) {
 #pragma unroll 1
       for (int e = t; e < (n - 1) * n; e += 128) {
         int i = gj_div(e, in);
         const int j = e - i * n;
         i += i >= k;
-        A[i * n + j] = csub(j == k ? cmk(0.0, 0.0) : A[i * n + j], cmul(S.col[i], A[k * n + j]));
+        const bool pc = j == k;
+        const double2 c = S.col[i], b = A[k * n + j], o = pc ? cmk(0.0, 0.0) : A[i * n + j];
+        double x = fma(pc ? c.y : c.x, pc ? b.y : b.x, -__dmul_rn(pc ? c.x : c.y, pc ? b.x : b.y));
+        if (pc) x = -x;
+        A[i * n + j] = cmk(__dsub_rn(o.x, x), __dsub_rn(o.y, fma(c.y, b.x, __dmul_rn(c.x, b.y))));
       }
     } else {
       const int m = n - k - 1;

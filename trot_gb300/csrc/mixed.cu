@@ -6,6 +6,7 @@
 //    combined in float-float (FP32 pairs) arithmetic — near-FP64 accuracy;
 //  * VHS = x_shifted . chol: 3-term BF16 split on tcgen05, FP32 accumulation;
 //  * one-body half steps and the Taylor series: FP32 on the CUDA cores.
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -29,11 +30,12 @@ static constexpr int kMaxOccGJ = 16;  // largest n of the float-float kernels
 // alone would cost more than the rest of the kernel.  One CTA per (walker, spin).
 __global__ void __launch_bounds__(256)
 green_ff_kernel(Spins sp, int N, const double2* __restrict__ wa, const double2* __restrict__ wb,
-                double2* __restrict__ green, double2* __restrict__ e1_out) {
+                double2* __restrict__ green, double2* __restrict__ e1_out, int* __restrict__ status) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ double2 red[32];
   __shared__ GjScratch gj;
   const int b = blockIdx.x, s = blockIdx.y, tid = threadIdx.x, nt = blockDim.x;
+  if (b == 0 && s == 0 && tid == 0) *status = 0;  // this call's status word (the sticky one persists)
   const int nmax = sp.n[0] > sp.n[1] ? sp.n[0] : sp.n[1];
   ffc* Wf = reinterpret_cast<ffc*>(smem_raw);                    // N x n
   ff* Cf = reinterpret_cast<ff*>(Wf + (size_t)N * nmax);          // N x n
@@ -119,7 +121,7 @@ green_ff_kernel(Spins sp, int N, const double2* __restrict__ wa, const double2* 
 }
 
 static int launch_green_ff(const Spins& sp, int W, int N, const double2* wa, const double2* wb, double2* green,
-                           double2* e1_out, cudaStream_t st) {
+                           double2* e1_out, int* status, cudaStream_t st) {
   const int nmax = sp.n[0] > sp.n[1] ? sp.n[0] : sp.n[1];
   const size_t smem = (size_t)N * nmax * (sizeof(ffc) + sizeof(ff)) + 16 + (size_t)nmax * nmax * 2 * 16;
   if (nmax > kMaxOccGJ) {
@@ -131,7 +133,7 @@ static int launch_green_ff(const Spins& sp, int W, int N, const double2* wa, con
     return TROT_ERR_UNSUPPORTED;
   }
   if (smem > 40 * 1024) cudaFuncSetAttribute(green_ff_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  green_ff_kernel<<<dim3(W, sp.nspin), 256, smem, st>>>(sp, N, wa, wb, green, e1_out);
+  green_ff_kernel<<<dim3(W, sp.nspin), 256, smem, st>>>(sp, N, wa, wb, green, e1_out, status);
   TROT_CHECK_LAUNCH("green_ff_kernel");
   return TROT_OK;
 }
@@ -197,13 +199,10 @@ struct MixedBuffers {
   float4* cs[2];     // per spin: traces c_g per (walker, g) as float-float (re.hi, re.lo, im.hi, im.lo)
   ExFixed* xpart;    // exchange partial sums per (walker, Cholesky tile)
   double2* fb;
-  double2* xs;
   double2 *shift_term, *fb_term;
   uint16_t* xq;
   float* vhs;
   uint16_t* vimg;  // [Vr | Vi] operand images of the tensor-core Trotter kernel
-  double2* ov_new; // overlaps of the propagated walkers (tensor-core Trotter, step mode)
-  double2* ovp;    // det(M_s)^mult_s per (spin, walker) of the propagated walkers
   int* node_flag;
   int* status;
   int nblk_total, mpad;
@@ -227,18 +226,13 @@ static size_t carve_mixed(const trot_system* s, const Spins& sp, Carver& c, Mixe
       m.nblk_total += L.nblk;
     }
     m.xpart = c.take<ExFixed>(W * m.nblk_total);
-    m.fb = c.take<double2>(W * G);
+    if (op == TROT_OP_LOCAL_ENERGY) m.fb = c.take<double2>(W * G);
   }
   if (op == TROT_OP_APPLY_TROTTER || op == TROT_OP_PROP_STEP) {
     m.mpad = (int)((2 * W + 127) / 128 * 128);
-    m.xs = c.take<double2>(W * G);
     m.xq = c.take<uint16_t>((size_t)s->mixed->vhs_slices * m.mpad * s->mixed->gpad);
     m.vhs = c.take<float>((size_t)m.mpad * s->mixed->n2pad);
-    if (s->mixed->exp_h1_half_img) {
-      m.vimg = c.take<uint16_t>(W * (kTcImgBytes / 2));
-      m.ov_new = c.take<double2>(W);
-      m.ovp = c.take<double2>(2 * W);
-    }
+    if (s->mixed->exp_h1_half_img) m.vimg = c.take<uint16_t>(W * (kTcImgBytes / 2));
     m.shift_term = c.take<double2>(W);
     m.fb_term = c.take<double2>(W);
     m.node_flag = c.take<int>(W);
@@ -872,6 +866,91 @@ x_slices_kernel(int W, int G, int gpad, int mpad, const C2* __restrict__ xs, uin
 #pragma unroll
       for (int sl = 0; sl < 3; ++sl)
         *reinterpret_cast<uint4*>(o + (size_t)sl * kVSlice + c * 16) = make_uint4(w[c][sl][0], w[c][sl][1], w[c][sl][2], w[c][sl][3]);
+  }
+}
+
+// Force bias, shifted fields, their operand image and the local energy of a step, one CTA per walker (and per padding
+// row pair of the image): fb = sum_s mult_s c_s, the fields as in fields_kernel, E as in energy_combine_kernel.  Four
+// kernels of 2 to 5 us each for a few hundred walkers, and the gaps between them, before: with the weights moved into
+// the overlap kernel 188 -> 159 us for a step of 64 walkers of 24 orbitals.  A thread takes one g; the split terms go through shared memory so that eight g leave as one
+// 16-byte store.
+struct StepFieldsArgs {
+  int W, G, gpad, nspin, mult[2], nchunks;
+  double sqrt_dt, h0;
+  const float4 *c0, *c1;
+  const double *mf_im, *x;
+  const double2* e1;
+  const ExFixed* xpart;
+  const int* status;
+  uint16_t* xq;
+  double2 *shift_term, *fb_term, *energy;  // energy: null if not wanted
+};
+
+__global__ void __launch_bounds__(256) step_fields_kernel(StepFieldsArgs a) {
+  __shared__ __align__(16) uint16_t sh[3][2][256];
+  __shared__ double red[64], sums[8];
+  const int b = blockIdx.x, tid = threadIdx.x, row = 2 * b, nkc = a.gpad / kVK;
+  double v[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};  // shift term, fb term, fb^2, exchange
+  unsigned char* img = reinterpret_cast<unsigned char*>(a.xq) + (size_t)(row >> 7) * nkc * 3 * kVSlice;
+  for (int g0 = 0; g0 < a.gpad; g0 += 256) {
+    const int g = g0 + tid;
+    float re = 0.f, im = 0.f;
+    if (b < a.W && g < a.G) {
+      const size_t k = (size_t)b * a.G + g;
+      const float4 c = a.c0[k];
+      double2 f = cscale(cmk(ff_d(ff{c.x, c.y}), ff_d(ff{c.z, c.w})), (double)a.mult[0]);
+      if (a.nspin == 2) {
+        const float4 d = a.c1[k];
+        f = cadd(f, cscale(cmk(ff_d(ff{d.x, d.y}), ff_d(ff{d.z, d.w})), (double)a.mult[1]));
+      }
+      const double mf = a.mf_im[g], xv = a.x[k];
+      // s = -sqrt(dt) (i fb - i mf); rounded product by product, as the FP32 operand must not depend on the form
+      const double2 s = cmk(__dmul_rn(f.y, a.sqrt_dt), __dmul_rn(f.x - mf, -a.sqrt_dt));
+      const double2 xs = cmk(__dsub_rn(xv, s.x), -s.y);
+      re = d2f_bits(xs.x);
+      im = d2f_bits(xs.y);
+      v[0] = fma(-xs.y, mf, v[0]);
+      v[1] = fma(xs.x, mf, v[1]);
+      v[2] = fma(s.x, fma(-0.5, s.x, xv), fma(0.5 * s.y, s.y, v[2]));  // x s - s^2 / 2
+      v[3] = fma(s.y, xv - s.x, v[3]);
+      if (a.energy) {
+        v[4] = fma(f.x, f.x, fma(-f.y, f.y, v[4]));
+        v[5] = fma(2.0 * f.x, f.y, v[5]);
+      }
+    }
+    uint16_t h[2][3];
+    split3_bf16(re, h[0][0], h[0][1], h[0][2]);
+    split3_bf16(im, h[1][0], h[1][1], h[1][2]);
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+      for (int sl = 0; sl < 3; ++sl) sh[sl][c][tid] = h[c][sl];
+    __syncthreads();
+    const int sl = tid >> 6, c = tid & 1, kk = g0 + ((tid >> 1) & 31) * 8;
+    if (tid < 192 && kk < a.gpad)
+      *reinterpret_cast<uint4*>(img + ((size_t)(kk / kVK) * 3 + sl) * kVSlice + tc::tile_off(row & 127, kk % kVK) +
+                                c * 16) = *reinterpret_cast<const uint4*>(&sh[sl][c][kk - g0]);
+    __syncthreads();
+  }
+  if (b >= a.W) return;
+  const double nan = __longlong_as_double(0x7FF8000000000000ll);
+  if (a.energy)
+    for (int k = tid; k < a.nchunks; k += 256) {
+      const ExFixed f = a.xpart[(size_t)b * a.nchunks + k];
+#pragma unroll
+      for (int c = 0; c < 2; ++c)  // v 2^-s, with 2^-s formed from its exponent bits (|s| < 1000)
+        v[6 + c] += f.s[c] == kExchangeNonFinite ? nan : (double)f.v[c] * pow2d(-f.s[c]);
+    }
+  block_sum8(v, red, sums);
+  if (tid == 0) {
+    a.shift_term[b] = cmk(sums[0], sums[1]);
+    a.fb_term[b] = cmk(sums[2], sums[3]);
+    if (a.energy) {
+      double2 e = a.e1[b];
+      if (a.nspin == 2) e = cadd(e, a.e1[(size_t)a.W + b]);
+      e = cmk(a.h0 + e.x + 0.5 * sums[4] - 0.5 * sums[6], e.y + 0.5 * sums[5] - 0.5 * sums[7]);
+      a.energy[b] = *a.status != 0 ? cmk(nan, nan) : e;  // the exchange / force-bias kernel timed out: no numbers
+    }
   }
 }
 
@@ -1530,18 +1609,14 @@ __global__ void vhs_image_kernel(int W, int N, int n2pad, int packed, const floa
 }
 
 // phaseless weights from overlaps computed after the propagation
-__global__ void tc_weight_kernel(TrotterArgs a, const double2* __restrict__ ov_new) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b < a.W) phaseless_update(a, b, ov_new[b]);
-}
-
 // New overlaps of the propagated walkers and their phaseless weights:
 // M_s = C_s^T w'_s in float-float (four independent accumulators per element),
-// det by FP64 Gauss-Jordan; one CTA per (walker, spin) writes det(M_s)^mult_s, then
-// overlap_weight_finish_kernel multiplies the spins and applies phaseless_update.
-__global__ void __launch_bounds__(256) overlap_weight_ff_kernel(Spins sp, TrotterArgs a, double2* __restrict__ ovp) {
+// det by FP64 elimination; one CTA per (walker, spin), the two spins of a walker in a cluster, whose first CTA
+// multiplies det(M_s)^mult_s and applies phaseless_update (a kernel of its own for that took 10 us at any size).
+__global__ void __launch_bounds__(256) overlap_weight_ff_kernel(Spins sp, TrotterArgs a) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ GjScratch gj;
+  __shared__ double2 dets;  // det(M_s)^mult_s
   const int b = blockIdx.x, s = blockIdx.y, tid = threadIdx.x, nt = blockDim.x;
   const int N = a.N;
   const int nmax = sp.n[0] > sp.n[1] ? sp.n[0] : sp.n[1];
@@ -1589,17 +1664,18 @@ __global__ void __launch_bounds__(256) overlap_weight_ff_kernel(Spins sp, Trotte
   __syncthreads();
   if (tid < 128) {  // LU determinant in FP64
     const double2 det = gauss_jordan(Md, n, false, gj, b);
-    if (tid == 0) ovp[(size_t)s * a.W + b] = (s ? sp.mult[1] : sp.mult[0]) == 2 ? cmul(det, det) : det;
+    if (tid == 0) dets = (s ? sp.mult[1] : sp.mult[0]) == 2 ? cmul(det, det) : det;
   }
-}
-
-// overlap = prod_s det(M_s)^mult_s, then the phaseless weight update
-__global__ void overlap_weight_finish_kernel(int nspin, TrotterArgs a, const double2* __restrict__ ovp) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= a.W) return;
-  double2 ov = cmul(cmk(1.0, 0.0), ovp[b]);
-  if (nspin == 2) ov = cmul(ov, ovp[(size_t)a.W + b]);
-  phaseless_update(a, b, ov);
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  double2 ov = cmk(0.0, 0.0);
+  if (sp.nspin == 2) cl.sync();
+  if (s == 0 && tid == 0) {
+    ov = cmul(cmk(1.0, 0.0), dets);
+    if (sp.nspin == 2) ov = cmul(ov, *cl.map_shared_rank(&dets, 1));
+  }
+  if (sp.nspin == 2) cl.sync();  // the other CTA's determinant stays readable until here
+  if (s == 0 && tid == 0) phaseless_update(a, b, ov);
 }
 
 // ------------------------------------------------------------------ host orchestration
@@ -1676,9 +1752,13 @@ static int run_slices_and_exchange(const trot_system* s, const Spins& sp, MixedB
     dim3 grid(std::min(a.n_items, gknob > 0 ? gknob : 152));
     TROT_TIMED("exchange_exact_tc", st, launch_exchange_exact(L.n_pad, grid, a, st));
   }
-  const int n = W * G;
+  return TROT_OK;
+}
+
+static int run_fb_combine(const trot_system* s, const Spins& sp, double2* fb, MixedBuffers& m, cudaStream_t st) {
+  const int n = s->n_walkers * s->nchol;
   fb_combine_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, sp.nspin, sp.mult[0], sp.mult[1], m.cs[0],
-                                                     sp.nspin == 2 ? m.cs[1] : nullptr, m.fb);
+                                                     sp.nspin == 2 ? m.cs[1] : nullptr, fb);
   TROT_CHECK_LAUNCH("fb_combine_kernel");
   return TROT_OK;
 }
@@ -1718,14 +1798,21 @@ int launch_split3_gemm(int rows, int K, int kpad, int ncols, int npad, const flo
   return split3_gemm(rows, K, kpad, ncols, npad, x, b_image, xq, D, status, st);
 }
 
-static int run_vhs(const trot_system* s, MixedBuffers& m, const double2* xs, cudaStream_t st) {
-  const int W = s->n_walkers, G = s->nchol;
+static int check_vhs_layout(const trot_system* s) {
   const trot_mixed* mx = s->mixed;
   if (mx->vhs_slices != 3 || mx->vhs_order != 2 || mx->gpad % kVK || mx->n2pad % 128) {
     set_error("mixed context: VHS operand layout mismatch");
     return TROT_ERR_BAD_SHAPE;
   }
-  TROT_TIMED("x_slices", st, launch_x_slices(W, G, mx->gpad, m.mpad, xs, m.xq, st));
+  return TROT_OK;
+}
+
+// xs = null: the operand image is there already
+static int run_vhs(const trot_system* s, MixedBuffers& m, const double2* xs, cudaStream_t st) {
+  const int W = s->n_walkers, G = s->nchol;
+  const trot_mixed* mx = s->mixed;
+  TROT_TRY(check_vhs_layout(s));
+  if (xs) TROT_TIMED("x_slices", st, launch_x_slices(W, G, mx->gpad, m.mpad, xs, m.xq, st));
   vhs_gemm_attr();
   const int mtiles = m.mpad / 128, N = s->norb;
   const int ncols = std::min(mx->n2pad, mx->vhs_packed ? N * (N + 1) / 2 : N * N);
@@ -1809,10 +1896,21 @@ static int run_trotter_tc(const trot_system* s, const Spins& sp, const TrotterAr
     if (smem > 40 * 1024)
       cudaFuncSetAttribute(overlap_weight_ff_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     TROT_TIMED("overlap_weight_ff", st, ([&]() -> int {
-      overlap_weight_ff_kernel<<<dim3(W, sp.nspin), 256, smem, st>>>(sp, t, m.ovp);
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3(W, sp.nspin);
+      cfg.blockDim = dim3(256);
+      cfg.dynamicSmemBytes = smem;
+      cfg.stream = st;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = 1;
+      at[0].val.clusterDim.y = sp.nspin;
+      at[0].val.clusterDim.z = 1;
+      cfg.attrs = at;
+      cfg.numAttrs = sp.nspin == 2 ? 1 : 0;
+      const cudaError_t rc = cudaLaunchKernelEx(&cfg, overlap_weight_ff_kernel, sp, t);
+      if (rc != cudaSuccess) return cuda_status(rc, "overlap_weight_ff_kernel");
       TROT_CHECK_LAUNCH("overlap_weight_ff_kernel");
-      overlap_weight_finish_kernel<<<(W + 127) / 128, 128, 0, st>>>(sp.nspin, t, m.ovp);
-      TROT_CHECK_LAUNCH("overlap_weight_finish_kernel");
       return TROT_OK;
     })());
   }
@@ -1834,7 +1932,6 @@ static int begin(const trot_system* s, const Spins& sp, Carver& c, MixedBuffers&
     set_error("workspace too small: %zu < %zu", c.size, c.used);
     return TROT_ERR_WORKSPACE_TOO_SMALL;
   }
-  cudaMemsetAsync(m.status, 0, sizeof(int), st);  // this call's status word (the sticky one persists)
   return TROT_OK;
 }
 
@@ -1843,11 +1940,9 @@ int mixed_force_bias(const trot_system* s, const Spins& sp, const double2* wa, c
   Carver c(ws, ws_bytes);
   MixedBuffers m;
   TROT_TRY(begin(s, sp, c, m, TROT_OP_FORCE_BIAS, st));
-  TROT_TRY(launch_green_ff(sp, s->n_walkers, s->norb, wa, wb, m.green, nullptr, st));
+  TROT_TRY(launch_green_ff(sp, s->n_walkers, s->norb, wa, wb, m.green, nullptr, m.status, st));
   TROT_TRY(run_slices_and_exchange(s, sp, m, st));
-  cudaMemcpyAsync(fb_out, m.fb, (size_t)s->n_walkers * s->nchol * sizeof(double2), cudaMemcpyDeviceToDevice, st);
-  TROT_CHECK_LAUNCH("cudaMemcpyAsync");
-  return TROT_OK;
+  return run_fb_combine(s, sp, fb_out, m, st);
 }
 
 int mixed_local_energy(const trot_system* s, const Spins& sp, const double2* wa, const double2* wb,
@@ -1855,8 +1950,9 @@ int mixed_local_energy(const trot_system* s, const Spins& sp, const double2* wa,
   Carver c(ws, ws_bytes);
   MixedBuffers m;
   TROT_TRY(begin(s, sp, c, m, TROT_OP_LOCAL_ENERGY, st));
-  TROT_TRY(launch_green_ff(sp, s->n_walkers, s->norb, wa, wb, m.green, m.e1, st));
+  TROT_TRY(launch_green_ff(sp, s->n_walkers, s->norb, wa, wb, m.green, m.e1, m.status, st));
   TROT_TRY(run_slices_and_exchange(s, sp, m, st));
+  TROT_TRY(run_fb_combine(s, sp, m.fb, m, st));
   return launch_energy_combine(s->n_walkers, s->nchol, m.nblk_total, s->h0, m.fb, m.e1, sp.nspin, nullptr, energy,
                                st, m.status, m.xpart);
 }
@@ -1882,15 +1978,21 @@ int mixed_prop_step(const trot_system* s, const Spins& sp, const trot_state* sta
   TROT_TRY(begin(s, sp, c, m, TROT_OP_PROP_STEP, st));
   double2* wa = (double2*)state->walkers_a;
   double2* wb = (double2*)state->walkers_b;
-  TROT_TIMED("green_ff", st, launch_green_ff(sp, W, N, wa, wb, m.green, energy_out ? m.e1 : nullptr, st));
+  TROT_TIMED("green_ff", st, launch_green_ff(sp, W, N, wa, wb, m.green, energy_out ? m.e1 : nullptr, m.status, st));
   TROT_TRY(run_slices_and_exchange(s, sp, m, st));
-  if (energy_out)
-    TROT_TIMED("energy_combine", st,
-               launch_energy_combine(W, G, m.nblk_total, s->h0, m.fb, m.e1, sp.nspin, nullptr, energy_out, st,
-                                     m.status, m.xpart));
-  TROT_TIMED("fields", st, launch_fields(W, G, s->sqrt_dt, m.fb, s->mf_shifts_im, fields, m.xs, m.shift_term,
-                                         m.fb_term, st));
-  TROT_TRY(run_vhs(s, m, m.xs, st));
+  StepFieldsArgs f{};
+  f.W = W; f.G = G; f.gpad = s->mixed->gpad; f.nspin = sp.nspin; f.mult[0] = sp.mult[0]; f.mult[1] = sp.mult[1];
+  f.nchunks = m.nblk_total; f.sqrt_dt = s->sqrt_dt; f.h0 = s->h0;
+  f.c0 = m.cs[0]; f.c1 = sp.nspin == 2 ? m.cs[1] : nullptr;
+  f.mf_im = s->mf_shifts_im; f.x = fields; f.e1 = m.e1; f.xpart = m.xpart; f.status = m.status;
+  f.xq = m.xq; f.shift_term = m.shift_term; f.fb_term = m.fb_term; f.energy = energy_out;
+  TROT_TRY(check_vhs_layout(s));
+  TROT_TIMED("step_fields", st, ([&]() -> int {
+    step_fields_kernel<<<m.mpad / 2, 256, 0, st>>>(f);
+    TROT_CHECK_LAUNCH("step_fields_kernel");
+    return TROT_OK;
+  })());
+  TROT_TRY(run_vhs(s, m, nullptr, st));
   TrotterArgs a{};
   a.W = W; a.N = N; a.G = G; a.nterms = s->n_exp_terms; a.sqrt_dt = s->sqrt_dt; a.expH = s->exp_h1_half;
   a.in_a = wa; a.in_b = wb; a.out_a = wa; a.out_b = wb;

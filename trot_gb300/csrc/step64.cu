@@ -163,7 +163,8 @@ step_finalize_kernel(int W, double* __restrict__ weights, double* __restrict__ s
 
 int launch_step_finalize(int W, double* weights, double* scalars, long long* nodes, const int* node_flag,
                          double damping, double dt, cudaStream_t st, const int* status) {
-  step_finalize_kernel<<<1, 1024, 0, st>>>(W, weights, scalars, nodes, node_flag, damping, dt, status);
+  // no more warps than add up to eight walkers a thread: each adds FP64 shuffles to one SM's pipes
+  step_finalize_kernel<<<1, W <= 2048 ? 256 : 1024, 0, st>>>(W, weights, scalars, nodes, node_flag, damping, dt, status);
   TROT_CHECK_LAUNCH("step_finalize_kernel");
   return TROT_OK;
 }

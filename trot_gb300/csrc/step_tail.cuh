@@ -7,17 +7,35 @@ namespace trot {
 
 // Phaseless importance weight of walker b given its new trial overlap
 // (trot/prop/afqmc.py:111-130): weights, overlaps and node flag are updated in place.
+//   imp_ph = |e^(u) rho| cos(arg(e^(v) rho)),  rho = new / old overlap, v = -sqrt(dt) shift, u = v + fb term + ...
+// Away from overflow that is e^(Re u) Re(rho e^(i Im v)): one exponential and one sine / cosine pair instead of two of
+// each, an arc tangent, another cosine and a square root, all of which wait on one another in the FP64 pipe (10 us for
+// one warp, however few walkers).  Beyond the bounds, the formula as it stands.
+static __device__ __noinline__ double phaseless_factor_general(double2 ratio, double2 expo, double2 v) {
+  const double2 imp = cmul(cexp(expo), ratio);
+  const double2 ph = cmul(cexp(v), ratio);
+  const double theta = atan2(ph.y, ph.x);
+  return hypot(imp.x, imp.y) * cos(theta);
+}
+__device__ __forceinline__ int exponent_of(double x) { return ((__double2hiint(x) >> 20) & 0x7FF) - 1023; }
 __device__ __forceinline__ void phaseless_update(const TrotterArgs& a, int b, double2 ov_new) {
   const double2 ov_old = a.overlaps[b];
   const double2 ratio = cdiv(ov_new, ov_old);
   const double2 shift = a.shift_term[b];
   const double2 fbt = a.fb_term[b];
   const double e_shift = a.scalars[0];
-  const double2 expo = cadd(cadd(cscale(shift, -a.sqrt_dt), fbt), cmk(a.dt * (e_shift + a.h0_prop), 0.0));
-  const double2 imp = cmul(cexp(expo), ratio);
-  const double2 ph = cmul(cexp(cscale(shift, -a.sqrt_dt)), ratio);
-  const double theta = atan2(ph.y, ph.x);
-  double imp_ph = hypot(imp.x, imp.y) * cos(theta);
+  const double2 v = cscale(shift, -a.sqrt_dt);
+  const double2 expo = cadd(cadd(v, fbt), cmk(a.dt * (e_shift + a.h0_prop), 0.0));
+  const int er = max(exponent_of(ratio.x), exponent_of(ratio.y));
+  double imp_ph;
+  if (exponent_of(expo.x) < 8 && exponent_of(expo.y) < 8 && exponent_of(v.x) < 8 && exponent_of(v.y) < 8 && er < 100 &&
+      er > -100) {
+    double s, c;
+    sincos(v.y, &s, &c);
+    imp_ph = exp(expo.x) * (ratio.x * c - ratio.y * s);
+  } else {
+    imp_ph = phaseless_factor_general(ratio, expo, v);
+  }
   if (!isfinite(imp_ph) || imp_ph < a.w_floor) imp_ph = 0.0;
   a.node_flag[b] = imp_ph <= 0.0 ? 1 : 0;
   if (imp_ph > a.w_cap) imp_ph = 0.0;

@@ -104,3 +104,24 @@ def test_prop_ctx_numeric_guard():
         ctx.prop_ctx(ss.h0, h1 * 1e15, ss.chol, rdm1, 1.0)
     # the library stays usable after a guarded failure
     ctx.prop_ctx(ss.h0, h1, ss.chol, rdm1, 0.01)
+
+
+@pytest.mark.parametrize("N,G,dt,scale", [(1, 1, 0.1, 1.0), (19, 7, 0.1, 1.0), (20, 1, 0.1, 30.0), (21, 33, 0.02, 1.0),
+                                          (63, 5, 0.3, 8.0), (65, 3, 0.01, 1.0), (127, 9, 0.05, 3.0), (129, 2, 0.05, 0.0)])
+def test_prop_ctx_general_matrices(N, G, dt, scale):
+    """Unsymmetric L_g and h1 at the edges of the squares' and the exponential's tiles, with 0 to 10 squarings, against
+    float64 on the host.  Rounding of A (1e-16 |A|) enters the exponential amplified by its condition, below |A| here."""
+    import scipy.linalg as sl
+
+    from trot_gb300 import ctx
+
+    rng = np.random.default_rng(N)
+    h1 = scale * rng.standard_normal((N, N)) / np.sqrt(N)
+    chol = rng.standard_normal((G, N, N)) / np.sqrt(N * G)
+    rho = rng.standard_normal((N, N)) / N
+    mf_im, h0p, eh, _ = ctx.prop_ctx(0.3, h1, chol, rho, dt)
+    t = np.einsum("gij,ji->g", chol, rho)
+    h_eff = h1 - 0.5 * np.einsum("gik,gkj->ij", chol, chol) + np.einsum("g,gij->ij", t, chol)
+    ref = sl.expm(-0.5 * dt * h_eff)
+    assert np.max(np.abs(cpu(mf_im) - t)) <= 1e-12 * max(1.0, np.max(np.abs(t)))
+    assert rel(cpu(eh), ref) <= 1e-12 * max(1.0, np.linalg.norm(0.5 * dt * h_eff, 1))

@@ -9,13 +9,18 @@
 // The matrix exponential is scaling and squaring of a degree-16 Taylor
 // polynomial: s = the smallest power of two with ||A||_1 / 2^s <= 1/2, the
 // Taylor sum of B = A / 2^s by Horner's rule (remainder < 0.5^17 / 17! ~ 2e-20
-// relative), then s squarings.  s is chosen on the device, so the launches are a
-// fixed sequence (no host round trip; squarings past s return at once).
+// relative), then s squarings, all in one cooperative kernel (s is chosen on the
+// device, no host round trip).
 //
 // Half rotation (trot/runtime_layout.py:200-245; trot/meas/rhf.py:308-319):
 //   rot_h1 = C^T h1 (n, N),  rot_chol[g] = C^T L_g (n, N)   for a real trial C (N, n).
 // CISD (trot/runtime_layout.py:248-292; trot/meas/cisd.py:92-110):
 //   lci1[g][i][p] = sum_t L_g[i][nocc + t] ci1[p][t]   (G, N, nocc).
+#include <cooperative_groups.h>
+
+#include <algorithm>
+
+#include "digits.h"
 #include "kernels.h"
 
 namespace trot {
@@ -126,89 +131,111 @@ __global__ void ctx_heff_kernel(int N, int S, double dt, const double* __restric
   }
 }
 
-// P = I (Horner's starting value)
-__global__ void ctx_eye_kernel(int n, double* __restrict__ P) {
-  const size_t nn = (size_t)n * n;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < nn; e += (size_t)gridDim.x * blockDim.x)
-    P[e] = (e / n == e % n) ? 1.0 : 0.0;
+// part[s][i][j] (+)= sum of t_g L_g[i][j] - 1/2 (L_g L_g)[i][j] over every S-th of the `count` vectors from s on, with
+// the squares given as pairs of rows (launch_square_dg)
+__global__ void ctx_v_sum_kernel(int N, int count, int add, const double* __restrict__ chol, const double* __restrict__ t,
+                                 const double2* __restrict__ sq, double* __restrict__ part) {
+  const size_t nn = (size_t)N * N, ld = (size_t)((N + 1) / 2) * N;
+  const int S = gridDim.y, s = blockIdx.y;
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < nn; e += (size_t)gridDim.x * blockDim.x) {
+    const int i = (int)(e / N), j = (int)(e - (size_t)i * N);
+    double v = add ? part[s * nn + e] : 0.0;
+    const double* q = reinterpret_cast<const double*>(sq + (size_t)(i >> 1) * N + j) + (i & 1);
+    for (int g = s; g < count; g += S) v = fma(t[g], chol[g * nn + e], fma(-0.5, q[2 * (size_t)g * ld], v));
+    part[s * nn + e] = v;
+  }
 }
 
-// ||A||_1 (max column sum) -> number of squarings; status on a non-finite or huge norm
-__global__ void ctx_norm_kernel(int N, const double* __restrict__ A, int* __restrict__ status) {
-  __shared__ double red[256];
-  double m = 0.0;
-  bool finite = true;
-  for (int j = threadIdx.x; j < N; j += blockDim.x) {
-    double c = 0.0;
-    for (int i = 0; i < N; ++i) c += fabs(A[(size_t)i * N + j]);
-    if (!(c <= 1.7e308)) finite = false;  // NaN or inf
-    m = fmax(m, c);
-  }
-  red[threadIdx.x] = finite ? m : -1.0;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) {
-      const double x = red[threadIdx.x], y = red[threadIdx.x + o];
-      red[threadIdx.x] = (x < 0.0 || y < 0.0) ? -1.0 : fmax(x, y);
+// out = expm(A).  One cooperative launch: the 16 Horner products and the squarings were 56 launches, most of them
+// squarings past s that only returned, and a 32 x 32 tile per CTA left all but 9 to 25 SMs idle at N = 80 (1.54 ms of two
+// exponentials of N = 80 and 2 N = 160, 0.36 ms like this; the 32 products and 5 squarings of FP64 0.15).  Tiles of 8 x 8, two halves of K: a CTA's four
+// warps are one per FP64 pipe of its SM.  Products of other CTAs are read past L1.
+static constexpr int kExpmK = 64;
+__device__ __forceinline__ void expm_product(int n, const double* X, const double* Y, double scale, bool identity, double* Z) {
+  __shared__ double As[8][kExpmK + 1], Bs[kExpmK][9], half[64];
+  const int tid = threadIdx.x, h = tid >> 6, r = (tid & 63) >> 3, c = tid & 7, nt = (n + 7) / 8;
+  for (int tile = blockIdx.x; tile < nt * nt; tile += gridDim.x) {
+    const int i0 = tile / nt * 8, j0 = tile % nt * 8;
+    double acc[2] = {0.0, 0.0}, xa[4], xb[4];
+    auto fetch = [&](int k0) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int e = tid + q * 128, i = i0 + e / kExpmK, ka = k0 + e % kExpmK, kb = k0 + e / 8, j = j0 + e % 8;
+        xa[q] = i < n && ka < n ? __ldcg(X + (size_t)i * n + ka) : 0.0;
+        xb[q] = kb < n && j < n ? __ldcg(Y + (size_t)kb * n + j) : 0.0;
+      }
+    };
+    fetch(0);
+    for (int k0 = 0; k0 < n; k0 += kExpmK) {
+      __syncthreads();
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int e = tid + q * 128;
+        As[e / kExpmK][e % kExpmK] = xa[q];
+        Bs[e / 8][e % 8] = xb[q];
+      }
+      __syncthreads();
+      if (k0 + kExpmK < n) fetch(k0 + kExpmK);
+#pragma unroll 8
+      for (int k = h * (kExpmK / 2); k < (h + 1) * (kExpmK / 2); k += 2) {
+        acc[0] = fma(As[r][k], Bs[k][c], acc[0]);
+        acc[1] = fma(As[r][k + 1], Bs[k + 1][c], acc[1]);
+      }
     }
+    if (h) half[tid & 63] = acc[0] + acc[1];
     __syncthreads();
+    const int i = i0 + r, j = j0 + c;
+    if (!h && i < n && j < n)
+      Z[(size_t)i * n + j] = (identity && i == j ? 1.0 : 0.0) + (acc[0] + acc[1] + half[tid]) * scale;
   }
-  if (threadIdx.x == 0) {
-    double nrm = red[0];
-    int s = 0;
-    if (nrm < 0.0) {
-      status[0] = TROT_ERR_NUMERIC_GUARD;
-    } else {
-      while (nrm > 0.5 && s < kMaxSquarings) { nrm *= 0.5; ++s; }
-      if (nrm > 0.5) status[0] = TROT_ERR_NUMERIC_GUARD;
-    }
+}
+
+__global__ void __launch_bounds__(128) ctx_expm_kernel(int n, const double* A, double* out, double* P0, double* P1,
+                                                       int* status) {
+  namespace cg = cooperative_groups;
+  cg::grid_group grid = cg::this_grid();
+  __shared__ unsigned long long top;
+  const int tid = threadIdx.x, lane = tid & 31;
+  // ||A||_1, the largest column sum (columns into P0): NaN and infinity are the largest words
+  for (int j = blockIdx.x * 4 + (tid >> 5); j < n; j += gridDim.x * 4) {
+    double s = 0.0;
+    for (int i = lane; i < n; i += 32) s += fabs(A[(size_t)i * n + j]);
+    s = warp_sum(s);
+    if (lane == 0) P0[j] = s;
+  }
+  if (tid == 0) top = 0;
+  grid.sync();
+  unsigned long long m = 0;
+  for (int j = tid; j < n; j += 128)
+    m = max(m, (unsigned long long)__double_as_longlong(__ldcg(P0 + j)) & 0x7FFFFFFFFFFFFFFFull);
+  atomicMax(&top, m);
+  __syncthreads();
+  double nrm = __longlong_as_double((long long)top);
+  int s = 0;
+  bool bad = !(nrm <= 1.7e308);
+  if (!bad) {
+    while (nrm > 0.5 && s < kMaxSquarings) { nrm *= 0.5; ++s; }
+    bad = nrm > 0.5;
+  }
+  if (blockIdx.x == 0 && tid == 0) {
+    if (bad) status[0] = TROT_ERR_NUMERIC_GUARD;
     status[1] = s;
   }
-}
-
-// mode 0 (Horner): Z = I + (A Y) * (2^-s * kinv);  mode 1 (squaring number q): Z = Y Y if q < s.
-// grid (j tiles, i tiles), 256 threads.
-__global__ void __launch_bounds__(256) ctx_gemm_kernel(int N, int mode, int q, double kinv,
-                                                       const double* __restrict__ A, const double* __restrict__ Y,
-                                                       double* __restrict__ Z, const int* __restrict__ status) {
-  const int s = status[1];
-  if (mode == 1 && q >= s) return;
-  const double* X = mode == 0 ? A : Y;
-  __shared__ double As[kCtxT][kCtxT + 1], Bs[kCtxT][kCtxT + 1];
-  const int j0 = blockIdx.x * kCtxT, i0 = blockIdx.y * kCtxT;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  double acc[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int k0 = 0; k0 < N; k0 += kCtxT) {
-#pragma unroll
-    for (int r = ty; r < kCtxT; r += 8) {
-      const int i = i0 + r, k = k0 + tx, kk = k0 + r, j = j0 + tx;
-      As[r][tx] = (i < N && k < N) ? X[(size_t)i * N + k] : 0.0;
-      Bs[r][tx] = (kk < N && j < N) ? Y[(size_t)kk * N + j] : 0.0;
-    }
-    __syncthreads();
-#pragma unroll 8
-    for (int k = 0; k < kCtxT; ++k) {
-      const double bv = Bs[k][tx];
-#pragma unroll
-      for (int r = 0; r < 4; ++r) acc[r] = fma(As[ty + 8 * r][k], bv, acc[r]);
-    }
-    __syncthreads();
+  grid.sync();
+  // T <- I + B T / k for k = 16 .. 1 (the first with T = I), B = A / 2^s
+  const double b = ldexp(1.0, -s);
+  const size_t nn = (size_t)n * n;
+  for (size_t e = blockIdx.x * (size_t)128 + tid; e < nn; e += (size_t)gridDim.x * 128)
+    P0[e] = (e / n == e % n ? 1.0 : 0.0) + A[e] * (b / kTaylorDeg);
+  double *from = P0, *to = P1;
+  for (int k = kTaylorDeg - 1; k >= 1 - s; --k) {  // k <= 0: squarings
+    grid.sync();
+    double* z = k == 1 - s ? out : to;
+    if (k >= 1) expm_product(n, A, from, b / k, true, z);
+    else expm_product(n, from, from, 1.0, false, z);
+    to = from;
+    from = z;
   }
-  const double scale = mode == 0 ? ldexp(kinv, -s) : 1.0;
-#pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const int i = i0 + ty + 8 * r, j = j0 + tx;
-    if (i < N && j < N) Z[(size_t)i * N + j] = (mode == 0 ? (i == j ? 1.0 : 0.0) : 0.0) + acc[r] * scale;
-  }
-}
-
-// exp_h1_half = P[s & 1] (Horner leaves its sum in P0; squaring q reads P[q & 1])
-__global__ void ctx_final_kernel(int N, const double* __restrict__ P0, const double* __restrict__ P1,
-                                 const int* __restrict__ status, double* __restrict__ out) {
-  const double* P = (status[1] & 1) ? P1 : P0;
-  const size_t nn = (size_t)N * N;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < nn; e += (size_t)gridDim.x * blockDim.x)
-    out[e] = P[e];
 }
 
 // out[g][p][j] = sum_i C[i][p] M_g[i][j] for p in [p0, p0 + 16): grid (G, ceil(n / 16)), 128 threads
@@ -311,27 +338,49 @@ __global__ void ctx_frechet_take_kernel(int N, const double* __restrict__ E, dou
 // TROT_ERR_NUMERIC_GUARD on a non-finite or huge norm, status[1] receives s.
 // p0, p1: n x n scratch.  Used by the propagation context and its adjoint.
 int launch_expm(int n, const double* A, double* out, double* p0, double* p1, int* status, cudaStream_t st) {
-  const size_t nn = (size_t)n * n;
-  const int eb = (int)((nn + 255) / 256 < 1024 ? (nn + 255) / 256 : 1024);
-  const int nt = (n + kCtxT - 1) / kCtxT;
-  ctx_norm_kernel<<<1, 256, 0, st>>>(n, A, status);
-  TROT_CHECK_LAUNCH("ctx_norm_kernel");
-  ctx_eye_kernel<<<eb, 256, 0, st>>>(n, p0);
-  TROT_CHECK_LAUNCH("ctx_eye_kernel");
-  double* P[2] = {p0, p1};
-  // Horner: T <- I + B T / k for k = 16 .. 1, ping-pong P0 -> P1 -> ... -> P0 (16 steps)
-  for (int idx = 0; idx < kTaylorDeg; ++idx) {
-    const int k = kTaylorDeg - idx;
-    ctx_gemm_kernel<<<dim3(nt, nt), 256, 0, st>>>(n, 0, 0, 1.0 / k, A, P[idx & 1], P[(idx + 1) & 1], status);
-    TROT_CHECK_LAUNCH("ctx_gemm_kernel");
+  int dev = 0, sms = 0, per = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, ctx_expm_kernel, 128, 0);
+  const long long nt = (n + 7) / 8, tiles = nt * nt;
+  const int grid = (int)std::min<long long>(tiles, (long long)sms * std::max(1, std::min(per, 4)));
+  void* args[] = {&n, &A, &out, &p0, &p1, &status};
+  const cudaError_t e = cudaLaunchCooperativeKernel((const void*)ctx_expm_kernel, dim3(grid), dim3(128), args, 0, st);
+  if (e != cudaSuccess) return cuda_status(e, "ctx_expm_kernel");
+  TROT_CHECK_LAUNCH("ctx_expm_kernel");
+  return TROT_OK;
+}
+
+// Scratch of the squares' digit products, at the end of a workspace (none for sizes that keep the FP64 kernel)
+static DgScratch carve_squares(int N, int G, Carver& c, int* status) {
+  DgScratch d;
+  if (!dg_takes(N) || N > 1024) return d;
+  const size_t bytes = square_dg_bytes(N, square_dg_count(N, G));
+  d.p = c.take<char>(bytes);
+  d.bytes = bytes;
+  d.status = status;
+  return d;
+}
+
+// part[s] for S slices: sum_g t_g L_g - 1/2 L_g L_g.  400 vectors of 80 orbitals: 880 us with FP64 tiles, 110 us from the
+// digit products.
+static int launch_v(int N, int G, int S, int gper, const double* chol, const double* t, double* part, const DgScratch& d,
+                    cudaStream_t st) {
+  if (!d.p) {
+    const int nt = (N + kCtxT - 1) / kCtxT;
+    ctx_v_partial_kernel<<<dim3(nt, nt, S), 256, 0, st>>>(N, G, gper, chol, t, part);
+    TROT_CHECK_LAUNCH("ctx_v_partial_kernel");
+    return TROT_OK;
   }
-  static_assert((kTaylorDeg & 1) == 0, "Horner must end in P0");
-  for (int q = 0; q < kMaxSquarings; ++q) {
-    ctx_gemm_kernel<<<dim3(nt, nt), 256, 0, st>>>(n, 1, q, 1.0, nullptr, P[q & 1], P[(q + 1) & 1], status);
-    TROT_CHECK_LAUNCH("ctx_gemm_kernel");
+  const int per = square_dg_count(N, G);
+  const size_t nn = (size_t)N * N;
+  for (int g = 0; g < G; g += per) {
+    const int count = std::min(per, G - g);
+    double2* sq = nullptr;
+    TROT_TRY(launch_square_dg(N, count, chol + g * nn, d, &sq, st));
+    ctx_v_sum_kernel<<<dim3((unsigned)((nn + 255) / 256), S), 256, 0, st>>>(N, count, g > 0, chol + g * nn, t + g, sq, part);
+    TROT_CHECK_LAUNCH("ctx_v_sum_kernel");
   }
-  ctx_final_kernel<<<eb, 256, 0, st>>>(n, p0, p1, status, out);
-  TROT_CHECK_LAUNCH("ctx_final_kernel");
   return TROT_OK;
 }
 
@@ -345,7 +394,9 @@ size_t trot_prop_ctx_workspace_size(int norb, int nchol) {
   if (norb < 1 || nchol < 1) { set_error("bad shape: norb %d, nchol %d", norb, nchol); return 0; }
   Carver c(nullptr, 0);
   CtxBuffers b;
-  return carve_ctx(norb, nchol, c, b) + 256;
+  carve_ctx(norb, nchol, c, b);
+  carve_squares(norb, nchol, c, b.status);
+  return c.used + 256;
 }
 
 int trot_build_prop_ctx(int norb, int nchol, double h0, double dt, const double* h1, const double* chol,
@@ -361,6 +412,7 @@ int trot_build_prop_ctx(int norb, int nchol, double h0, double dt, const double*
   Carver c(ws, ws_bytes);
   CtxBuffers b;
   carve_ctx(N, G, c, b);
+  const DgScratch dg = carve_squares(N, G, c, b.status);
   if (!c.ok) { set_error("workspace too small: %zu < %zu", ws_bytes, c.used); return TROT_ERR_WORKSPACE_TOO_SMALL; }
   int S, gper;
   ctx_slices(N, G, S, gper);
@@ -371,9 +423,7 @@ int trot_build_prop_ctx(int norb, int nchol, double h0, double dt, const double*
   TROT_CHECK_LAUNCH("ctx_mf_kernel");
   ctx_h0_kernel<<<1, 256, 0, st>>>(G, h0, mf_im, h0_prop);
   TROT_CHECK_LAUNCH("ctx_h0_kernel");
-  const int nt = (N + kCtxT - 1) / kCtxT;
-  ctx_v_partial_kernel<<<dim3(nt, nt, S), 256, 0, st>>>(N, G, gper, chol, mf_im, b.part);
-  TROT_CHECK_LAUNCH("ctx_v_partial_kernel");
+  TROT_TRY(launch_v(N, G, S, gper, chol, mf_im, b.part, dg, st));
   const size_t nn = (size_t)N * N;
   const int eb = (int)((nn + 255) / 256 < 1024 ? (nn + 255) / 256 : 1024);
   ctx_heff_kernel<<<eb, 256, 0, st>>>(N, S, dt, h1, b.part, b.a);
@@ -390,6 +440,7 @@ size_t trot_prop_ctx_vjp_workspace_size(int norb, int nchol) {
   const size_t m = (size_t)4 * norb * norb;
   c.take<double>(nchol);      // mean-field traces
   for (int k = 0; k < 4; ++k) c.take<double>(m);  // M, P0, P1, expm(M)
+  carve_squares(norb, nchol, c, b.status);
   return c.used + 256;
 }
 
@@ -411,6 +462,7 @@ int trot_prop_ctx_vjp(int norb, int nchol, double dt, const double* h1, const do
   double* q0 = c.take<double>(m);
   double* q1 = c.take<double>(m);
   double* E = c.take<double>(m);
+  const DgScratch dg = carve_squares(N, G, c, b.status);
   if (!c.ok) { set_error("workspace too small: %zu < %zu", ws_bytes, c.used); return TROT_ERR_WORKSPACE_TOO_SMALL; }
   int S, gper;
   ctx_slices(N, G, S, gper);
@@ -419,9 +471,7 @@ int trot_prop_ctx_vjp(int norb, int nchol, double dt, const double* h1, const do
   if (e != cudaSuccess) return cuda_status(e, "trot_prop_ctx_vjp memset");
   ctx_mf_kernel<<<G, 256, 0, st>>>(N, chol, rdm1, t);
   TROT_CHECK_LAUNCH("ctx_mf_kernel");
-  const int nt = (N + kCtxT - 1) / kCtxT;
-  ctx_v_partial_kernel<<<dim3(nt, nt, S), 256, 0, st>>>(N, G, gper, chol, t, b.part);
-  TROT_CHECK_LAUNCH("ctx_v_partial_kernel");
+  TROT_TRY(launch_v(N, G, S, gper, chol, t, b.part, dg, st));
   const size_t nn = (size_t)N * N;
   const int eb = (int)((nn + 255) / 256 < 1024 ? (nn + 255) / 256 : 1024);
   ctx_heff_kernel<<<eb, 256, 0, st>>>(N, S, dt, h1, b.part, b.a);

@@ -630,6 +630,44 @@ int launch_zgemm_dg(int M, int Nn, int K, double alpha, const double2* A, int ld
   return TROT_OK;
 }
 
+// ------------------------------------------------------------------ squares of real matrices
+static size_t square_dg_each(size_t N) {  // scratch of one matrix
+  const size_t rows = (2 * ((N + 1) / 2) + kDgP - 1) / kDgP * kDgP + (N + 127) / 128 * 128;
+  return rows * (kDgRowBytes((N + 15) / 16) + 2) + (N + 1) / 2 * N * sizeof(double2);
+}
+int square_dg_count(size_t N, size_t G) {
+  return (int)std::max<size_t>(1, std::min<size_t>({G, (size_t(128) << 20) / square_dg_each(N), 65535}));
+}
+size_t square_dg_bytes(size_t N, size_t count) { return count * square_dg_each(N) + 6 * 256; }
+
+int launch_square_dg(int N, int count, const double* L, const DgScratch& s, double2** C, cudaStream_t st) {
+  if (s.bytes < square_dg_bytes(N, count)) { set_error("squares: scratch %zu", s.bytes); return TROT_ERR_WORKSPACE_TOO_SMALL; }
+  char* p = reinterpret_cast<char*>(((uintptr_t)s.p + 255) & ~(uintptr_t)255);
+  auto take = [&](size_t n) {
+    char* r = p;
+    p += (n + 255) & ~(size_t)255;
+    return r;
+  };
+  const int mh = (N + 1) / 2, tiles = (2 * mh + kDgP - 1) / kDgP, nrt = (N + 127) / 128;
+  const size_t ra = (size_t)count * tiles * kDgP, rb = (size_t)count * nrt * 128, bytes = kDgRowBytes((N + 15) / 16);
+  DgArgs a{};
+  uint16_t* ia = reinterpret_cast<uint16_t*>(take(ra * bytes));
+  uint16_t* ib = reinterpret_cast<uint16_t*>(take(rb * bytes));
+  int16_t* ea = reinterpret_cast<int16_t*>(take(ra * 2));
+  int16_t* eb = reinterpret_cast<int16_t*>(take(rb * 2));
+  *C = reinterpret_cast<double2*>(take((size_t)count * mh * N * sizeof(double2)));
+  DgSrc sa = dg_src(L, 0, N, N, kDgP, N, 1, ia, ea);
+  sa.rpad = tiles * kDgP; sa.nblk = count; sa.bstride = (long long)N * N;
+  TROT_TRY(dg_rows_launch(sa, (int)(ra / 8), st));
+  DgSrc sb = dg_src(L, 0, N, N, 128, 1, N, ib, eb);
+  sb.rpad = nrt * 128; sb.nblk = count; sb.bstride = (long long)N * N;
+  TROT_TRY(dg_rows_launch(sb, (int)(rb / 8), st));
+  a.imgA = ia; a.exA = ea; a.imgB = ib; a.exB = eb;
+  a.Nn = N; a.M = mh; a.nrt = a.bB = nrt; a.ntile = tiles; a.nbatch = count; a.cstride = (long long)mh * N;
+  a.nk16 = (N + 15) / 16; a.shift = 1; a.C = *C; a.ldc = N; a.salpha = 1; a.status = s.status;
+  return dg_gemm<false>(a, st);
+}
+
 // ------------------------------------------------------------------ exchange
 // f_g[i][j] = sum_p rot_chol_g[i][p] G[j][p] of a chunk of walkers as one product F (rows (b, j), columns (g, i)), then
 // per walker sum_g sum_ij f_gij f_gji and the traces tr f_g (trot/meas/rhf.py:33-60,119-125).  F of a chunk stays in

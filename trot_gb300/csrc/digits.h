@@ -27,6 +27,12 @@ size_t exchange_dg_bytes(const Spins& sp, size_t W, size_t N, size_t G);
 int launch_exchange_dg(const Spins& sp, int W, int N, int G, const double2* green, double2* partial, double2* fb,
                        const DgScratch& s, cudaStream_t st);
 
+// C[g][m][j] = (row 2 m, row 2 m + 1) of L_g L_g for `count` real N x N matrices, m < ceil(N / 2) (N even or odd: the
+// odd last row's partner is zero).  square_dg_count: matrices a call takes with a scratch of square_dg_bytes.
+int square_dg_count(size_t N, size_t G);
+size_t square_dg_bytes(size_t N, size_t count);
+int launch_square_dg(int N, int count, const double* L, const DgScratch& s, double2** C, cudaStream_t st);
+
 // Trotter propagation (with overlaps and weights in step mode) by digit products; same results as launch_trotter.
 size_t trotter_dg_bytes(const Spins& sp, size_t W, size_t N);
 int launch_trotter_dg(const Spins& sp, const TrotterArgs& a, const DgScratch& s, cudaStream_t st);

@@ -150,8 +150,11 @@ __global__ void ctx_v_sum_kernel(int N, int count, int add, const double* __rest
 // squarings past s that only returned, and a 32 x 32 tile per CTA left all but 9 to 25 SMs idle at N = 80 (1.54 ms of two
 // exponentials of N = 80 and 2 N = 160, 0.36 ms like this; the 32 products and 5 squarings of FP64 0.15).  Tiles of 8 x 8, two halves of K: a CTA's four
 // warps are one per FP64 pipe of its SM.  Products of other CTAs are read past L1.
+// The sums are kept as R = T - I (R <- (B + B R) / k, R <- 2 R + R^2), rounded relative to R and not to I, which the
+// squarings would amplify; I is added at the end.
 static constexpr int kExpmK = 64;
-__device__ __forceinline__ void expm_product(int n, const double* X, const double* Y, double scale, bool identity, double* Z) {
+// Z = (by X + X Y) scale (+ I)
+__device__ __forceinline__ void expm_product(int n, const double* X, const double* Y, double scale, double by, bool last, double* Z) {
   __shared__ double As[8][kExpmK + 1], Bs[kExpmK][9], half[64];
   const int tid = threadIdx.x, h = tid >> 6, r = (tid & 63) >> 3, c = tid & 7, nt = (n + 7) / 8;
   for (int tile = blockIdx.x; tile < nt * nt; tile += gridDim.x) {
@@ -186,7 +189,8 @@ __device__ __forceinline__ void expm_product(int n, const double* X, const doubl
     __syncthreads();
     const int i = i0 + r, j = j0 + c;
     if (!h && i < n && j < n)
-      Z[(size_t)i * n + j] = (identity && i == j ? 1.0 : 0.0) + (acc[0] + acc[1] + half[tid]) * scale;
+      Z[(size_t)i * n + j] = fma(by, __ldcg(X + (size_t)i * n + j), acc[0] + acc[1] + half[tid]) * scale +
+                             (last && i == j ? 1.0 : 0.0);
   }
 }
 
@@ -222,17 +226,17 @@ __global__ void __launch_bounds__(128) ctx_expm_kernel(int n, const double* A, d
     status[1] = s;
   }
   grid.sync();
-  // T <- I + B T / k for k = 16 .. 1 (the first with T = I), B = A / 2^s
+  // R <- (B + B R) / k for k = 16 .. 1 (the first with R = 0), B = A / 2^s
   const double b = ldexp(1.0, -s);
   const size_t nn = (size_t)n * n;
-  for (size_t e = blockIdx.x * (size_t)128 + tid; e < nn; e += (size_t)gridDim.x * 128)
-    P0[e] = (e / n == e % n ? 1.0 : 0.0) + A[e] * (b / kTaylorDeg);
+  for (size_t e = blockIdx.x * (size_t)128 + tid; e < nn; e += (size_t)gridDim.x * 128) P0[e] = A[e] * (b / kTaylorDeg);
   double *from = P0, *to = P1;
   for (int k = kTaylorDeg - 1; k >= 1 - s; --k) {  // k <= 0: squarings
     grid.sync();
-    double* z = k == 1 - s ? out : to;
-    if (k >= 1) expm_product(n, A, from, b / k, true, z);
-    else expm_product(n, from, from, 1.0, false, z);
+    const bool last = k == 1 - s;
+    double* z = last ? out : to;
+    if (k >= 1) expm_product(n, A, from, b / k, 1.0, last, z);
+    else expm_product(n, from, from, 1.0, 2.0, last, z);
     to = from;
     from = z;
   }

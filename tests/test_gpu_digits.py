@@ -197,3 +197,19 @@ def test_trotter_from_digit_products(kind, N, na, nb, terms, W):
     st = S.step(S.state(S.walkers(w), np.ones(W), ov, -1.0, -1.0), dev(x))
     assert np.max(np.abs(cpu(st.overlaps) - o.overlaps)) <= 1e-10 * np.max(np.abs(o.overlaps))
     assert np.allclose(cpu(st.weights), o.weights, rtol=1e-9, atol=1e-12)
+
+
+def test_more_row_groups_than_a_grid_dimension_holds():
+    """4100 walkers of 60 orbitals make 65600 groups of eight operand rows, past the 65535 of a grid's y and z; every
+    walker keeps the bits of a run of its own."""
+    from trot_gb300.prop import make_trotter_ops
+
+    N, n, G, W = 60, 5, 24, 4100
+    ss = synthetic.make_system(N, (n, n), G, seed=4)
+    S = Setup("rhf_r", ss.h0, ss.h1, ss.chol, ss.mo_a, ss.mo_b, 0.01, W)
+    w = dev(synthetic.perturbed_walkers(ss.mo_a, W, 0.1, 3))
+    xs = dev(np.random.default_rng(2).standard_normal((W, G)) + 0j)
+    op = make_trotter_ops("restricted", "restricted").apply_trotter
+    full = op(w, xs, S.prop_ctx, 6)
+    for a, b in ((0, 3), (2047, 2050), (4093, 4100)):
+        assert torch.equal(full[a:b], op(w[a:b].contiguous(), xs[a:b].contiguous(), S.prop_ctx, 6))

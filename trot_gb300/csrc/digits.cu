@@ -166,15 +166,28 @@ static DgSrc dg_src(const double* p, int cplx, int rows, int K, int R, long long
   return DgSrc{p, K, (K + 15) / 16, R, cplx, 0, rows, kDgOneBlock, 1, 0, rst, kst, kDgOneBlock, nullptr, 0, 0, img, ex};
 }
 
-__global__ void __launch_bounds__(256) dg_rows_kernel(DgSrc a) {
+// Up to four sources of the same K in one launch: most are small (3 to 10 us, half of it the launch and the tail), and
+// the operands of a product do not depend on one another.  FP64 energy of 67 orbitals, 200 walkers: 7 launches -> 4.
+struct DgRows {
+  static constexpr int kMax = 4;
+  DgSrc s[kMax];
+  int first[kMax + 1];  // first group of eight rows of each
+  int count, ks;        // ks: CTAs of a cluster, one after the other in the grid
+};
+
+__global__ void __launch_bounds__(256) dg_rows_kernel(const __grid_constant__ DgRows q) {
+  const int KS = q.ks, rank = (int)blockIdx.x % KS;
+  int src = 0, group = (int)blockIdx.x / KS;
+  while (src + 1 < q.count && group >= q.first[src + 1]) ++src;
+  group -= q.first[src];
+  const DgSrc& a = q.s[src];
   __shared__ unsigned smx[8][8], cmx[8];
   __shared__ float sl1[8][8], cl1[8];
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
-  const int KS = (int)gridDim.x, rank = (int)blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int rl = lane & 7, kg = lane >> 3;
-  const int row = blockIdx.y * 8 + rl;
+  const int row = group * 8 + rl;
   const int blk = row / a.rpad, rr = row - blk * a.rpad;
   const bool valid = blk < a.nblk && rr < a.rpb, flip = a.conj && (rr & 1);
   const double* p = a.p;
@@ -257,12 +270,15 @@ __global__ void __launch_bounds__(256) dg_rows_kernel(DgSrc a) {
 // a warp per 32 k, eight at most
 static int dg_row_threads(int nk16) { return 32 * std::min(8, (nk16 + 1) / 2); }
 
-static int dg_rows_launch(const DgSrc& a, int groups, cudaStream_t st) {
+static int dg_rows_launch(DgRows q, cudaStream_t st) {
+  const int groups = q.first[q.count], nk16 = q.s[0].nk16;
+  if (groups == 0) return TROT_OK;
   int ks = 1;
-  while (ks < 8 && a.nk16 * 16 > 256 * ks && groups * ks < 304) ks *= 2;
+  while (ks < 8 && nk16 * 16 > 256 * ks && groups * ks < 304) ks *= 2;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(ks, groups);
-  cfg.blockDim = dim3(dg_row_threads(a.nk16));
+  q.ks = ks;
+  cfg.gridDim = dim3((unsigned)ks * (unsigned)groups);
+  cfg.blockDim = dim3(dg_row_threads(nk16));
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -271,10 +287,20 @@ static int dg_rows_launch(const DgSrc& a, int groups, cudaStream_t st) {
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = ks > 1 ? 1 : 0;
-  const cudaError_t rc = cudaLaunchKernelEx(&cfg, dg_rows_kernel, a);
+  const cudaError_t rc = cudaLaunchKernelEx(&cfg, dg_rows_kernel, q);
   if (rc != cudaSuccess) return cuda_status(rc, "dg_rows_kernel");
   TROT_CHECK_LAUNCH("dg_rows_kernel");
   return TROT_OK;
+}
+static void dg_rows_add(DgRows& q, const DgSrc& a, int groups) {
+  q.s[q.count] = a;
+  q.first[q.count + 1] = q.first[q.count] + groups;
+  ++q.count;
+}
+static int dg_rows_launch(const DgSrc& a, int groups, cudaStream_t st) {
+  DgRows q{};
+  dg_rows_add(q, a, groups);
+  return dg_rows_launch(q, st);
 }
 
 // ------------------------------------------------------------------ product
@@ -605,7 +631,6 @@ int launch_zgemm_dg(int M, int Nn, int K, double alpha, const double2* A, int ld
   uint16_t* imgA = reinterpret_cast<uint16_t*>(take(2 * mc * kDgRowBytes(nk16)));
   int16_t* exB = reinterpret_cast<int16_t*>(take((size_t)nrt * 128 * 2));
   int16_t* exA = reinterpret_cast<int16_t*>(take(2 * mc * 2));
-  TROT_TRY(dg_rows_launch(dg_src(B, 0, Nn, K, 128, b_is_nk ? ldb : 1, b_is_nk ? 1 : ldb, imgB, exB), nrt * 16, st));
   int lk = 0;
   while ((1 << lk) < K) ++lk;
   a.imgB = imgB; a.exB = exB; a.imgA = imgA; a.exA = exA;
@@ -621,8 +646,11 @@ int launch_zgemm_dg(int M, int Nn, int K, double alpha, const double2* A, int ld
   for (size_t m0 = 0; m0 < (size_t)M; m0 += mc) {
     const int mm = (int)std::min(mc, (size_t)M - m0);
     a.ntile = (2 * mm + kDgP - 1) / kDgP;
-    TROT_TRY(dg_rows_launch(dg_src(reinterpret_cast<const double*>(A + (long long)m0 * lda), 1, 2 * mm, K, kDgP, 2ll * lda,
-                                   2, imgA, exA), a.ntile * 4, st));
+    DgRows rows{};
+    dg_rows_add(rows, dg_src(reinterpret_cast<const double*>(A + (long long)m0 * lda), 1, 2 * mm, K, kDgP, 2ll * lda, 2,
+                             imgA, exA), a.ntile * 4);
+    if (m0 == 0) dg_rows_add(rows, dg_src(B, 0, Nn, K, 128, b_is_nk ? ldb : 1, b_is_nk ? 1 : ldb, imgB, exB), nrt * 16);
+    TROT_TRY(dg_rows_launch(rows, st));
     a.M = mm;
     a.C = C + (long long)m0 * ldc;
     TROT_TRY(dg_gemm<false>(a, st));
@@ -658,10 +686,12 @@ int launch_square_dg(int N, int count, const double* L, const DgScratch& s, doub
   *C = reinterpret_cast<double2*>(take((size_t)count * mh * N * sizeof(double2)));
   DgSrc sa = dg_src(L, 0, N, N, kDgP, N, 1, ia, ea);
   sa.rpad = tiles * kDgP; sa.nblk = count; sa.bstride = (long long)N * N;
-  TROT_TRY(dg_rows_launch(sa, (int)(ra / 8), st));
+  DgRows rows{};
+  dg_rows_add(rows, sa, (int)(ra / 8));
   DgSrc sb = dg_src(L, 0, N, N, 128, 1, N, ib, eb);
   sb.rpad = nrt * 128; sb.nblk = count; sb.bstride = (long long)N * N;
-  TROT_TRY(dg_rows_launch(sb, (int)(rb / 8), st));
+  dg_rows_add(rows, sb, (int)(rb / 8));
+  TROT_TRY(dg_rows_launch(rows, st));
   a.imgA = ia; a.exA = ea; a.imgB = ib; a.exB = eb;
   a.Nn = N; a.M = mh; a.nrt = a.bB = nrt; a.ntile = tiles; a.nbatch = count; a.cstride = (long long)mh * N;
   a.nk16 = (N + 15) / 16; a.shift = 1; a.C = *C; a.ldc = N; a.salpha = 1; a.status = s.status;
@@ -774,15 +804,16 @@ int launch_exchange_dg(const Spins& sp, int W, int N, int G, const double2* gree
   for (int q = 0; q < sp.nspin; ++q) {
     const int n = sp.n[q], Gn = G * n;
     a.nrt = (Gn + 127) / 128;
-    if (q == 0 || sp.rot_chol[q] != sp.rot_chol[0] || n != sp.n[0]) {
-      TROT_TRY(dg_rows_launch(dg_src(sp.rot_chol[q], 0, Gn, N, 128, N, 1, imgB, exB), a.nrt * 16, st));
-    }
+    DgRows rows{};
+    if (q == 0 || sp.rot_chol[q] != sp.rot_chol[0] || n != sp.n[0])
+      dg_rows_add(rows, dg_src(sp.rot_chol[q], 0, Gn, N, 128, N, 1, imgB, exB), a.nrt * 16);
     const int tiles = (2 * W * n + kDgP - 1) / kDgP;
     DgSrc sa = dg_src(reinterpret_cast<const double*>(green + (size_t)sp.off[q] * N), 1, 2 * n, N, kDgP, 2ll * N, 2, imgA, exA);
     sa.rpad = 2 * n;
     sa.nblk = W;
     sa.bstride = 2ll * sp.ntot * N;
-    TROT_TRY(dg_rows_launch(sa, tiles * 4, st));
+    dg_rows_add(rows, sa, tiles * 4);
+    TROT_TRY(dg_rows_launch(rows, st));
     a.imgB = imgB; a.exB = exB;
     a.Nn = Gn; a.nk16 = nk16; a.nbatch = 1; a.shift = 1;  // N <= 1024
     a.C = F; a.ldc = Gn; a.salpha = 1; a.ealpha = 0; a.accumulate = 0; a.status = s.status;
@@ -956,8 +987,9 @@ int launch_trotter_dg(const Spins& sp, const TrotterArgs& t, const DgScratch& s,
   sv.rpad = pl.vtiles * 128;
   sv.nblk = W;
   sv.bstride = 2ll * N * N;
-  if (t.nterms > 0) TROT_TRY(dg_rows_launch(sv, W * pl.vtiles * 16, st));
-  TROT_TRY(dg_rows_launch(dg_src(t.expH, 0, N, N, 128, N, 1, eimg, eex), (int)erows / 8, st));
+  DgRows rows{};
+  if (t.nterms > 0) dg_rows_add(rows, sv, W * pl.vtiles * 16);
+  dg_rows_add(rows, dg_src(t.expH, 0, N, N, 128, N, 1, eimg, eex), (int)erows / 8);
   DgSrc sw = dg_src(reinterpret_cast<const double*>(t.in_a), 1, 2 * nc, N, kDgP, 2, 2ll * sp.n[0], uimg, uex);
   sw.rpad = pl.rpad;
   sw.nblk = W;
@@ -968,7 +1000,8 @@ int launch_trotter_dg(const Spins& sp, const TrotterArgs& t, const DgScratch& s,
     sw.bstride2 = 2ll * N * sp.n[1];
     sw.kst2 = 2ll * sp.n[1];
   }
-  TROT_TRY(dg_rows_launch(sw, W * pl.tiles * 4, st));
+  dg_rows_add(rows, sw, W * pl.tiles * 4);
+  TROT_TRY(dg_rows_launch(rows, st));
   DgArgs e{};  // E x
   e.imgB = eimg; e.exB = eex; e.imgA = uimg; e.exA = uex;
   e.Nn = N; e.M = nc; e.nrt = (N + 127) / 128; e.ntile = pl.tiles; e.nk16 = pl.nk16; e.shift = 1;
@@ -1031,8 +1064,10 @@ void adjoint_dg_carve(DgAdjoint& d, int W, int N, int nc, int K2, const DgScratc
 
 int adjoint_dg_e(const DgAdjoint& d, const double* E, cudaStream_t st) {
   const int groups = (int)adj_rows(d.N, 128) / 8;
-  TROT_TRY(dg_rows_launch(dg_src(E, 0, d.N, d.N, 128, d.N, 1, d.eimg, d.eex), groups, st));
-  return dg_rows_launch(dg_src(E, 0, d.N, d.N, 128, 1, d.N, d.etimg, d.etex), groups, st);
+  DgRows rows{};
+  dg_rows_add(rows, dg_src(E, 0, d.N, d.N, 128, d.N, 1, d.eimg, d.eex), groups);
+  dg_rows_add(rows, dg_src(E, 0, d.N, d.N, 128, 1, d.N, d.etimg, d.etex), groups);
+  return dg_rows_launch(rows, st);
 }
 
 int adjoint_dg_v(const DgAdjoint& d, const double2* V, bool transposed, cudaStream_t st) {
@@ -1104,12 +1139,14 @@ int adjoint_dg_gv(const DgAdjoint& d, const double2* S, long long sstride, const
   s.rpad = rpad;
   s.nblk = d.W;
   s.bstride = 2 * sstride;
-  TROT_TRY(dg_rows_launch(s, d.W * (rpad / 8), st));
+  DgRows rows{};
+  dg_rows_add(rows, s, d.W * (rpad / 8));
   DgSrc u = dg_src(reinterpret_cast<const double*>(U), 1, 2 * N, d.K2, 128, 2, 2ll * N, d.vimg, d.vex);
   u.rpad = vpad;
   u.nblk = d.W;
   u.bstride = 2 * ustride;
-  TROT_TRY(dg_rows_launch(u, d.W * (vpad / 8), st));
+  dg_rows_add(rows, u, d.W * (vpad / 8));
+  TROT_TRY(dg_rows_launch(rows, st));
   DgArgs a{};
   a.imgA = d.uimg; a.exA = d.uex; a.imgB = d.vimg; a.exB = d.vex;
   a.Nn = 2 * N; a.M = N; a.nrt = a.bB = vpad / 128; a.ntile = rpad / kDgP; a.nbatch = d.W;
@@ -1190,8 +1227,8 @@ cisd_pairs_kernel(int n, int G, int gsub, int nchunk, const double2* __restrict_
   }
 }
 
-static int cisd_lg_rows(const CisdGammaArgs& c, uint16_t* irow, int16_t* erow, uint16_t* ilc, int16_t* elc,
-                        cudaStream_t st);
+static void cisd_lg_rows(DgRows& rows, const CisdGammaArgs& c, uint16_t* irow, int16_t* erow, uint16_t* ilc,
+                         int16_t* elc);
 
 static size_t cgd_chunk(size_t W, size_t N, size_t n, size_t G) {
   const size_t wc = std::max<size_t>(1, (size_t(64) << 20) / (n * G * N * sizeof(double2)));
@@ -1239,8 +1276,9 @@ int launch_cisd_gamma_dg(const CisdGammaArgs& c, const DgScratch& s, cudaStream_
   // rows (g, i) = columns of L_g; (g, p) = rows p < n of L_g; (g, a) = columns of lci1_g
   DgSrc sc = dg_src(c.chol, 0, N, N, 128, 1, N, b.icol, b.ecol);
   sc.rpad = N; sc.nblk = G; sc.bstride = (long long)N * N;
-  TROT_TRY(dg_rows_launch(sc, (int)(adj_rows((size_t)G * N, 128) / 8), st));
-  TROT_TRY(cisd_lg_rows(c, b.irow, b.erow, b.ilc, b.elc, st));
+  DgRows first{};
+  dg_rows_add(first, sc, (int)(adj_rows((size_t)G * N, 128) / 8));
+  cisd_lg_rows(first, c, b.irow, b.erow, b.ilc, b.elc);
   const int gsub = std::max(1, std::min(kPairsChunk, 256 / nn)), nchunk = cisd_gamma_dg_chunks(G);
   const size_t smem = (size_t)(gsub + 1) * nn * sizeof(double2);
   if (smem > 40 * 1024) cudaFuncSetAttribute(cisd_pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1249,8 +1287,9 @@ int launch_cisd_gamma_dg(const CisdGammaArgs& c, const DgScratch& s, cudaStream_
     const int wn = std::min(wc, W - w0);
     const double2* gr = c.green + (size_t)w0 * n * N;
     const int tiles = (2 * wn * n + kDgP - 1) / kDgP;
-    TROT_TRY(dg_rows_launch(dg_src(reinterpret_cast<const double*>(gr), 1, 2 * wn * n, N, kDgP, 2ll * N, 2, b.ig, b.eg),
-                            tiles * 4, st));
+    DgRows rows = w0 == 0 ? first : DgRows{};
+    dg_rows_add(rows, dg_src(reinterpret_cast<const double*>(gr), 1, 2 * wn * n, N, kDgP, 2ll * N, 2, b.ig, b.eg), tiles * 4);
+    TROT_TRY(dg_rows_launch(rows, st));
     DgArgs a{};
     a.imgA = b.ig; a.exA = b.eg; a.M = wn * n; a.ntile = tiles; a.nbatch = 1;
     a.nk16 = (N + 15) / 16; a.shift = 1; a.salpha = 1; a.status = s.status;
@@ -1265,10 +1304,12 @@ int launch_cisd_gamma_dg(const CisdGammaArgs& c, const DgScratch& s, cudaStream_
     TROT_CHECK_LAUNCH("cisd_q_kernel");
     DgSrc sq = dg_src(reinterpret_cast<const double*>(b.Q), 1, 2 * N, N, 128, 2, 2ll * N, b.iq, b.eq);
     sq.rpad = qpad; sq.nblk = wn; sq.bstride = 2ll * N * N;
-    TROT_TRY(dg_rows_launch(sq, wn * (qpad / 8), st));
+    DgRows pair{};
+    dg_rows_add(pair, sq, wn * (qpad / 8));
     DgSrc s2 = dg_src(reinterpret_cast<const double*>(b.gl), 1, 2 * G * n, N, kDgP, 2ll * N, 2, b.igl, b.egl);
     s2.rpad = glpad; s2.nblk = wn; s2.bstride = 2ll * n * G * N;
-    TROT_TRY(dg_rows_launch(s2, wn * (glpad / 8), st));
+    dg_rows_add(pair, s2, wn * (glpad / 8));
+    TROT_TRY(dg_rows_launch(pair, st));
     DgArgs q{};
     q.imgA = b.igl; q.exA = b.egl; q.imgB = b.iq; q.exB = b.eq;
     q.M = G * n; q.ntile = glpad / kDgP; q.Nn = 2 * N; q.nrt = q.bB = qpad / 128; q.nbatch = wn;
@@ -1311,25 +1352,27 @@ size_t cisd_lg_dg_bytes(size_t W, size_t N, size_t n, size_t G) {
 }
 
 // digits of the rows p < n of every L_g and of the columns of every lci1_g
-static int cisd_lg_rows(const CisdGammaArgs& c, uint16_t* irow, int16_t* erow, uint16_t* ilc, int16_t* elc,
-                        cudaStream_t st) {
+static void cisd_lg_rows(DgRows& rows, const CisdGammaArgs& c, uint16_t* irow, int16_t* erow, uint16_t* ilc,
+                         int16_t* elc) {
   const int N = c.N, n = c.n, G = c.G, groups = (int)(adj_rows((size_t)G * n, 128) / 8);
   DgSrc sr = dg_src(c.chol, 0, n, N, 128, N, 1, irow, erow);
   sr.rpad = n; sr.nblk = G; sr.bstride = (long long)N * N;
-  TROT_TRY(dg_rows_launch(sr, groups, st));
+  dg_rows_add(rows, sr, groups);
   DgSrc sl = dg_src(c.lci1, 0, n, N, 128, 1, n, ilc, elc);
   sl.rpad = n; sl.nblk = G; sl.bstride = (long long)N * n;
-  return dg_rows_launch(sl, groups, st);
+  dg_rows_add(rows, sl, groups);
 }
 
 int launch_cisd_lg_dg(const CisdGammaArgs& c, const DgScratch& s, double2** F1, double2** F2, cudaStream_t st) {
   const int W = c.W, N = c.N, n = c.n, G = c.G;
   ClgBuffers b;
   if (s.bytes < clg_carve(b, W, N, n, G, s.p)) { set_error("CISD terms: scratch %zu", s.bytes); return TROT_ERR_WORKSPACE_TOO_SMALL; }
-  TROT_TRY(cisd_lg_rows(c, b.irow, b.erow, b.ilc, b.elc, st));
+  DgRows rows{};
+  cisd_lg_rows(rows, c, b.irow, b.erow, b.ilc, b.elc);
   const int tiles = (2 * W * n + kDgP - 1) / kDgP;
-  TROT_TRY(dg_rows_launch(dg_src(reinterpret_cast<const double*>(c.green), 1, 2 * W * n, N, kDgP, 2ll * N, 2, b.ig, b.eg),
-                          tiles * 4, st));
+  dg_rows_add(rows, dg_src(reinterpret_cast<const double*>(c.green), 1, 2 * W * n, N, kDgP, 2ll * N, 2, b.ig, b.eg),
+              tiles * 4);
+  TROT_TRY(dg_rows_launch(rows, st));
   DgArgs a{};
   a.imgA = b.ig; a.exA = b.eg; a.M = W * n; a.ntile = tiles; a.nbatch = 1;
   a.nk16 = (N + 15) / 16; a.shift = 1; a.salpha = 1; a.status = s.status;

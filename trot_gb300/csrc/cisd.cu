@@ -608,8 +608,11 @@ cisd_gamma_f32_kernel(int N, int n, int v, int G, const double2* __restrict__ gr
 // walker, lg1 and the n x n sums stay in the warp's shared memory, no CTA barrier between vectors.  What is left per
 // vector is gl P2 and glgp in FP32 (7 n N + 4 n^2 v operations) and n^3 float-float products; the two float-float
 // products over N that cisd_gamma_f32_kernel forms per vector were 3/4 of its work.
+// Latency bounds it (a vector's loads, products and stores follow one another in its warp): 32 warps an SM and rows of
+// glgp in fours rather than eights (64 instead of 128 registers) take 450 us for 256 walkers of 60 orbitals, 8 + 8
+// electrons and 300 vectors, 16 warps and eights 584.
 static constexpr int kGammaChunk = 32;  // vectors per CTA
-static constexpr int kGammaTile = 8;    // rows p of glgp at a time
+static constexpr int kGammaTile = 4;    // rows p of glgp at a time
 
 static size_t cisd_gamma_w_shared(int N, int n) { return (size_t)2 * n * N * sizeof(float2) + (size_t)n * (n | 1) * 16; }
 static size_t cisd_gamma_w_warp(int N, int n) { return ((size_t)n * N * sizeof(float2) + 15) / 16 * 16 + (size_t)n * (n | 1) * 16; }
@@ -619,7 +622,7 @@ static int cisd_gamma_w_warps(int N, int n) {
                                                                            : (56 * 1024 - sh) / pw));
 }
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)
 cisd_gamma_w_kernel(int N, int n, int v, int G, const double2* __restrict__ green, const float* __restrict__ gld, int ldd,
                     const double2* __restrict__ F1, const double2* __restrict__ F2, const double2* __restrict__ p2,
                     const double2* __restrict__ ci1g1, double2* __restrict__ xg, float2* __restrict__ xf,

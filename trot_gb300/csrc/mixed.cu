@@ -1717,6 +1717,25 @@ static int launch_exchange_exact(int n_pad, dim3 grid, const ExArgs& a, cudaStre
   return TROT_OK;
 }
 
+// Walker tiles per item (an item: a Cholesky tile and a run of walker tiles): the busiest CTA has
+// ceil(items / CTAs) items, so the run is chosen to leave the last round full.  A tile takes 4.2 us; an item of one tile
+// waits for its Cholesky tile about 1 us, of two 0.2 us, longer ones hide it.  Runs of eight, as before / by this rule:
+// N = 24, n = 5, 120 vectors, 64 walkers 40.2 / 10.7 us; N = 97, n = 12, 388, 128: 106 / 83; N = 40, n = 6, 160, 512:
+// 76.6 / 46.6; N = 120, n = 12 + 10, 720, 1024: 1621 / 1602.
+static int exchange_run(int ntiles, int nblk, int ctas) {
+  int best = 1;
+  double cost = 1e300;
+  for (int t = 1; t <= std::min(ntiles, 16); ++t) {
+    const long long items = (long long)nblk * ((ntiles + t - 1) / t);
+    const double c = (double)((items + ctas - 1) / ctas) * (t + 0.25 / t);
+    if (c <= cost) {
+      cost = c;
+      best = t;
+    }
+  }
+  return best;
+}
+
 static int run_slices_and_exchange(const trot_system* s, const Spins& sp, MixedBuffers& m, cudaStream_t st) {
   const int W = s->n_walkers, N = s->norb, G = s->nchol;
   for (int q = 0; q < sp.nspin; ++q) {
@@ -1734,9 +1753,9 @@ static int run_slices_and_exchange(const trot_system* s, const Spins& sp, MixedB
     ExArgs a{};
     a.L = L;
     a.G = G; a.W = W; a.mult = sp.mult[q];
-    // persistent grid: one CTA per SM walks (Cholesky tile, run of 8 walker tiles) items
-    const int tpi = tune_get(TROT_TUNE_EXCHANGE_TILES);
-    a.tiles_per_item = std::min(tpi > 0 ? tpi : 8, L.ntiles);
+    // persistent grid: one CTA per SM walks (Cholesky tile, run of walker tiles) items
+    const int tpi = tune_get(TROT_TUNE_EXCHANGE_TILES), gknob = tune_get(TROT_TUNE_EXCHANGE_GRID);
+    a.tiles_per_item = std::min(tpi > 0 ? tpi : exchange_run(L.ntiles, L.nblk, gknob > 0 ? gknob : 152), L.ntiles);
     a.chunks = (L.ntiles + a.tiles_per_item - 1) / a.tiles_per_item;
     a.n_items = L.nblk * a.chunks;
     a.rot_img = s->mixed->rot_slices[mq];
@@ -1748,7 +1767,6 @@ static int run_slices_and_exchange(const trot_system* s, const Spins& sp, MixedB
     a.nblk_total = m.nblk_total;
     a.status = m.status;
     a.test_timeout_polls = tune_get(TROT_TUNE_TEST_TIMEOUT);
-    const int gknob = tune_get(TROT_TUNE_EXCHANGE_GRID);
     dim3 grid(std::min(a.n_items, gknob > 0 ? gknob : 152));
     TROT_TIMED("exchange_exact_tc", st, launch_exchange_exact(L.n_pad, grid, a, st));
   }

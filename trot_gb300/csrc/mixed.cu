@@ -1295,6 +1295,7 @@ struct TrotTcArgs {
   const uint16_t* vimg;  // (W, 8 chunks, 3, 128, 32) bf16 image of [Vr | Vi]
   const uint16_t* eimg;  // (4 chunks, 3, 128, 32) bf16 image of E
   int* status;
+  int wpc;               // walkers per CTA, 1 or kTcWPC
 };
 
 // B element (row j, k < 128) = x as 3 slices; B image = [kchunk][slice][NB rows][32]
@@ -1339,8 +1340,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) trotter_tc_kernel(Spins sp, Tro
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int N = a.N, nc = sp.ntot, nterms = a.nterms;
   const int nsteps = nterms + 2;  // E, V x nterms, E
-  const int b0 = blockIdx.x * WPC;
-  const int nw = min(WPC, a.W - b0);
+  const int nkc = (N + kTcKC - 1) / kTcKC;  // K chunks of E, Vr and Vi that are not all padding
+  const int b0 = blockIdx.x * g.wpc;
+  const int nw = min(g.wpc, a.W - b0);
   if (warp == 16) tc::tmem_alloc(&tslot, X::TmemCols);
   if (tid < 18) coefs[tid] = tid == 0 ? 1.f : (float)(a.sqrt_dt / (double)tid);
   if (tid == kTcEpi) {
@@ -1376,13 +1378,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) trotter_tc_kernel(Spins sp, Tro
       int c = 0;
       for (int step = 0; step < nsteps && ok; ++step) {
         const bool vterm = step > 0 && step <= nterms;
-        const int nk = vterm ? 8 : 4;
+        const int nk = vterm ? 2 * nkc : nkc;
         for (int wi = 0; wi < nw && ok; ++wi) {
           const uint32_t bw = sb + (uint32_t)wi * kBBytes;
           // this walker's B operand for the step is written by the epilogue
           ok = tc::mbar_wait(&b_ready[wi], (uint32_t)(step & 1));
-          for (int kc = 0; kc < nk && ok; ++kc, ++c) {
-            const int st = c % S;
+          for (int kk = 0; kk < nk && ok; ++kk, ++c) {
+            const int st = c % S, kc = kk < nkc ? kk : 4 + kk - nkc;
             ok = tc::mbar_wait(&full[st], (uint32_t)((c / S) & 1));
             if (!ok) break;
             tc::fence_after_sync();
@@ -1427,11 +1429,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) trotter_tc_kernel(Spins sp, Tro
       int last = -1;  // this loader's last issued chunk
       int c = 0;
       for (int step = 0; step < nsteps && ok; ++step) {
-        const int nk = (step > 0 && step <= nterms) ? 8 : 4;
+        const int nk = (step > 0 && step <= nterms) ? 2 * nkc : nkc;
         for (int wi = 0; wi < nw && ok; ++wi)
-          for (int kc = 0; kc < nk; ++kc, ++c) {
+          for (int kk = 0; kk < nk; ++kk, ++c) {
             if (c % kTcLoaders != w) continue;
-            const int st = c % S;
+            const int st = c % S, kc = kk < nkc ? kk : 4 + kk - nkc;
             if (c >= S) {  // the MMAs of chunk c - S have read the slot
               const uint32_t par = (uint32_t)(((c / S) - 1) & 1);
               uint32_t polls = 0;
@@ -1581,10 +1583,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) trotter_tc_kernel(Spins sp, Tro
 // 16-byte stores.
 __global__ void vhs_image_kernel(int W, int N, int n2pad, int packed, const float* __restrict__ D,
                                  uint16_t* __restrict__ img) {
-  const size_t total = (size_t)W * 8 * 128 * 4;
+  const int nkc = (N + kTcKC - 1) / kTcKC;  // chunks past the orbitals are not read
+  const size_t total = (size_t)W * 2 * nkc * 128 * 4;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-    const int kg = (int)(e & 3), p = (int)((e >> 2) & 127), kc = (int)((e >> 9) & 7);
-    const size_t b = e >> 12;
+    const int kg = (int)(e & 3), p = (int)((e >> 2) & 127);
+    const size_t b = (e >> 9) / (2 * nkc);
+    const int kk = (int)((e >> 9) - b * (2 * nkc)), kc = kk < nkc ? kk : 4 + kk - nkc;
     const int k0 = kc * kTcKC + kg * 8;              // 0..255
     const int im = k0 >= 128 ? 1 : 0, q0 = k0 & 127;
     const float* src = D + (2 * b + im) * (size_t)n2pad;
@@ -1874,7 +1878,7 @@ template <int NB>
 static void trotter_tc_launch(const Spins& sp, const TrotTcArgs& g, int W, cudaStream_t st) {
   constexpr size_t smem = TcShape<NB>::smem;
   cudaFuncSetAttribute(trotter_tc_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  trotter_tc_kernel<NB><<<(W + kTcWPC - 1) / kTcWPC, kTcThreads, smem, st>>>(sp, g);
+  trotter_tc_kernel<NB><<<(W + g.wpc - 1) / g.wpc, kTcThreads, smem, st>>>(sp, g);
 }
 
 static int run_trotter_tc(const trot_system* s, const Spins& sp, const TrotterArgs& t, const MixedBuffers& m,
@@ -1887,7 +1891,7 @@ static int run_trotter_tc(const trot_system* s, const Spins& sp, const TrotterAr
   }
   static_assert(kTcImgBytes == 8 * (size_t)kTcChunk, "operand image size");
   TROT_TIMED("vhs_image", st, ([&]() -> int {
-    const size_t threads = (size_t)W * 8 * 128 * 4;
+    const size_t threads = (size_t)W * 2 * ((N + kTcKC - 1) / kTcKC) * 128 * 4;
     const int blocks = (int)std::min<size_t>((threads + 255) / 256, 152 * 32);
     vhs_image_kernel<<<blocks, 256, 0, st>>>(W, N, s->mixed->n2pad, s->mixed->vhs_packed, m.vhs, m.vimg);
     TROT_CHECK_LAUNCH("vhs_image_kernel");
@@ -1898,6 +1902,9 @@ static int run_trotter_tc(const trot_system* s, const Spins& sp, const TrotterAr
   g.vimg = m.vimg;
   g.eimg = s->mixed->exp_h1_half_img;
   g.status = m.status;
+  // one walker alone in a CTA takes 0.59 of the time of two (N = 24, n = 5: 27 / 47 us; N = 120, n = 15: 31 / 51), so two
+  // share one only if that saves rounds: 304 walkers 53 / 47 us, 456 79.6 / 93.3, 608 108 / 96
+  g.wpc = 0.59 * ((W + 151) / 152) < (W + 303) / 304 ? 1 : kTcWPC;
   TROT_TIMED("trotter_tc", st, ([&]() -> int {
     switch (NB) {
       case 16: trotter_tc_launch<16>(sp, g, W, st); break;

@@ -314,6 +314,7 @@ green_slices_kernel(int N, int n, int n_pad, int P, int WB, int W, int ntot, int
 #pragma unroll
     for (int k = 0; k < kKP / 32; ++k) {
       const int p = lane + 32 * k;
+      if (p >> 4 >= (N + 15) >> 4) break;  // K16 steps past the orbitals are not read
       long long v = rint_scaled(x[k], kGreenBits - e);
       uint16_t* dst = out + (size_t)(p >> 4) * unit;
 #pragma unroll
@@ -334,6 +335,8 @@ green_slices_kernel(int N, int n, int n_pad, int P, int WB, int W, int ntot, int
 // (trot/meas/rhf.py:33-60) and the traces c_g = sum_i f_gii (Coulomb / force bias,
 // trot/meas/rhf.py:119-125).
 //
+// K16 steps past the last orbital are neither loaded nor multiplied (N = 24: 2 of 8; 10.7 -> 7.9 us at 64 walkers).
+//
 // A persistent CTA walks work items = (Cholesky tile: gb vectors x n orbitals = up to
 // 128 MMA rows (g, i), run of walker tiles of P columns).  Warp 16 (one lane) is the
 // producer.  The rot_chol digits of the item's tile (5 planes x 128 rows x 128 orbitals)
@@ -353,6 +356,7 @@ green_slices_kernel(int N, int n, int n_pad, int P, int WB, int W, int ntot, int
 // A_d in float-float, stages f in shared memory for the transposed products f_gji, and
 // reduces the exchange and the traces in fixed order.
 struct ExArgs {
+  int nks;                   // K16 steps of the orbitals, <= kKS
   SpinLayout L;
   int G, W, mult;
   int tiles_per_item, chunks, n_items;  // work item = (Cholesky tile, run of walker tiles)
@@ -427,12 +431,14 @@ struct ExShape {
   static constexpr size_t bytes = offBar + 40 * 8 + 1024;                      // + base alignment
 };
 
-template <int NP>
+// FULL: kKS steps, as a constant (a loop of a.nks steps takes 2 % longer at 120 orbitals)
+template <int NP, bool FULL>
 __global__ void __launch_bounds__(kExThreads, 1) exchange_exact_kernel(ExArgs a) {
   using X = ExShape<NP>;
   constexpr int P = X::P, WBT = X::WBT, JH = X::JH, FS = X::FS;
   constexpr uint32_t UB = X::UB, UU = X::UU;
-  constexpr int kUnits = kKS / kExKU;  // ring units per walker tile
+  static_assert(kExKU == 1, "a ring unit is one K16 step");
+  const int nks = FULL ? kKS : a.nks;  // K16 steps that are not all padding, ring units per walker tile
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = smem_raw + ((1024 - (tc::smem_u32(smem_raw) & 1023)) & 1023);
   unsigned char* sA = base;
@@ -506,7 +512,7 @@ __global__ void __launch_bounds__(kExThreads, 1) exchange_exact_kernel(ExArgs a)
             if (!ok) break;
           }
           const uint32_t dcol = taddr + (uint32_t)(buf * 256);
-          for (int k = 0; k < kKS; ++k, ++gs) {
+          for (int k = 0; k < nks; ++k, ++gs) {
             if (i == 0) {
               ok = tc::mbar_wait(&a_full[k], (uint32_t)(kitem & 1));
               if (!ok) break;
@@ -557,7 +563,7 @@ __global__ void __launch_bounds__(kExThreads, 1) exchange_exact_kernel(ExArgs a)
       int last_b = -1;  // this loader's last issued unit
       auto units_of = [&](int item) {
         const int t0 = (item % a.chunks) * a.tiles_per_item;
-        return (min(L.ntiles, t0 + a.tiles_per_item) - t0) * kUnits;
+        return (min(L.ntiles, t0 + a.tiles_per_item) - t0) * nks;
       };
       int btot = bi < a.n_items ? units_of(bi) : 0;
       auto advance_b = [&]() {
@@ -575,7 +581,7 @@ __global__ void __launch_bounds__(kExThreads, 1) exchange_exact_kernel(ExArgs a)
           const int slot = bg % kExSlots;
           if (bg < kExSlots || tc::mbar_test_wait(&empty[slot], (uint32_t)((bg / kExSlots - 1) & 1))) {
             const int t0 = (bi % a.chunks) * a.tiles_per_item;
-            const int ti = t0 + bu / kUnits, tk = (bu % kUnits) * kExKU;
+            const int ti = t0 + bu / nks, tk = bu % nks;
             tc::mbar_expect_tx(&full[slot], UU);
             tc::bulk_g2s(ring + (size_t)slot * UU, a.green_img + ((size_t)ti * kKS + tk) * (UB / 2), UU, &full[slot]);
             last_b = bg;
@@ -590,7 +596,7 @@ __global__ void __launch_bounds__(kExThreads, 1) exchange_exact_kernel(ExArgs a)
                        &a_full[ak]);
           pend_mask |= 1u << ak;
           pend_par = (pend_par & ~(1u << ak)) | ((uint32_t)(ka & 1) << ak);
-          if (++ak == kKS) {
+          if (++ak == nks) {
             ak = 0;
             ai += gridDim.x;
             ++ka;
@@ -1697,16 +1703,21 @@ static int check_mixed_shapes(const trot_system* s, const Spins& sp) {
   return TROT_OK;
 }
 
-template <int NP>
+template <int NP, bool FULL>
 static void exchange_exact_launch(dim3 grid, const ExArgs& a, cudaStream_t st) {
   constexpr size_t smem = ExShape<NP>::bytes;
   static_assert(smem <= 232448, "exchange kernel: shared memory above the 227 KB limit");
   static bool attr_set = false;
   if (!attr_set) {
-    cudaFuncSetAttribute(exchange_exact_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(exchange_exact_kernel<NP, FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     attr_set = true;
   }
-  exchange_exact_kernel<NP><<<grid, kExThreads, smem, st>>>(a);
+  exchange_exact_kernel<NP, FULL><<<grid, kExThreads, smem, st>>>(a);
+}
+template <int NP>
+static void exchange_exact_launch(dim3 grid, const ExArgs& a, cudaStream_t st) {
+  if (a.nks == kKS) exchange_exact_launch<NP, true>(grid, a, st);
+  else exchange_exact_launch<NP, false>(grid, a, st);
 }
 
 static int launch_exchange_exact(int n_pad, dim3 grid, const ExArgs& a, cudaStream_t st) {
@@ -1722,10 +1733,10 @@ static int launch_exchange_exact(int n_pad, dim3 grid, const ExArgs& a, cudaStre
 }
 
 // Walker tiles per item (an item: a Cholesky tile and a run of walker tiles): the busiest CTA has
-// ceil(items / CTAs) items, so the run is chosen to leave the last round full.  A tile takes 4.2 us; an item of one tile
+// ceil(items / CTAs) items, so the run is chosen to leave the last round full.  A tile takes 4 us; an item of one tile
 // waits for its Cholesky tile about 1 us, of two 0.2 us, longer ones hide it.  Runs of eight, as before / by this rule:
-// N = 24, n = 5, 120 vectors, 64 walkers 40.2 / 10.7 us; N = 97, n = 12, 388, 128: 106 / 83; N = 40, n = 6, 160, 512:
-// 76.6 / 46.6; N = 120, n = 12 + 10, 720, 1024: 1621 / 1602.
+// N = 24, n = 5, 120 vectors, 64 walkers 32.9 / 7.9 us; N = 97, n = 12, 388, 128: 99.7 / 77.6; N = 40, n = 6, 160, 512:
+// 68.4 / 42.0; N = 120, n = 12 + 10, 720, 1024: 1621 / 1602.
 static int exchange_run(int ntiles, int nblk, int ctas) {
   int best = 1;
   double cost = 1e300;
@@ -1756,7 +1767,7 @@ static int run_slices_and_exchange(const trot_system* s, const Spins& sp, MixedB
     const int mq = (s->kind == TROT_UHF_U) ? q : 0;
     ExArgs a{};
     a.L = L;
-    a.G = G; a.W = W; a.mult = sp.mult[q];
+    a.G = G; a.W = W; a.mult = sp.mult[q]; a.nks = (N + 15) / 16;
     // persistent grid: one CTA per SM walks (Cholesky tile, run of walker tiles) items
     const int tpi = tune_get(TROT_TUNE_EXCHANGE_TILES), gknob = tune_get(TROT_TUNE_EXCHANGE_GRID);
     a.tiles_per_item = std::min(tpi > 0 ? tpi : exchange_run(L.ntiles, L.nblk, gknob > 0 ? gknob : 152), L.ntiles);
@@ -1902,8 +1913,8 @@ static int run_trotter_tc(const trot_system* s, const Spins& sp, const TrotterAr
   g.vimg = m.vimg;
   g.eimg = s->mixed->exp_h1_half_img;
   g.status = m.status;
-  // one walker alone in a CTA takes 0.59 of the time of two (N = 24, n = 5: 27 / 47 us; N = 120, n = 15: 31 / 51), so two
-  // share one only if that saves rounds: 304 walkers 53 / 47 us, 456 79.6 / 93.3, 608 108 / 96
+  // one walker alone in a CTA takes 0.59 of the time of two (N = 97, n = 12: 30 / 50 us; N = 120, n = 15: 31 / 51), so two
+  // share one only if that saves rounds: N = 97, 304 walkers 61 / 51 us, 456 91 / 100, 608 122 / 104
   g.wpc = 0.59 * ((W + 151) / 152) < (W + 303) / 304 ? 1 : kTcWPC;
   TROT_TIMED("trotter_tc", st, ([&]() -> int {
     switch (NB) {

@@ -1736,7 +1736,7 @@ static int launch_exchange_exact(int n_pad, dim3 grid, const ExArgs& a, cudaStre
 // ceil(items / CTAs) items, so the run is chosen to leave the last round full.  A tile takes 4 us; an item of one tile
 // waits for its Cholesky tile about 1 us, of two 0.2 us, longer ones hide it.  Runs of eight, as before / by this rule:
 // N = 24, n = 5, 120 vectors, 64 walkers 32.9 / 7.9 us; N = 97, n = 12, 388, 128: 99.7 / 77.6; N = 40, n = 6, 160, 512:
-// 68.4 / 42.0; N = 120, n = 12 + 10, 720, 1024: 1621 / 1602.
+// 68.4 / 42.0; N = 120, n = 12 + 10, 600, 1024: 1621 / 1602.
 static int exchange_run(int ntiles, int nblk, int ctas) {
   int best = 1;
   double cost = 1e300;

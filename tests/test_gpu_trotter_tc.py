@@ -28,3 +28,21 @@ def test_chunks_and_walkers_per_cta(N, n):
     assert rel(cpu(full), cpu(ref)) <= 2e-5
     for m in (1, 151, 153, 304):
         assert torch.equal(op(w[:m].contiguous(), xs[:m].contiguous(), S.prop_ctx, 6), full[:m])
+
+
+@pytest.mark.parametrize("terms", [1, 31, 32, 33, 64])
+def test_many_terms(terms):
+    """The FP64 kernel's coefficients, 32 at a time, against the oracle (1e-10, the FP64 path's tolerance)."""
+    import trot_gb300 as tg
+    from oracle import afqmc_oracle as orc
+    from trot_gb300 import synthetic
+
+    N, n, G, W = 9, 2, 12, 3
+    ss = synthetic.make_system(N, (n, n), G, decay=30.0, seed=2, h0=0.2)
+    S = Setup("rhf_r", ss.h0, ss.h1, ss.chol, ss.mo_a, ss.mo_b, 0.01, W)
+    w = synthetic.perturbed_walkers(ss.mo_a, W, 0.1, 3)
+    rng = np.random.default_rng(5)
+    xs = rng.normal(size=(W, G)) + 0.3j * rng.normal(size=(W, G))
+    got = tg.make_trotter_ops("restricted", "restricted").apply_trotter(dev(w), dev(xs), S.prop_ctx, terms)
+    ref = orc.apply_trotter_r(w, xs, orc.build_prop_ctx(ss.h0, ss.h1, ss.chol, ss.rdm1(), 0.01), terms)
+    assert rel(cpu(got), ref) <= 1e-10

@@ -858,7 +858,7 @@ cisd_energy_kernel(int G, int nchunk, double h0, const double2* __restrict__ wsc
                    const double2* __restrict__ lg, const double2* __restrict__ lcs,
                    const double2* __restrict__ gpart, const double2* __restrict__ l2part,
                    double2* __restrict__ energy, const int* __restrict__ status) {
-  __shared__ double2 red[32];
+  __shared__ double red[64], sums[2][8];
   const int b = blockIdx.x;
   if (status[0] != 0) {  // a tensor-core product of this call timed out: no numbers
     const double nan = __longlong_as_double(0x7FF8000000000000ll);
@@ -874,10 +874,14 @@ cisd_energy_kernel(int G, int nchunk, double h0, const double2* __restrict__ wsc
   double2 p[4] = {cmk(0.0, 0.0), cmk(0.0, 0.0), cmk(0.0, 0.0), cmk(0.0, 0.0)};
   for (int c = threadIdx.x; c < nchunk; c += blockDim.x)
     for (int k = 0; k < 4; ++k) p[k] = cadd(p[k], gpart[((size_t)b * nchunk + c) * 4 + k]);
-  lglg = block_sum2(lglg, red);
-  lslg = block_sum2(lslg, red);
-  for (int k = 0; k < 4; ++k) p[k] = block_sum2(p[k], red);
+  double u[8] = {lglg.x, lglg.y, lslg.x, lslg.y, 0.0, 0.0, 0.0, 0.0};
+  double v[8] = {p[0].x, p[0].y, p[1].x, p[1].y, p[2].x, p[2].y, p[3].x, p[3].y};
+  block_sum8(u, red, sums[0]);
+  block_sum8(v, red, sums[1]);
   if (threadIdx.x == 0) {
+    lglg = cmk(sums[0][0], sums[0][1]);
+    lslg = cmk(sums[0][2], sums[0][3]);
+    for (int k = 0; k < 4; ++k) p[k] = cmk(sums[1][2 * k], sums[1][2 * k + 1]);
     const double2 ci1g = wsc[(size_t)b * 8 + 0], gci2g = wsc[(size_t)b * 8 + 1];
     const double2 e1_1_2 = wsc[(size_t)b * 8 + 2], e1_2_2 = wsc[(size_t)b * 8 + 3];
     double2 l2ci2 = cmk(0.0, 0.0);

@@ -14,7 +14,7 @@ __global__ void __launch_bounds__(256)
 fields_kernel(int G, double sqrt_dt, const double2* __restrict__ fb, const double* __restrict__ mf_im,
               const double* __restrict__ x, double2* __restrict__ xs, double2* __restrict__ shift_term,
               double2* __restrict__ fb_term) {
-  __shared__ double2 red[32];
+  __shared__ double red[64], sums[8];
   const int b = blockIdx.x;
   double2 st = cmk(0.0, 0.0), ft = cmk(0.0, 0.0);
   for (int g = threadIdx.x; g < G; g += blockDim.x) {
@@ -28,11 +28,11 @@ fields_kernel(int G, double sqrt_dt, const double2* __restrict__ fb, const doubl
     st = cadd(st, cmul(xsv, mf));
     ft = cadd(ft, csub(cscale(s, xv), cscale(cmul(s, s), 0.5)));
   }
-  st = block_sum2(st, red);
-  ft = block_sum2(ft, red);
+  double v[8] = {st.x, st.y, ft.x, ft.y, 0.0, 0.0, 0.0, 0.0};
+  block_sum8(v, red, sums);
   if (threadIdx.x == 0) {
-    shift_term[b] = st;
-    fb_term[b] = ft;
+    shift_term[b] = cmk(sums[0], sums[1]);
+    fb_term[b] = cmk(sums[2], sums[3]);
   }
 }
 
@@ -257,7 +257,7 @@ energy_combine_kernel(int G, int nchunks, double h0, const double2* __restrict__
                       const double2* __restrict__ e1, int e1_parts, const double2* __restrict__ partial,
                       double2* __restrict__ energy, const int* __restrict__ status,
                       const ExFixed* __restrict__ xfixed) {
-  __shared__ double2 red[32];
+  __shared__ double red[64], sums[8];
   const int b = blockIdx.x;
   if (status && status[0] != 0) {  // the exchange / force-bias kernel timed out: no numbers
     const double nan = __longlong_as_double(0x7FF8000000000000ll);
@@ -282,9 +282,11 @@ energy_combine_kernel(int G, int nchunks, double h0, const double2* __restrict__
   } else {
     for (int k = threadIdx.x; k < nchunks; k += blockDim.x) x = cadd(x, partial[(size_t)b * nchunks + k]);
   }
-  c = block_sum2(c, red);
-  x = block_sum2(x, red);
+  double v8[8] = {c.x, c.y, x.x, x.y, 0.0, 0.0, 0.0, 0.0};
+  block_sum8(v8, red, sums);
   if (threadIdx.x == 0) {
+    c = cmk(sums[0], sums[1]);
+    x = cmk(sums[2], sums[3]);
     double2 e = e1[b];
     for (int k = 1; k < e1_parts; ++k) e = cadd(e, e1[(size_t)k * gridDim.x + b]);
     energy[b] = cmk(h0 + e.x + 0.5 * c.x - 0.5 * x.x, e.y + 0.5 * c.y - 0.5 * x.y);

@@ -62,21 +62,32 @@ TROT_D double warp_sum(double v) {
 }
 TROT_D double2 warp_sum2(double2 v) { return cmk(warp_sum(v.x), warp_sum(v.y)); }
 
-// Block-wide sum in a fixed order (deterministic).  `red` holds >= 32 double2.
+// Block-wide sum in a fixed order (deterministic).  `red` holds >= 32 double2.  The halves of a warp take one component
+// each after the first exchange: 5 + 3 dependent FP64 additions for 256 threads instead of 20, at about 60 cycles each.
 TROT_D double2 block_sum2(double2 v, double2* red) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-  v = warp_sum2(v);
+  const bool im = lane & 16;
+  double a = (im ? v.y : v.x) + __shfl_xor_sync(0xffffffffu, im ? v.x : v.y, 16);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+  double* rd = reinterpret_cast<double*>(red) + (im ? 1 : 0);
   __syncthreads();
-  if (lane == 0) red[wid] = v;
+  if ((lane & 15) == 0) rd[2 * wid] = a;
   __syncthreads();
-  double2 t = cmk(0.0, 0.0);
-  if (wid == 0) {
-    t = lane < nw ? red[lane] : cmk(0.0, 0.0);
-    t = warp_sum2(t);
-    if (lane == 0) red[0] = t;
+  if (nw > 1) {
+    if (wid == 0) {
+      const int k = lane & 15;
+      a = k < nw ? rd[2 * k] : 0.0;
+      if (nw > 16) a += k + 16 < nw ? rd[2 * (k + 16)] : 0.0;
+#pragma unroll 1
+      for (int o = 8; o > 0; o >>= 1)
+        if (nw > o) a += __shfl_xor_sync(0xffffffffu, a, o);
+      __syncwarp();
+      if (k == 0) rd[0] = a;
+    }
+    __syncthreads();
   }
-  __syncthreads();
-  t = red[0];
+  const double2 t = red[0];
   __syncthreads();
   return t;
 }

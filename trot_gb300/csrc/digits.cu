@@ -707,7 +707,7 @@ int launch_square_dg(int N, int count, const double* L, const DgScratch& s, doub
 // exchange_pairs_kernel, one CTA per (64 Cholesky vectors, walker): the vectors' n x n blocks in shared memory, row i
 // takes the pairs (i, i + k mod n), k <= n / 2, each product once (weight 2 off the diagonal), four FP64 FMAs each:
 // 0.6 ms of the FP64 pipe at 120 orbitals, 12 + 10 electrons, 600 vectors, 1024 walkers, which bounds it.  The CTA's
-// own reduction (20 FP64 additions per warp) costs as much as 16 vectors' products, hence 64 vectors per CTA.
+// own reduction (8 FP64 additions in a row) costs as much as 6 vectors' products, hence 64 vectors per CTA.
 static constexpr int kExgChunk = 64;     // vectors per partial sum
 static constexpr int kExgThreads = 128;  // a thread per (vector, i) of the vectors in shared memory
 
@@ -747,12 +747,15 @@ exchange_pairs_kernel(int n, int G, int gsub, int nchunks, int mult, int add, co
         cfma(once, sm[j * lds + tid], row[j]);
       }
     }
-    if (tid < ng) {
-      double2 t = cmk(0.0, 0.0);
-      for (int r = 0; r < n; ++r) t = cadd(t, sm[r * lds + tid * n + r]);
-      if (mult == 2) t = cadd(t, t);
-      double2* o = fb + (size_t)b * G + gs + tid;
-      *o = add ? cadd(*o, t) : t;
+    // the traces, a thread per vector and component (a thread per vector issued twice the FP64 instructions of one warp,
+    // which the others waited for: 54 us a chunk of 12-electron walkers, 50 like this)
+    for (int q = tid; q < 2 * ng; q += kExgThreads) {
+      const double* d = reinterpret_cast<const double*>(sm + (q >> 1) * n) + (q & 1);
+      double t = 0.0;
+      for (int r = 0; r < n; ++r) t += d[2 * r * (lds + 1)];
+      if (mult == 2) t += t;
+      double* o = reinterpret_cast<double*>(fb + (size_t)b * G + gs) + q;
+      *o = add ? *o + t : t;
     }
   }
   once = cadd(once, cadd(twice, twice));

@@ -336,91 +336,6 @@ TROT_D double2 gauss_jordan(double2* A, int n, bool inverse, GjScratch& S, int t
   return threadIdx.x < 32 ? warp_lu(A, n) : cmk(0.0, 0.0);
 }
 
-// Small-matrix LU with partial pivoting on an n x n complex matrix in shared
-// memory (row-major, leading dimension ld), executed by the whole block.
-// Returns det(A) to all threads; A is overwritten by its LU factors.
-// If `inv` is non-null it receives A^{-1} (Gauss-Jordan on [A | I]).
-TROT_D double2 block_gauss_jordan(double2* A, int n, int ld, double2* inv, int* piv_s, double2* red) {
-  const int tid = threadIdx.x, nt = blockDim.x;
-  if (inv) {
-    for (int e = tid; e < n * n; e += nt) {
-      int i = e / n, j = e % n;
-      inv[i * ld + j] = cmk(i == j ? 1.0 : 0.0, 0.0);
-    }
-  }
-  __shared__ double2 det_s, rp_s;  // running determinant; reciprocal of the current pivot
-  if (tid == 0) det_s = cmk(1.0, 0.0);
-  __syncthreads();
-  for (int k = 0; k < n; ++k) {
-    // pivot search: warp 0 finds argmax |A[i][k]|, i >= k (first max wins)
-    if (tid < 32) {
-      double best = -1.0;
-      int bi = k;
-      for (int i = k + tid; i < n; i += 32) {
-        double a = cabs2(A[i * ld + k]);
-        if (a > best) { best = a; bi = i; }
-      }
-      for (int o = 16; o > 0; o >>= 1) {
-        double ob = __shfl_xor_sync(0xffffffffu, best, o);
-        int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-      }
-      if (tid == 0) *piv_s = bi;
-    }
-    __syncthreads();
-    const int p = *piv_s;
-    if (p != k) {
-      for (int j = tid; j < n; j += nt) {
-        double2 t = A[k * ld + j]; A[k * ld + j] = A[p * ld + j]; A[p * ld + j] = t;
-        if (inv) { t = inv[k * ld + j]; inv[k * ld + j] = inv[p * ld + j]; inv[p * ld + j] = t; }
-      }
-    }
-    __syncthreads();
-    const double2 piv = A[k * ld + k];
-    if (tid == 0) {
-      det_s = cmul(p != k ? cmk(-det_s.x, -det_s.y) : det_s, piv);
-      rp_s = cdiv(cmk(1.0, 0.0), piv);  // one division per pivot, shared by all threads
-    }
-    __syncthreads();
-    const double2 rp = rp_s;
-    if (inv) {
-      // Gauss-Jordan: normalise row k, eliminate column k from every other row
-      for (int j = tid; j < n; j += nt) {
-        A[k * ld + j] = cmul(A[k * ld + j], rp);
-        inv[k * ld + j] = cmul(inv[k * ld + j], rp);
-      }
-      __syncthreads();
-      for (int e = tid; e < n * n; e += nt) {
-        int i = e / n, j = e % n;
-        if (i == k) continue;
-        double2 f = A[i * ld + k];
-        // column k of A itself is updated last (j == k) by the thread that owns it
-        if (j != k) A[i * ld + j] = csub(A[i * ld + j], cmul(f, A[k * ld + j]));
-        inv[i * ld + j] = csub(inv[i * ld + j], cmul(f, inv[k * ld + j]));
-      }
-      __syncthreads();
-      for (int i = tid; i < n; i += nt)
-        if (i != k) A[i * ld + k] = cmk(0.0, 0.0);
-      __syncthreads();
-    } else {
-      // plain LU elimination below the pivot: multipliers once per row (stored in column k)
-      for (int i = k + 1 + tid; i < n; i += nt) A[i * ld + k] = cmul(A[i * ld + k], rp);
-      __syncthreads();
-      const int m = n - k - 1;
-      for (int e = tid; e < m * m; e += nt) {
-        const int i = k + 1 + e / m, j = k + 1 + e % m;
-        A[i * ld + j] = csub(A[i * ld + j], cmul(A[i * ld + k], A[k * ld + j]));
-      }
-      __syncthreads();
-    }
-  }
-  __syncthreads();
-  double2 d = det_s;
-  __syncthreads();
-  (void)red;
-  return d;
-}
-
 // ---------------------------------------------------------------- errors
 namespace trot {
 void set_error(const char* fmt, ...);

@@ -932,8 +932,6 @@ __global__ void __launch_bounds__(256) dg_taylor_kernel(DgTaylor a) {
 // propagated walkers from the transposed w'[j][p]; in step mode their overlap and weight
 __global__ void __launch_bounds__(256) dg_trotter_tail_kernel(Spins sp, TrotterArgs a, const double2* __restrict__ wt) {
   extern __shared__ double2 smem[];
-  __shared__ double2 red[32];
-  __shared__ int piv;
   const int b = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
   const int N = a.N, nc = sp.ntot;
   double2* W2 = smem;           // N x nc
@@ -947,7 +945,7 @@ __global__ void __launch_bounds__(256) dg_trotter_tail_kernel(Spins sp, TrotterA
     for (int e = tid; e < N * n; e += nt) w[e] = W2[(e / n) * nc + sp.off[s] + e % n];
   }
   if (a.overlaps == nullptr) return;
-  overlap_and_weight(sp, a, N, nc, W2, Ms, &piv, red);
+  overlap_and_weight(sp, a, N, nc, W2, Ms);
 }
 
 struct DgTrotterPlan {

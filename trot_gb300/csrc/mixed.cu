@@ -1183,8 +1183,6 @@ struct Trot32Args {
 
 __global__ void __launch_bounds__(256) trotter32_kernel(Spins sp, Trot32Args a32) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  __shared__ double2 red[32];
-  __shared__ int piv;
   const TrotterArgs& a = a32.t;
   const int b = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
   const int N = a.N, nc = sp.ntot;
@@ -1237,7 +1235,7 @@ __global__ void __launch_bounds__(256) trotter32_kernel(Spins sp, Trot32Args a32
   if (a.overlaps == nullptr) return;
   // n x n scratch over the dead O, T, T2 tiles (16-byte aligned, n^2 * 16 <= 2 * tbytes)
   double2* Ms = reinterpret_cast<double2*>(smem_raw + vbytes);
-  overlap_and_weight(sp, a, N, nc, W2, Ms, &piv, red);
+  overlap_and_weight(sp, a, N, nc, W2, Ms);
 }
 
 // ------------------------------------------------------------------ tensor-core Trotter propagation

@@ -66,8 +66,6 @@ __device__ void real_mm(int N, int nc, const double* __restrict__ E, const doubl
 __global__ void __launch_bounds__(kTrotThreads)
 trotter_kernel(Spins sp, TrotterArgs a) {
   extern __shared__ double2 smem[];
-  __shared__ double2 red[32];
-  __shared__ int piv;
   // sqrt_dt / k of 32 terms at a time, a division a thread of the last warp (one per term in every warp took 3 us of a
   // block's 46 at N = 24, n = 5)
   __shared__ double coef[32];
@@ -119,7 +117,7 @@ trotter_kernel(Spins sp, TrotterArgs a) {
     for (int e = tid; e < N * n; e += nt) w[e] = T2[(e / n) * nc + sp.off[s] + e % n];
   }
   if (a.overlaps == nullptr) return;
-  overlap_and_weight(sp, a, N, nc, T2, O, &piv, red);
+  overlap_and_weight(sp, a, N, nc, T2, O);
 }
 
 // The chain of digit products takes 19 launches, 150 us at least; this kernel's time is the FP64 pipe's, one walker's

@@ -47,7 +47,7 @@ __device__ __forceinline__ void phaseless_update(const TrotterArgs& a, int b, do
 
 // W2: propagated walker columns (N x nc, FP64, shared memory); Ms: n x n scratch.
 __device__ __forceinline__ void overlap_and_weight(const Spins& sp, const TrotterArgs& a, int N, int nc,
-                                                   const double2* W2, double2* Ms, int* piv, double2* red) {
+                                                   const double2* W2, double2* Ms) {
   __shared__ GjScratch gj;
   const int b = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
   // new overlap: prod_s det(C_s^T w'_s)^mult  (trot/trial/rhf.py:45-54, trot/trial/uhf.py:54-58)
@@ -64,10 +64,7 @@ __device__ __forceinline__ void overlap_and_weight(const Spins& sp, const Trotte
     }
     __syncthreads();
     double2 det = cmk(0.0, 0.0);
-    if (n > kGjMax)
-      det = block_gauss_jordan(Ms, n, n, nullptr, piv, red);
-    else if (tid < 128)
-      det = gauss_jordan(Ms, n, false, gj, b);
+    if (tid < 128) det = gauss_jordan(Ms, n, false, gj, b);  // n <= kGjMax: the step's Green's functions take no more
     det_all = cmul(det_all, sp.mult[s] == 2 ? cmul(det, det) : det);
   }
   if (tid == 0) phaseless_update(a, b, det_all);

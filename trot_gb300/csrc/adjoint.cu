@@ -949,7 +949,7 @@ int trot_prop_step_vjp(const trot_system* s, const trot_state* in, const double*
     TROT_TRY(adjoint_dg_v(b.ad, b.V, false, st));
     TROT_TRY(adjoint_dg_from_walkers(b.ad, kDgE, w[0], a.n[0], two ? w[1] : nullptr, a.n[1], false, b.Ut, sU, st));
     for (int l = 0; l < K; ++l)
-      TROT_TRY(adjoint_dg_from_rows(b.ad, kDgV, b.Ut + l * per1, sU, b.Ut + (l + 1) * per1, sU, st));
+      TROT_TRY(adjoint_dg_from_rows(b.ad, kDgV, b.Ut + l * per1, sU, b.Ut + (l + 1) * per1, sU, st, l));
     adj_chain_sum_kernel<<<grid_of(W * per1), 256, 0, st>>>(W, per1, co, b.Ut, b.Ot);
     TROT_CHECK_LAUNCH("adj_chain_sum_kernel");
     TROT_TRY(adjoint_dg_from_rows(b.ad, kDgE, b.Ot, (long long)per1, b.Tt, (long long)per1, st));

@@ -115,6 +115,15 @@ TROT_D void dg_store8(const double* x, int e, uint16_t* o, size_t plane) {
   for (int t = 0; t < kDgS; ++t) *reinterpret_cast<uint4*>(o + t * plane) = w[t];
 }
 
+// x 2^k by its exponent bits (below the normal range: 0)
+TROT_D double dg_shift(double x, int k) {
+  const int hi = __double2hiint(x), e = (hi >> 20) & 0x7FF;
+  if (e == 0x7FF) return x;
+  if (e == 0 || e + k <= 0) return 0.0;
+  if (e + k >= 0x7FF) return __hiloint2double(0x7FF00000, 0);
+  return __hiloint2double(hi + k * (1 << 20), __double2loint(x));
+}
+
 TROT_D double dg_neg(double x) { return __hiloint2double(__double2hiint(x) ^ (int)0x80000000u, __double2loint(x)); }
 
 // high word of the largest |x| so far, and sum of |x| as a float from its high word (the range only matters near
@@ -158,12 +167,20 @@ struct DgSrc {
   long long bstride2, kst2;
   uint16_t* img;
   int16_t* ex;
+  // balanced sums (mode 2): element k of block b times 2^(ksign kexp[b kld + k])
+  const int16_t* kexp;
+  int kld, ksign;
+  // exponent of the larger part of complex row r of block b at cexp[b cld + r] (mode 1; null: not wanted)
+  int16_t* cexp;
+  int cld;
 };
+static constexpr int kDgZeroTerm = -0x4000;  // exponent of a zero row: 2^e of it makes anything 0
 static constexpr int kDgOneBlock = 1 << 30;
 // `rows` rows of stride rst (complex ones count twice), one block
 static DgSrc dg_src(const double* p, int cplx, int rows, int K, int R, long long rst, long long kst, uint16_t* img,
                     int16_t* ex) {
-  return DgSrc{p, K, (K + 15) / 16, R, cplx, 0, rows, kDgOneBlock, 1, 0, rst, kst, kDgOneBlock, nullptr, 0, 0, img, ex};
+  return DgSrc{p, K, (K + 15) / 16, R, cplx, 0, rows, kDgOneBlock, 1, 0, rst, kst, kDgOneBlock, nullptr, 0, 0, img, ex,
+               nullptr, 0, 0, nullptr, 0};
 }
 
 // Up to four sources of the same K in one launch: most are small (3 to 10 us, half of it the launch and the tail), and
@@ -175,6 +192,8 @@ struct DgRows {
   int count, ks;        // ks: CTAs of a cluster, one after the other in the grid
 };
 
+// MODE 1: a source may write cexp; 2: use kexp (in the plain kernel their tests alone cost 3 % of an FP64 step)
+template <int MODE>
 __global__ void __launch_bounds__(256) dg_rows_kernel(const __grid_constant__ DgRows q) {
   const int KS = q.ks, rank = (int)blockIdx.x % KS;
   int src = 0, group = (int)blockIdx.x / KS;
@@ -202,6 +221,7 @@ __global__ void __launch_bounds__(256) dg_rows_kernel(const __grid_constant__ Dg
       p += blk * a.bstride + rr * a.rst;
     }
   }
+  const int16_t* kexp = MODE == 2 ? a.kexp + (size_t)(valid ? blk : 0) * a.kld : nullptr;
   const int nwarp = (int)blockDim.x >> 5, kpad = a.nk16 * 16, kstep = nwarp * 32 * KS;
   unsigned mx = 0;
   float l1 = 0.f;
@@ -213,6 +233,7 @@ __global__ void __launch_bounds__(256) dg_rows_kernel(const __grid_constant__ Dg
       const int k = k0 + kg * 8 + i;
       x[i] = (valid && k < a.K) ? p[k * kst] : 0.0;
       if (flip) x[i] = dg_neg(x[i]);
+      if (MODE == 2 && k < a.K) x[i] = dg_shift(x[i], a.ksign * kexp[k]);
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i) dg_row_max(x[i], mx, s);
@@ -244,6 +265,11 @@ __global__ void __launch_bounds__(256) dg_rows_kernel(const __grid_constant__ Dg
   }
   const int e = dg_exponent(mx, l1);
   if (rank == 0 && warp == 0 && lane < 8) a.ex[row] = (int16_t)e;
+  if (MODE == 1 && a.cexp && rank == 0 && warp == 0) {
+    const unsigned both = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));  // real and imaginary part
+    if (lane < 8 && !(lane & 1) && valid)
+      a.cexp[(size_t)blk * a.cld + (rr >> 1)] = (int16_t)(both >> 20 ? (int)(both >> 20) - 1022 : kDgZeroTerm);
+  }
   const bool live = valid && e != kDgNonFinite;
   const int r = row % a.R;
   uint16_t* out = a.img + (size_t)(row / a.R) * a.nk16 * kDgS * a.R * 16;
@@ -256,6 +282,7 @@ __global__ void __launch_bounds__(256) dg_rows_kernel(const __grid_constant__ Dg
       for (int i = 0; i < 8; ++i) {
         x[i] = (live && kb + i < a.K) ? p[(kb + i) * kst] : 0.0;
         if (flip) x[i] = dg_neg(x[i]);
+        if (MODE == 2 && kb + i < a.K) x[i] = dg_shift(x[i], a.ksign * kexp[kb + i]);
       }
     }
     if (!live) {
@@ -270,7 +297,7 @@ __global__ void __launch_bounds__(256) dg_rows_kernel(const __grid_constant__ Dg
 // a warp per 32 k, eight at most
 static int dg_row_threads(int nk16) { return 32 * std::min(8, (nk16 + 1) / 2); }
 
-static int dg_rows_launch(DgRows q, cudaStream_t st) {
+static int dg_rows_launch(DgRows q, cudaStream_t st, int mode = 0) {
   const int groups = q.first[q.count], nk16 = q.s[0].nk16;
   if (groups == 0) return TROT_OK;
   int ks = 1;
@@ -287,7 +314,8 @@ static int dg_rows_launch(DgRows q, cudaStream_t st) {
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = ks > 1 ? 1 : 0;
-  const cudaError_t rc = cudaLaunchKernelEx(&cfg, dg_rows_kernel, q);
+  const cudaError_t rc = cudaLaunchKernelEx(
+      &cfg, mode == 0 ? dg_rows_kernel<0> : mode == 1 ? dg_rows_kernel<1> : dg_rows_kernel<2>, q);
   if (rc != cudaSuccess) return cuda_status(rc, "dg_rows_kernel");
   TROT_CHECK_LAUNCH("dg_rows_kernel");
   return TROT_OK;
@@ -297,10 +325,10 @@ static void dg_rows_add(DgRows& q, const DgSrc& a, int groups) {
   q.first[q.count + 1] = q.first[q.count] + groups;
   ++q.count;
 }
-static int dg_rows_launch(const DgSrc& a, int groups, cudaStream_t st) {
+static int dg_rows_launch(const DgSrc& a, int groups, cudaStream_t st, int mode = 0) {
   DgRows q{};
   dg_rows_add(q, a, groups);
-  return dg_rows_launch(q, st);
+  return dg_rows_launch(q, st, mode);
 }
 
 // ------------------------------------------------------------------ product
@@ -1040,7 +1068,7 @@ size_t adjoint_dg_bytes(size_t W, size_t N, size_t nc, size_t K2) {
   DgAdjoint d{};
   DgScratch s{};
   adjoint_dg_carve(d, (int)W, (int)N, (int)nc, (int)K2, s);
-  return (size_t)((char*)d.etex - (char*)nullptr) + adj_rows(N, 128) * 2 + 512;
+  return (size_t)((char*)d.cexp - (char*)nullptr) + W * K2 * 2 + 512;
 }
 
 // (with s.p null the pointers are offsets from the start, for the size)
@@ -1063,6 +1091,7 @@ void adjoint_dg_carve(DgAdjoint& d, int W, int N, int nc, int K2, const DgScratc
   d.uex = reinterpret_cast<int16_t*>(take(std::max(ur, gr) * 2));
   d.eex = reinterpret_cast<int16_t*>(take(er * 2));
   d.etex = reinterpret_cast<int16_t*>(take(er * 2));
+  d.cexp = reinterpret_cast<int16_t*>(take((size_t)W * K2 * 2));
 }
 
 int adjoint_dg_e(const DgAdjoint& d, const double* E, cudaStream_t st) {
@@ -1101,7 +1130,7 @@ static int adj_apply(const DgAdjoint& d, DgOperand op, DgSrc s, double2* out, lo
   const int rpad = (int)adj_rows(2 * d.nc, kDgP);
   s.rpad = rpad;
   s.nblk = d.W;
-  TROT_TRY(dg_rows_launch(s, d.W * (rpad / 8), st));
+  TROT_TRY(dg_rows_launch(s, d.W * (rpad / 8), st, s.cexp ? 1 : 0));
   DgArgs a{};
   a.imgA = d.uimg; a.exA = d.uex;
   a.imgB = op == kDgV ? d.vimg : op == kDgE ? d.eimg : d.etimg;
@@ -1129,12 +1158,22 @@ int adjoint_dg_from_walkers(const DgAdjoint& d, DgOperand op, const double2* wa,
 }
 
 int adjoint_dg_from_rows(const DgAdjoint& d, DgOperand op, const double2* src, long long sstride, double2* out,
-                         long long ostride, cudaStream_t st) {
+                         long long ostride, cudaStream_t st, int term) {
   DgSrc s = dg_src(reinterpret_cast<const double*>(src), 1, 2 * d.nc, d.N, kDgP, 2ll * d.N, 2, d.uimg, d.uex);
   s.bstride = 2 * sstride;
+  if (term >= 0) {
+    s.cexp = d.cexp + term * d.nc;
+    s.cld = d.K2;
+  }
   return adj_apply(d, op, s, out, ostride, st);
 }
 
+// A term k = (l, j) of the sum is column j of V^l E w times one of its cotangent: the first grows like |V|^l, the second
+// falls like sqrt(dt)^(l + 1) / (l + 1)!, and their columns' scales are each other's inverse.  A digit row has one
+// exponent, so as they stand the large l of U (at the small l of S) would leave the leading terms few digits: with
+// sqrt(dt) |V| = 1.4 (80 orbitals) the error was 7.7e-12 of the largest element, 1.9e-9 with 2.8 (120 orbitals).
+// Therefore U_k 2^-e and S_k 2^e with e the exponent of column k of U: all columns of U peak at 1/2 to 1, and the row
+// maxima of S are those of the terms (2e-16 at both).
 int adjoint_dg_gv(const DgAdjoint& d, const double2* S, long long sstride, const double2* U, long long ustride,
                   double2* gv, cudaStream_t st) {
   const int N = d.N, rpad = (int)adj_rows(2 * N, kDgP), vpad = (int)adj_rows(2 * N, 128);
@@ -1142,14 +1181,20 @@ int adjoint_dg_gv(const DgAdjoint& d, const double2* S, long long sstride, const
   s.rpad = rpad;
   s.nblk = d.W;
   s.bstride = 2 * sstride;
+  s.kexp = d.cexp;
+  s.kld = d.K2;
+  s.ksign = 1;
   DgRows rows{};
   dg_rows_add(rows, s, d.W * (rpad / 8));
   DgSrc u = dg_src(reinterpret_cast<const double*>(U), 1, 2 * N, d.K2, 128, 2, 2ll * N, d.vimg, d.vex);
   u.rpad = vpad;
   u.nblk = d.W;
   u.bstride = 2 * ustride;
+  u.kexp = d.cexp;
+  u.kld = d.K2;
+  u.ksign = -1;
   dg_rows_add(rows, u, d.W * (vpad / 8));
-  TROT_TRY(dg_rows_launch(rows, st));
+  TROT_TRY(dg_rows_launch(rows, st, 2));
   DgArgs a{};
   a.imgA = d.uimg; a.exA = d.uex; a.imgB = d.vimg; a.exB = d.vex;
   a.Nn = 2 * N; a.M = N; a.nrt = a.bB = vpad / 128; a.ntile = rpad / kDgP; a.nbatch = d.W;

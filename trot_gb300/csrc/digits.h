@@ -43,6 +43,7 @@ struct DgAdjoint {
   int W, N, nc, K2;                    // K2: terms (l, j) of the cotangent of V
   uint16_t *vimg, *uimg, *eimg, *etimg;
   int16_t *vex, *uex, *eex, *etex;
+  int16_t* cexp;                       // (W, K2): exponents of the chain's columns u_l[j], k = (l, j)
   int* status;
 };
 enum DgOperand { kDgE, kDgET, kDgV };
@@ -56,10 +57,10 @@ int adjoint_dg_v_active(const DgAdjoint& d, const int* act, cudaStream_t st);
 // out[b][j][p] (walkers ostride apart) = op . columns of wa (W, N, na) and wb (W, N, nb), conjugated if conj
 int adjoint_dg_from_walkers(const DgAdjoint& d, DgOperand op, const double2* wa, int na, const double2* wb, int nb,
                             bool conj, double2* out, long long ostride, cudaStream_t st);
-// the same from an array (walker, j, p), walkers sstride apart
+// the same from an array (walker, j, p), walkers sstride apart; term l >= 0: src is u_l, whose exponents gv wants
 int adjoint_dg_from_rows(const DgAdjoint& d, DgOperand op, const double2* src, long long sstride, double2* out,
-                         long long ostride, cudaStream_t st);
-// gv[b][p][q] = sum_{k < K2} S[b][k][p] U[b][k][q] (the digits of V are overwritten)
+                         long long ostride, cudaStream_t st, int term = -1);
+// gv[b][p][q] = sum_{k < K2} S[b][k][p] U[b][k][q], U[b][k] the u_l noted above (the digits of V are overwritten)
 int adjoint_dg_gv(const DgAdjoint& d, const double2* S, long long sstride, const double2* U, long long ustride,
                   double2* gv, cudaStream_t st);
 

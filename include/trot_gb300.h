@@ -210,16 +210,17 @@ int trot_apply_trotter(const trot_system* sys, const double* walkers_a, const do
 int trot_prop_step(const trot_system* sys, const trot_state* state, const double* fields,
                    double* energy_out, void* workspace, size_t workspace_bytes, void* stream);
 
-/* Device status of the last mixed-precision op that used this workspace
- * (its first bytes): TROT_OK, or TROT_ERR_DEVICE_TIMEOUT when a tensor-core
- * kernel's completion wait ran out (the kernel then skipped its output, freed
- * its tensor memory and returned, and the op wrote NaN results: the local
- * energies, or the step's weights and population shift).  Synchronous
- * (cudaMemcpy). */
+/* Device status of the last op that used this workspace (its first bytes):
+ * TROT_OK, or TROT_ERR_DEVICE_TIMEOUT when a tensor-core kernel's completion
+ * wait ran out (the kernel then skipped its output, freed its tensor memory
+ * and returned, and the op wrote NaN results: the local energies, the step's
+ * weights and population shift, the gradients of a vector-Jacobian product,
+ * elsewhere at least the values that were skipped).  FP64 ops from 20 orbitals
+ * on use tensor-core kernels too.  Synchronous (cudaMemcpy). */
 int trot_workspace_status(const void* workspace, int* status_out);
 
-/* Sticky device status of every mixed-precision op that used this workspace
- * since the sticky word (the fourth int of the workspace) was last cleared:
+/* Sticky device status of every op that used this workspace since the sticky
+ * word (the fourth int of the workspace) was last cleared:
  * TROT_ERR_DEVICE_TIMEOUT if any of them timed out as above, else TROT_OK.
  * A workspace whose first 16 bytes were zero-filled starts clear; clear != 0
  * resets the word after reading it.  Lets a caller that issues many
@@ -247,7 +248,8 @@ int trot_sr_resample(const trot_system* sys, const double* weights_in, const dou
 
 /* Block energy on the device (trot/prop/blocks.py:236-257): clamps Re(E_L)
  * to e_estimate when non-finite or further than sqrt(2/dt) from it, zeroes the
- * weights of non-finite walkers (in place), forms the weighted block energy
+ * weights of non-finite walkers (in place; the energies of a call that timed
+ * out, see trot_workspace_status, make all weights and the block NaN), forms the weighted block energy
  * and updates e_estimate (scalars[1]) with the shift_ema moving average.
  * obs_out (float64 [2], device) receives [e_block, sum of weights]. */
 int trot_block_energy(int n_walkers, const double* energy, double* weights, double* scalars, double dt,
@@ -291,9 +293,8 @@ int trot_split_key(int64_t* key, void* stream);
  * before any stream capture.  With CUDA's lazy module loading that first call
  * also reserves the 32 MiB: make it before a framework pre-allocates the GPU,
  * or set CUDA_MODULE_LOADING=EAGER.  All calls share the array, so calls that
- * overlap on the GPU race.  A mixed-precision call whose tensor-core kernel
- * timed out writes NaN energies; mixed-precision callers check
- * trot_local_energy_noalloc_status.  No counterpart in the reference. */
+ * overlap on the GPU race.  A call whose tensor-core kernel timed out writes
+ * NaN energies; callers check trot_local_energy_noalloc_status.  No counterpart in the reference. */
 int trot_local_energy_noalloc(const trot_system* sys, const double* walkers_a, const double* walkers_b,
                               double* energy_out, void* stream);
 
@@ -501,7 +502,8 @@ int trot_tc_gemm_bf16(const uint16_t* A, const uint16_t* B, float* D, int M, int
  * A (M x K) and C (M x N) complex row-major (lda, ldc complex elements), B real,
  * (N x K) row-major if b_is_nk, else (K x N) (ldb elements); alpha a power of two
  * (or its negative); K <= 2^17.  A row of A or column of B with a NaN or an
- * infinity gives NaN outputs.  workspace: trot_zgemm_digits_workspace bytes.
+ * infinity gives NaN outputs, and so does a timeout (trot_workspace_status).
+ * workspace: trot_zgemm_digits_workspace bytes.
  * The building block of the FP64 contractions; no counterpart in the reference. */
 size_t trot_zgemm_digits_workspace(int M, int N, int K);
 int trot_zgemm_digits(int M, int N, int K, double alpha, const double* A, int lda, const double* B, int ldb,
@@ -515,10 +517,11 @@ int trot_zgemm_digits(int M, int N, int K, double alpha, const double* A, int ld
  *     exchange kernel (default 8);
  *   TROT_TUNE_EXCHANGE_GRID: persistent CTAs of that kernel (default 152);
  *   TROT_TUNE_TEST_TIMEOUT: test switch of the device-timeout path, not a
- *     tuning knob: when v > 0 the exchange kernel's first wait is on a barrier
- *     nothing arrives on, limited to v polls, so it takes its timeout path
- *     (status TROT_ERR_DEVICE_TIMEOUT, no copies or MMAs issued, NaN energies)
- *     on every call until the knob is set back to 0. */
+ *     tuning knob: when v > 0 the first wait of the exchange kernel and of the
+ *     FP64 digit products is on a barrier nothing arrives on, limited to v
+ *     polls, so they take their timeout path (status TROT_ERR_DEVICE_TIMEOUT, no
+ *     copies or MMAs issued, NaN results) on every call until the knob is set
+ *     back to 0. */
 typedef enum {
   TROT_TUNE_EXCHANGE_TILES = 0,
   TROT_TUNE_EXCHANGE_GRID = 1,

@@ -844,6 +844,28 @@ static int from_rows(int W, int N, int n, int nc, int off, bool conj, const doub
   return TROT_OK;
 }
 
+// The gradients of a call whose digit products timed out: NaN
+struct AdjOutputs {
+  double* p[6];
+  size_t len[6];
+};
+__global__ void adj_poison_kernel(const int* __restrict__ status, AdjOutputs o) {
+  if (status[0] == 0) return;
+  for (int k = 0; k < 6; ++k)
+    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < o.len[k]; e += (size_t)gridDim.x * blockDim.x)
+      o.p[k][e] = timeout_nan();
+}
+static int poison_if_timed_out(const int* status, const AdjOutputs& o, cudaStream_t st) {
+  adj_poison_kernel<<<152, 256, 0, st>>>(status, o);
+  TROT_CHECK_LAUNCH("adj_poison_kernel");
+  return TROT_OK;
+}
+// this call's status word (the sticky one persists)
+static int clear_status(int* status, cudaStream_t st) {
+  const cudaError_t e = cudaMemsetAsync(status, 0, sizeof(int), st);
+  return e == cudaSuccess ? TROT_OK : cuda_status(e, "adjoint memset");
+}
+
 static int dcopy(void* dst, const void* src, size_t bytes, cudaStream_t st) {
   cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, st);
   return e == cudaSuccess ? TROT_OK : cuda_status(e, "adjoint copy");
@@ -908,6 +930,7 @@ int trot_prop_step_vjp(const trot_system* s, const trot_state* in, const double*
   }
   if (!c.ok) { set_error("workspace too small: %zu < %zu", ws_bytes, c.used); return TROT_ERR_WORKSPACE_TOO_SMALL; }
   cudaStream_t st = (cudaStream_t)stream;
+  TROT_TRY(clear_status(c.status(), st));
   const int W = a.W, N = a.N, G = a.G, K = a.K;
   const size_t NN = (size_t)N * N;
   const double2 one = cmk(1.0, 0.0), zero = cmk(0.0, 0.0);
@@ -1092,6 +1115,11 @@ int trot_prop_step_vjp(const trot_system* s, const trot_state* in, const double*
                           (int)a.nN[q], false, b.dg, st));
     TROT_TRY(green_vjp_launch(a, q, x.green, x.gG, x.P, gin[q], st));
   }
+  if (b.dg.p || b.chain) {
+    const size_t w2 = 2 * (size_t)W;
+    return poison_if_timed_out(c.status(), {{g_walkers_in_a, g_walkers_in_b, g_weights_in, g_overlaps_in, g_scalars_in, g_exp_h1_half},
+                                            {2 * a.wn[0], two ? 2 * a.wn[1] : 0, w2 / 2, w2, 2, NN}}, st);
+  }
   return TROT_OK;
 }
 
@@ -1117,6 +1145,7 @@ int trot_local_energy_vjp(const trot_system* s, const double* walkers_a, const d
   if (!c.ok) { set_error("workspace too small: %zu < %zu", ws_bytes, c.used); return TROT_ERR_WORKSPACE_TOO_SMALL; }
   cudaStream_t st = (cudaStream_t)stream;
   const int W = a.W, N = a.N, G = a.G;
+  TROT_TRY(clear_status(c.status(), st));
   const double2* w[2] = {(const double2*)walkers_a, (const double2*)walkers_b};
   double2* gw[2] = {(double2*)g_walkers_a, (double2*)g_walkers_b};
   adj_act_from_cotangent_kernel<<<(W + 127) / 128, 128, 0, st>>>(W, g_energy, 0, b.act);
@@ -1157,6 +1186,9 @@ int trot_local_energy_vjp(const trot_system* s, const double* walkers_a, const d
     adj_h1_direct_kernel<<<grid_of((size_t)N * N), 256, 0, st>>>(N, n, m, a.mo[q], b.H, g_h1);
     TROT_CHECK_LAUNCH("adj_h1_direct_kernel");
   }
+  if (b.dg.p)
+    return poison_if_timed_out(c.status(), {{g_walkers_a, g_walkers_b, g_h1},
+                                            {2 * a.wn[0], a.nspin == 2 ? 2 * a.wn[1] : 0, (size_t)N * N}}, st);
   return TROT_OK;
 }
 

@@ -69,6 +69,7 @@ static size_t digit_bytes(const trot_system* s, const Spins& sp, int op) {
 static size_t carve_step(const trot_system* s, const Spins& sp, Carver& c, StepBuffers& b, int op, bool digits) {
   const size_t W = s->n_walkers, N = s->norb, G = s->nchol;
   b = StepBuffers{};
+  b.status = c.status();
   if (op == TROT_OP_SR) { c.take<double>(W); return c.used; }
   if (op == TROT_OP_QR) return c.used;
   b.green = c.take<double2>(W * sp.ntot * N);
@@ -89,7 +90,7 @@ static size_t carve_step(const trot_system* s, const Spins& sp, Carver& c, StepB
   if (nd) {
     b.dg.p = c.take<char>(nd);
     b.dg.bytes = nd;
-    b.dg.status = c.status();
+    b.dg.status = b.status;
   }
   return c.used;
 }
@@ -308,7 +309,7 @@ int trot_force_bias(const trot_system* s, const double* wa, const double* wb, do
   StepBuffers b;
   TROT_TRY(carve_ws(s, sp, ws, ws_bytes, b, TROT_OP_FORCE_BIAS));
   TROT_TRY(launch_green(sp, s->n_walkers, s->norb, (const double2*)wa, (const double2*)wb, b.green, nullptr,
-                        nullptr, st));
+                        nullptr, st, b.status));
   return force_bias_from_green(s, sp, b.green, (double2*)out, b.dg, st);
 }
 
@@ -325,10 +326,10 @@ int trot_local_energy(const trot_system* s, const double* wa, const double* wb, 
   StepBuffers b;
   TROT_TRY(carve_ws(s, sp, ws, ws_bytes, b, TROT_OP_LOCAL_ENERGY));
   const int W = s->n_walkers, N = s->norb, G = s->nchol;
-  TROT_TRY(launch_green(sp, W, N, (const double2*)wa, (const double2*)wb, b.green, nullptr, b.e1, st));
+  TROT_TRY(launch_green(sp, W, N, (const double2*)wa, (const double2*)wb, b.green, nullptr, b.e1, st, b.status));
   int nchunks = 0;
   TROT_TRY(force_bias_and_exchange(s, sp, b, nchunks, st));
-  return launch_energy_combine(W, G, nchunks, s->h0, b.fb, b.e1, 1, b.exc, (double2*)out, st);
+  return launch_energy_combine(W, G, nchunks, s->h0, b.fb, b.e1, 1, b.exc, (double2*)out, st, b.status);
 }
 
 int trot_apply_trotter(const trot_system* s, const double* wa, const double* wb, const double* xs,
@@ -347,6 +348,8 @@ int trot_apply_trotter(const trot_system* s, const double* wa, const double* wb,
   if (s->precision == TROT_MIXED) return mixed_apply_trotter(s, sp, (const double2*)xs, a, ws, ws_bytes, st);
   StepBuffers b;
   TROT_TRY(carve_ws(s, sp, ws, ws_bytes, b, TROT_OP_APPLY_TROTTER));
+  const cudaError_t e = cudaMemsetAsync(b.status, 0, sizeof(int), st);  // this call's word; the sticky one persists
+  if (e != cudaSuccess) return cuda_status(e, "trot_apply_trotter memset");
   TROT_TRY(launch_vhs64(W, N, G, (const double2*)xs, s->chol_flat, s->chol_packed, b.vp, b.vhs, b.dg, st));
   a.vhs = b.vhs;
   return launch_trotter(sp, a, b.dg, st);
@@ -373,7 +376,7 @@ int trot_prop_step(const trot_system* s, const trot_state* state, const double* 
   double2* wa = (double2*)state->walkers_a;
   double2* wb = (double2*)state->walkers_b;
   // 1. Green's functions (+ one-body energy) of the current walkers
-  TROT_TIMED("green", st, launch_green(sp, W, N, wa, wb, b.green, nullptr, energy_out ? b.e1 : nullptr, st));
+  TROT_TIMED("green", st, launch_green(sp, W, N, wa, wb, b.green, nullptr, energy_out ? b.e1 : nullptr, st, b.status));
   // 2. force bias, 3. optional local energy of the current walkers (reuses G; f_g gives both)
   if (!energy_out) {
     TROT_TIMED("force_bias_fp64", st, force_bias_from_green(s, sp, b.green, b.fb, b.dg, st));
@@ -381,7 +384,7 @@ int trot_prop_step(const trot_system* s, const trot_state* state, const double* 
     int nchunks = 0;
     TROT_TRY(force_bias_and_exchange(s, sp, b, nchunks, st));
     TROT_TIMED("energy_combine", st,
-               launch_energy_combine(W, G, nchunks, s->h0, b.fb, b.e1, 1, b.exc, (double2*)energy_out, st));
+               launch_energy_combine(W, G, nchunks, s->h0, b.fb, b.e1, 1, b.exc, (double2*)energy_out, st, b.status));
   }
   // 4. shifted fields
   TROT_TIMED("fields", st, launch_fields(W, G, s->sqrt_dt, b.fb, s->mf_shifts_im, fields, b.xs, b.shift_term, b.fb_term, st));
@@ -397,7 +400,7 @@ int trot_prop_step(const trot_system* s, const trot_state* state, const double* 
   TROT_TIMED("trotter_fp64", st, launch_trotter(sp, a, b.dg, st));
   // 7. population-control shift, node count
   TROT_TIMED("step_finalize", st, launch_step_finalize(W, state->weights, state->scalars, (long long*)state->node_encounters,
-                                                       b.node_flag, s->pop_control_damping, s->dt, st));
+                                                       b.node_flag, s->pop_control_damping, s->dt, st, b.status));
   return TROT_OK;
 }
 

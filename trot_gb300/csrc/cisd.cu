@@ -861,7 +861,7 @@ cisd_energy_kernel(int G, int nchunk, double h0, const double2* __restrict__ wsc
   __shared__ double red[64], sums[2][8];
   const int b = blockIdx.x;
   if (status[0] != 0) {  // a tensor-core product of this call timed out: no numbers
-    const double nan = __longlong_as_double(0x7FF8000000000000ll);
+    const double nan = timeout_nan();
     if (threadIdx.x == 0) energy[b] = cmk(nan, nan);
     return;
   }
@@ -979,11 +979,12 @@ static bool cisd_wants_m2(const trot_cisd* c, const CisdBuffers& b, int stage) {
 }
 
 // green, x, C_c / C_e, scalars; stage 0 = overlap only, 1 = + N x N matrices and chol contractions, 2 = + energy terms
-static int cisd_run(const trot_cisd* c, int W, const double2* w, CisdBuffers& b, int stage, cudaStream_t st) {
+// (begin: the call's first run, which clears its status word)
+static int cisd_run(const trot_cisd* c, int W, const double2* w, CisdBuffers& b, int stage, cudaStream_t st,
+                    bool begin = true) {
   const int N = c->norb, n = c->nocc, v = c->nvir, G = c->nchol, nv = n * v;
   Spins sp = cisd_spins(c);
-  if (stage > 0) cudaMemsetAsync(b.status, 0, sizeof(int), st);  // this call's word; the sticky one persists
-  TROT_TIMED("cisd_green", st, launch_green(sp, W, N, w, nullptr, b.green, b.det2, b.hg2, st));
+  TROT_TIMED("cisd_green", st, launch_green(sp, W, N, w, nullptr, b.green, b.det2, b.hg2, st, begin ? b.status : nullptr));
   CISD_LAUNCH("cisd_x", cisd_x_kernel, W, 256, 0, st, N, n, v, b.green, c->ci1, b.x,
               stage >= 1 ? b.ci1g1 : nullptr, b.wsc);
   TROT_TIMED("cisd_ci2g", st,
@@ -1243,7 +1244,7 @@ int trot_cisd_prop_step(const trot_cisd* c, const trot_system* prop, const trot_
     TROT_TIMED("trotter_fp64", st, launch_trotter(sp, a, b.dg, st));
   }
   // 5. CISD overlaps of the new walkers, weights, population shift
-  TROT_TRY(cisd_run(c, W, w, b, 0, st));
+  TROT_TRY(cisd_run(c, W, w, b, 0, st, false));
   CISD_LAUNCH("cisd_overlap", cisd_overlap_kernel, W, 256, 0, st, c->nocc * c->nvir, b.x, b.cg, b.wsc, b.det2,
               b.ov_new);
   a.overlaps = (double2*)state->overlaps; a.weights = state->weights; a.scalars = state->scalars;

@@ -9,15 +9,19 @@
 #define TROT_D __device__ __forceinline__
 
 // ---------------------------------------------------------------- device status words
-// A mixed-precision workspace starts with int[4] status words: [0] the status of
-// the current call (reset when the call begins), [3] a sticky copy that only
-// trot_workspace_timeouts clears.  A tensor-core kernel whose bounded wait ran out
-// records TROT_ERR_DEVICE_TIMEOUT in both, skips its outputs and returns; the
-// kernels that combine its results then write NaN instead of numbers.
+// A workspace starts with int[4] status words: [0] the status of the current call
+// (reset when the call begins), [3] a sticky copy that only trot_workspace_timeouts
+// clears.  A tensor-core kernel whose bounded wait ran out records
+// TROT_ERR_DEVICE_TIMEOUT in both, skips its outputs (digit products: makes them NaN)
+// and returns; the kernels that combine its results then write NaN instead of numbers.
 TROT_D void report_timeout(int* status) {
   atomicExch(status, (int)TROT_ERR_DEVICE_TIMEOUT);
   atomicExch(status + 3, (int)TROT_ERR_DEVICE_TIMEOUT);
 }
+// The NaN of those results.  A walker's own NaN energy costs it its weight and no more (block_energy_kernel); an energy
+// with this one means that the whole call gave no numbers.
+static constexpr long long kTimeoutNan = 0x7FF8000074696D65ll;
+TROT_D double timeout_nan() { return __longlong_as_double(kTimeoutNan); }
 
 // ---------------------------------------------------------------- complex (double2)
 TROT_HD double2 cmk(double r, double i) { return make_double2(r, i); }

@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(128) ctx_expm_kernel(int n, const double* A, d
     bad = nrm > 0.5;
   }
   if (blockIdx.x == 0 && tid == 0) {
-    if (bad) status[0] = TROT_ERR_NUMERIC_GUARD;
+    if (bad && status[0] == TROT_OK) status[0] = TROT_ERR_NUMERIC_GUARD;  // (a timed-out product's NaN: its own status)
     status[1] = s;
   }
   grid.sync();

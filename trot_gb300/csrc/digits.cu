@@ -351,6 +351,7 @@ struct DgArgs {
   long long ldc;
   int salpha, ealpha, accumulate;  // alpha = salpha 2^ealpha, salpha = +-1
   int* status;
+  int test_timeout_polls;          // TEST: the MMA thread's first wait is on a barrier nothing arrives on
 };
 
 // q 2^(ex - 1075) for results next to or outside the normal range
@@ -379,7 +380,8 @@ __device__ __noinline__ void dg_add(double2* o, double2 v) { *o = cadd(*o, v); }
 
 // PAIR: the 128-row tiles hold complex rows (row 2 p = real, 2 p + 1 = imaginary part of V[p]) and the product is the
 // complex V T: C[m][p] = V_p . A_m.  Lanes 2 p and 2 p + 1 exchange the cross terms; each stores its part.
-template <bool PAIR>
+// TEST: the kernel of the timeout switch (its test in the MMA loop's function made every product 6 % slower)
+template <bool PAIR, bool TEST>
 __global__ void __launch_bounds__(kDgThreads, 1) dg_gemm_kernel(DgArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   unsigned char* base = smem_raw + ((128 - (tc::smem_u32(smem_raw) & 127)) & 127);
@@ -429,6 +431,7 @@ __global__ void __launch_bounds__(kDgThreads, 1) dg_gemm_kernel(DgArgs a) {
       const uint64_t bd0 = tc::smem_desc(tc::smem_u32(sB), 128, 256);
       const uint32_t adlo = (uint32_t)ad0, bdlo = (uint32_t)bd0, dhi = (uint32_t)(ad0 >> 32);
       int ca = 0, cs = 0;  // K16 step and slab counters of this CTA
+      if (TEST) ok = tc::mbar_wait(drain, 0u, (uint32_t)a.test_timeout_polls);
       for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
         for (int s = 0; s < nslab && ok; ++s, ++cs) {
           const int ks = min(kDgSlab, nk - s * kDgSlab), buf = cs & 1, bs = cs % kDgBSlots;
@@ -478,7 +481,7 @@ __global__ void __launch_bounds__(kDgThreads, 1) dg_gemm_kernel(DgArgs a) {
       const int slots = la ? kDgASlots : kDgBSlots;
       uint64_t* full = la ? a_full : b_full;
       uint64_t* free_ = la ? a_free : b_free;
-      bool ok = true;
+      bool ok = !TEST;
       int c = 0;
       for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
         const int bt = item / (a.nrt * a.ntile);
@@ -512,7 +515,7 @@ __global__ void __launch_bounds__(kDgThreads, 1) dg_gemm_kernel(DgArgs a) {
         }
       }
       if (!ok) {
-        if (!*abort_flag && a.status) report_timeout(a.status);
+        if (!*abort_flag && a.status && !TEST) report_timeout(a.status);
         for (int u = c - 1; u >= 0 && u >= c - slots; --u)  // bounded drain of the copies in flight
           tc::mbar_wait(&full[u % slots], (uint32_t)((u / slots) & 1), 1000000u);
       }
@@ -631,10 +634,12 @@ size_t dg_scratch_bytes(size_t M, size_t Nn, size_t K) {
 }
 
 template <bool PAIR>
-static int dg_gemm(const DgArgs& a, cudaStream_t st) {
-  cudaFuncSetAttribute(dg_gemm_kernel<PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgSmem);
+static int dg_gemm(DgArgs a, cudaStream_t st) {
+  a.test_timeout_polls = tune_get(TROT_TUNE_TEST_TIMEOUT);
+  const auto kernel = a.test_timeout_polls > 0 ? dg_gemm_kernel<PAIR, true> : dg_gemm_kernel<PAIR, false>;
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgSmem);
   const int items = a.nrt * a.ntile * a.nbatch;
-  dg_gemm_kernel<PAIR><<<items < 152 ? items : 152, kDgThreads, kDgSmem, st>>>(a);
+  kernel<<<items < 152 ? items : 152, kDgThreads, kDgSmem, st>>>(a);
   TROT_CHECK_LAUNCH("dg_gemm_kernel");
   return TROT_OK;
 }
@@ -1454,6 +1459,8 @@ extern "C" int trot_zgemm_digits(int M, int N, int K, double alpha, const double
   s.p = c.take<char>(s.bytes);
   s.status = c.status();
   if (!c.ok) { set_error("workspace too small: %zu < %zu", ws_bytes, c.used); return TROT_ERR_WORKSPACE_TOO_SMALL; }
+  const cudaError_t e = cudaMemsetAsync(s.status, 0, sizeof(int), (cudaStream_t)stream);
+  if (e != cudaSuccess) return cuda_status(e, "trot_zgemm_digits memset");
   return launch_zgemm_dg(M, N, K, alpha, (const double2*)A, lda, B, ldb, b_is_nk != 0, (double2*)C, ldc,
                          accumulate != 0, s, (cudaStream_t)stream);
 }

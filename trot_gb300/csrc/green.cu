@@ -22,7 +22,8 @@ static constexpr int kMaxOcc = 64;
 
 __global__ void __launch_bounds__(kGreenThreads)
 green_kernel(Spins sp, int N, int padded, const double2* __restrict__ wa, const double2* __restrict__ wb,
-             double2* __restrict__ green, double2* __restrict__ ovlp_out, double2* __restrict__ e1_out) {
+             double2* __restrict__ green, double2* __restrict__ ovlp_out, double2* __restrict__ e1_out,
+             int* __restrict__ status) {
   extern __shared__ double2 smem[];
   __shared__ double2 red[32];
   __shared__ double2 sums[2];  // det^mult, mult e1 of this spin
@@ -31,6 +32,7 @@ green_kernel(Spins sp, int N, int padded, const double2* __restrict__ wa, const 
   cg::cluster_group cl = cg::this_cluster();
   const int s = sp.nspin == 2 ? blockIdx.x & 1 : 0, b = sp.nspin == 2 ? blockIdx.x >> 1 : blockIdx.x;
   const int tid = threadIdx.x, nt = blockDim.x;
+  if (status && blockIdx.x == 0 && tid == 0) *status = 0;  // this call's status word (the sticky one persists)
   const bool want_green = green != nullptr || e1_out != nullptr;
   const int n = s ? sp.n[1] : sp.n[0], ld = padded ? n | 1 : n;
   const double2* w = (s ? wb : wa) + (size_t)b * N * n;
@@ -89,7 +91,7 @@ green_kernel(Spins sp, int N, int padded, const double2* __restrict__ wa, const 
 }
 
 int launch_green(const Spins& sp, int W, int N, const double2* wa, const double2* wb, double2* green,
-                 double2* ovlp_out, double2* e1_out, cudaStream_t st) {
+                 double2* ovlp_out, double2* e1_out, cudaStream_t st, int* status) {
   int nmax = sp.n[0] > sp.n[1] ? sp.n[0] : sp.n[1];
   if (nmax > kMaxOcc) {
     set_error("green: nocc %d > %d unsupported", nmax, kMaxOcc);
@@ -118,7 +120,8 @@ int launch_green(const Spins& sp, int W, int N, const double2* wa, const double2
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = sp.nspin == 2 ? 1 : 0;
-  const cudaError_t rc = cudaLaunchKernelEx(&cfg, green_kernel, sp, N, pad ? 1 : 0, wa, wb, green, ovlp_out, e1_out);
+  const cudaError_t rc = cudaLaunchKernelEx(&cfg, green_kernel, sp, N, pad ? 1 : 0, wa, wb, green, ovlp_out, e1_out,
+                                            status);
   if (rc != cudaSuccess) return cuda_status(rc, "green_kernel");
   TROT_CHECK_LAUNCH("green_kernel");
   return TROT_OK;

@@ -38,6 +38,7 @@ struct DgScratch {
 };
 
 struct StepBuffers {
+  int* status;  // the workspace's status words
   double2 *green, *e1, *fb, *xs, *shift_term, *fb_term, *vhs, *exc;
   double2* vp;  // packed upper triangle of the VHS (W, N(N+1)/2) when chol_packed is set
   int* node_flag;
@@ -53,8 +54,9 @@ size_t fp64_min_workspace(const trot_system* s, int op);
 // green: complex (W, ntot*N) half Green's functions, spin blocks concatenated
 // (may be null); det_out: complex (W) overlap = prod_s det(C_s^T w_s)^mult_s (may be null);
 // e1_out: complex (W) sum_s mult_s sum(G_s o rot_h1_s) (may be null).
+// status: the call's status word, which the op's first kernel clears (may be null).
 int launch_green(const Spins& sp, int W, int N, const double2* wa, const double2* wb,
-                 double2* green, double2* ovlp_out, double2* e1_out, cudaStream_t st);
+                 double2* green, double2* ovlp_out, double2* e1_out, cudaStream_t st, int* status = nullptr);
 
 // C[m][n] (+)= alpha * sum_k A[m][k] * B(k, n), A complex (lda), C complex (ldc).
 // b_is_nk: B stored (N, K) row-major (ldb) — otherwise (K, N) row-major.
@@ -100,9 +102,8 @@ struct TrotterArgs {
 // by digit products where `dg` holds their scratch and trotter_takes_digits, else on the FP64 pipe
 bool trotter_takes_digits(const Spins& sp, int N);
 int launch_trotter(const Spins& sp, const TrotterArgs& a, const DgScratch& dg, cudaStream_t st);
-// status (optional): the mixed-precision status words of the step (int[4], see
-// report_timeout); when status[0] is set the step's weights and population shift
-// become NaN instead of numbers computed from skipped tensor-core results
+// status (optional): the status words of the step (int[4], see report_timeout);
+// when status[0] is set the step's weights and population shift become NaN instead of numbers computed from skipped tensor-core results
 int launch_step_finalize(int W, double* weights, double* scalars, long long* nodes,
                          const int* node_flag, double damping, double dt, cudaStream_t st,
                          const int* status = nullptr);

@@ -955,7 +955,7 @@ __global__ void __launch_bounds__(256) step_fields_kernel(StepFieldsArgs a) {
       double2 e = a.e1[b];
       if (a.nspin == 2) e = cadd(e, a.e1[(size_t)a.W + b]);
       e = cmk(a.h0 + e.x + 0.5 * sums[4] - 0.5 * sums[6], e.y + 0.5 * sums[5] - 0.5 * sums[7]);
-      a.energy[b] = *a.status != 0 ? cmk(nan, nan) : e;  // the exchange / force-bias kernel timed out: no numbers
+      a.energy[b] = *a.status != 0 ? cmk(timeout_nan(), timeout_nan()) : e;  // the exchange / force-bias kernel timed out: no numbers
     }
   }
 }

@@ -151,7 +151,7 @@ step_finalize_kernel(int W, double* __restrict__ weights, double* __restrict__ s
                      const int* __restrict__ status) {
   __shared__ double2 red[32];
   if (status && status[0] != 0) {  // a tensor-core kernel of this step timed out: no numbers
-    const double nan = __longlong_as_double(0x7FF8000000000000ll);
+    const double nan = timeout_nan();
     for (int i = threadIdx.x; i < W; i += blockDim.x) weights[i] = nan;
     if (threadIdx.x == 0) scalars[0] = nan;
     return;
@@ -258,7 +258,7 @@ energy_combine_kernel(int G, int nchunks, double h0, const double2* __restrict__
   __shared__ double red[64], sums[8];
   const int b = blockIdx.x;
   if (status && status[0] != 0) {  // the exchange / force-bias kernel timed out: no numbers
-    const double nan = __longlong_as_double(0x7FF8000000000000ll);
+    const double nan = timeout_nan();
     if (threadIdx.x == 0) energy[b] = cmk(nan, nan);
     return;
   }

@@ -387,7 +387,8 @@ int launch_sr(const Spins& sp, int W, int N, const double* weights, const double
 // Block tail of trot/prop/blocks.py:236-257 on the device: E = Re(E_L); walkers
 // with non-finite E get weight 0; E is clamped to e_ref when |E - e_ref| >
 // sqrt(2/dt); e_block = sum w E / sum w (e_ref if sum w == 0);
-// e_estimate <- (1 - ema) e_estimate + ema e_block.  obs = [e_block, sum w].
+// e_estimate <- (1 - ema) e_estimate + ema e_block.  obs = [e_block, sum w].  Energies of a call that timed out
+// (timeout_nan): weights, e_estimate and obs become NaN too.
 __global__ void __launch_bounds__(1024)
 block_energy_kernel(int W, const double2* __restrict__ energy, double* __restrict__ weights,
                     double* __restrict__ scalars, double dt, double ema, double* __restrict__ obs) {
@@ -395,14 +396,21 @@ block_energy_kernel(int W, const double2* __restrict__ energy, double* __restric
   const double e_ref = scalars[1];
   const double thresh = sqrt(2.0 / dt);
   double2 acc = cmk(0.0, 0.0);  // (sum w E, sum w)
+  bool timed_out = false;
   for (int i = threadIdx.x; i < W; i += blockDim.x) {
     double e = energy[i].x;
     const bool bad = !isfinite(e);
+    timed_out |= __double_as_longlong(e) == kTimeoutNan;
     if (bad || fabs(e - e_ref) > thresh) e = e_ref;
     double w = weights[i];
     if (bad) { w = 0.0; weights[i] = 0.0; }
     acc.x += w * e;
     acc.y += w;
+  }
+  if (__syncthreads_or(timed_out)) {  // the energies are no numbers (report_timeout): nor is the block
+    for (int i = threadIdx.x; i < W; i += blockDim.x) weights[i] = timeout_nan();
+    if (threadIdx.x == 0) scalars[1] = obs[0] = obs[1] = timeout_nan();
+    return;
   }
   acc = block_sum2(acc, red);
   if (threadIdx.x == 0) {

@@ -65,6 +65,8 @@ def prop_ctx(h0: float, h1, chol, rdm1, dt: float):
     torch.cuda.current_stream().synchronize()
     st = ctypes.c_int(0)
     _lib.call("trot_workspace_status", ws.data_ptr(), ctypes.addressof(st))
+    if st.value == 6:
+        raise _lib.TrotError(st.value, "propagation context: a tensor-core kernel's bounded wait ran out")
     if st.value != _lib.OK:
         raise _lib.TrotError(st.value, "propagation context: h1_eff has a non-finite entry or "
                                        "dt/2 ||h1_eff||_1 > 2^39")

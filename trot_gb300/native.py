@@ -58,7 +58,9 @@ def raise_on_timeout(ws_ptr: int, what: str) -> None:
 def check_device_timeouts(what: str = "trot_gb300") -> None:
     """raise_on_timeout for every cached workspace of the current device (one
     check per block or per graph replay covers all the asynchronous steps
-    before it)."""
+    before it).  The mixed-precision energies and force biases check by
+    themselves; FP64 calls do not wait for the device, so a timed-out one shows
+    in its NaN results (and those of the block around it) and here."""
     dev = torch.cuda.current_device()
     for (d, _), buf in list(_workspaces.items()):
         if d == dev:

@@ -48,14 +48,19 @@ Spins make_spins(const trot_system* s) {
   return sp;
 }
 
+// f_g of every vector by digit products: the force bias is their traces, with or without an energy
+static bool takes_traces(int N) { return dg_takes(N) && N <= 1024; }
+
 // Scratch of the op's tensor-core digit products (the largest of them; they run one after another).
 static size_t digit_bytes(const trot_system* s, const Spins& sp, int op) {
   const size_t W = s->n_walkers, N = s->norb, G = s->nchol;
   size_t n = 0;
-  if (op == TROT_OP_FORCE_BIAS || op == TROT_OP_LOCAL_ENERGY || op == TROT_OP_PROP_STEP)
+  if ((op == TROT_OP_FORCE_BIAS || op == TROT_OP_LOCAL_ENERGY || op == TROT_OP_PROP_STEP) && !takes_traces((int)N))
     for (int q = 0; q < sp.nspin; ++q)
       if (dg_takes(sp.n[q] * (int)N)) n = std::max(n, dg_scratch_bytes(W, G, sp.n[q] * N));
-  if ((op == TROT_OP_LOCAL_ENERGY || op == TROT_OP_PROP_STEP) && dg_takes((int)N) && N <= 1024)
+  if ((op == TROT_OP_FORCE_BIAS || op == TROT_OP_PROP_STEP) && takes_traces((int)N))
+    n = std::max(n, fb_dg_bytes(sp, W, N, G));
+  if ((op == TROT_OP_LOCAL_ENERGY || op == TROT_OP_PROP_STEP) && takes_traces((int)N))
     n = std::max(n, exchange_dg_bytes(sp, W, N, G));
   if ((op == TROT_OP_APPLY_TROTTER || op == TROT_OP_PROP_STEP) && dg_takes((int)G))
     n = std::max(n, dg_scratch_bytes(W, N * N, G));  // full or packed
@@ -157,10 +162,11 @@ static int check_prop(const trot_system* s) {
 }
 
 
-// force bias from the half Green's functions: fb = sum_s mult_s rot_chol_s G_s
+// force bias from the half Green's functions: fb = sum_s mult_s rot_chol_s G_s (the bits of force_bias_and_exchange)
 static int force_bias_from_green(const trot_system* s, const Spins& sp, const double2* green, double2* fb,
-                                 const DgScratch& dg, cudaStream_t st) {
+                                 FbParts* parts, const DgScratch& dg, cudaStream_t st) {
   const int W = s->n_walkers, N = s->norb, G = s->nchol, K = sp.ntot * N;
+  if (dg.p && takes_traces(N)) return launch_fb_dg(sp, W, N, G, green, fb, parts, dg, st);
   for (int q = 0; q < sp.nspin; ++q) {
     TROT_TRY(launch_zgemm(W, G, sp.n[q] * N, (double)sp.mult[q], green + (size_t)sp.off[q] * N, K, sp.rot_chol[q],
                           sp.n[q] * N, true, fb, G, q > 0, dg, st));
@@ -174,13 +180,13 @@ static int force_bias_and_exchange(const trot_system* s, const Spins& sp, const 
                                    cudaStream_t st) {
   const int W = s->n_walkers, N = s->norb, G = s->nchol;
   TROT_TRY(check_exchange_tile(sp, N));
-  if (b.dg.p && dg_takes(N) && N <= 1024) {
+  if (b.dg.p && takes_traces(N)) {
     nchunks = exchange_dg_chunks(G);
     TROT_TIMED("exchange_digits", st, launch_exchange_dg(sp, W, N, G, b.green, b.exc, b.fb, b.dg, st));
     return TROT_OK;
   }
   nchunks = exchange_chunks(G);
-  TROT_TIMED("force_bias_fp64", st, force_bias_from_green(s, sp, b.green, b.fb, b.dg, st));
+  TROT_TIMED("force_bias_fp64", st, force_bias_from_green(s, sp, b.green, b.fb, nullptr, b.dg, st));
   TROT_TIMED("exchange_fp64", st, launch_exchange(sp, W, N, G, b.green, b.exc, st));
   return TROT_OK;
 }
@@ -310,7 +316,7 @@ int trot_force_bias(const trot_system* s, const double* wa, const double* wb, do
   TROT_TRY(carve_ws(s, sp, ws, ws_bytes, b, TROT_OP_FORCE_BIAS));
   TROT_TRY(launch_green(sp, s->n_walkers, s->norb, (const double2*)wa, (const double2*)wb, b.green, nullptr,
                         nullptr, st, b.status));
-  return force_bias_from_green(s, sp, b.green, (double2*)out, b.dg, st);
+  return force_bias_from_green(s, sp, b.green, (double2*)out, nullptr, b.dg, st);
 }
 
 int trot_local_energy(const trot_system* s, const double* wa, const double* wb, double* out, void* ws,
@@ -378,8 +384,9 @@ int trot_prop_step(const trot_system* s, const trot_state* state, const double* 
   // 1. Green's functions (+ one-body energy) of the current walkers
   TROT_TIMED("green", st, launch_green(sp, W, N, wa, wb, b.green, nullptr, energy_out ? b.e1 : nullptr, st, b.status));
   // 2. force bias, 3. optional local energy of the current walkers (reuses G; f_g gives both)
+  FbParts parts{};
   if (!energy_out) {
-    TROT_TIMED("force_bias_fp64", st, force_bias_from_green(s, sp, b.green, b.fb, b.dg, st));
+    TROT_TIMED("force_bias_fp64", st, force_bias_from_green(s, sp, b.green, b.fb, &parts, b.dg, st));
   } else {
     int nchunks = 0;
     TROT_TRY(force_bias_and_exchange(s, sp, b, nchunks, st));
@@ -387,7 +394,7 @@ int trot_prop_step(const trot_system* s, const trot_state* state, const double* 
                launch_energy_combine(W, G, nchunks, s->h0, b.fb, b.e1, 1, b.exc, (double2*)energy_out, st, b.status));
   }
   // 4. shifted fields
-  TROT_TIMED("fields", st, launch_fields(W, G, s->sqrt_dt, b.fb, s->mf_shifts_im, fields, b.xs, b.shift_term, b.fb_term, st));
+  TROT_TIMED("fields", st, launch_fields(W, G, s->sqrt_dt, b.fb, s->mf_shifts_im, fields, b.xs, b.shift_term, b.fb_term, st, &parts));
   // 5. VHS
   TROT_TIMED("vhs_fp64", st, launch_vhs64(W, N, G, b.xs, s->chol_flat, s->chol_packed, b.vp, b.vhs, b.dg, st));
   // 6. propagation + overlaps + weights

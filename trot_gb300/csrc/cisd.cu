@@ -973,9 +973,10 @@ static Spins cisd_spins(const trot_cisd* c) {
     return TROT_OK;                                             \
   })())
 
-// ci2_green by itself is read by cisd_gamma_kernel only
-static bool cisd_wants_m2(const trot_cisd* c, const CisdBuffers& b, int stage) {
-  return stage == 2 && c->gl_precision != TROT_MIXED && !(b.dg.p && cisd_gamma_digits(c));
+// ci2_green by itself is read by cisd_gamma_kernel only.  (Without an energy nothing reads it, but the force bias has
+// its bits from the same two sums then.)
+static bool cisd_wants_m2(const trot_cisd* c, const CisdBuffers& b) {
+  return c->gl_precision != TROT_MIXED && !(b.dg.p && cisd_gamma_digits(c));
 }
 
 // green, x, C_c / C_e, scalars; stage 0 = overlap only, 1 = + N x N matrices and chol contractions, 2 = + energy terms
@@ -994,7 +995,7 @@ static int cisd_run(const trot_cisd* c, int W, const double2* w, CisdBuffers& b,
   const size_t smem = cisd_mats_smem(N, n, v);
   if (smem > 40 * 1024) cudaFuncSetAttribute(cisd_mats_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   CISD_LAUNCH("cisd_mats", cisd_mats_kernel, W, 256, smem, st, N, n, v, b.green, c->ci1, b.cg, b.x, c->h1, b.ms,
-              cisd_wants_m2(c, b, stage) ? b.m2 : nullptr, b.p2, b.wsc);
+              cisd_wants_m2(c, b) ? b.m2 : nullptr, b.p2, b.wsc);
   // lg = rot_chol . G  (rot_chol rows g: chol[g][:n][:] = first n N entries of chol_flat row g)
   TROT_TIMED("cisd_chol_gemm", st,
              launch_zgemm(W, G, n * N, 1.0, b.green, n * N, c->chol, N * N, true, b.lg, G, false, b.dg, st, b.kpart,

@@ -873,6 +873,89 @@ int launch_exchange_dg(const Spins& sp, int W, int N, int G, const double2* gree
   return TROT_OK;
 }
 
+// The traces alone, for a force bias without an energy: the diagonal elements f_gii of every occupied orbital i as one
+// batch (rows: walkers, columns: vectors), then the sums over i in exchange_pairs_kernel's order, so that a step moves its
+// walkers by the same bits whether or not it reports their energy.  The sums are left to the kernel that forms the fields
+// (FbParts) where all f_gii fit a cap; they are FP64 additions, 43 us of that pipe at 22 columns, 600 vectors, 1024 walkers.
+// One product over (i, p), of other roundings, takes about as long: its K is n times as long and its tiles are fewer (N =
+// 135, n = 16, 540 vectors, 128 walkers leave 112 SMs without one).
+static constexpr size_t kFbCap = size_t(256) << 20;
+static size_t fb_chunk(const Spins& sp, size_t W, size_t G) {  // walkers per pass, a multiple of 16
+  size_t wc = kFbCap / (sp.ntot * G * sizeof(double2)) / 16 * 16;
+  if (wc < 16) wc = 16;
+  return std::min(wc, (W + 15) / 16 * 16);
+}
+
+size_t fb_dg_bytes(const Spins& sp, size_t W, size_t N, size_t G) {
+  const size_t rb = kDgRowBytes((N + 15) / 16), wc = fb_chunk(sp, W, G);
+  const size_t nmax = std::max(sp.n[0], sp.nspin == 2 ? sp.n[1] : 0);
+  return nmax * ((2 * wc + 31) / 32 * 32 + (G + 127) / 128 * 128) * (rb + 2) + sp.ntot * wc * G * sizeof(double2) + 6 * 256;
+}
+
+__global__ void __launch_bounds__(256) fb_traces_kernel(FbParts f, double2* __restrict__ fb) {
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < f.len; e += (size_t)gridDim.x * blockDim.x)
+    fb[e] = fb_trace(f, e);
+}
+
+int launch_fb_dg(const Spins& sp, int W, int N, int G, const double2* green, double2* fb, FbParts* parts,
+                 const DgScratch& s, cudaStream_t st) {
+  if (s.bytes < fb_dg_bytes(sp, W, N, G)) { set_error("force bias: scratch %zu", s.bytes); return TROT_ERR_WORKSPACE_TOO_SMALL; }
+  const size_t rb = kDgRowBytes((N + 15) / 16);
+  const int gpad = (G + 127) / 128 * 128, wc = (int)fb_chunk(sp, W, G), nmax = std::max(sp.n[0], sp.nspin == 2 ? sp.n[1] : 0);
+  const size_t rows = (size_t)nmax * ((2 * wc + 31) / 32 * 32);
+  char* p = reinterpret_cast<char*>(((uintptr_t)s.p + 255) & ~(uintptr_t)255);
+  auto take = [&](size_t n) {
+    char* r = p;
+    p += (n + 255) & ~(size_t)255;
+    return r;
+  };
+  DgArgs a{};
+  uint16_t* imgB = reinterpret_cast<uint16_t*>(take((size_t)nmax * gpad * rb));
+  uint16_t* imgA = reinterpret_cast<uint16_t*>(take(rows * rb));
+  int16_t* exB = reinterpret_cast<int16_t*>(take((size_t)nmax * gpad * 2));
+  int16_t* exA = reinterpret_cast<int16_t*>(take(rows * 2));
+  double2* F = reinterpret_cast<double2*>(p);
+  const double* held = nullptr;  // whose digits imgB holds
+  int held_n = 0;
+  for (int w0 = 0; w0 < W; w0 += wc) {
+    const int wn = std::min(wc, W - w0), apad = (2 * wn + kDgP - 1) / kDgP * kDgP;
+    FbParts f{};
+    f.nspin = sp.nspin;
+    f.len = (size_t)wn * G;
+    for (int q = 0; q < sp.nspin; ++q) {
+      const int n = sp.n[q];
+      DgRows r{};
+      if (sp.rot_chol[q] != held || n != held_n) {
+        held = sp.rot_chol[q];
+        held_n = n;
+        DgSrc sb = dg_src(sp.rot_chol[q], 0, G, N, 128, (long long)n * N, 1, imgB, exB);
+        sb.rpad = gpad; sb.nblk = n; sb.bstride = N;
+        dg_rows_add(r, sb, n * (gpad / 8));
+      }
+      DgSrc sa = dg_src(reinterpret_cast<const double*>(green + ((size_t)w0 * sp.ntot + sp.off[q]) * N), 1, 2 * wn, N,
+                        kDgP, 2ll * sp.ntot * N, 2, imgA, exA);
+      sa.rpad = apad; sa.nblk = n; sa.bstride = 2ll * N;
+      dg_rows_add(r, sa, n * (apad / 8));
+      TROT_TRY(dg_rows_launch(r, st));
+      a.imgB = imgB; a.exB = exB; a.imgA = imgA; a.exA = exA;
+      a.Nn = G; a.M = wn; a.nrt = a.bB = gpad / 128; a.ntile = apad / kDgP; a.nbatch = n;
+      a.cstride = (long long)f.len; a.nk16 = (N + 15) / 16; a.shift = 1;  // N <= 1024
+      a.C = F + sp.off[q] * f.len; a.ldc = G; a.salpha = 1; a.status = s.status;
+      TROT_TRY(dg_gemm<false>(a, st));
+      f.F[q] = a.C;
+      f.n[q] = n;
+      f.mult[q] = sp.mult[q];
+    }
+    if (parts && wc >= W) {
+      *parts = f;
+      return TROT_OK;
+    }
+    fb_traces_kernel<<<(unsigned)std::min<size_t>((f.len + 255) / 256, 152 * 8), 256, 0, st>>>(f, fb + (size_t)w0 * G);
+    TROT_CHECK_LAUNCH("fb_traces_kernel");
+  }
+  return TROT_OK;
+}
+
 // ------------------------------------------------------------------ Trotter propagation
 // w' = E sum_k ((i sqrt(dt))^k / k!) V^k E w of every walker (trot/prop/chol_afqmc_ops.py:198-222,
 // trot/prop/utils.py:20-30) as a chain of batched digit products: per walker V (2 N rows, re / im interleaved) against

@@ -27,6 +27,12 @@ size_t exchange_dg_bytes(const Spins& sp, size_t W, size_t N, size_t G);
 int launch_exchange_dg(const Spins& sp, int W, int N, int G, const double2* green, double2* partial, double2* fb,
                        const DgScratch& s, cudaStream_t st);
 
+// The same fb, bit for bit, without the exchange sums.  With parts, where all f_gii are there at once, they are handed
+// over in it instead (inside the scratch; parts->nspin stays 0 otherwise).
+size_t fb_dg_bytes(const Spins& sp, size_t W, size_t N, size_t G);
+int launch_fb_dg(const Spins& sp, int W, int N, int G, const double2* green, double2* fb, FbParts* parts,
+                 const DgScratch& s, cudaStream_t st);
+
 // C[g][m][j] = (row 2 m, row 2 m + 1) of L_g L_g for `count` real N x N matrices, m < ceil(N / 2) (N even or odd: the
 // odd last row's partner is zero).  square_dg_count: matrices a call takes with a scratch of square_dg_bytes.
 int square_dg_count(size_t N, size_t G);

@@ -80,9 +80,36 @@ int launch_vhs64(int W, int N, int G, const double2* xs, const double* chol_flat
 // Mp = the packed upper triangle of M + M^T (diagonal once), W matrices of N x N.
 int launch_pack_sym(int N, int W, const double2* m, double2* mp, cudaStream_t st);
 
-// step64.cu
+// Diagonal elements f_gii whose sums are the force bias (digits.cu): spin q's of orbital i at F[q] + i len complex
+// values, (W, G) each.  nspin 0: none.
+struct FbParts {
+  const double2* F[2];
+  size_t len;
+  int n[2], mult[2], nspin;
+};
+// element e of fb = sum_q mult_q sum_i f_gii, added in exchange_pairs_kernel's order
+TROT_D double2 fb_trace(const FbParts& f, size_t e) {
+  double2 v = make_double2(0.0, 0.0);
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    if (q >= f.nspin) break;
+    const double2* p = f.F[q] + e;
+    double2 t = make_double2(0.0, 0.0);
+#pragma unroll 4
+    for (int i = 0; i < f.n[q]; ++i) {
+      const double2 x = __ldg(p + i * f.len);
+      t = make_double2(__dadd_rn(t.x, x.x), __dadd_rn(t.y, x.y));
+    }
+    if (f.mult[q] == 2) t = make_double2(__dadd_rn(t.x, t.x), __dadd_rn(t.y, t.y));
+    v = q ? make_double2(__dadd_rn(v.x, t.x), __dadd_rn(v.y, t.y)) : t;
+  }
+  return v;
+}
+
+// step64.cu (the force bias from fb, or from parts where given)
 int launch_fields(int W, int G, double sqrt_dt, const double2* fb, const double* mf_im,
-                  const double* x, double2* xs, double2* shift_term, double2* fb_term, cudaStream_t st);
+                  const double* x, double2* xs, double2* shift_term, double2* fb_term, cudaStream_t st,
+                  const FbParts* parts = nullptr);
 
 struct TrotterArgs {
   int W, N, G, nterms;

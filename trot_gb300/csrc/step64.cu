@@ -10,15 +10,16 @@ namespace trot {
 //   s = -sqrt(dt) (i fb - mf),  xs = x - s,
 //   shift_term = sum_g xs mf,   fb_term = sum_g (x s - s^2 / 2)
 // mf = i * mf_im (purely imaginary).  One CTA per walker.
+template <bool PARTS>
 __global__ void __launch_bounds__(256)
-fields_kernel(int G, double sqrt_dt, const double2* __restrict__ fb, const double* __restrict__ mf_im,
+fields_kernel(int G, double sqrt_dt, FbParts parts, const double2* __restrict__ fb, const double* __restrict__ mf_im,
               const double* __restrict__ x, double2* __restrict__ xs, double2* __restrict__ shift_term,
               double2* __restrict__ fb_term) {
   __shared__ double red[64], sums[8];
   const int b = blockIdx.x;
   double2 st = cmk(0.0, 0.0), ft = cmk(0.0, 0.0);
   for (int g = threadIdx.x; g < G; g += blockDim.x) {
-    const double2 f = fb[(size_t)b * G + g];
+    const double2 f = PARTS ? fb_trace(parts, (size_t)b * G + g) : fb[(size_t)b * G + g];
     const double2 mf = cmk(0.0, mf_im[g]);
     const double2 ifb = cmk(-f.y, f.x);
     const double2 s = cscale(csub(ifb, mf), -sqrt_dt);
@@ -37,8 +38,11 @@ fields_kernel(int G, double sqrt_dt, const double2* __restrict__ fb, const doubl
 }
 
 int launch_fields(int W, int G, double sqrt_dt, const double2* fb, const double* mf_im, const double* x,
-                  double2* xs, double2* shift_term, double2* fb_term, cudaStream_t st) {
-  fields_kernel<<<W, 256, 0, st>>>(G, sqrt_dt, fb, mf_im, x, xs, shift_term, fb_term);
+                  double2* xs, double2* shift_term, double2* fb_term, cudaStream_t st, const FbParts* parts) {
+  if (parts && parts->nspin)
+    fields_kernel<true><<<W, 256, 0, st>>>(G, sqrt_dt, *parts, fb, mf_im, x, xs, shift_term, fb_term);
+  else
+    fields_kernel<false><<<W, 256, 0, st>>>(G, sqrt_dt, FbParts{}, fb, mf_im, x, xs, shift_term, fb_term);
   TROT_CHECK_LAUNCH("fields_kernel");
   return TROT_OK;
 }

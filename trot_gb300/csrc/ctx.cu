@@ -355,12 +355,18 @@ int launch_expm(int n, const double* A, double* out, double* p0, double* p1, int
   return TROT_OK;
 }
 
-// Scratch of the squares' digit products, at the end of a workspace (none for sizes that keep the FP64 kernel)
+// Scratch of the squares' digit products, at the end of a workspace (none for sizes that keep the FP64 kernel, or where
+// the rest of a caller's workspace is too small for it)
 static DgScratch carve_squares(int N, int G, Carver& c, int* status) {
   DgScratch d;
   if (!dg_takes(N) || N > 1024) return d;
+  const Carver before = c;
   const size_t bytes = square_dg_bytes(N, square_dg_count(N, G));
   d.p = c.take<char>(bytes);
+  if (before.base && before.ok && !c.ok) {
+    c = before;
+    return DgScratch{};
+  }
   d.bytes = bytes;
   d.status = status;
   return d;

@@ -410,11 +410,14 @@ int trot_fp_step(const trot_system* sys, const trot_state* state, const double* 
  *   mf_im[g]    = tr(L_g rdm1)           (mf_shifts = i mf_im, nchol doubles)
  *   *h0_prop    = -h0 + 1/2 sum_g mf_im[g]^2
  *   exp_h1_half = expm(-dt/2 (h1 - 1/2 sum_g L_g L_g + sum_g mf_im[g] L_g))   (norb, norb)
- * Workspace: trot_prop_ctx_workspace_size(norb, nchol) bytes; after the stream
+ * Workspace: trot_prop_ctx_workspace_size(norb, nchol) bytes; with
+ * trot_prop_ctx_workspace_size_digits of them the squares L_g L_g run on the
+ * tensor cores (the same numbers to rounding).  After the stream
  * reaches the end of the call, trot_workspace_status(workspace) is
  * TROT_ERR_NUMERIC_GUARD when h1_eff had a non-finite entry or
  * dt/2 ||h1_eff||_1 > 2^39 (outputs undefined then), else TROT_OK. */
 size_t trot_prop_ctx_workspace_size(int norb, int nchol);
+size_t trot_prop_ctx_workspace_size_digits(int norb, int nchol);
 int trot_build_prop_ctx(int norb, int nchol, double h0, double dt, const double* h1, const double* chol,
                         const double* rdm1, double* mf_im, double* h0_prop, double* exp_h1_half,
                         void* workspace, size_t workspace_bytes, void* stream);
@@ -479,8 +482,9 @@ int trot_orthonormalize_vjp(const trot_system* sys, const double* walkers_a, con
 /* Adjoint of the propagation context's exp(-dt/2 h1_eff) with respect to h1:
  * adds the Frechet-derivative adjoint of expm applied to g_exp_h1_half, times
  * -dt/2, into g_h1 (N x N); same inputs as trot_build_prop_ctx.  Workspace:
- * trot_prop_ctx_vjp_workspace_size(norb, nchol). */
+ * trot_prop_ctx_vjp_workspace_size(norb, nchol), or _digits as there. */
 size_t trot_prop_ctx_vjp_workspace_size(int norb, int nchol);
+size_t trot_prop_ctx_vjp_workspace_size_digits(int norb, int nchol);
 int trot_prop_ctx_vjp(int norb, int nchol, double dt, const double* h1, const double* chol, const double* rdm1,
                       const double* g_exp_h1_half, double* g_h1, void* workspace, size_t workspace_bytes,
                       void* stream);

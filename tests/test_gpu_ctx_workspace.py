@@ -32,8 +32,9 @@ def test_small_workspace(N, G, vjp):
     h1, rho, gE = (dev(rng.standard_normal((N, N)) / N) for _ in range(3))
     chol = dev(rng.standard_normal((G, N, N)) / np.sqrt(N * G))
     lib = _lib.load()
-    full = (lib.trot_prop_ctx_vjp_workspace_size if vjp else lib.trot_prop_ctx_workspace_size)(N, G)
+    full = (lib.trot_prop_ctx_vjp_workspace_size_digits if vjp else lib.trot_prop_ctx_workspace_size_digits)(N, G)
     least = _need(N, G, vjp)
+    assert least <= (lib.trot_prop_ctx_vjp_workspace_size if vjp else lib.trot_prop_ctx_workspace_size)(N, G) <= least + 256
     assert least < full // 4
     new = lambda *s: torch.zeros(s, dtype=torch.float64, device="cuda")
 

@@ -118,6 +118,7 @@ _SIGNATURES = {
     "trot_fp_workspace_size": (ctypes.c_size_t, [ctypes.POINTER(TrotSystem)]),
     "trot_fp_step": (_i, [ctypes.POINTER(TrotSystem), ctypes.POINTER(TrotState), _p, _p, _p, ctypes.c_size_t, _p]),
     "trot_prop_ctx_workspace_size": (ctypes.c_size_t, [_i, _i]),
+    "trot_prop_ctx_workspace_size_digits": (ctypes.c_size_t, [_i, _i]),
     "trot_build_prop_ctx": (_i, [_i, _i, _d, _d, _p, _p, _p, _p, _p, _p, _p, ctypes.c_size_t, _p]),
     "trot_half_rotate": (_i, [_i, _i, _i, _p, _p, _p, _p, _p, _p]),
     "trot_cisd_lci1": (_i, [_i, _i, _i, _p, _p, _p, _p]),
@@ -128,6 +129,7 @@ _SIGNATURES = {
     "trot_overlap_vjp": (_i, [ctypes.POINTER(TrotSystem), _p, _p, _p, _p, _p, _p, ctypes.c_size_t, _p]),
     "trot_orthonormalize_vjp": (_i, [ctypes.POINTER(TrotSystem), _p, _p, _p, _p, _p, _p, _p, _p, _p]),
     "trot_prop_ctx_vjp_workspace_size": (ctypes.c_size_t, [_i, _i]),
+    "trot_prop_ctx_vjp_workspace_size_digits": (ctypes.c_size_t, [_i, _i]),
     "trot_prop_ctx_vjp": (_i, [_i, _i, _d, _p, _p, _p, _p, _p, _p, ctypes.c_size_t, _p]),
     "trot_set_tuning": (_i, [_i, _i]),
     "trot_get_tuning": (_i, [_i]),

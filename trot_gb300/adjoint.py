@@ -170,7 +170,7 @@ class ExpH1Half(torch.autograd.Function):
         N, G = prob.norb, prob.nchol
         rd = ctx_dev._spin_summed(prob.rdm1)
         gh1 = torch.zeros((N, N), dtype=torch.float64, device=h1.device)
-        ws = _ws(_lib.load().trot_prop_ctx_vjp_workspace_size(N, G))
+        ws = _ws(_lib.load().trot_prop_ctx_vjp_workspace_size_digits(N, G))
         g = g.contiguous()
         _lib.call("trot_prop_ctx_vjp", N, G, float(prob.params.dt), h1.detach().contiguous().data_ptr(),
                   prob.chol.data_ptr(), rd.data_ptr(), g.data_ptr(), gh1.data_ptr(), ws.data_ptr(), ws.numel(),

@@ -400,14 +400,16 @@ using namespace trot;
 
 extern "C" {
 
-size_t trot_prop_ctx_workspace_size(int norb, int nchol) {
+static size_t ctx_workspace(int norb, int nchol, bool digits) {
   if (norb < 1 || nchol < 1) { set_error("bad shape: norb %d, nchol %d", norb, nchol); return 0; }
   Carver c(nullptr, 0);
   CtxBuffers b;
   carve_ctx(norb, nchol, c, b);
-  carve_squares(norb, nchol, c, b.status);
+  if (digits) carve_squares(norb, nchol, c, b.status);
   return c.used + 256;
 }
+size_t trot_prop_ctx_workspace_size(int norb, int nchol) { return ctx_workspace(norb, nchol, false); }
+size_t trot_prop_ctx_workspace_size_digits(int norb, int nchol) { return ctx_workspace(norb, nchol, true); }
 
 int trot_build_prop_ctx(int norb, int nchol, double h0, double dt, const double* h1, const double* chol,
                         const double* rdm1, double* mf_im, double* h0_prop, double* exp_h1_half, void* ws,
@@ -442,7 +444,7 @@ int trot_build_prop_ctx(int norb, int nchol, double h0, double dt, const double*
   return TROT_OK;
 }
 
-size_t trot_prop_ctx_vjp_workspace_size(int norb, int nchol) {
+static size_t ctx_vjp_workspace(int norb, int nchol, bool digits) {
   if (norb < 1 || nchol < 1) { set_error("bad shape: norb %d, nchol %d", norb, nchol); return 0; }
   Carver c(nullptr, 0);
   CtxBuffers b;
@@ -450,9 +452,11 @@ size_t trot_prop_ctx_vjp_workspace_size(int norb, int nchol) {
   const size_t m = (size_t)4 * norb * norb;
   c.take<double>(nchol);      // mean-field traces
   for (int k = 0; k < 4; ++k) c.take<double>(m);  // M, P0, P1, expm(M)
-  carve_squares(norb, nchol, c, b.status);
+  if (digits) carve_squares(norb, nchol, c, b.status);
   return c.used + 256;
 }
+size_t trot_prop_ctx_vjp_workspace_size(int norb, int nchol) { return ctx_vjp_workspace(norb, nchol, false); }
+size_t trot_prop_ctx_vjp_workspace_size_digits(int norb, int nchol) { return ctx_vjp_workspace(norb, nchol, true); }
 
 int trot_prop_ctx_vjp(int norb, int nchol, double dt, const double* h1, const double* chol, const double* rdm1,
                       const double* g_exp_h1_half, double* g_h1, void* ws, size_t ws_bytes, void* stream) {

@@ -53,7 +53,7 @@ def prop_ctx(h0: float, h1, chol, rdm1, dt: float):
     if tuple(chol.shape) != (G, N, N) or tuple(h1.shape) != (N, N) or tuple(dm.shape) != (N, N):
         raise ValueError(f"shapes h1 {tuple(h1.shape)}, chol {tuple(chol.shape)}, rdm1 {tuple(dm.shape)}")
     lib = _lib.load()
-    nbytes = lib.trot_prop_ctx_workspace_size(N, G)
+    nbytes = lib.trot_prop_ctx_workspace_size_digits(N, G)
     if nbytes == 0:
         _lib.check(1)  # TROT_ERR_BAD_SHAPE, message from the library
     ws = torch.empty(nbytes, dtype=torch.uint8, device=chol.device)

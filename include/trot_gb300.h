@@ -164,8 +164,13 @@ typedef struct {
 const char* trot_last_error(void);
 int trot_abi_version(void);
 
-/* Bytes of workspace the given op needs for this system. */
+/* Bytes of workspace the given op wants for this system. */
 size_t trot_workspace_size(const trot_system* sys, int op);
+/* Bytes with which the op runs at all: without the scratch of the FP64 digit
+ * products, on the slower FP64 pipe (the same numbers to rounding).  Any
+ * workspace between the two is accepted.  Likewise the other *_size_least
+ * functions below. */
+size_t trot_workspace_size_least(const trot_system* sys, int op);
 
 /* Trial overlaps of all walkers (complex128 out (W)).
  * Replaces overlap_r / overlap_u: trot/trial/rhf.py:45-54, trot/trial/uhf.py:48-58. */
@@ -249,8 +254,8 @@ int trot_sr_resample(const trot_system* sys, const double* weights_in, const dou
 /* Block energy on the device (trot/prop/blocks.py:236-257): clamps Re(E_L)
  * to e_estimate when non-finite or further than sqrt(2/dt) from it, zeroes the
  * weights of non-finite walkers (in place; the energies of a call that timed
- * out, see trot_workspace_status, make all weights and the block NaN), forms the weighted block energy
- * and updates e_estimate (scalars[1]) with the shift_ema moving average.
+ * out, see trot_workspace_status, make all weights and the block NaN), forms
+ * the weighted block energy and updates e_estimate (scalars[1]) with the shift_ema moving average.
  * obs_out (float64 [2], device) receives [e_block, sum of weights]. */
 int trot_block_energy(int n_walkers, const double* energy, double* weights, double* scalars, double dt,
                       double shift_ema, double* obs_out, void* stream);
@@ -286,7 +291,7 @@ int trot_split_key(int64_t* key, void* stream);
  * loads it, until the process exits).  For callers that cannot allocate
  * device memory, e.g. a JAX custom call inside a process whose GPU memory
  * XLA has pre-allocated.  Systems needing more scratch than 32 MiB
- * (trot_workspace_size(sys, TROT_OP_LOCAL_ENERGY)) are rejected with
+ * (trot_workspace_size_least(sys, TROT_OP_LOCAL_ENERGY)) are rejected with
  * TROT_ERR_WORKSPACE_TOO_SMALL.  A call outside stream capture resolves the
  * array's address on the current device (cudaGetSymbolAddress) and caches it;
  * calls under capture use the cache, so the first call on a device must come
@@ -352,6 +357,7 @@ typedef struct {
  * sizes.  The local energy needs 2 W nchol nocc nvir complex values for the
  * l2ci2 quadratic forms. */
 size_t trot_cisd_workspace_size(const trot_cisd* cisd, int n_walkers, int op);
+size_t trot_cisd_workspace_size_least(const trot_cisd* cisd, int n_walkers, int op);
 /* walkers: complex128 (W, norb, nocc); out complex128 (W).
  * overlap_r_high (trot/trial/cisd.py:148-186). */
 int trot_cisd_overlap(const trot_cisd* cisd, int n_walkers, const double* walkers, double* overlap_out,
@@ -399,6 +405,7 @@ int trot_cisd_prop_step(const trot_cisd* cisd, const trot_system* prop, const tr
  * weights are updated in place; overlaps, scalars and node count are not read.
  * Workspace: trot_fp_workspace_size(sys) bytes. */
 size_t trot_fp_workspace_size(const trot_system* sys);
+size_t trot_fp_workspace_size_least(const trot_system* sys);
 int trot_fp_step(const trot_system* sys, const trot_state* state, const double* fields, const double* zeta_dev,
                  void* workspace, size_t workspace_bytes, void* stream);
 
@@ -464,6 +471,7 @@ int trot_cisd_lci1(int norb, int nchol, int nocc, const double* ci1, const doubl
  * trot_orthonormalize_vjp: g_w = g_q (w^H q)^-1 per spin for q the orthonormalised
  * walkers (everything downstream is invariant under q -> q M). */
 size_t trot_vjp_workspace_size(const trot_system* sys, int op);
+size_t trot_vjp_workspace_size_least(const trot_system* sys, int op);
 int trot_prop_step_vjp(const trot_system* sys, const trot_state* state_in, const double* fields,
                        const double* g_walkers_out_a, const double* g_walkers_out_b, const double* g_weights_out,
                        const double* g_overlaps_out, const double* g_scalars_out, double* g_walkers_in_a,

@@ -86,6 +86,7 @@ _SIGNATURES = {
     "trot_last_error": (ctypes.c_char_p, []),
     "trot_abi_version": (_i, []),
     "trot_workspace_size": (ctypes.c_size_t, [ctypes.POINTER(TrotSystem), _i]),
+    "trot_workspace_size_least": (ctypes.c_size_t, [ctypes.POINTER(TrotSystem), _i]),
     "trot_overlap": (_i, [ctypes.POINTER(TrotSystem), _p, _p, _p, _p]),
     "trot_half_green": (_i, [ctypes.POINTER(TrotSystem), _p, _p, _p, _p, _p]),
     "trot_force_bias": (_i, [ctypes.POINTER(TrotSystem), _p, _p, _p, _p, ctypes.c_size_t, _p]),
@@ -109,6 +110,7 @@ _SIGNATURES = {
     "trot_zgemm_digits_workspace": (ctypes.c_size_t, [_i, _i, _i]),
     "trot_zgemm_digits": (_i, [_i, _i, _i, _d, _p, _i, _p, _i, _i, _p, _i, _i, _p, ctypes.c_size_t, _p]),
     "trot_cisd_workspace_size": (ctypes.c_size_t, [ctypes.POINTER(TrotCisd), _i, _i]),
+    "trot_cisd_workspace_size_least": (ctypes.c_size_t, [ctypes.POINTER(TrotCisd), _i, _i]),
     "trot_cisd_overlap": (_i, [ctypes.POINTER(TrotCisd), _i, _p, _p, _p, ctypes.c_size_t, _p]),
     "trot_cisd_force_bias": (_i, [ctypes.POINTER(TrotCisd), _i, _p, _p, _p, ctypes.c_size_t, _p]),
     "trot_cisd_local_energy": (_i, [ctypes.POINTER(TrotCisd), _i, _p, _p, _p, ctypes.c_size_t, _p]),
@@ -116,6 +118,7 @@ _SIGNATURES = {
     "trot_cisd_prop_step": (_i, [ctypes.POINTER(TrotCisd), ctypes.POINTER(TrotSystem), ctypes.POINTER(TrotState),
                                  _p, _p, _p, ctypes.c_size_t, _p]),
     "trot_fp_workspace_size": (ctypes.c_size_t, [ctypes.POINTER(TrotSystem)]),
+    "trot_fp_workspace_size_least": (ctypes.c_size_t, [ctypes.POINTER(TrotSystem)]),
     "trot_fp_step": (_i, [ctypes.POINTER(TrotSystem), ctypes.POINTER(TrotState), _p, _p, _p, ctypes.c_size_t, _p]),
     "trot_prop_ctx_workspace_size": (ctypes.c_size_t, [_i, _i]),
     "trot_prop_ctx_workspace_size_digits": (ctypes.c_size_t, [_i, _i]),
@@ -123,6 +126,7 @@ _SIGNATURES = {
     "trot_half_rotate": (_i, [_i, _i, _i, _p, _p, _p, _p, _p, _p]),
     "trot_cisd_lci1": (_i, [_i, _i, _i, _p, _p, _p, _p]),
     "trot_vjp_workspace_size": (ctypes.c_size_t, [ctypes.POINTER(TrotSystem), _i]),
+    "trot_vjp_workspace_size_least": (ctypes.c_size_t, [ctypes.POINTER(TrotSystem), _i]),
     "trot_prop_step_vjp": (_i, [ctypes.POINTER(TrotSystem), ctypes.POINTER(TrotState), _p, _p, _p, _p, _p, _p, _p,
                                 _p, _p, _p, _p, _p, _p, ctypes.c_size_t, _p]),
     "trot_local_energy_vjp": (_i, [ctypes.POINTER(TrotSystem), _p, _p, _p, _p, _p, _p, _p, ctypes.c_size_t, _p]),

@@ -133,14 +133,15 @@ def _ptr(t) -> int:
     return 0 if t is None or t.numel() == 0 else t.data_ptr()
 
 
-def _ws(nbytes: int) -> torch.Tensor:
+def _ws(nbytes: int, least: int) -> torch.Tensor:
     if nbytes == 0:
         raise _lib.TrotError(1, _lib.load().trot_last_error().decode())
-    return torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+    return native.empty_or_least(nbytes, least)
 
 
 def _vjp_ws(s, op) -> torch.Tensor:
-    return _ws(_lib.load().trot_vjp_workspace_size(ctypes.byref(s), op))
+    lib = _lib.load()
+    return _ws(lib.trot_vjp_workspace_size(ctypes.byref(s), op), lib.trot_vjp_workspace_size_least(ctypes.byref(s), op))
 
 
 def _empty(like: torch.Tensor) -> torch.Tensor:
@@ -170,7 +171,8 @@ class ExpH1Half(torch.autograd.Function):
         N, G = prob.norb, prob.nchol
         rd = ctx_dev._spin_summed(prob.rdm1)
         gh1 = torch.zeros((N, N), dtype=torch.float64, device=h1.device)
-        ws = _ws(_lib.load().trot_prop_ctx_vjp_workspace_size_digits(N, G))
+        lib = _lib.load()
+        ws = _ws(lib.trot_prop_ctx_vjp_workspace_size_digits(N, G), lib.trot_prop_ctx_vjp_workspace_size(N, G))
         g = g.contiguous()
         _lib.call("trot_prop_ctx_vjp", N, G, float(prob.params.dt), h1.detach().contiguous().data_ptr(),
                   prob.chol.data_ptr(), rd.data_ptr(), g.data_ptr(), gh1.data_ptr(), ws.data_ptr(), ws.numel(),

@@ -877,16 +877,16 @@ using namespace trot;
 
 extern "C" {
 
-size_t trot_vjp_workspace_size(const trot_system* s, int op) {
+static size_t vjp_workspace(const trot_system* s, int op, bool digits) {
   if (check_adj(s) != TROT_OK) return 0;
   const AdjCommon a = common_of(s);
   Carver c(nullptr, 0);
   if (op == TROT_OP_PROP_STEP) {
     StepWs b;
-    carve_step(a, c, b, true);
+    carve_step(a, c, b, digits);
   } else if (op == TROT_OP_LOCAL_ENERGY) {
     EnergyWs b;
-    carve_energy(a, c, b, true);
+    carve_energy(a, c, b, digits);
   } else if (op == TROT_OP_OVERLAP) {
     for (int q = 0; q < a.nspin; ++q) {
       c.take<double2>(a.W * a.nN[q]);
@@ -902,6 +902,8 @@ size_t trot_vjp_workspace_size(const trot_system* s, int op) {
   }
   return c.used + 256;
 }
+size_t trot_vjp_workspace_size(const trot_system* s, int op) { return vjp_workspace(s, op, true); }
+size_t trot_vjp_workspace_size_least(const trot_system* s, int op) { return vjp_workspace(s, op, false); }
 
 int trot_prop_step_vjp(const trot_system* s, const trot_state* in, const double* fields, const double* g_walkers_out_a,
                        const double* g_walkers_out_b, const double* g_weights_out, const double* g_overlaps_out,

@@ -112,13 +112,6 @@ static int carve_ws(const trot_system* s, const Spins& sp, void* ws, size_t ws_b
   return TROT_ERR_WORKSPACE_TOO_SMALL;
 }
 
-size_t fp64_min_workspace(const trot_system* s, int op) {
-  const Spins sp = make_spins(s);
-  Carver c(nullptr, 0);
-  StepBuffers b;
-  return carve_step(s, sp, c, b, op, false) + 256;
-}
-
 static int check_system(const trot_system* s) {
   if (!s) { set_error("null system"); return TROT_ERR_NULL_PTR; }
   if (s->kind < TROT_RHF_R || s->kind > TROT_UHF_U) { set_error("bad kind %d", s->kind); return TROT_ERR_BAD_SHAPE; }
@@ -245,7 +238,7 @@ extern "C" {
 const char* trot_last_error(void) { return g_err; }
 int trot_abi_version(void) { return TROT_ABI_VERSION; }
 
-size_t trot_workspace_size(const trot_system* s, int op) {
+static size_t workspace_size(const trot_system* s, int op, bool digits) {
   if (check_system(s) != TROT_OK) return 0;
   Spins sp = make_spins(s);
   Carver c(nullptr, 0);
@@ -255,9 +248,12 @@ size_t trot_workspace_size(const trot_system* s, int op) {
     if (!s->mixed) return 0;
     return mixed_workspace_size(s, op) + 256;
   }
-  size_t n = carve_step(s, sp, c, b, op, true);
+  size_t n = carve_step(s, sp, c, b, op, digits);
   return n + 256;
 }
+
+size_t trot_workspace_size(const trot_system* s, int op) { return workspace_size(s, op, true); }
+size_t trot_workspace_size_least(const trot_system* s, int op) { return workspace_size(s, op, false); }
 
 int trot_block_rdm1(const trot_system* s, const double* green, const double* weights, const double* obs,
                     double* rdm1_out, void* ws, size_t ws_bytes, void* stream) {

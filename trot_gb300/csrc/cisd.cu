@@ -1100,7 +1100,7 @@ using namespace trot;
 
 extern "C" {
 
-size_t trot_cisd_workspace_size(const trot_cisd* c, int n_walkers, int op) {
+static size_t cisd_workspace(const trot_cisd* c, int n_walkers, int op, bool digits) {
   if (check_cisd(c, n_walkers, false) != TROT_OK) return 0;
   if (op != TROT_OP_OVERLAP && op != TROT_OP_FORCE_BIAS && op != TROT_OP_LOCAL_ENERGY && op != TROT_OP_PROP_STEP) {
     set_error("CISD workspace: unsupported op %d", op);
@@ -1108,7 +1108,11 @@ size_t trot_cisd_workspace_size(const trot_cisd* c, int n_walkers, int op) {
   }
   Carver cv(nullptr, 0);
   CisdBuffers b;
-  return carve_cisd(c, n_walkers, op, cv, b, true) + 256;
+  return carve_cisd(c, n_walkers, op, cv, b, digits) + 256;
+}
+size_t trot_cisd_workspace_size(const trot_cisd* c, int n_walkers, int op) { return cisd_workspace(c, n_walkers, op, true); }
+size_t trot_cisd_workspace_size_least(const trot_cisd* c, int n_walkers, int op) {
+  return cisd_workspace(c, n_walkers, op, false);
 }
 
 int trot_cisd_overlap(const trot_cisd* c, int W, const double* walkers, double* out, void* ws, size_t ws_bytes,

@@ -1066,8 +1066,12 @@ __global__ void __launch_bounds__(256) dg_trotter_tail_kernel(Spins sp, TrotterA
 
 struct DgTrotterPlan {
   int nk16, vtiles, tiles, rpad;  // K16 steps; 128-row tiles of V, 32-row tiles and rows of U per walker
+  int wc;                         // walkers per pass
   size_t rb, bytes;
 };
+// The digits of V are 1.5 times the size of V and more (rows up to a multiple of 128), so they are kept for a pass of
+// walkers only, 1 GB of them (1800 walkers of 120 orbitals: many times what fills the chip).
+static constexpr size_t kDgTrotterCap = size_t(1) << 30;
 static DgTrotterPlan dg_trotter_plan(const Spins& sp, size_t W, size_t N) {
   DgTrotterPlan p{};
   p.nk16 = (int)((N + 15) / 16);
@@ -1076,15 +1080,18 @@ static DgTrotterPlan dg_trotter_plan(const Spins& sp, size_t W, size_t N) {
   p.rpad = p.tiles * kDgP;
   p.rb = kDgRowBytes(p.nk16);
   const size_t erows = (N + 127) / 128 * 128;
-  p.bytes = (W * p.vtiles * 128 + W * p.rpad + erows) * (p.rb + 2) + 2 * W * sp.ntot * N * sizeof(double2) + 10 * 256;
+  const size_t rows = p.vtiles * 128 + p.rpad, each = rows * (p.rb + 2) + 2 * sp.ntot * N * sizeof(double2);
+  const size_t wc = std::max<size_t>(1, std::min<size_t>(W, kDgTrotterCap / each));
+  p.wc = (int)((W + (W + wc - 1) / wc - 1) / ((W + wc - 1) / wc));  // passes of equal size
+  p.bytes = p.wc * each + erows * (p.rb + 2) + 10 * 256;
   return p;
 }
 
 size_t trotter_dg_bytes(const Spins& sp, size_t W, size_t N) { return dg_trotter_plan(sp, W, N).bytes; }
 
 int launch_trotter_dg(const Spins& sp, const TrotterArgs& t, const DgScratch& s, cudaStream_t st) {
-  const int W = t.W, N = t.N, nc = sp.ntot;
-  const DgTrotterPlan pl = dg_trotter_plan(sp, W, N);
+  const int N = t.N, nc = sp.ntot;
+  const DgTrotterPlan pl = dg_trotter_plan(sp, t.W, N);
   if (s.bytes < pl.bytes) { set_error("trotter: scratch %zu < %zu", s.bytes, pl.bytes); return TROT_ERR_WORKSPACE_TOO_SMALL; }
   char* p = reinterpret_cast<char*>(((uintptr_t)s.p + 255) & ~(uintptr_t)255);
   auto take = [&](size_t n) {
@@ -1092,60 +1099,78 @@ int launch_trotter_dg(const Spins& sp, const TrotterArgs& t, const DgScratch& s,
     p += (n + 255) & ~(size_t)255;
     return r;
   };
-  const size_t vrows = (size_t)W * pl.vtiles * 128, urows = (size_t)W * pl.rpad, erows = (size_t)(N + 127) / 128 * 128;
+  const size_t vrows = (size_t)pl.wc * pl.vtiles * 128, urows = (size_t)pl.wc * pl.rpad, erows = (size_t)(N + 127) / 128 * 128;
   uint16_t* vimg = reinterpret_cast<uint16_t*>(take(vrows * pl.rb));
   uint16_t* uimg = reinterpret_cast<uint16_t*>(take(urows * pl.rb));
   uint16_t* eimg = reinterpret_cast<uint16_t*>(take(erows * pl.rb));
   int16_t* vex = reinterpret_cast<int16_t*>(take(vrows * 2));
   int16_t* uex = reinterpret_cast<int16_t*>(take(urows * 2));
   int16_t* eex = reinterpret_cast<int16_t*>(take(erows * 2));
-  double2* U = reinterpret_cast<double2*>(take((size_t)W * nc * N * sizeof(double2)));
-  double2* O = reinterpret_cast<double2*>(take((size_t)W * nc * N * sizeof(double2)));
-  // digits of V (walker, 2 p + c), of E and of the walkers (walker, 2 j + c; K along the orbitals)
-  DgSrc sv = dg_src(reinterpret_cast<const double*>(t.vhs), 1, 2 * N, N, 128, 2ll * N, 2, vimg, vex);
-  sv.rpad = pl.vtiles * 128;
-  sv.nblk = W;
-  sv.bstride = 2ll * N * N;
-  DgRows rows{};
-  if (t.nterms > 0) dg_rows_add(rows, sv, W * pl.vtiles * 16);
-  dg_rows_add(rows, dg_src(t.expH, 0, N, N, 128, N, 1, eimg, eex), (int)erows / 8);
-  DgSrc sw = dg_src(reinterpret_cast<const double*>(t.in_a), 1, 2 * nc, N, kDgP, 2, 2ll * sp.n[0], uimg, uex);
-  sw.rpad = pl.rpad;
-  sw.nblk = W;
-  sw.bstride = 2ll * N * sp.n[0];
-  if (sp.nspin == 2) {
-    sw.split = 2 * sp.n[0];
-    sw.p2 = reinterpret_cast<const double*>(t.in_b);
-    sw.bstride2 = 2ll * N * sp.n[1];
-    sw.kst2 = 2ll * sp.n[1];
-  }
-  dg_rows_add(rows, sw, W * pl.tiles * 4);
-  TROT_TRY(dg_rows_launch(rows, st));
-  DgArgs e{};  // E x
-  e.imgB = eimg; e.exB = eex; e.imgA = uimg; e.exA = uex;
-  e.Nn = N; e.M = nc; e.nrt = (N + 127) / 128; e.ntile = pl.tiles; e.nk16 = pl.nk16; e.shift = 1;
-  e.nbatch = W; e.bB = 0; e.cstride = (long long)nc * N;
-  e.C = U; e.ldc = N; e.salpha = 1; e.status = s.status;
-  DgArgs v = e;  // V x
-  v.imgB = vimg; v.exB = vex; v.Nn = 2 * N; v.nrt = v.bB = pl.vtiles;
-  TROT_TRY(dg_gemm<false>(e, st));
-  DgTaylor ty{W, N, nc, pl.rpad, 0, t.nterms == 0, 1.0, (const double*)U, (double*)O, uimg, uex};
-  for (int k = 0;; ++k) {
-    ty.k = k;
-    ty.last = k == t.nterms;
-    dg_taylor_kernel<<<W * pl.tiles * 4, dg_row_threads(pl.nk16), 0, st>>>(ty);
-    TROT_CHECK_LAUNCH("dg_taylor_kernel");
-    if (k == t.nterms) break;
-    TROT_TRY(dg_gemm<true>(v, st));
-    ty.coef *= t.sqrt_dt / (double)(k + 1);
-  }
-  TROT_TRY(dg_gemm<false>(e, st));
+  double2* U = reinterpret_cast<double2*>(take((size_t)pl.wc * nc * N * sizeof(double2)));
+  double2* O = reinterpret_cast<double2*>(take((size_t)pl.wc * nc * N * sizeof(double2)));
   const int nmax = std::max(sp.n[0], sp.nspin == 2 ? sp.n[1] : 0);
   const size_t smem = (size_t)(N * nc + nmax * nmax) * sizeof(double2);
-  if (smem > 40 * 1024)
-    cudaFuncSetAttribute(dg_trotter_tail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  dg_trotter_tail_kernel<<<W, 256, smem, st>>>(sp, t, U);
-  TROT_CHECK_LAUNCH("dg_trotter_tail_kernel");
+  for (int w0 = 0; w0 < t.W; w0 += pl.wc) {
+    const int W = std::min(pl.wc, t.W - w0);
+    TrotterArgs a = t;  // of this pass
+    a.W = W;
+    a.vhs += (size_t)w0 * N * N;
+    for (int q = 0; q < sp.nspin; ++q) {
+      const size_t off = (size_t)w0 * N * sp.n[q];
+      (q ? a.in_b : a.in_a) += off;
+      (q ? a.out_b : a.out_a) += off;
+    }
+    if (a.overlaps) {
+      a.overlaps += w0;
+      a.weights += w0;
+      a.shift_term += w0;
+      a.fb_term += w0;
+      a.node_flag += w0;
+    }
+    // digits of V (walker, 2 p + c), of E and of the walkers (walker, 2 j + c; K along the orbitals)
+    DgSrc sv = dg_src(reinterpret_cast<const double*>(a.vhs), 1, 2 * N, N, 128, 2ll * N, 2, vimg, vex);
+    sv.rpad = pl.vtiles * 128;
+    sv.nblk = W;
+    sv.bstride = 2ll * N * N;
+    DgRows rows{};
+    if (t.nterms > 0) dg_rows_add(rows, sv, W * pl.vtiles * 16);
+    if (w0 == 0) dg_rows_add(rows, dg_src(t.expH, 0, N, N, 128, N, 1, eimg, eex), (int)erows / 8);
+    DgSrc sw = dg_src(reinterpret_cast<const double*>(a.in_a), 1, 2 * nc, N, kDgP, 2, 2ll * sp.n[0], uimg, uex);
+    sw.rpad = pl.rpad;
+    sw.nblk = W;
+    sw.bstride = 2ll * N * sp.n[0];
+    if (sp.nspin == 2) {
+      sw.split = 2 * sp.n[0];
+      sw.p2 = reinterpret_cast<const double*>(a.in_b);
+      sw.bstride2 = 2ll * N * sp.n[1];
+      sw.kst2 = 2ll * sp.n[1];
+    }
+    dg_rows_add(rows, sw, W * pl.tiles * 4);
+    TROT_TRY(dg_rows_launch(rows, st));
+    DgArgs e{};  // E x
+    e.imgB = eimg; e.exB = eex; e.imgA = uimg; e.exA = uex;
+    e.Nn = N; e.M = nc; e.nrt = (N + 127) / 128; e.ntile = pl.tiles; e.nk16 = pl.nk16; e.shift = 1;
+    e.nbatch = W; e.bB = 0; e.cstride = (long long)nc * N;
+    e.C = U; e.ldc = N; e.salpha = 1; e.status = s.status;
+    DgArgs v = e;  // V x
+    v.imgB = vimg; v.exB = vex; v.Nn = 2 * N; v.nrt = v.bB = pl.vtiles;
+    TROT_TRY(dg_gemm<false>(e, st));
+    DgTaylor ty{W, N, nc, pl.rpad, 0, t.nterms == 0, 1.0, (const double*)U, (double*)O, uimg, uex};
+    for (int k = 0;; ++k) {
+      ty.k = k;
+      ty.last = k == t.nterms;
+      dg_taylor_kernel<<<W * pl.tiles * 4, dg_row_threads(pl.nk16), 0, st>>>(ty);
+      TROT_CHECK_LAUNCH("dg_taylor_kernel");
+      if (k == t.nterms) break;
+      TROT_TRY(dg_gemm<true>(v, st));
+      ty.coef *= t.sqrt_dt / (double)(k + 1);
+    }
+    TROT_TRY(dg_gemm<false>(e, st));
+    if (smem > 40 * 1024)
+      cudaFuncSetAttribute(dg_trotter_tail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    dg_trotter_tail_kernel<<<W, 256, smem, st>>>(sp, a, U);
+    TROT_CHECK_LAUNCH("dg_trotter_tail_kernel");
+  }
   return TROT_OK;
 }
 

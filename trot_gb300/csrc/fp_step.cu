@@ -71,8 +71,17 @@ static size_t carve_fp(const trot_system* s, const Spins& sp, Carver& c, FpBuffe
   return c.used;
 }
 
-static size_t trotter_bytes(const trot_system* s) {
-  return (trot_workspace_size(s, TROT_OP_APPLY_TROTTER) + 255) & ~(size_t)255;
+static size_t trotter_bytes(const trot_system* s, bool digits) {
+  return ((digits ? trot_workspace_size(s, TROT_OP_APPLY_TROTTER) : trot_workspace_size_least(s, TROT_OP_APPLY_TROTTER)) +
+          255) & ~(size_t)255;
+}
+static size_t fp_workspace(const trot_system* s, bool digits) {
+  const size_t tb = trotter_bytes(s, digits);
+  if (tb == 0) return 0;
+  Spins sp = make_spins(s);
+  Carver c(nullptr, 0);
+  FpBuffers f;
+  return tb + carve_fp(s, sp, c, f) + 256;
 }
 
 }  // namespace trot
@@ -81,14 +90,8 @@ using namespace trot;
 
 extern "C" {
 
-size_t trot_fp_workspace_size(const trot_system* s) {
-  const size_t tb = trotter_bytes(s);
-  if (tb == 0) return 0;
-  Spins sp = make_spins(s);
-  Carver c(nullptr, 0);
-  FpBuffers f;
-  return tb + carve_fp(s, sp, c, f) + 256;
-}
+size_t trot_fp_workspace_size(const trot_system* s) { return fp_workspace(s, true); }
+size_t trot_fp_workspace_size_least(const trot_system* s) { return fp_workspace(s, false); }
 
 int trot_fp_step(const trot_system* s, const trot_state* state, const double* fields, const double* zeta_dev,
                  void* ws, size_t ws_bytes, void* stream) {
@@ -98,10 +101,10 @@ int trot_fp_step(const trot_system* s, const trot_state* state, const double* fi
     return TROT_ERR_NULL_PTR;
   }
   if (!s->mf_shifts_im) { set_error("null propagation context"); return TROT_ERR_NULL_PTR; }
-  size_t tb = trotter_bytes(s);
+  size_t tb = trotter_bytes(s, true);
   if (tb == 0) return TROT_ERR_BAD_SHAPE;  // trot_workspace_size recorded the reason
   if (s->precision == TROT_FP64 && ws_bytes < trot_fp_workspace_size(s))  // too small for the digit products' scratch
-    tb = (fp64_min_workspace(s, TROT_OP_APPLY_TROTTER) + 255) & ~(size_t)255;
+    tb = trotter_bytes(s, false);
   if (ws_bytes < tb) { set_error("workspace too small: %zu < %zu", ws_bytes, tb); return TROT_ERR_WORKSPACE_TOO_SMALL; }
   Spins sp = make_spins(s);
   Carver c(ws ? static_cast<char*>(ws) + tb : nullptr, ws_bytes - tb);

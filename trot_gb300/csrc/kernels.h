@@ -47,8 +47,6 @@ struct StepBuffers {
 
 Spins make_spins(const trot_system* s);
 int tune_get(int knob);  // tune.cu: 0 = default
-// bytes with which an FP64 op runs at all: its workspace without the digit products' scratch
-size_t fp64_min_workspace(const trot_system* s, int op);
 
 // Green's function / overlap per walker (green.cu).
 // green: complex (W, ntot*N) half Green's functions, spin blocks concatenated

@@ -92,7 +92,7 @@ extern "C" int trot_local_energy_noalloc(const trot_system* sys, const double* w
   if (need == 0) return trot_local_energy(sys, walkers_a, walkers_b, energy_out, nullptr, 0, stream);
   // an FP64 system whose digit products do not fit runs without them
   if (need > kNoAllocScratchBytes && sys->precision == TROT_FP64)
-    need = fp64_min_workspace(sys, TROT_OP_LOCAL_ENERGY);
+    need = trot_workspace_size_least(sys, TROT_OP_LOCAL_ENERGY);
   if (need > kNoAllocScratchBytes) {
     set_error("trot_local_energy_noalloc: this system needs %zu bytes of scratch but the built-in scratch "
               "array holds %zu bytes; call trot_local_energy with a caller workspace",

@@ -56,7 +56,8 @@ def prop_ctx(h0: float, h1, chol, rdm1, dt: float):
     nbytes = lib.trot_prop_ctx_workspace_size_digits(N, G)
     if nbytes == 0:
         _lib.check(1)  # TROT_ERR_BAD_SHAPE, message from the library
-    ws = torch.empty(nbytes, dtype=torch.uint8, device=chol.device)
+    ws = native.empty_or_least(nbytes, lib.trot_prop_ctx_workspace_size(N, G))
+    nbytes = ws.numel()
     mf_im = torch.empty(G, dtype=torch.float64, device=chol.device)
     h0p = torch.empty(1, dtype=torch.float64, device=chol.device)
     eh = torch.empty((N, N), dtype=torch.float64, device=chol.device)

@@ -9,6 +9,7 @@ import torch
 from . import _lib
 
 _workspaces: dict = {}
+_refused: dict = {}  # (device, stream): bytes that did not fit beside the rest of the program
 
 
 def stream_ptr() -> int:
@@ -19,21 +20,55 @@ def ptr(t) -> int:
     return 0 if t is None else t.data_ptr()
 
 
-def workspace(nbytes: int) -> torch.Tensor:
+def empty_or_least(nbytes: int, least: int) -> torch.Tensor:
+    """A new uint8 device buffer of ``nbytes``, or of ``least`` where that much memory is not there."""
+    try:
+        return torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+    except torch.cuda.OutOfMemoryError:
+        if least >= nbytes:
+            raise
+    return torch.empty(least, dtype=torch.uint8, device="cuda")
+
+
+def _fits(nbytes: int) -> bool:
+    dev = torch.cuda.current_device()
+    free = torch.cuda.mem_get_info(dev)[0]
+    return nbytes <= free + torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
+
+
+def workspace(nbytes: int, least: int | None = None) -> torch.Tensor:
     """A cached uint8 device buffer of at least ``nbytes``, one per (device,
     stream): calls on one stream are ordered and may share it, calls running
     concurrently on different streams (fragment batches) get their own.  The
     256-byte status block at the start of a new buffer is zero-filled, so its
     sticky timeout word starts clear (a buffer replaced by a larger one starts
-    a new record)."""
+    a new record).  Where ``nbytes`` are not free, ``least`` bytes (the
+    library's ``*_size_least``) do, until they are."""
     dev = torch.cuda.current_device()
     key = (dev, torch.cuda.current_stream().cuda_stream)
     buf = _workspaces.get(key)
-    if buf is None or buf.numel() < nbytes:
-        buf = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=f"cuda:{dev}")
-        buf[:256].zero_()
-        _workspaces[key] = buf
-    return buf
+    if buf is not None:
+        if buf.numel() >= nbytes:
+            return buf
+        if least is not None and least <= buf.numel() and nbytes >= _refused.get(key, nbytes + 1) and not _fits(nbytes):
+            return buf
+    if least is None:
+        least = nbytes
+    try:
+        new = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=f"cuda:{dev}")
+        _refused.pop(key, None)
+    except torch.cuda.OutOfMemoryError:
+        if least >= nbytes:
+            raise
+        _refused[key] = min(nbytes, _refused.get(key, nbytes))
+        if buf is not None and buf.numel() >= least:
+            return buf
+        _workspaces.pop(key, None)
+        buf = None  # the smaller buffer's memory may be part of what is missing
+        new = torch.empty(max(least, 256), dtype=torch.uint8, device=f"cuda:{dev}")
+    new[:256].zero_()
+    _workspaces[key] = new
+    return new
 
 
 def capturing() -> bool:
@@ -150,5 +185,5 @@ def ws_for(s: _lib.TrotSystem, op: int) -> tuple[int, int]:
     n = _lib.load().trot_workspace_size(ctypes.byref(s), op)
     if n == 0:
         raise _lib.TrotError(1, _lib.load().trot_last_error().decode())
-    buf = workspace(n)
+    buf = workspace(n, _lib.load().trot_workspace_size_least(ctypes.byref(s), op))
     return buf.data_ptr(), buf.numel()

@@ -95,6 +95,12 @@ def _system(kind, walkers_a, mo_a, mo_b, *, rot_h1=(None, None), rot_chol=(None,
     return s
 
 
+def _vjp_workspace(s, op):
+    lib = _lib.load()
+    return native.workspace(lib.trot_vjp_workspace_size(ctypes.byref(s), op),
+                            lib.trot_vjp_workspace_size_least(ctypes.byref(s), op))
+
+
 # ---------------------------------------------------------------- overlap
 
 
@@ -124,8 +130,7 @@ def _overlap_backward(ctx, g):
     wa, wb, mo_a, mo_b = ctx.saved_tensors
     s = _system(ctx.kind, wa, mo_a, mo_b)
     ga, gb = torch.zeros_like(wa), torch.zeros_like(wb)
-    nbytes = _lib.load().trot_vjp_workspace_size(ctypes.byref(s), _lib.OP_OVERLAP)
-    ws = native.workspace(nbytes)
+    ws = _vjp_workspace(s, _lib.OP_OVERLAP)
     _lib.call("trot_overlap_vjp", ctypes.byref(s), wa.data_ptr(), _ptr(wb), g.contiguous().data_ptr(), ga.data_ptr(),
               _ptr(gb), ws.data_ptr(), ws.numel(), native.stream_ptr())
     return ga, gb, None, None, None
@@ -194,8 +199,7 @@ def _energy_backward(ctx, g):
     ga, gb = torch.zeros_like(wa), torch.zeros_like(wb)
     N = int(mo_a.shape[0])
     gh1 = torch.zeros((N, N), dtype=torch.float64, device=wa.device)  # through rot_h1 = C^T h1: not returned
-    nbytes = _lib.load().trot_vjp_workspace_size(ctypes.byref(s), _lib.OP_LOCAL_ENERGY)
-    ws = native.workspace(nbytes)
+    ws = _vjp_workspace(s, _lib.OP_LOCAL_ENERGY)
     _lib.call("trot_local_energy_vjp", ctypes.byref(s), wa.data_ptr(), _ptr(wb), gre.data_ptr(), ga.data_ptr(),
               _ptr(gb), gh1.data_ptr(), ws.data_ptr(), ws.numel(), native.stream_ptr())
     return ga, gb, None, None, None, None, None, None, None, None, None
@@ -368,7 +372,7 @@ def _step_backward(ctx, gwa, gwb, gwt, gov, gsc):
     gwa_in, gwb_in = torch.empty_like(wa), torch.empty_like(wb)
     gwt_in, gov_in, gsc_in = torch.empty_like(wt), torch.empty_like(ov), torch.empty_like(scal)
     geh = torch.zeros_like(eh)
-    ws = native.workspace(_lib.load().trot_vjp_workspace_size(ctypes.byref(s), _lib.OP_PROP_STEP))
+    ws = _vjp_workspace(s, _lib.OP_PROP_STEP)
     _lib.call("trot_prop_step_vjp", ctypes.byref(s), ctypes.byref(st), x.contiguous().data_ptr(), gwa.data_ptr(),
               _ptr(gwb), native.ptr(gwt), native.ptr(gov), gsc.data_ptr(), gwa_in.data_ptr(), _ptr(gwb_in),
               gwt_in.data_ptr(), gov_in.data_ptr(), gsc_in.data_ptr(), geh.data_ptr(), ws.data_ptr(), ws.numel(),

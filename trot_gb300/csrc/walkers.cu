@@ -67,9 +67,11 @@ __device__ double qr_gram_schmidt(int N, int n, int ld, double2* Q, double2* coe
   return prod;
 }
 
-// Cholesky S = R^H R of the Hermitian n x n S (its upper triangle is read) and X = R^-1 (upper) by one warp; rdiag[j] =
-// R_jj.  Returns false (in every lane) where a pivot is not above 1e-4 S_jj.
-__device__ bool warp_cholesky_inverse(double2* S, double2* X, int n, double* rdiag) {
+// Cholesky S = R^H R of the Hermitian n x n S (its upper triangle is read) and X = R^-1 (upper) by one warp; rdiag[j] (1 +
+// rcorr[j].x) = 1 / X_jj, the R_jj that belongs to v X (d rsqrt(d) alone is off by twice the error of rsqrt(d), which the
+// norm's product collects over the columns: 1.07e-15 RMS at n = 12).  Returns false (in every lane) where a pivot is not
+// above 1e-4 S_jj.
+__device__ bool warp_cholesky_inverse(double2* S, double2* X, int n, double* rdiag, double2* rcorr) {
   const int lane = threadIdx.x & 31;
   bool ok = true;
   for (int k = 0; k < n; ++k) {
@@ -79,8 +81,10 @@ __device__ bool warp_cholesky_inverse(double2* S, double2* X, int n, double* rdi
       const double d = S[k * n + k].x;
       ok = d > 1e-4 * rdiag[k];  // rdiag[k] holds S_kk until the pivot is known
       rk = rsqrt(d);
-      rdiag[k] = d * rk;
-      S[k * n + k] = cmk(d * rk, 0.0);
+      const double r = d * rk;
+      S[k * n + k] = cmk(r, 0.0);
+      rdiag[k] = r;
+      rcorr[k].x = fma(-r, rk, 1.0);
     }
     ok = __shfl_sync(0xffffffffu, ok, 0);
     if (!ok) return false;
@@ -198,7 +202,7 @@ qr_kernel(Spins sp, int N, double2* __restrict__ wa, double2* __restrict__ wb, d
       }
       __syncthreads();
       if (tid < 32) {
-        const bool ok = warp_cholesky_inverse(S, X, n, rdiag);
+        const bool ok = warp_cholesky_inverse(S, X, n, rdiag, coef);
         if (tid == 0 && !ok) bad = 1;
       }
       __syncthreads();
@@ -227,6 +231,7 @@ qr_kernel(Spins sp, int N, double2* __restrict__ wa, double2* __restrict__ wb, d
         int i = 0, j = 0;
         if (e < np) {
           qr_pair(e, n, i, j);
+          if (i == j) acc.x = -0.125;  // the eight lanes' shares of - I: the sums end near 0 and round little
           for (int p = opart; p < N; p += 8) {
             const double2 x = Q[p * ld + i];
             cfma(acc, cmk(x.x, -x.y), Q[p * ld + j]);
@@ -239,7 +244,7 @@ qr_kernel(Spins sp, int N, double2* __restrict__ wa, double2* __restrict__ wb, d
         }
         if (e < np && opart == 0) {
           if (i == j) {
-            acc = cmk(0.5 * (acc.x - 1.0), 0.0);
+            acc = cmk(0.5 * acc.x, 0.0);
             X[i * n + i] = acc;
           }
           const float2 xf = make_float2(qr_f32(acc.x), qr_f32(acc.y));
@@ -267,7 +272,7 @@ qr_kernel(Spins sp, int N, double2* __restrict__ wa, double2* __restrict__ wb, d
         }
       }
       if (tid == 0)
-        for (int j = 0; j < n; ++j) prod *= ldexp(rdiag[j] * (1.0 + X[j * n + j].x), cexp[j] - 1023);
+        for (int j = 0; j < n; ++j) prod *= ldexp(fma(rdiag[j], X[j * n + j].x + coef[j].x, rdiag[j]), cexp[j] - 1023);
       __syncthreads();
     } else {
       __syncthreads();

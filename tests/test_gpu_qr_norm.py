@@ -44,3 +44,15 @@ def test_norm_roundings(N, n, W):
     rms = np.sqrt(np.mean(err ** 2))
     print(f"N={N} n={n}: rms {rms:.2e}, mean {err.mean():.2e}, bound {2 * np.sqrt(n) * 2.0 ** -53:.2e}")
     assert rms <= 2 * np.sqrt(n) * 2.0 ** -53 * (1 + 4 / np.sqrt(2 * W))
+
+
+@pytest.mark.parametrize("N,n", [(31, 30), (128, 7), (129, 7), (160, 9), (161, 2), (256, 5), (257, 33)])
+def test_gram_schmidt_rows(N, n):
+    """Walkers that only Gram-Schmidt orthogonalises, at the edges of the block sizes, beside one that it does not."""
+    from tests.test_gpu_qr import check
+
+    rng = np.random.default_rng(N + n)
+    w = rng.standard_normal((3, N, n)) + 1j * rng.standard_normal((3, N, n))
+    w[0, :, n - 1] = (1 - 2j) * w[0, :, 0] + 1e-5 * w[0, :, n - 1]
+    w[2, :, 1] = w[2, :, 0] + 1e-3 * w[2, :, 1]
+    check(w)

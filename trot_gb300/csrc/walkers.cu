@@ -1,4 +1,6 @@
 // Walker QR orthonormalisation and stochastic reconfiguration (FP64).
+#include <algorithm>
+
 #include "ff.cuh"
 #include "kernels.h"
 
@@ -27,30 +29,38 @@ TROT_D double qr_scale(double x, int k) {
 // A walker whose columns are too close to dependent for step 1 (a pivot below 1e-4 of its column, E above 2e-10) or not
 // finite takes twice-iterated classical Gram-Schmidt, as do all where the two n x n matrices do not fit beside the walker
 // (gs_only).
-static constexpr int kQrThreads = 128;
+// A thread per row, 128 at least (fewer rows leave the dot products and pairs to more warps) and 256 at most: 135 rows on 128
+// threads were two rounds of every column.
+static int qr_threads(int N) { return std::min(256, std::max(128, (N + 31) / 32 * 32)); }
 
-// twice-iterated classical Gram-Schmidt in shared memory (row stride ld); returns prod ||v||
-__device__ double qr_gram_schmidt(int N, int n, int ld, double2* Q, double2* coef, double2* red) {
+// Twice-iterated classical Gram-Schmidt in shared memory (row stride ld); returns prod ||v||.  Bound by its FP64
+// instructions and the waits between them: four fused multiply-adds per complex product and five additions per dot product
+// (six and ten before) pay for the first pass of a walker that ends here: condition 1e6, 1024 walkers of 120 x (12 + 10) 1290
+// -> 875 us, of 160 x (24 + 24) 6958 -> 4239.  Out of line, so that its registers are not the fast route's.
+static __device__ __noinline__ double qr_gram_schmidt(int N, int n, int ld, double2* Q, double2* coef, double2* red) {
   const int tid = threadIdx.x, nt = blockDim.x;
   const int lane = tid & 31, wid = tid >> 5, nw = nt >> 5;
   double prod = 1.0;
   for (int j = 0; j < n; ++j) {
     for (int pass = 0; pass < 2; ++pass) {
-      // coef[i] = <Q_i, v> for i < j  (one warp per i)
+      // coef[i] = -<Q_i, v> for i < j  (one warp per i)
       for (int i = wid; i < j; i += nw) {
         double2 acc = cmk(0.0, 0.0);
         for (int p = lane; p < N; p += 32) {
           const double2 q = Q[p * ld + i], v = Q[p * ld + j];
-          acc.x += q.x * v.x + q.y * v.y;
-          acc.y += q.x * v.y - q.y * v.x;
+          cfma(acc, cmk(q.x, -q.y), v);
         }
-        acc = warp_sum2(acc);
-        if (lane == 0) coef[i] = acc;
+        // a half warp per component after the first exchange
+        const bool im = lane & 16;
+        double a = (im ? acc.y : acc.x) + __shfl_xor_sync(0xffffffffu, im ? acc.x : acc.y, 16);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        if ((lane & 15) == 0) (im ? coef[i].y : coef[i].x) = -a;
       }
       __syncthreads();
       for (int p = tid; p < N; p += nt) {
         double2 v = Q[p * ld + j];
-        for (int i = 0; i < j; ++i) v = csub(v, cmul(Q[p * ld + i], coef[i]));
+        for (int i = 0; i < j; ++i) cfma(v, Q[p * ld + i], coef[i]);
         Q[p * ld + j] = v;
       }
       __syncthreads();
@@ -134,7 +144,7 @@ TROT_D void qr_pair(int e, int n, int& i, int& j) {
   j = i + e;
 }
 
-__global__ void __launch_bounds__(kQrThreads)
+__global__ void __launch_bounds__(256)
 qr_kernel(Spins sp, int N, double2* __restrict__ wa, double2* __restrict__ wb, double2* __restrict__ norm, int write_q,
           int gs_only) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -303,7 +313,7 @@ int launch_qr(const Spins& sp, int W, int N, double2* wa, double2* wb, double2* 
   const bool gs_only = smem > 220 * 1024;
   if (gs_only) smem = (size_t)N * nmax * sizeof(double2);
   if (smem > 40 * 1024) cudaFuncSetAttribute(qr_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  qr_kernel<<<W, kQrThreads, smem, st>>>(sp, N, wa, wb, norm_out, write_q ? 1 : 0, gs_only ? 1 : 0);
+  qr_kernel<<<W, qr_threads(N), smem, st>>>(sp, N, wa, wb, norm_out, write_q ? 1 : 0, gs_only ? 1 : 0);
   TROT_CHECK_LAUNCH("qr_kernel");
   return TROT_OK;
 }

@@ -183,7 +183,7 @@ def _workspace(c: _lib.TrotCisd, W: int, op: int) -> tuple[int, int]:
     n = _lib.load().trot_cisd_workspace_size(ctypes.byref(c), W, op)
     if n == 0:
         raise _lib.TrotError(1, _lib.load().trot_last_error().decode())
-    buf = native.workspace(n, _lib.load().trot_cisd_workspace_size_least(ctypes.byref(c), W, op))
+    buf = native.workspace(n, lambda: _lib.load().trot_cisd_workspace_size_least(ctypes.byref(c), W, op))
     return buf.data_ptr(), buf.numel()
 
 
@@ -328,8 +328,8 @@ def afqmc_step(state: PropState, *, params, ham_data, trial_data: CisdTrial, mea
     n = _lib.load().trot_cisd_workspace_size(ctypes.byref(c), W, _lib.OP_PROP_STEP)
     if n == 0:
         raise _lib.TrotError(1, _lib.load().trot_last_error().decode())
-    least = _lib.load().trot_cisd_workspace_size_least(ctypes.byref(c), W, _lib.OP_PROP_STEP)
-    buf = native.workspace(n + 256 + extra, least + 256 + extra)
+    buf = native.workspace(n + 256 + extra, lambda: 256 + extra + _lib.load().trot_cisd_workspace_size_least(
+        ctypes.byref(c), W, _lib.OP_PROP_STEP))
     ws, nws = buf.data_ptr(), buf.numel()
     _lib.call("trot_cisd_prop_step", ctypes.byref(c), ctypes.byref(s), ctypes.byref(st), fields.data_ptr(),
               native.ptr(energy_out), ws, nws, native.stream_ptr())

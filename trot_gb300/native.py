@@ -36,24 +36,22 @@ def _fits(nbytes: int) -> bool:
     return nbytes <= free + torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
 
 
-def workspace(nbytes: int, least: int | None = None) -> torch.Tensor:
+def workspace(nbytes: int, least=None) -> torch.Tensor:
     """A cached uint8 device buffer of at least ``nbytes``, one per (device,
     stream): calls on one stream are ordered and may share it, calls running
     concurrently on different streams (fragment batches) get their own.  The
     256-byte status block at the start of a new buffer is zero-filled, so its
     sticky timeout word starts clear (a buffer replaced by a larger one starts
-    a new record).  Where ``nbytes`` are not free, ``least`` bytes (the
+    a new record).  Where ``nbytes`` are not free, ``least()`` bytes (the
     library's ``*_size_least``) do, until they are."""
     dev = torch.cuda.current_device()
     key = (dev, torch.cuda.current_stream().cuda_stream)
     buf = _workspaces.get(key)
-    if buf is not None:
-        if buf.numel() >= nbytes:
-            return buf
-        if least is not None and least <= buf.numel() and nbytes >= _refused.get(key, nbytes + 1) and not _fits(nbytes):
-            return buf
-    if least is None:
-        least = nbytes
+    if buf is not None and buf.numel() >= nbytes:
+        return buf
+    least = nbytes if least is None else least()
+    if buf is not None and least <= buf.numel() and nbytes >= _refused.get(key, nbytes + 1) and not _fits(nbytes):
+        return buf
     try:
         new = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=f"cuda:{dev}")
         _refused.pop(key, None)
@@ -185,5 +183,5 @@ def ws_for(s: _lib.TrotSystem, op: int) -> tuple[int, int]:
     n = _lib.load().trot_workspace_size(ctypes.byref(s), op)
     if n == 0:
         raise _lib.TrotError(1, _lib.load().trot_last_error().decode())
-    buf = workspace(n, _lib.load().trot_workspace_size_least(ctypes.byref(s), op))
+    buf = workspace(n, lambda: _lib.load().trot_workspace_size_least(ctypes.byref(s), op))
     return buf.data_ptr(), buf.numel()

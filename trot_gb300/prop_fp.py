@@ -48,7 +48,7 @@ def afqmc_step_fp(state: PropState, sys: System, *, params, ham_data, trial_data
     n = _lib.load().trot_fp_workspace_size(ctypes.byref(s))
     if n == 0:
         raise _lib.TrotError(1, _lib.load().trot_last_error().decode())
-    buf = native.workspace(n, _lib.load().trot_fp_workspace_size_least(ctypes.byref(s)))
+    buf = native.workspace(n, lambda: _lib.load().trot_fp_workspace_size_least(ctypes.byref(s)))
     _lib.call("trot_fp_step", ctypes.byref(s), ctypes.byref(st), fields.data_ptr(), zeta.data_ptr(),
               buf.data_ptr(), buf.numel(), native.stream_ptr())
     return state

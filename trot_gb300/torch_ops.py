@@ -98,7 +98,7 @@ def _system(kind, walkers_a, mo_a, mo_b, *, rot_h1=(None, None), rot_chol=(None,
 def _vjp_workspace(s, op):
     lib = _lib.load()
     return native.workspace(lib.trot_vjp_workspace_size(ctypes.byref(s), op),
-                            lib.trot_vjp_workspace_size_least(ctypes.byref(s), op))
+                            lambda: lib.trot_vjp_workspace_size_least(ctypes.byref(s), op))
 
 
 # ---------------------------------------------------------------- overlap

@@ -13,10 +13,16 @@
 //    and less, where the last bit does not matter;
 //  * after each slab the seven sums are added into one 64-bit integer per output, which is converted to FP64 once.
 //
-// Error against a long-double product, on the force bias, exchange, VHS and CISD operands of systems of 24 to 135
-// orbitals (K = 24 ... 2160): 1.0e-16 ... 6.1e-16 of the result, against 1.7e-16 ... 1.5e-15 for an FP64 sum over k
-// (0.2 to 0.86 of it; five digits, or orders d <= 5 only, are worse than FP64 where one element dominates its
-// row).  The result does not depend on the tiling or on the other rows.
+// The slices are those of the error-free transformation of Ozaki, Ogita, Oishi and Rump (Numer. Algorithms 59, 2012), with
+// digits of fixed width instead of rounded remainders.
+//
+// The error is relative to the maxima of the two rows, about 2^-54 of their product per term, not to the terms as in an
+// FP64 sum: rows whose large elements meet zeros or small elements of the other operand lose what the FP64 sum keeps (a
+// factor of 10^s against 10^-s, K = 120: 2.4e-15 of the result at s = 2, 2.3e-11 at s = 6).  The operands here have
+// no such rows but for the step adjoint's, which are balanced first (adjoint_dg_gv).  On the force bias, exchange, VHS and
+// CISD operands of systems of 24 to 135 orbitals (K = 24 ... 2160), against a long-double product: 1.0e-16 ... 6.1e-16 of
+// the result, an FP64 sum over k 1.7e-16 ... 1.5e-15 (0.2 to 0.86 of it; five digits, or orders d <= 5 only, are worse
+// than FP64 where one element dominates its row).  The result does not depend on the tiling or on the other rows.
 //
 // Rate (1024 x 7260, K = 600, the VHS of 120 orbitals): 0.455 ms + 0.040 ms for the digits = 36 TFLOP/s, against
 // 14.5 ms on the FP64 pipe; bound by the MMAs' operand reads from shared memory (about 50 cycles per MMA and 0.75 per

@@ -725,8 +725,8 @@ static void carve_step(const AdjCommon& a, Carver& c, StepWs& b, bool digits) {
     x.Pn = c.take<double2>(W * n * n);
     x.detn = c.take<double2>(W);
     x.gwn = c.take<double2>(wn);
-    x.gw2 = c.take<double2>(wn);
     if (!b.chain) {
+      x.gw2 = c.take<double2>(wn);
       x.Vv = c.take<double2>((size_t)(a.K + 1) * wn);
       x.S = c.take<double2>((size_t)a.K * wn);
     }
@@ -739,7 +739,7 @@ static void carve_step(const AdjCommon& a, Carver& c, StepWs& b, bool digits) {
   b.st = c.take<double2>(W);
   b.ft = c.take<double2>(W);
   b.V = c.take<double2>(W * NN);
-  b.Bc = c.take<double2>(NN);
+  if (!b.chain) b.Bc = c.take<double2>(NN);
   b.gV = c.take<double2>(W * NN);
   if (a.chol_packed) b.vp = c.take<double2>(W * ((size_t)a.N * (a.N + 1) / 2));
   b.gxsv = c.take<double2>(W * G);

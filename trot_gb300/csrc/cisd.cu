@@ -791,11 +791,6 @@ cisd_l2_reduce_kernel(int G, int nv, const double2* __restrict__ xg, const doubl
 }
 
 // ------------------------------------------------------------------ combines
-__device__ __forceinline__ double2 cdot_row(const double2* a, const double2* b, int n) {
-  double2 s = cmk(0.0, 0.0);
-  for (int k = 0; k < n; ++k) cfma(s, a[k], b[k]);
-  return s;
-}
 
 // overlap = (1 + 2 ci1g + gci2g) det0^2, gci2g = sum ci2g o x; one CTA per walker
 __global__ void cisd_overlap_kernel(int nv, const double2* __restrict__ x, const double2* __restrict__ cg,

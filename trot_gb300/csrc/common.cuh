@@ -64,7 +64,6 @@ TROT_D double warp_sum(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-TROT_D double2 warp_sum2(double2 v) { return cmk(warp_sum(v.x), warp_sum(v.y)); }
 
 // Block-wide sum in a fixed order (deterministic).  `red` holds >= 32 double2.  The halves of a warp take one component
 // each after the first exchange: 5 + 3 dependent FP64 additions for 256 threads instead of 20, at about 60 cycles each.

@@ -14,7 +14,7 @@ inline bool dg_takes(int K) { return K >= kDgMinK && K <= kDgMaxK; }
 // Bytes that launch_zgemm_dg wants for C (M x Nn) = alpha A (M x K complex) B (K x Nn real).
 size_t dg_scratch_bytes(size_t M, size_t Nn, size_t K);
 
-// C[m][n] (+)= alpha sum_k A[m][k] B(k, n) as launch_zgemm_cr, with both operands as six
+// C[m][n] (+)= alpha sum_k A[m][k] B(k, n) as launch_zgemm_cr_splitk, with both operands as six
 // FP16 digit planes per row and 26 exact tensor-core products.
 int launch_zgemm_dg(int M, int Nn, int K, double alpha, const double2* A, int lda, const double* B, int ldb,
                     bool b_is_nk, double2* C, long long ldc, bool accumulate, const DgScratch& s, cudaStream_t st);

@@ -103,11 +103,6 @@ __global__ void zgemm_splitk_reduce_kernel(int M, int Nn, int S, double alpha, c
   }
 }
 
-int launch_zgemm_cr(int M, int Nn, int K, double alpha, const double2* A, int lda, const double* B,
-                    int ldb, bool b_is_nk, double2* C, int ldc, bool accumulate, cudaStream_t st) {
-  return launch_zgemm_cr_splitk(M, Nn, K, alpha, A, lda, B, ldb, b_is_nk, C, ldc, accumulate, nullptr, 1, st);
-}
-
 int launch_zgemm_cr_splitk(int M, int Nn, int K, double alpha, const double2* A, int lda, const double* B, int ldb,
                            bool b_is_nk, double2* C, int ldc, bool accumulate, double2* part, int S,
                            cudaStream_t st) {

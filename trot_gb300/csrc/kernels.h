@@ -58,11 +58,8 @@ int launch_green(const Spins& sp, int W, int N, const double2* wa, const double2
 
 // C[m][n] (+)= alpha * sum_k A[m][k] * B(k, n), A complex (lda), C complex (ldc).
 // b_is_nk: B stored (N, K) row-major (ldb) — otherwise (K, N) row-major.
-int launch_zgemm_cr(int M, int Nn, int K, double alpha, const double2* A, int lda,
-                    const double* B, int ldb, bool b_is_nk, double2* C, int ldc, bool accumulate,
-                    cudaStream_t st);
-// Same with K split into S slices computed by separate CTAs (for small M x Nn and long K):
-// part holds S * M * Nn complex partials, reduced in slice order into C.
+// part (may be null): K split into S slices computed by separate CTAs (for small M x Nn
+// and long K); part holds S * M * Nn complex partials, reduced in slice order into C.
 int launch_zgemm_cr_splitk(int M, int Nn, int K, double alpha, const double2* A, int lda, const double* B, int ldb,
                            bool b_is_nk, double2* C, int ldc, bool accumulate, double2* part, int S,
                            cudaStream_t st);

@@ -1616,7 +1616,6 @@ __global__ void vhs_image_kernel(int W, int N, int n2pad, int packed, const floa
   }
 }
 
-// phaseless weights from overlaps computed after the propagation
 // New overlaps of the propagated walkers and their phaseless weights:
 // M_s = C_s^T w'_s in float-float (four independent accumulators per element),
 // det by FP64 elimination; one CTA per (walker, spin), the two spins of a walker in a cluster, whose first CTA

@@ -127,7 +127,9 @@ trotter_kernel(Spins sp, TrotterArgs a) {
 // The chain of digit products takes 19 launches, 150 us at least; this kernel's time is the FP64 pipe's, one walker's
 // N^2 nc products on one SM at a time.  Measured (6 terms; FP64 kernel / digit products, us): N = 24, 5 columns: 60 / 150
 // (64 walkers), 216 / 355 (1024); N = 40, 7: 150 / 152, 654 / 427; N = 50, 8: 190 / 168, 1110 / 479; N = 64, 10: 345 /
-// 164, 2107 / 550; N = 96, 12: 843 / 193, 5505 / 1003.
+// 164, 2107 / 550; N = 96, 12: 843 / 193, 5505 / 1003.  The line is where 64 walkers break even and looks at one walker's
+// work only, so that its numbers do not depend on the size of the batch; 1024 walkers just below it (N = 40) would be faster
+// with the products.
 bool trotter_takes_digits(const Spins& sp, int N) {
   return dg_takes(N) && N <= 1024 && (long long)N * N * sp.ntot >= 14000;
 }
